@@ -89,7 +89,7 @@ def core() -> ctypes.CDLL:
         lib.rb_rmsnorm_rows_ld.argtypes = [P, I, P, I, F, F, P, I, I, I, I, P]
         lib.rb_rmsnorm_rows_ld.restype = c_int
         lib.rb_swiglu.argtypes = [P, P, I, I, I, I, I, P]
-        lib.rb_gemm_f32.argtypes = [P, P, P, I, I, I, I, I, I, P]
+        lib.rb_gemm_f32.argtypes = [P, P, P, I, I, I, I, I, I, I, P]
         lib.rb_gemm_skinny.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P]
         lib.rb_gemm_skinny.restype = c_int
         lib.rb_gemm_skinny_act.argtypes = [P, P, P, I, I, P, I, I, I, I, I, I, I, P]
@@ -305,15 +305,16 @@ def softcap(x: torch.Tensor, cap: float) -> None:
 
 # ------------------------------------------------------------------------------- matrix products
 
-def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = x[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K)."""
+def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int = -1) -> None:
+    """out[M, N] = x[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K).  ``kind``: 0-3 one size of tile, 4 the
+    kernel for up to 4 rows, -1 the one that suits the sizes; all give the same bits."""
     M, K = x.shape
     N = w.shape[0]
     assert x.dtype == w.dtype == out.dtype == torch.float32
     assert w.shape[1] == K and out.shape == (M, N)
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     _check(core().rb_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                              _stream()), "gemm_f32")
+                              kind, _stream()), "gemm_f32")
 
 
 SKINNY_KERNEL_MAX_ROWS = 32     # what the kernel takes

@@ -1,5 +1,6 @@
 """Each CUDA kernel alone against its plain float32 reference, at sizes other than the engine's."""
 import math
+import types
 
 import pytest
 import torch
@@ -115,6 +116,26 @@ def test_gemm_f32_is_exact_float32(M, N, K):
     o2 = torch.empty(1, 1, device=DEV)
     ops.gemm_f32(x2, w2, o2)
     assert o2.item() == 1.0 + 2.0 ** -12
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 33, 132), (2, 64, 4), (4, 100, 1030), (5, 65, 36), (33, 129, 100), (130, 257, 31), (257, 96, 256)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_gemm_f32_kernels_agree(M, N, K, offset):
+    """Every tile size and the kernel for few rows against each other (bit by bit) and against float64, at the edges of tiles and
+    stages; ``offset`` puts the operands off 16-byte boundaries.  A sum of K products in float32 is off by at most K / 2^24 times
+    the sum of their sizes."""
+    ops = _ops()
+    wide = torch.randn(M + N, K + 3, device=DEV)
+    x, w = wide[:M, offset:offset + K], wide[M:, offset:offset + K]
+    if offset == 0 and K % 4 == 0:
+        x, w = x.contiguous(), w.contiguous()
+    outs = []
+    for kind in (-1, 0, 1, 2, 3) + ((4,) if M <= 4 else ()):
+        outs.append(torch.full((M, N), float("nan"), device=DEV))
+        ops.gemm_f32(x, w, outs[-1], kind=kind)
+        assert torch.equal(outs[-1], outs[0])
+    bound = (x.double().abs() @ w.double().abs().T) * K * 2.0 ** -24
+    assert ((outs[0].double() - x.double() @ w.double().T).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 32])
@@ -243,6 +264,26 @@ def test_attention_simt(dtype, Hq, Hkv, D, P, window):
     scale = 0.7 / math.sqrt(D)
     ops.attention_simt(pg.qkv, pg.kpool, pg.vpool, pg.pos, pg.tok_seg, pg.bt, P, out, Hq, Hkv, D, scale, window or 0)
     assert torch.allclose(out.float().cpu(), pg.reference(scale, window), **_tol(dtype))
+
+
+@pytest.mark.parametrize("Hq,Hkv,D,P", [(4, 2, 16, 16), (8, 1, 80, 8), (40, 1, 32, 16), (3, 1, 256, 64)])
+@pytest.mark.parametrize("window,keep", [(None, 0), (37, 0), (40, 5), (33, 70)])
+def test_attention_simt_rows_do_not_depend_on_their_block(Hq, Hkv, D, P, window, keep):
+    """Tokens that share a CTA get the bits that each gets alone, whatever lies in the cache behind them."""
+    ops = _ops()
+    pg = Paged([130, 70, 200, 1], [130, 3, 17, 1], Hq, Hkv, D, P, torch.float32, seed=D)
+    def run(rows):
+        q, pos, seg = pg.qkv[rows].contiguous(), pg.pos[rows].contiguous(), pg.tok_seg[rows].contiguous()
+        out = torch.full((len(rows), Hq * D), float("nan"), device=DEV)
+        batch = types.SimpleNamespace(pos=pos, tok_seg=seg)
+        ops.paged_attention(q, pg.kpool, pg.vpool, batch, pg.bt, P, out, Hq, Hkv, D, D ** -0.5, window, keep=keep)
+        return out
+    rows = torch.arange(sum(pg.q_lens))
+    whole = run(rows)
+    assert torch.isfinite(whole).all()
+    for t in (0, 15, 16, 17, 64, 129, 130, 132, 133, 149, 150):
+        assert torch.equal(run(rows[t:t + 1])[0], whole[t]), t
+    assert torch.equal(run(rows.flip(0)), whole.flip(0))                    # no two neighbours at following positions
 
 
 @pytest.mark.parametrize("Hq,Hkv,D,P", ATT_SHAPES)
