@@ -55,6 +55,7 @@ struct ScanArgs {
     const int* cu_q; const int* seg_slot;
     float* out;               // [T, H*V]
     int H, G, D, V;
+    int below;                // segments of this many tokens and more are left alone (0: none)
 };
 
 __device__ __forceinline__ float ld_elem(const void* p, int f32, size_t i) {
@@ -97,6 +98,7 @@ linear_scan_kernel(const ScanArgs a) {
     const int kvh = h / (H / a.G);
     const int nrd = (D + 7) >> 3;                      // row groups that exist
     const int t0 = a.cu_q[seg], t1 = a.cu_q[seg + 1];
+    if (a.below > 0 && t1 - t0 >= a.below) return;     // recurrent_chunks.cu takes it
     float* st = a.state + (long long)a.seg_slot[seg] * a.state_stride;
     float* Sg = st + a.s_off + (size_t)h * nrd * 8 * V;
     const bool col = j < V;
@@ -342,13 +344,13 @@ RB_EXPORT int rb_linear_scan(int mode, const void* q, const void* k, const void*
                              const float* extra, float cap,
                              float q_scale, float* state, long long state_stride, int s_off, int n_off, int m_off,
                              int f_off, const int* cu_q, const int* seg_slot, float* out, int H, int G, int D, int V,
-                             int segments, cudaStream_t st) {
+                             int segments, int below, cudaStream_t st) {
     ScanArgs a;
     a.q = q; a.k = k; a.v = v; a.q_ld = q_ld; a.k_ld = k_ld; a.v_ld = v_ld;
     a.q_f32 = q_f32; a.k_f32 = k_f32; a.v_f32 = v_f32;
     a.gate_a = gate_a; a.gate_b = gate_b; a.extra = extra; a.cap = cap; a.q_scale = q_scale;
     a.state = state; a.state_stride = state_stride; a.s_off = s_off; a.n_off = n_off; a.m_off = m_off; a.f_off = f_off;
-    a.cu_q = cu_q; a.seg_slot = seg_slot; a.out = out; a.H = H; a.G = G; a.D = D; a.V = V;
+    a.cu_q = cu_q; a.seg_slot = seg_slot; a.out = out; a.H = H; a.G = G; a.D = D; a.V = V; a.below = below;
     if (mode == MODE_DECAY) return launch_scan<MODE_DECAY>(a, segments, st);
     if (mode == MODE_MEMORY) return launch_scan<MODE_MEMORY>(a, segments, st);
     if (mode == MODE_DELTA) return launch_scan<MODE_DELTA>(a, segments, st);

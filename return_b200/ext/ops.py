@@ -1118,7 +1118,7 @@ def tanh_joint(x_in, x_out, y, post, nxt, out, shift=None, batch=None, rows=None
 # ------------------------------------------------------------------------------- mixers with a matrix state
 
 _recurrent = None
-_RECURRENT_SOURCES = ["recurrent.cu"]
+_RECURRENT_SOURCES = ["recurrent.cu", "recurrent_chunks.cu"]
 SCAN_DECAY, SCAN_MEMORY, SCAN_DELTA, SCAN_BONUS, SCAN_SSM, SCAN_DELTA_HEAD = 0, 1, 2, 3, 4, 5
 SCAN_MAX_KEY_DIM = 256
 
@@ -1130,7 +1130,9 @@ def recurrent_lib() -> ctypes.CDLL:
     if _recurrent is None:
         lib = build.load("return_recurrent", _RECURRENT_SOURCES, {"RB_PDL_MODE": PDL_MODE})
         P, I, F, L = c_void_p, c_int, c_float, ctypes.c_longlong
-        lib.rb_linear_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, F, P, L, I, I, I, I, P, P, P, I, I, I, I, I, P]
+        lib.rb_linear_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, F, P, L, I, I, I, I, P, P, P, I, I, I, I, I, I, P]
+        lib.rb_chunked_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, P, L, I, P, P, P, P] + [I] * 8 + [P, P]
+        lib.rb_chunked_scan_floats.argtypes, lib.rb_chunked_scan_floats.restype = [I, I, I], L
         lib.rb_token_shift_mix.argtypes = [P, I, P, I, I, P, L, I, P, P, P, P, I, I, I, P]
         lib.rb_ssm_prep.argtypes = [P, I, I, I, P, P, I, I, P, L, I, P, P, P, P, I, I, P, P, I, P, P, I, I, P]
         lib.rb_gated_part_norm.argtypes = [P, P, I, P, I, F, P, I, I, I, I, P]
@@ -1156,7 +1158,7 @@ def recurrent_lib() -> ctypes.CDLL:
         lib.rb_head_norm_gate.argtypes = [P, P, I, P, I, I, I, F, P, I, I, I, I, P]
         lib.rb_add_dual_norm.argtypes = [P, P, I, F, P, I, F, P, P, P, I, F, F, P, P, I, I, I, P]
         lib.rb_scaled_sum.argtypes = [P, I, F, P, I, F, P, I, L, P]
-        for name in ("rb_linear_scan", "rb_rotary_to_f32", "rb_delta_prep", "rb_conv_state_update",
+        for name in ("rb_linear_scan", "rb_chunked_scan", "rb_rotary_to_f32", "rb_delta_prep", "rb_conv_state_update",
                      "rb_head_norm_gate", "rb_add_dual_norm", "rb_scaled_sum", "rb_token_shift_mix", "rb_ssm_prep",
                      "rb_gated_part_norm"):
             getattr(lib, name).restype = c_int
@@ -1173,8 +1175,10 @@ def _is_f32(t: torch.Tensor) -> int:
 
 
 def linear_scan(mode: int, q, k, v, gate_a, gate_b, state, offsets, batch, out, heads: int, kv_heads: int,
-                dim: int, vdim: int, q_scale: float = 1.0, cap: float = 0.0, forgot_offset: int = -1, extra=None) -> None:
-    """The recurrence of a mixer with a [dim, vdim] state per head, over every segment of the step, token by token.
+                dim: int, vdim: int, q_scale: float = 1.0, cap: float = 0.0, forgot_offset: int = -1, extra=None,
+                below: int = 0) -> None:
+    """The recurrence of a mixer with a [dim, vdim] state per head, over every segment of the step, token by token
+    (``below`` > 0: over the segments of fewer tokens only).
 
     q, k: [T, >= kv_heads * dim] views (float32 or bfloat16, unit stride along a row), v: [T, >= heads * vdim];
     ``state``: float32 [slots, n], the row of a segment is ``batch.seg_slot``; ``offsets`` = (S, n, m): where the
@@ -1199,8 +1203,47 @@ def linear_scan(mode: int, q, k, v, gate_a, gate_b, state, offsets, batch, out, 
     _check(recurrent_lib().rb_linear_scan(
         mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _is_f32(q), _is_f32(k), _is_f32(v),
         _ptr(gate_a), _ptr(gate_b), _ptr(extra), cap, q_scale, _ptr(state), state.stride(0), offsets[0], offsets[1], offsets[2],
-        forgot_offset, _ptr(batch.cu_q), _ptr(batch.seg_slot), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, _stream()),
-        "linear_scan")
+        forgot_offset, _ptr(batch.cu_q), _ptr(batch.seg_slot), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, below,
+        _stream()), "linear_scan")
+
+
+CHUNK_TOKENS = 32                          # tokens of a chunk (csrc/recurrent_chunks.cu)
+# Scratch that a chunked scan asks for at most: a longer step goes through it in windows, one after the other.  What the first
+# kernel leaves there then still lies in L2 (126 MB) when the second reads it.
+CHUNK_SCRATCH_BYTES = 64 << 20
+
+
+def chunked_scan_ok(mode: int, heads: int, dim: int) -> bool:
+    """Whether ``chunked_scan`` takes this mode and key size."""
+    return recurrent_lib().rb_chunked_scan_floats(mode, heads, dim) > 0
+
+
+def chunked_scan(mode: int, q, k, v, gate_a, gate_b, state, s_off: int, batch, chunks: int, min_tokens: int, out, heads: int,
+                 kv_heads: int, dim: int, vdim: int, extra=None, buffer=None) -> None:
+    """``linear_scan`` for the segments of at least ``min_tokens`` tokens, 32 tokens at a time (every mode but SCAN_MEMORY, keys up
+    to 128).  ``chunks``: how many chunks of 32 these segments have between them.  ``buffer(name, shape, dtype, device)`` gives
+    the scratch."""
+    assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
+    assert out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == heads * vdim
+    assert q.stride(1) == 1 and k.stride(1) == 1 and v.stride(1) == 1
+    assert gate_a.dtype == torch.float32 and gate_a.is_contiguous()
+    if gate_b is not None:
+        assert gate_b.dtype == torch.float32 and gate_b.is_contiguous()
+    if mode in (SCAN_BONUS, SCAN_SSM):
+        assert extra is not None and extra.dtype == torch.float32 and extra.is_contiguous()
+        assert extra.numel() == (heads * dim if mode == SCAN_BONUS else heads)
+    lib = recurrent_lib()
+    _tc5_launched.add(out.device)
+    per = lib.rb_chunked_scan_floats(mode, heads, dim)
+    window = max(1, min(chunks, CHUNK_SCRATCH_BYTES // (4 * per)))
+    scratch = (buffer or (lambda name, shape, dtype, device: torch.empty(shape, dtype=dtype, device=device)))(
+        "state_mixer.chunks", (window * per,), torch.float32, out.device)
+    for first in range(0, chunks, window):
+        _check(lib.rb_chunked_scan(
+            mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _is_f32(q), _is_f32(k), _is_f32(v),
+            _ptr(gate_a), _ptr(gate_b), _ptr(extra), 1.0, _ptr(state), state.stride(0), s_off, _ptr(batch.cu_q), _ptr(batch.seg_slot),
+            _ptr(scratch), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, min_tokens, first, min(window, chunks - first),
+            _ptr(tc5_status(out.device)), _stream()), "chunked_scan", 2)
 
 
 def scan_pieces_combine(pieces, state, s_off: int, decay, cu_piece, seg_first, seg_slot, per_head: int, total: int,

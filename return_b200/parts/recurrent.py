@@ -55,32 +55,91 @@ class _StateMixer(Mixer):
             return memo[key]
         plan = None
         lens = np.diff(host.cu_q).astype(np.int64)
-        if int(lens.max()) >= self.PIECES_MIN_TOKENS:
-            ctas = self.H * ((self.V + 31) // 32)
-            want = (2 * ops.num_sms()) // max(1, ctas * int((lens >= self.PIECES_MIN_TOKENS).sum()))
-            if want >= 3:                                   # two passes over the tokens: fewer pieces would not pay
-                cuts, first = [0], [0]
-                for start, n in zip(host.cu_q[:-1], lens):
-                    k = int(min(want, max(1, n // self.PIECE_MIN_TOKENS))) if n >= self.PIECES_MIN_TOKENS else 1
-                    edges = [int(start) + (int(n) * i) // k for i in range(1, k + 1)]
-                    cuts.extend(edges)
-                    first.append(first[-1] + k)
-                n_pieces = len(cuts) - 1
-                tables = torch.from_numpy(np.asarray(cuts + first + list(range(n_pieces)), np.int32)).to(
-                    self.env.device, non_blocking=True)
-                a, c = len(cuts), len(cuts) + len(first)
-                virtual = SimpleNamespace(cu_q=tables[:a], seg_slot=tables[c:], num_segments=n_pieces)
-                plan = (virtual, tables[a:c], n_pieces)
+        counts = self._piece_counts(lens)
+        if counts is not None:
+            cuts, first = [0], [0]
+            for start, n, k in zip(host.cu_q[:-1], lens, counts):
+                cuts.extend(int(start) + (int(n) * i) // k for i in range(1, k + 1))
+                first.append(first[-1] + k)
+            n_pieces = len(cuts) - 1
+            tables = torch.from_numpy(np.asarray(cuts + first + list(range(n_pieces)), np.int32)).to(
+                self.env.device, non_blocking=True)
+            a, c = len(cuts), len(cuts) + len(first)
+            virtual = SimpleNamespace(cu_q=tables[:a], seg_slot=tables[c:], num_segments=n_pieces)
+            plan = (virtual, tables[a:c], n_pieces)
         if memo is not None:
             memo[key] = plan
         return plan
 
+    def _piece_counts(self, lens):
+        """Into how many pieces segments of these lengths are cut, or None if none is."""
+        long = lens >= self.PIECES_MIN_TOKENS
+        if not long.any():
+            return None
+        want = (2 * ops.num_sms()) // max(1, self.H * ((self.V + 31) // 32) * int(long.sum()))
+        if want < 3:                                        # two passes over the tokens: fewer pieces would not pay
+            return None
+        return [int(min(want, max(1, n // self.PIECE_MIN_TOKENS))) if big else 1 for n, big in zip(lens, long)]
 
-    def _scan(self, mode, q, k, v, decay, step, ctx, out, groups, extra, by_row, pieces):
-        """The scan of a mixer whose decays differ from token to token (per head, or per head and key row with
-        ``by_row``).  With ``pieces`` the long segments are scanned in pieces side by side: every piece from zero, the
-        states handed on in order (a piece's transition is the product of its tokens' decays), every piece again."""
+    # A segment of at least this many tokens goes through the scan 32 tokens at a time (bfloat16 path only: the sums then take
+    # another order than token by token, which the float32 path never does).  Measured with 16 heads of 128 x 128 (delta rule with
+    # a decay per key row / fixed decay, us): 64 tokens 35 / 23 token by token, 31 / 27 in chunks (and a launch more); 96 tokens 49 / 31 and 33 / 28; 256 tokens 119 / 71 and 47 / 40;
+    # 2,048 tokens 900 / 515 and 219 / 150.
+    CHUNKED_MIN_TOKENS = 96
+    # Where a segment can be cut into pieces that are scanned side by side instead, that wins with many pieces: k pieces of a
+    # segment of n tokens take 2 n / k tokens' time (0.25 us each) and 20 us, chunks n / 32 times 1.6 us, so the two meet at
+    # k = 10 (16 heads of 128 values give 4 pieces, 8 heads 9, 4 heads 16); and with few key rows, because a chunk's matrices
+    # are padded to 64 while a token's time falls with them.
+    CHUNKED_MAX_PIECES = 12
+    CHUNKED_MIN_KEYS = 48
+
+    def _chunks(self, mode, batch):
+        """None, or (chunks of the step's long segments, whether there are short ones beside them).  Worked out once per step
+        and kind of scan."""
+        host = getattr(batch, "host", None)
+        if self.env.act_dtype == torch.float32 or host is None or not getattr(host, "num_multi", 0):
+            return None
+        memo = getattr(batch, "scratch", None)
+        linear = mode not in (ops.SCAN_DELTA, ops.SCAN_DELTA_HEAD)          # states of pieces can be handed on by their decays
+        key = ("state_mixer.chunks.plan", linear, self.H, self.D, self.V)
+        if memo is not None and key in memo:
+            return memo[key]
+        lens = np.diff(host.cu_q).astype(np.int64)
+        long = lens >= self.CHUNKED_MIN_TOKENS
+        plan = (int(((lens[long] + ops.CHUNK_TOKENS - 1) // ops.CHUNK_TOKENS).sum()), bool((~long).any())) if long.any() else None
+        if plan is not None and not ops.chunked_scan_ok(mode, self.H, self.D):
+            plan = None
+        counts = self._piece_counts(lens) if linear and plan is not None else None
+        if counts is not None and (max(counts) >= self.CHUNKED_MAX_PIECES or self.D < self.CHUNKED_MIN_KEYS):
+            plan = None
+        if memo is not None:
+            memo[key] = plan
+        return plan
+
+    def _scan_in_chunks(self, mode, q, k, v, gate_a, gate_b, ctx, out, groups, extra=None):
+        """The recurrence of the step's long segments in chunks, of the others token by token.  False (and nothing done) if the
+        step has no long segment, or on the float32 path."""
         b = ctx.batch
+        plan = self._chunks(mode, b)
+        if plan is None:
+            return False
+        chunks, others = plan
+        ops.chunked_scan(mode, q, k, v, gate_a, gate_b, ctx.state, 0, b, chunks, self.CHUNKED_MIN_TOKENS, out, self.H, groups,
+                         self.D, self.V, extra=extra, buffer=ctx.buffer)
+        if others:
+            ops.linear_scan(mode, q, k, v, gate_a, gate_b, ctx.state, (0, 0, 0), b, out, self.H, groups, self.D, self.V, extra=extra,
+                            below=self.CHUNKED_MIN_TOKENS)
+        return True
+
+    def _scan(self, mode, q, k, v, decay, step, ctx, out, groups, extra, by_row):
+        """The scan of a mixer whose decays differ from token to token (per head, or per head and key row with
+        ``by_row``).  Where it does not run in chunks (keys too long for them) the long segments are scanned in pieces side by
+        side: every piece from zero, the states handed on in order (a piece's transition is the product of its tokens' decays),
+        every piece again."""
+        b = ctx.batch
+        if self._scan_in_chunks(mode, q, k, v, decay, step, ctx, out, groups, extra):
+            return
+        pieces = self._pieces(b) if self.env.act_dtype != torch.float32 else None
         if pieces is None:
             ops.linear_scan(mode, q, k, v, decay, step, ctx.state, (0, 0, 0), b, out, self.H, groups, self.D, self.V, extra=extra)
             return
@@ -135,8 +194,11 @@ class Retention(_StateMixer):
             self._decay = torch.tensor(s.decay, dtype=torch.float32, device=dev)
         o = ctx.buffer("retention.o", (T, HV), torch.float32, dev)
         v = proj[:, 2 * HD:2 * HD + HV]
-        pieces = self._pieces(b) if x.dtype != torch.float32 else None
-        if pieces is None:
+        chunked = self._scan_in_chunks(ops.SCAN_DECAY, q32, k32, v, self._decay, None, ctx, o, self.H)
+        pieces = self._pieces(b) if x.dtype != torch.float32 and not chunked else None
+        if chunked:
+            pass
+        elif pieces is None:
             ops.linear_scan(ops.SCAN_DECAY, q32, k32, v, self._decay, None, ctx.state, (0, 0, 0), b, o,
                             self.H, self.H, self.D, self.V)
         else:
@@ -206,8 +268,9 @@ class ChannelDelta(_StateMixer):
                        self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5)
         ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
         o = ctx.buffer("channel_delta.o", (T, HV), torch.float32, dev)
-        ops.linear_scan(ops.SCAN_DELTA, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
-                        self.H, self.G, self.D, self.V)
+        if not self._scan_in_chunks(ops.SCAN_DELTA, q32, k32, v32, decay, beta, ctx, o, self.G):
+            ops.linear_scan(ops.SCAN_DELTA, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
+                            self.H, self.G, self.D, self.V)
         mixed = ctx.buffer("channel_delta.mixed", (T, HV), x.dtype, dev)
         ops.head_norm_gate(o, gate, self.p_norm, 1, 1, s.eps, mixed, self.H, self.V)
         return self._project_out(mixed, ctx)
@@ -324,8 +387,7 @@ class TimeMix(_StateMixer):
         decay = ctx.buffer("time_mix.decay", (T, HD), torch.float32, dev)
         ops.linear(low, self.p_decay_up, decay, act="neg_exp_exp", bias=self.p_decay_bias)
         o = ctx.buffer("time_mix.o", (T, HD), torch.float32, dev)
-        self._scan(ops.SCAN_BONUS, proj[0], proj[1], proj[2], decay, None, ctx, o, self.H, self._bonus32, True,
-                   self._pieces(b) if dt != torch.float32 else None)
+        self._scan(ops.SCAN_BONUS, proj[0], proj[1], proj[2], decay, None, ctx, o, self.H, self._bonus32, True)
         mixed = ctx.buffer("time_mix.mixed", (T, HD), dt, dev)
         ops.head_norm_gate(o, proj[3], self.p_norm, 2, 0, s.eps, mixed, self.H, self.V)
         return self._project_out(mixed, ctx)
@@ -387,7 +449,7 @@ class StateSpace(_StateMixer):
         ops.conv_state_update(proj[:, inner:], s.conv_taps, ctx.state, self.conv_off, b, C)   # after every token read the old one
         y = ctx.buffer("state_space.y", (T, inner), torch.float32, dev)
         self._scan(ops.SCAN_SSM, conv[:, inner + GN:], conv[:, inner:inner + GN], conv[:, :inner], decay, step, ctx, y,
-                   s.groups, self._skip32, False, self._pieces(b) if x.dtype != torch.float32 else None)
+                   s.groups, self._skip32, False)
         mixed = ctx.buffer("state_space.mixed", (T, inner), x.dtype, dev)
         ops.gated_part_norm(y, proj[:, :inner], self.p_norm, s.norm_groups, s.eps, mixed)
         return self._project_out(mixed, ctx)
@@ -444,8 +506,9 @@ class GatedDelta(_StateMixer):
                        self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5, head_decay=True)
         ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
         o = ctx.buffer("gated_delta.o", (T, HV), torch.float32, dev)
-        ops.linear_scan(ops.SCAN_DELTA_HEAD, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
-                        self.H, self.G, self.D, self.V)
+        if not self._scan_in_chunks(ops.SCAN_DELTA_HEAD, q32, k32, v32, decay, beta, ctx, o, self.G):
+            ops.linear_scan(ops.SCAN_DELTA_HEAD, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
+                            self.H, self.G, self.D, self.V)
         mixed = ctx.buffer("gated_delta.mixed", (T, HV), x.dtype, dev)
         ops.head_norm_gate(o, proj[:, C:], self.p_norm, 1, 0, s.eps, mixed, self.H, self.V)
         return self._project_out(mixed, ctx)

@@ -1,0 +1,110 @@
+"""The recurrences 32 tokens at a time against the plain recurrence in float64 and beside the walk token by token."""
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _ops():
+    from return_b200.ext import ops
+    return ops
+
+
+def plain(mode, ops, q, k, v, gate_a, gate_b, S, extra):
+    """One segment: q, k [T, H, D], v [T, H, V], S [H, D, V], all float64."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        g = gate_a[:, None, None] if mode == ops.SCAN_DECAY else gate_a[t].reshape(S.shape[0], -1, 1)
+        if mode == ops.SCAN_BONUS:
+            pair = k[t][:, :, None] * v[t][:, None]
+            out[t] = torch.bmm(q[t][:, None], S + extra[:, :, None] * pair)[:, 0]
+            S = g * S + pair
+            continue
+        S = g * S
+        u = v[t]
+        if mode in (ops.SCAN_DELTA, ops.SCAN_DELTA_HEAD):
+            u = gate_b[t][:, None] * (u - torch.bmm(k[t][:, None], S)[:, 0])
+        elif mode == ops.SCAN_SSM:
+            u = gate_b[t][:, None] * u
+        S = S + k[t][:, :, None] * u[:, None]
+        out[t] = torch.bmm(q[t][:, None], S)[:, 0]
+        if mode == ops.SCAN_SSM:
+            out[t] += extra[:, None] * v[t]
+    return out, S
+
+
+def rows(S):
+    """A state [H, D, V] in a slot's order: [head][row / 8][column][row % 8], rows padded with zeros."""
+    H, D, V = S.shape
+    padded = torch.zeros(H, (D + 7) // 8 * 8, V, dtype=S.dtype, device=S.device)
+    padded[:, :D] = S
+    return padded.view(H, -1, 8, V).transpose(2, 3).reshape(-1)
+
+
+@pytest.mark.parametrize("mode", ["DECAY", "DELTA", "BONUS", "SSM", "DELTA_HEAD"])
+@pytest.mark.parametrize("lens,H,G,D,V,decay,form", [
+    ([64, 1, 95, 96], 2, 2, 128, 16, 1.0, "float32"),          # whole chunks and remainders, a segment that is left alone
+    ([70, 200], 4, 2, 24, 40, 0.1, "bfloat16"),                # few key rows, columns that do not fill a CTA
+    ([97], 2, 1, 100, 24, 30.0, "unaligned"),                  # decays that underflow within a chunk; rows off 16-byte boundaries
+    ([129, 65], 3, 3, 64, 17, 0.0, "bfloat16"),                # no decay at all
+])
+def test_chunked_scan(mode, lens, H, G, D, V, decay, form, monkeypatch):
+    ops = _ops()
+    m = getattr(ops, "SCAN_" + mode)
+    delta = mode.startswith("DELTA")
+    T, n = sum(lens), len(lens)
+    gen = torch.Generator(device=DEV).manual_seed(D + V)
+    normal = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    dt = torch.bfloat16 if form == "bfloat16" else torch.float32
+    wide = torch.zeros(T, 2 * G * D + H * V + 5, dtype=dt, device=DEV)
+    lead = 3 if form == "unaligned" else 0
+    q, k, v = wide[:, lead:lead + G * D], wide[:, lead + G * D:lead + 2 * G * D], wide[:, lead + 2 * G * D:lead + 2 * G * D + H * V]
+    q.copy_(normal(T, G * D) * D ** -0.5)
+    k.copy_(unit(normal(T, G, D)).reshape(T, -1))
+    v.copy_(normal(T, H * V))
+    shape = {"DECAY": (H,), "DELTA": (T, H * D), "BONUS": (T, H * D)}.get(mode, (T, H))
+    gate_a = torch.exp(-decay * torch.nn.functional.softplus(normal(*shape)))
+    gate_b = torch.rand(T, H, generator=gen, device=DEV) if delta or mode == "SSM" else None
+    extra = normal(H, D) if mode == "BONUS" else normal(H) if mode == "SSM" else None
+    s_off, per = 1, H * ((D + 7) // 8 * 8) * V                  # a state that begins on an odd float of an odd row
+    starts = [normal(H, D, V) * 0.3 for _ in lens]
+    state = torch.zeros(n + 1, s_off + per + 2 - (per + s_off) % 2, device=DEV)
+    for i, S in enumerate(starts):
+        state[n - i, s_off:s_off + per] = rows(S)              # slots in another order than segments
+    cu = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    batch = SimpleNamespace(cu_q=torch.from_numpy(cu).to(DEV), num_segments=n,
+                            seg_slot=torch.tensor([n - i for i in range(n)], dtype=torch.int32, device=DEV))
+    chunks = sum((x + 31) // 32 for x in lens if x >= 64)
+
+    def run(in_chunks, scratch=None):
+        st, out = state.clone(), torch.full((T, H * V), float("nan"), device=DEV)
+        below = 0
+        if in_chunks:
+            if scratch is not None:
+                monkeypatch.setattr(ops, "CHUNK_SCRATCH_BYTES", scratch)
+            ops.chunked_scan(m, q, k, v, gate_a, gate_b, st, s_off, batch, chunks, 64, out, H, G, D, V, extra=extra)
+            below = 64
+        ops.linear_scan(m, q, k, v, gate_a, gate_b, st, (s_off, 0, 0), batch, out, H, G, D, V, extra=extra, below=below)
+        return out, st
+
+    got, walked = run(True), run(False)
+    windows = run(True, scratch=1)                             # a chunk at a time: the state goes through its slot in between
+    ops.check_status(DEV)
+    assert torch.equal(windows[0], got[0]) and torch.equal(windows[1], got[1])
+    f = lambda x: None if x is None else x.double()
+    heads = lambda x, d, g: x.double().reshape(-1, g, d).repeat_interleave(H // g, 1)
+    for i, (a, b) in enumerate(zip(cu[:-1], cu[1:])):
+        ga = f(gate_a) if mode == "DECAY" else f(gate_a[a:b])
+        want, S = plain(m, ops, heads(q[a:b], D, G), heads(k[a:b], D, G), heads(v[a:b], V, H), ga,
+                        None if gate_b is None else f(gate_b[a:b]), starts[i].double(), f(extra))
+        for x, y, w in ((got[0][a:b], walked[0][a:b], want.reshape(b - a, -1)),
+                        (got[1][n - i, s_off:s_off + per], walked[1][n - i, s_off:s_off + per], rows(S))):
+            off = lambda z: float((z.double() - w).norm() / w.norm())
+            # sums of up to 128 + 32 terms rounded to 24 bits, in other orders: a few 2^-24 either way
+            assert off(x) < 2.0 * off(y) + 2.0 ** -22, (i, off(x), off(y))
