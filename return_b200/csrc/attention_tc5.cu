@@ -45,9 +45,13 @@
 // (tanh_poly in common.cuh); else the hardware's 2^x and reciprocal, which take as long as the softmax's own three times over.  With a window it can
 // also keep the first `keep` positions visible for every later query: the key tiles are then walked in two runs, the tiles
 // of the kept positions that lie before the window's first tile, then the window's.
-// A step with too few such CTAs to fill the GPU (a short portion of a long prompt) splits the keys of every
-// block over gridDim.z CTAs; each leaves its unnormalised O with its reference maximum and sum in float32,
-// and a second kernel merges them (the same arithmetic as the decode kernel's merge).
+// A step with too few such CTAs to fill the GPU (a short portion of a long prompt), or one whose longest blocks would keep a few
+// SMs busy long after the others, splits the keys of its blocks over up to gridDim.z CTAs: as many as the block has shares of
+// `share` key tiles (0: all gridDim.z), so that a CTA's work is about the same whatever its block's context; the CTAs that a
+// short block does not need return at once.  Each leaves its unnormalised O with its reference maximum and sum in float32,
+// and a second kernel merges them (the same arithmetic as the decode kernel's merge); a block of one share writes its rows itself.
+// Measured (16 heads; 512 rows behind 7,680 keys, a prompt of 200, 61 rows behind 1,500): 65 us; every block in two
+// shares alike 86, one CTA a block 148.
 // *status is raised if a wait gave up.
 #include "tc5.cuh"
 
@@ -160,6 +164,22 @@ struct ScoreMod {
     int keep;                  // with a window: the first `keep` positions stay visible (0: none)
 };
 
+// The key tiles that a block of query rows from position p0 on walks: those of the window (or of the block of positions, or of
+// all keys) from jt_window on, and before them n_keep tiles of kept first positions.
+struct Walk {
+    int lo_min, jt_window, n_keep, jt_first;
+    __device__ __forceinline__ Walk(int p0, int window, int chunk, int keep) {
+        lo_min = window > 0 ? max(0, p0 - window + 1) : chunk > 0 ? (p0 / chunk) * chunk : 0;
+        jt_window = lo_min / KN;
+        n_keep = window > 0 ? min((keep + KN - 1) / KN, jt_window) : 0;
+        jt_first = jt_window - n_keep;
+    }
+};
+// Over how many CTAs a block of nt key tiles is split.
+__device__ __forceinline__ int shares_of(int nt, int n_split, int share) {
+    return share > 0 ? min(n_split, max(1, (nt + share - 1) / share)) : n_split;
+}
+
 template <bool MOD>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restrict__ kpool,
@@ -168,7 +188,7 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
                         const int* __restrict__ block_table, int bt_stride, int page_size,
                         bf16* __restrict__ out, int Hq, int Hkv, float scale_log2, int window,
                         float* __restrict__ part_o, float* __restrict__ part_ml, int total_rows,
-                        int* __restrict__ status, const float* __restrict__ sink, ScoreMod sm) {
+                        int* __restrict__ status, const float* __restrict__ sink, ScoreMod sm, int share) {
     // The swizzled tiles need 1024-byte alignment.  The kernel has no static shared memory, so the
     // dynamic window starts at the CTA's shared base; should it ever not be aligned, the kernel
     // reports it and does nothing.
@@ -192,10 +212,11 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     const int p0 = seg_pos0[seg] + row0;                  // position of the CTA's first query
     const int p_last = p0 + m_rows - 1;
     const int chunk = MOD ? sm.chunk : 0;
-    const int lo_min = window > 0 ? max(0, p0 - window + 1) : chunk > 0 ? (p0 / chunk) * chunk : 0;
     const int keep = MOD && window > 0 ? sm.keep : 0;
-    const int jt_window = lo_min / KN;                    // the first key tile of the window (or of all keys)
-    const int n_keep = MOD ? min((keep + KN - 1) / KN, jt_window) : 0;       // tiles of kept positions before it
+    const Walk walk(p0, window, chunk, keep);
+    const int lo_min = walk.lo_min;
+    const int jt_window = walk.jt_window;                 // the first key tile of the window (or of all keys)
+    const int n_keep = MOD ? walk.n_keep : 0;             // tiles of kept positions before it
     // the walk's tiles are numbered jt_first, jt_first + 1, ...; tile_of turns a number into a key tile.  With kept tiles they
     // come first: the numbers then start at n_keep tiles below the window's
     int jt_first = jt_window - n_keep;
@@ -204,7 +225,8 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     int na = min(p_last, p0 + QM - 1) / KN - jt_first + 1;
     int nb = m_rows > QM ? p_last / KN - jt_first + 1 : 0;
     int nt = max(na, nb);
-    const int n_split = gridDim.z, split = blockIdx.z;
+    const int n_split = shares_of(nt, gridDim.z, share), split = blockIdx.z;
+    if (split >= n_split) return;                         // a short block: fewer CTAs than the longest
     if (n_split > 1) {                                    // this CTA's share of the block's key tiles; it may be empty
         const int per = (nt + n_split - 1) / n_split;
         const int t0 = split * per;
@@ -220,6 +242,22 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     const unsigned bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * i; };
 
+    // The rows go to shared memory and back a whole row by neighbouring lanes, so that an instruction touches whole lines (a lane
+    // a row, 16 bytes at a time, took 4.4 us for the queries and 1.5 us for the outputs of a CTA, whose key tiles take 1.1 us
+    // each; a prompt of 2,048 tokens, 32 heads of 128: 58.6 -> 52.3 us).
+    constexpr int LPR = D / 8, RPI = 32 / LPR;            // lanes a row of 16-byte pieces, rows an instruction
+    const int rsel = lane / LPR, sub = lane % LPR;
+    if (warp < 2 * 4) {
+        const int qt = warp >> 2;
+        const unsigned tile = smem_u32(sQ) + qt * Q_BYTES + (unsigned)(sub >> 3) * (QM * 128);
+#pragma unroll
+        for (int i = 0; i < 32 / RPI; ++i) {
+            const int r = (warp & 3) * 32 + i * RPI + rsel, grow = qt * QM + r;
+            const bool there = grow < m_rows;             // rows that do not exist are zero
+            cp_async16(tile + sw128_offset(r, sub & 7), there ? q + (size_t)(q_begin + row0 + grow) * ld + (size_t)h * D + sub * 8 : q, there);
+        }
+        cp_async_commit();
+    }
     if (warp == W_MMA) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
     if (tid == 0) {
         for (int i = 0; i < N_BARS; ++i)
@@ -254,17 +292,8 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
         const float raw_max = capped ? TANH_POLY_MAX / k_cap : 0.f;            // up to this product the polynomial holds
         const float* bias_row = (MOD && sm.bias) ? sm.bias + (size_t)h * sm.bias_n : nullptr;
         const float bias_last_l = (MOD && sm.bias) ? bias_row[sm.bias_n - 1] * LOG2E : 0.f;
-        unsigned char* myQ = sQ + qt * Q_BYTES;
         unsigned char* myPs = sP + qt * 2 * P_BYTES;           // this query tile's two P buffers
-        {
-            const bf16* qrow = q + (size_t)(q_begin + row0 + grow) * ld + (size_t)h * D;
-#pragma unroll
-            for (int c = 0; c < D / 8; ++c) {
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (row_valid) v = *reinterpret_cast<const uint4*>(qrow + c * 8);
-                *reinterpret_cast<uint4*>(myQ + (c >> 3) * (QM * 128) + sw128_offset(r, c & 7)) = v;
-            }
-        }
+        cp_async_wait<0>();                                  // the query rows, asked for before anything else
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_Q_READY));
@@ -422,50 +451,60 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
             ok = mbar_wait(bar(B_PV_DONE + qt * 2 + ((n_mine - 1) & 1)), ((n_mine - 1) >> 1) & 1) && ok;
             fence_after_sync();
         }
-        const size_t token = (size_t)(q_begin + row0 + grow);
+        const size_t token0 = (size_t)(q_begin + row0 + qt * QM);     // the query tile's first row
+        // Finished rows pass through the tile's P buffers, which no MMA reads any more, 16-byte piece p of row r at p ^ (r % 8).
+        auto row_at = [&](int row, int piece, int pieces) { return reinterpret_cast<uint4*>(myPs + row * (pieces * 16) + ((piece ^ (row & 7)) << 4)); };
         if (n_split > 1) {
             // one of several CTAs over this row's keys: O as it stands, with the reference maximum and the sum
-            const size_t slot = ((size_t)split * total_rows + token) * Hq + h;
             if (row_valid) {
+                const size_t slot = ((size_t)split * total_rows + token0 + r) * Hq + h;
                 part_ml[2 * slot] = n_mine > 0 ? m_ref : -INFINITY;
                 part_ml[2 * slot + 1] = n_mine > 0 ? l_run : 0.f;
             }
             if (n_mine > 0) {
-                float* prow = part_o + slot * D;
 #pragma unroll 1
-                for (int c0 = 0; c0 < D; c0 += 32) {
+                for (int c0 = 0; c0 < D; c0 += 32) {       // 32 columns are eight pieces of four floats
                     unsigned o[32];
                     tmem_ld32(o_addr + c0, o);
                     tmem_ld_wait();
-                    if (row_valid) {
+                    __syncwarp();                            // the columns before these have been taken
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<uint4*>(prow + c0 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                    for (int i = 0; i < 8; ++i) *row_at(r, i, 8) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rr = (warp & 3) * 32 + i * 4 + (lane >> 3);
+                        if (qt * QM + rr < m_rows)
+                            *reinterpret_cast<uint4*>(part_o + (((size_t)split * total_rows + token0 + rr) * Hq + h) * D + c0 + (lane & 7) * 4) = *row_at(rr, lane & 7, 8);
                     }
                 }
             }
         } else if (n_mine > 0) {
             // a sink: a term of the denominator that has no key and no value, not scaled
             const float inv = 1.f / (sink != nullptr ? l_run + exp2f(sink[h] * LOG2E - m_ref) : l_run);
-            bf16* orow = out + token * ((size_t)Hq * D) + (size_t)h * D;
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 32) {
                 unsigned o[32];
                 tmem_ld32(o_addr + c0, o);
                 tmem_ld_wait();
-                if (row_valid) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 v;
-                        __nv_bfloat162 a0 = __floats2bfloat162_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                        __nv_bfloat162 a1 = __floats2bfloat162_rn(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                        __nv_bfloat162 a2 = __floats2bfloat162_rn(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                        __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                        v.x = *reinterpret_cast<unsigned*>(&a0); v.y = *reinterpret_cast<unsigned*>(&a1);
-                        v.z = *reinterpret_cast<unsigned*>(&a2); v.w = *reinterpret_cast<unsigned*>(&a3);
-                        *reinterpret_cast<uint4*>(orow + c0 + i) = v;
-                    }
+                for (int i = 0; i < 32; i += 8) {
+                    uint4 v;
+                    __nv_bfloat162 a0 = __floats2bfloat162_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                    __nv_bfloat162 a1 = __floats2bfloat162_rn(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                    __nv_bfloat162 a2 = __floats2bfloat162_rn(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                    __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                    v.x = *reinterpret_cast<unsigned*>(&a0); v.y = *reinterpret_cast<unsigned*>(&a1);
+                    v.z = *reinterpret_cast<unsigned*>(&a2); v.w = *reinterpret_cast<unsigned*>(&a3);
+                    *row_at(r, (c0 + i) >> 3, LPR) = v;
                 }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 32 / RPI; ++i) {
+                const int rr = (warp & 3) * 32 + i * RPI + rsel;
+                if (qt * QM + rr < m_rows)
+                    *reinterpret_cast<uint4*>(out + (token0 + rr) * ((size_t)Hq * D) + (size_t)h * D + sub * 8) = *row_at(rr, sub, LPR);
             }
         }
     } else if (warp == W_MMA || warp == W_MMA_B) {
@@ -569,8 +608,6 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
                 if ((j >= lo_min || j < keep) && j <= p_last && next_page[u] >= 0)
                     where[u] = reinterpret_cast<unsigned long long>(pool + (((size_t)next_page[u] * Hkv + kvh) * pg.page_size + pg.row(j)) * D);
             }
-            constexpr int LPR = D / 8, RPI = 32 / LPR;              // lanes a row, rows an instruction
-            const int sub = lane % LPR, rsel = lane / LPR;
             const unsigned piece = (unsigned)(sub >> 3) * (KN * 128), c7 = (unsigned)(sub & 7);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -616,13 +653,17 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
 // out[row, h] = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M) over the splits of the keys: one warp a (row, head).
 __global__ void __launch_bounds__(256)
 merge_key_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                        const int* __restrict__ tiles, const int* __restrict__ cu_q, int n_split, int total_rows,
+                        const int* __restrict__ tiles, const int* __restrict__ cu_q, const int* __restrict__ seg_pos0, int max_split,
+                        int share, int window, int chunk, int keep, int total_rows,
                         int Hq, bf16* __restrict__ out, const float* __restrict__ sink) {
     const int seg = tiles[2 * blockIdx.y], row0 = tiles[2 * blockIdx.y + 1];
     const int q_begin = cu_q[seg];
     const int m_rows = min(NQ * QM, cu_q[seg + 1] - q_begin - row0);
     const int r = blockIdx.z * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, h = blockIdx.x;
     if (r >= m_rows) return;
+    const int p0 = seg_pos0[seg] + row0;
+    const int n_split = shares_of((p0 + m_rows - 1) / KN - Walk(p0, window, chunk, keep).jt_first + 1, max_split, share);
+    if (n_split == 1) return;                              // the block's only CTA wrote its rows
     const size_t token = (size_t)(q_begin + row0 + r);
     constexpr int PER = D / 32;                            // floats of a row a lane holds: 2 or 4
     float m_all = -INFINITY;
@@ -657,7 +698,8 @@ RB_EXPORT long long rb_attn_tc5_split_floats(int n_split, int total_rows, int Hq
 }
 
 // tiles: [n_tiles, 2] = (segment, first row of a block of up to 256 query rows), the blocks with the
-// longest contexts first.  n_split > 1 splits the keys of every block over that many CTAs; ``scratch`` then
+// longest contexts first.  n_split > 1 splits the keys of every block over that many CTAs, or with share > 0 over one CTA for
+// every `share` key tiles, n_split at most; ``scratch`` then
 // holds rb_attn_tc5_split_floats(...) floats and total_rows is the number of rows of q.
 // chunk, softcap, slopes, bias, keep: the score options (0, 0, null, null, 0: the plain kernel); a window and a chunk exclude
 // each other, kept first positions go with a window.
@@ -666,11 +708,11 @@ RB_EXPORT int rb_attn_prefill_tc5_mod(const void* q, int ld, const void* kpool, 
                                       int bt_stride, int page_size, void* out, int Hq, int Hkv, float scale, int window,
                                       int n_split, void* scratch, int total_rows, int* status, const float* sink,
                                       int chunk, float softcap, const float* slopes, const float* bias, int bias_n,
-                                      int keep, cudaStream_t st) {
+                                      int keep, int share, cudaStream_t st) {
     if (n_tiles <= 0) return 0;
     if (bias != nullptr && bias_n < 1) return (int)cudaErrorInvalidValue;
     if (n_tiles > 65535 || n_split < 1 || n_split > 64 || (n_split > 1 && scratch == nullptr)) return (int)cudaErrorInvalidValue;
-    if ((window > 0 && chunk > 0) || keep < 0 || (keep > 0 && window <= 0)) return (int)cudaErrorInvalidValue;
+    if ((window > 0 && chunk > 0) || keep < 0 || (keep > 0 && window <= 0) || share < 0) return (int)cudaErrorInvalidValue;
     static PerDevice configured;
     const int rc = configured.once([](int) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
@@ -686,14 +728,15 @@ RB_EXPORT int rb_attn_prefill_tc5_mod(const void* q, int ld, const void* kpool, 
     if (chunk > 0 || softcap > 0.f || slopes != nullptr || bias != nullptr || keep > 0)
         attn_prefill_tc5_kernel<true><<<grid, THREADS, SMEM_BYTES, st>>>(
             (const bf16*)q, ld, (const bf16*)kpool, (const bf16*)vpool, tiles, cu_q, seg_pos0, block_table, bt_stride,
-            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm);
+            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm, share);
     else
         attn_prefill_tc5_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(
             (const bf16*)q, ld, (const bf16*)kpool, (const bf16*)vpool, tiles, cu_q, seg_pos0, block_table, bt_stride,
-            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm);
+            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm, share);
     if (n_split > 1) {
         dim3 mgrid(Hq, n_tiles, NQ * QM / 8);
-        merge_key_splits_kernel<<<mgrid, 256, 0, st>>>(part_o, part_ml, tiles, cu_q, n_split, total_rows, Hq, (bf16*)out, sink);
+        merge_key_splits_kernel<<<mgrid, 256, 0, st>>>(part_o, part_ml, tiles, cu_q, seg_pos0, n_split, share, window, chunk, keep, total_rows, Hq,
+                                                       (bf16*)out, sink);
     }
     return rb_launch_status();
 }
@@ -704,5 +747,5 @@ RB_EXPORT int rb_attn_prefill_tc5(const void* q, int ld, const void* kpool, cons
                                   int n_split, void* scratch, int total_rows, int* status, const float* sink,
                                   cudaStream_t st) {
     return rb_attn_prefill_tc5_mod(q, ld, kpool, vpool, tiles, n_tiles, cu_q, seg_pos0, block_table, bt_stride, page_size, out,
-                                   Hq, Hkv, scale, window, n_split, scratch, total_rows, status, sink, 0, 0.f, nullptr, nullptr, 0, 0, st);
+                                   Hq, Hkv, scale, window, n_split, scratch, total_rows, status, sink, 0, 0.f, nullptr, nullptr, 0, 0, 0, st);
 }

@@ -9,6 +9,7 @@ library (rollout/monkey_patch/qwen3.py:21-22,29-31,56).
 from __future__ import annotations
 
 import ctypes
+import heapq
 from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
@@ -707,7 +708,7 @@ def attention_tc5_lib(head_dim: int) -> ctypes.CDLL:
         lib = build.load(f"return_attn_tc5_d{head_dim}", ["attention_tc5.cu"], _attn_tc5_defines(head_dim))
         P, I, F = c_void_p, c_int, c_float
         lib.rb_attn_prefill_tc5.argtypes = [P, I, P, P, P, I, P, P, P, I, I, P, I, I, F, I, I, P, I, P, P, P]
-        lib.rb_attn_prefill_tc5_mod.argtypes = [P, I, P, P, P, I, P, P, P, I, I, P, I, I, F, I, I, P, I, P, P, I, F, P, P, I, I, P]
+        lib.rb_attn_prefill_tc5_mod.argtypes = [P, I, P, P, P, I, P, P, P, I, I, P, I, I, F, I, I, P, I, P, P, I, F, P, P, I, I, I, P]
         lib.rb_attn_prefill_tc5_mod.restype = c_int
         lib.rb_attn_tc5_split_floats.argtypes = [I, I, I]
         lib.rb_attn_tc5_split_floats.restype = ctypes.c_longlong
@@ -733,10 +734,11 @@ def _bias_args(bias, num_heads):
 
 def attention_prefill_tc5(qkv, k_pool, v_pool, tiles, cu_q, seg_pos0, block_table, page_size, out, num_heads,
                           num_kv_heads, head_dim, scale, window=0, num_splits=1, held=None, sink=None,
-                          chunk=0, softcap=0.0, slopes=None, bias=None, keep=0) -> None:
+                          chunk=0, softcap=0.0, slopes=None, bias=None, keep=0, share=0) -> None:
     """tcgen05 attention for the listed (segment, first row) blocks of up to TC5_TILE_ROWS query rows
     (the blocks with the longest contexts should come first: they take longest).  ``num_splits`` > 1 splits
-    every block's keys over that many CTAs and merges them in a second launch; ``held``: the step's map of
+    every block's keys over that many CTAs (with ``share`` > 0: over one CTA for every ``share`` key tiles of
+    PREFILL_KEY_TILE keys, ``num_splits`` at most) and merges them in a second launch; ``held``: the step's map of
     work buffers, so that the layers share the buffer of the partial results.  ``chunk``, ``softcap``, ``slopes``, ``bias``,
     ``keep``: the score options of ``paged_attention``."""
     assert qkv.dtype == torch.bfloat16 and k_pool.dtype == torch.bfloat16 and out.is_contiguous()
@@ -757,7 +759,7 @@ def attention_prefill_tc5(qkv, k_pool, v_pool, tiles, cu_q, seg_pos0, block_tabl
                                        block_table.stride(0), page_size, _ptr(out), num_heads, num_kv_heads, scale,
                                        int(window or 0), num_splits, _ptr(scratch), T, _ptr(tc5_status(qkv.device)),
                                        _sink_ptr(sink, num_heads), int(chunk or 0), float(softcap or 0.0),
-                                       _sink_ptr(slopes, num_heads), *_bias_args(bias, num_heads), int(keep or 0), _stream()),
+                                       _sink_ptr(slopes, num_heads), *_bias_args(bias, num_heads), int(keep or 0), int(share), _stream()),
            "attention_prefill_tc5", 2 if num_splits > 1 else 1)
 
 
@@ -771,20 +773,76 @@ def prefill_splits(n_ctas: int, longest_context: int) -> int:
     return max(1, min(num_sms() // max(1, n_ctas), longest_context // PREFILL_SPLIT_MIN_KEYS, 64))
 
 
-def _prefill_split_count(batch, num_heads, window) -> int:
+PREFILL_KEY_TILE = 64              # keys of a tile of the tcgen05 prefill attention kernel
+# What a CTA costs beside its key tiles (query rows in, tensor memory, the first scores, rows out) and what the merge of a split
+# costs, in key tiles of 1.1 us: measured 9 us and 4 us.
+PREFILL_CTA_TILES, PREFILL_MERGE_TILES = 8, 4
+PREFILL_SPLIT_SCRATCH_BYTES = 64 << 20
+
+
+def _launch_tiles(work, heads: int, sms: int) -> int:
+    """When a launch is done whose CTAs, ``heads`` alike of every length in ``work`` in this order, go one by one to the SM that
+    is free first."""
+    free = [(0, sms)]                                  # (time, SMs that are free then), a heap
+    done = 0
+    for length in work:
+        need = heads
+        while need:
+            at, n = heapq.heappop(free)
+            took = min(n, need)
+            if n > took:
+                heapq.heappush(free, (at, n - took))
+            heapq.heappush(free, (at + length, took))
+            done = max(done, at + length)
+            need -= took
+    return done
+
+
+def prefill_shares(tiles, heads: int, rows: int, head_dim: int):
+    """(CTAs that the longest block's keys are split over, key tiles of a CTA's share or 0 for no split) for blocks that walk
+    ``tiles`` key tiles each, all ``heads`` alike, ``rows`` query rows in all.  Among splits of the longest block into s shares (of
+    PREFILL_SPLIT_MIN_KEYS keys at least), with every other block cut into shares of about that size, the one whose launch is done
+    first (``_launch_tiles``; the kernel starts first shares of all blocks first, then second ones, ...).  The partial results of a
+    split stay under PREFILL_SPLIT_SCRATCH_BYTES."""
+    sms, longest = num_sms(), max(tiles)
+    even = heads * (sum(tiles) + len(tiles) * PREFILL_CTA_TILES) / sms
+    if len(tiles) > 256:                               # many blocks: whatever is uneven is short beside the rest
+        return 1, 0
+    best, best_done = (1, 0), _launch_tiles([t + PREFILL_CTA_TILES for t in tiles], heads, sms)
+    if best_done <= 1.25 * even:                       # the blocks keep the SMs busy as they are
+        return best
+    for s in (2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 32, 48, 64):
+        share = -(-longest // s)
+        if share * PREFILL_KEY_TILE < PREFILL_SPLIT_MIN_KEYS or s * rows * heads * (head_dim + 2) * 4 > PREFILL_SPLIT_SCRATCH_BYTES:
+            break
+        counts = [-(-t // share) for t in tiles]
+        if heads * sum(counts) > 3 * sms:              # more than SMs can take in a few rounds: the CTAs' own cost grows
+            break
+        work = [-(-t // c) + PREFILL_CTA_TILES for z in range(max(counts)) for t, c in zip(tiles, counts) if c > z]
+        d = _launch_tiles(work, heads, sms) + PREFILL_MERGE_TILES
+        if d < best_done:
+            best, best_done = (s, share), d
+    return best
+
+
+def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=0):
+    """``prefill_shares`` of this step's blocks, worked out once per step and kind of layer."""
     held = getattr(batch, "scratch", None)
-    key = ("attention.prefill_splits", num_heads, window)
+    key = ("attention.prefill_shares", num_heads, head_dim, window, chunk, keep)
     if held is not None and key in held:
         return held[key]
     host = batch.host
-    tiles = host.tiles[TILES_TC5]
-    longest = int(host.seg_kv_len[tiles[:, 0]].max())
-    if window:
-        longest = min(longest, int(window) + TC5_TILE_ROWS)
-    n = prefill_splits(tiles.shape[0] * num_heads, longest)
+    tiles = []
+    for seg, row0 in host.tiles[TILES_TC5].tolist():
+        p0 = int(host.seg_pos0[seg]) + row0
+        end = min(int(host.seg_kv_len[seg]), p0 + TC5_TILE_ROWS)
+        low = max(0, p0 - window + 1) if window else p0 // chunk * chunk if chunk else 0
+        kept = min(-(-keep // PREFILL_KEY_TILE), low // PREFILL_KEY_TILE) if window and keep else 0
+        tiles.append((end - 1) // PREFILL_KEY_TILE - low // PREFILL_KEY_TILE + 1 + kept)
+    shares = prefill_shares(tiles, num_heads, host.num_tokens, head_dim)
     if held is not None:
-        held[key] = n
-    return n
+        held[key] = shares
+    return shares
 
 
 def decode_splits(n_ctas_base: int, max_kv_len: int, ctas_per_sm: int = 2) -> int:
@@ -962,10 +1020,11 @@ def paged_attention(qkv, k_pool, v_pool, batch, block_table, page_size, out, num
     bound = keys_seen(window, keep) or chunk      # either bounds the keys a query can see
     if host.num_multi:
         if head_dim in TC5_ATTENTION_HEAD_DIMS:
+            splits, share = prefill_shares_of(batch, num_heads, head_dim, window, chunk, keep)
             attention_prefill_tc5(qkv, k_pool, v_pool, batch.tiles[TILES_TC5], batch.cu_q, batch.seg_pos0, block_table,
                                   page_size, out, num_heads, num_kv_heads, head_dim, scale, window or 0,
-                                  _prefill_split_count(batch, num_heads, bound), getattr(batch, "scratch", None), sink,
-                                  chunk, softcap, slopes, bias, keep)
+                                  splits, getattr(batch, "scratch", None), sink,
+                                  chunk, softcap, slopes, bias, keep, share)
         else:
             attention_prefill_mma(qkv, k_pool, v_pool, batch.tiles[TILES_MMA], batch.cu_q, batch.seg_pos0, block_table,
                                   page_size, out, num_heads, num_kv_heads, head_dim, scale, window or 0, sink,

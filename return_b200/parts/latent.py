@@ -155,9 +155,9 @@ class LatentAttention(Mixer):
         qx = ctx.buffer("latent.x_q", (T, H * head), dt, dev)
         ops.latent_expand_query(q, q_abs, self.width, C, qx, H, D, R)
         ox = ctx.buffer("latent.x_o", (T, H * head), dt, dev)
+        splits, share = ops.prefill_shares_of(b, H, head, s.window)
         ops.attention_prefill_tc5(qx, pools[0], pools[1], b.tiles[ops.TILES_TC5], b.cu_q, b.seg_pos0, kv.block_table,
-                                  kv.page_size, ox, H, H, head, s.scale, s.window or 0,
-                                  ops._prefill_split_count(b, H, s.window), b.scratch, self.sink_f32)
+                                  kv.page_size, ox, H, H, head, s.scale, s.window or 0, splits, b.scratch, self.sink_f32, share=share)
         ops.latent_take_values(ox, b, packed, H, Vd)
 
     # ------------------------------------------------------------------ one step

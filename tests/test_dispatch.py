@@ -26,6 +26,46 @@ def test_prefill_key_splits():
             assert 1 <= s <= 64 and (s == 1 or (s * ctas <= ops.num_sms() and keys // s >= ops.PREFILL_SPLIT_MIN_KEYS))
 
 
+def test_prefill_key_shares():
+    """Shares keep enough keys, cover the longest block and stay within the scratch; even work is left alone."""
+    import random
+    from types import SimpleNamespace
+
+    import numpy as np
+    from return_b200.ext import ops
+    assert ops.prefill_shares([4 * i for i in range(8, 0, -1)], 32, 2048, 128) == (1, 0)        # a whole prompt, 32 heads
+    assert ops.prefill_shares([8], 4, 200, 128) == (1, 0)                                       # a share would have too few keys
+    rng = random.Random(0)
+    for _ in range(300):
+        tiles = [rng.randint(1, 400) for _ in range(rng.randint(1, 40))]
+        heads, rows = rng.choice((4, 16, 32)), 256 * len(tiles)
+        s, share = ops.prefill_shares(tiles, heads, rows, 128)
+        if s == 1:
+            assert share == 0
+            continue
+        assert 1 < s <= 64 and share * ops.PREFILL_KEY_TILE >= ops.PREFILL_SPLIT_MIN_KEYS
+        assert -(-max(tiles) // share) <= s and s * rows * heads * 130 * 4 <= ops.PREFILL_SPLIT_SCRATCH_BYTES
+    # the tiles that the kernel walks for a block, counted key by key
+    for _ in range(100):
+        pos0, n = rng.randint(0, 600), rng.randint(2, 700)
+        window, chunk, keep = rng.choice(((None, None, 0), (rng.randint(1, 300), None, 0), (rng.randint(1, 300), None, rng.randint(1, 300)),
+                                          (None, rng.randint(1, 300), 0)))
+        blocks = np.array([(0, r) for r in range(0, n, ops.TC5_TILE_ROWS)], np.int32)
+        seen = []
+        real, ops.prefill_shares = ops.prefill_shares, lambda tiles, *rest: (seen.append(tiles), (1, 0))[1]
+        try:
+            ops.prefill_shares_of(SimpleNamespace(host=SimpleNamespace(tiles={ops.TILES_TC5: blocks}, seg_pos0=np.array([pos0]),
+                                                                       seg_kv_len=np.array([pos0 + n]), num_tokens=n)), 4, 128, window, chunk, keep)
+        finally:
+            ops.prefill_shares = real
+        for got, (_, r0) in zip(seen[0], blocks):
+            first = pos0 + r0
+            last = min(first + ops.TC5_TILE_ROWS, pos0 + n) - 1
+            low = max(0, first - window + 1) if window else first // chunk * chunk if chunk else 0
+            walked = {j // 64 for j in range(low, last + 1)} | {j // 64 for j in range(min(keep, low // 64 * 64))}
+            assert got == len(walked)
+
+
 def test_decode_key_splits():
     from return_b200.ext import ops
     for base in (1, 8, 64, 296, 512, 2000):

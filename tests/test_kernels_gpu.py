@@ -325,6 +325,27 @@ def test_attention_prefill_tc5(Hq, Hkv, D, P, window, splits):
     assert torch.allclose(out.float().cpu(), pg.reference(scale, window), atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("window,keep,softcap", [(None, 0, 0.0), (150, 0, 0.0), (130, 70, 0.0), (None, 0, 5.0)])
+@pytest.mark.parametrize("share", [1, 3, 4])
+def test_attention_prefill_tc5_shares(D, window, keep, softcap, share):
+    """Blocks split over as many CTAs as they have shares of key tiles: one, several or the most, a last share of fewer tiles,
+    against the same blocks unsplit (the plain kernel's own result; the sums differ in their order only)."""
+    ops = _ops()
+    Hq, Hkv, P = 4, 2, 16
+    kv_lens, q_lens = [2, 64, 65, 700, 1000, 300], [2, 64, 3, 300, 70, 257]
+    pg = Paged(kv_lens, q_lens, Hq, Hkv, D, P, torch.bfloat16, seed=D + 7)
+    tiles = torch.tensor([(i, r0) for i, ql in enumerate(q_lens) for r0 in range(0, ql, ops.TC5_TILE_ROWS)], dtype=torch.int32, device=DEV)
+    outs = []
+    for splits, per in ((1, 0), (5, share)):
+        outs.append(torch.full((sum(q_lens), Hq * D), float("nan"), device=DEV, dtype=torch.bfloat16))
+        ops.attention_prefill_tc5(pg.qkv, pg.kpool, pg.vpool, tiles, pg.cu_q, pg.seg_pos0, pg.bt, P, outs[-1], Hq, Hkv, D, D ** -0.5,
+                                  window or 0, num_splits=splits, softcap=softcap, keep=keep, share=per)
+    ops.check_status(DEV)
+    # probabilities are rounded to bfloat16 against another reference maximum, at most 2^-8 of a value either way
+    assert torch.allclose(outs[1].float(), outs[0].float(), atol=2.0 ** -6, rtol=2.0 ** -6)
+
+
 def test_prefill_split_choice():
     """Keys are split only while blocks x heads leave SMs idle and every share keeps enough keys."""
     ops = _ops()
