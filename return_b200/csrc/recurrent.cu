@@ -512,6 +512,24 @@ RB_EXPORT int rb_memory_pieces_combine(float* pieces, long long piece_stride, fl
                          state, state_stride, m_off, f_off, seg_first, seg_slot, H);
 }
 
+// ---------------------------------------------------------------- four elements at a time
+// The kernels around a scan only move rows, so what bounds them is memory.  Where sizes and addresses allow, a lane takes four
+// neighbouring elements in one access (16 bytes of float32, 8 of bfloat16); the element-wise kernels beside them take the rest.
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld4(const bf16* p) {
+    const uint2 b = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(b.x << 16), __uint_as_float(b.x & 0xffff0000u), __uint_as_float(b.y << 16), __uint_as_float(b.y & 0xffff0000u));
+}
+__device__ __forceinline__ float4 ld4(const void* p, int dtype, size_t i) { return dtype == RB_F32 ? ld4((const float*)p + i) : ld4((const bf16*)p + i); }
+__device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void st4(bf16* p, const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+// Whether four elements at p, and at p plus any multiple of four, can be taken at once.
+static inline bool fours(const float* p) { return ((uintptr_t)p % 16) == 0; }
+static inline bool fours(const void* p, int dtype) { return ((uintptr_t)p % (dtype == RB_F32 ? 16 : 8)) == 0; }
+
 // ---------------------------------------------------------------- rotation of q and k into float32
 // x: two runs of `heads` heads of size D inside rows of a projection buffer (q at q_off, k at k_off).  The first
 // `rot` elements of a head turn by the angle of the token's position (tables cos, sin [positions, rot/2]), element
@@ -546,11 +564,46 @@ __global__ void rotary_to_f32_kernel(const TA* __restrict__ x, int ld, int q_off
     }
 }
 
+// Heads that turn whole: a CTA a token, a thread four pairs of one head.  2,048 tokens of 16 + 16 heads of 128: ROT_NEW us (element by
+// element, a CTA a token and head: 36.5 us).
+template <typename TA>
+__global__ void __launch_bounds__(256)
+rotary_to_f32_vec_kernel(const TA* __restrict__ x, int ld, int q_off, int k_off, const float* __restrict__ cos_t,
+                         const float* __restrict__ sin_t, const int* __restrict__ pos, float* __restrict__ q32, float* __restrict__ k32,
+                         int heads, int D, float q_scale, float k_scale) {
+    pdl_wait();
+    const int t = blockIdx.x, half = D >> 1, per = half >> 2;
+    const size_t p = (size_t)pos[t] * half;
+    for (int e = threadIdx.x; e < 2 * heads * per; e += blockDim.x) {
+        const int hh = e / per, i = (e - hh * per) * 4;
+        const bool is_k = hh >= heads;
+        const int h = is_k ? hh - heads : hh;
+        const TA* src = x + (size_t)t * ld + (is_k ? k_off : q_off) + (size_t)h * D + i;
+        const float scale = is_k ? k_scale : q_scale;
+        const float4 u = ld4(src), v = ld4(src + half), c = ld4(cos_t + p + i), s = ld4(sin_t + p + i);
+        float* dst = (is_k ? k32 : q32) + ((size_t)t * heads + h) * D + i;
+        st4(dst, make_float4((u.x * c.x - v.x * s.x) * scale, (u.y * c.y - v.y * s.y) * scale, (u.z * c.z - v.z * s.z) * scale, (u.w * c.w - v.w * s.w) * scale));
+        st4(dst + half, make_float4((v.x * c.x + u.x * s.x) * scale, (v.y * c.y + u.y * s.y) * scale, (v.z * c.z + u.z * s.z) * scale, (v.w * c.w + u.w * s.w) * scale));
+    }
+}
+
+template <typename TA>
+static int launch_rotary_vec(const void* x, int ld, int q_off, int k_off, const float* cos_t, const float* sin_t, const int* pos, float* q32,
+                             float* k32, int T, int heads, int D, float q_scale, float k_scale, cudaStream_t st) {
+    const int tasks = 2 * heads * (D / 8);
+    return rb_launch_pdl(rotary_to_f32_vec_kernel<TA>, dim3(T), dim3(tasks < 256 ? (tasks + 31) / 32 * 32 : 256), 0, st, (const TA*)x, ld, q_off, k_off,
+                         cos_t, sin_t, pos, q32, k32, heads, D, q_scale, k_scale);
+}
+
 RB_EXPORT int rb_rotary_to_f32(const void* x, int ld, int q_off, int k_off, const float* cos_t, const float* sin_t,
                                int rot, const int* pos, float* q32, float* k32, int act_dtype, int T, int heads, int D,
                                float q_scale, float k_scale, cudaStream_t st) {
     if (T <= 0) return 0;
     if (rot > D || (rot & 1)) return (int)cudaErrorInvalidValue;
+    if (rot == D && D % 8 == 0 && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && fours(x, act_dtype) && fours(cos_t) && fours(sin_t) && fours(q32) &&
+        fours(k32))
+        return (act_dtype == RB_F32 ? launch_rotary_vec<float> : launch_rotary_vec<bf16>)(x, ld, q_off, k_off, cos_t, sin_t, pos, q32, k32, T, heads,
+                                                                                          D, q_scale, k_scale, st);
     dim3 grid(T, 2 * heads);
     const int threads = D <= 32 ? 32 : D <= 64 ? 64 : 128;
     if (act_dtype == RB_F32)
@@ -652,6 +705,139 @@ delta_prep_kernel(const TA* __restrict__ x, int ld, const void* __restrict__ tap
     }
 }
 
+// The same with four channels a lane: a warp takes one unit (a query, key or value head of up to 256 channels) of TOK tokens one after
+// the other, the inputs that the taps reach back to in registers, so that a token costs one read of its row.  Taps up to four.  The
+// CTAs behind those of the heads take the decays, 1,024 a CTA and round, and the betas.  2,048 tokens of 4 + 4 + 16 heads of 128
+// with a decay per key row: PREP_NEW us (a CTA a token and unit, element by element: 77).
+#define PREP_MAX_TAPS 4
+template <typename TA, int NV, int TOK>
+__global__ void __launch_bounds__(256)
+delta_prep_vec_kernel(const TA* __restrict__ x, int ld, const void* __restrict__ taps, int taps_dtype, int K,
+                      const float* __restrict__ state, long long state_stride, int conv_off,
+                      const int* __restrict__ tok_seg, const int* __restrict__ cu_q, const int* __restrict__ seg_slot,
+                      float* __restrict__ q32, float* __restrict__ k32, float* __restrict__ v32,
+                      float* __restrict__ a, const void* __restrict__ A_log, const void* __restrict__ dt_bias, int vec_dtype,
+                      float* __restrict__ b, int T, int H, int G, int D, int V, float q_scale, int DA, int conv_ctas, int decay_ctas) {
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    if ((int)blockIdx.x >= conv_ctas) {
+        const int cta = blockIdx.x - conv_ctas;
+        const long long n = (long long)T * H * DA;
+        if (cta >= decay_ctas) {
+            for (long long e = (long long)(cta - decay_ctas) * 256 + threadIdx.x; e < (long long)T * H; e += (long long)(gridDim.x - conv_ctas - decay_ctas) * 256)
+                b[e] = sigmoid_f(b[e]);
+        } else if (DA % 4 == 0) {
+            for (long long e = ((long long)cta * 256 + threadIdx.x) * 4; e < n; e += (long long)decay_ctas * 1024) {
+                const int c = (int)(e % (H * DA));
+                const float rate = expf(load_as_f32(A_log, vec_dtype, c / DA));
+                const float4 y = ld4(a + e), d = ld4(dt_bias, vec_dtype, c);
+                st4(a + e, make_float4(expf(-rate * softplus_f(y.x + d.x)), expf(-rate * softplus_f(y.y + d.y)), expf(-rate * softplus_f(y.z + d.z)),
+                                       expf(-rate * softplus_f(y.w + d.w))));
+            }
+        } else {
+            for (long long e = (long long)cta * 256 + threadIdx.x; e < n; e += (long long)decay_ctas * 256) {
+                const int c = (int)(e % (H * DA));
+                a[e] = expf(-expf(load_as_f32(A_log, vec_dtype, c / DA)) * softplus_f(a[e] + load_as_f32(dt_bias, vec_dtype, c)));
+            }
+        }
+        return;
+    }
+    const int units = 2 * G + H, task = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int unit = task % units, tb = (task / units) * TOK;
+    if (tb >= T) return;
+    int c0, len;
+    float* dst;                                           // of token 0
+    size_t dst_ld;
+    if (unit < G) { c0 = unit * D; len = D; dst = q32 + (size_t)unit * D; dst_ld = (size_t)G * D; }
+    else if (unit < 2 * G) { c0 = unit * D; len = D; dst = k32 + (size_t)(unit - G) * D; dst_ld = (size_t)G * D; }
+    else { c0 = 2 * G * D + (unit - 2 * G) * V; len = V; dst = v32 + (size_t)(unit - 2 * G) * V; dst_ld = (size_t)H * V; }
+    const bool normed = unit < 2 * G;
+    const float scale = unit < G ? q_scale : 1.0f;
+    float w[NV][4][PREP_MAX_TAPS], back[NV][PREP_MAX_TAPS - 1][4];       // back[.][m]: the input m + 1 tokens before
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+#pragma unroll
+            for (int j = 0; j < PREP_MAX_TAPS; ++j) {
+                const int i = 128 * n + 4 * lane + ch;
+                w[n][ch][j] = i < len && j < K ? load_as_f32(taps, taps_dtype, (size_t)(c0 + i) * K + (K - 1 - j)) : 0.f;   // of the input j tokens back
+            }
+    int seg = -1;
+#pragma unroll 1
+    for (int u = 0; u < TOK && tb + u < T; ++u) {
+        const int t = tb + u, s = tok_seg[t];
+        const TA* row = x + (size_t)t * ld + c0 + 4 * lane;
+        if (s != seg) {                                   // the first token here, or of its segment: what came before it
+            seg = s;
+            const int l = t - cu_q[s];                    // tokens of the segment before t
+            const float* cs = state + (long long)seg_slot[s] * state_stride + conv_off;
+#pragma unroll
+            for (int n = 0; n < NV; ++n)
+#pragma unroll
+                for (int m = 0; m < PREP_MAX_TAPS - 1; ++m) {
+                    const int j = m + 1, i = 128 * n + 4 * lane;
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (i < len && j < K) {
+                        if (j <= l) {
+                            v = ld4(row - (size_t)j * ld + 128 * n);
+                        } else {
+                            const float* at = cs + (size_t)(c0 + i) * (K - 1) + (K - 1 - (j - l));
+                            v = make_float4(at[0], at[K - 1], at[2 * (K - 1)], at[3 * (K - 1)]);
+                        }
+                    }
+                    back[n][m][0] = v.x; back[n][m][1] = v.y; back[n][m][2] = v.z; back[n][m][3] = v.w;
+                }
+        }
+        float y[NV][4], ss = 0.f;
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+            const bool live = 128 * n + 4 * lane < len;
+            const float4 v4 = live ? ld4(row + 128 * n) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float now[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) {
+                float z = 0.f;                            // oldest first; taps that do not exist are left out
+#pragma unroll
+                for (int j = PREP_MAX_TAPS - 1; j > 0; --j)
+                    if (j < K) z = fmaf(w[n][ch][j], back[n][j - 1][ch], z);
+                z = fmaf(w[n][ch][0], now[ch], z);
+                z = live ? z / (1.0f + expf(-z)) : 0.f;
+                y[n][ch] = z;
+                ss = fmaf(z, z, ss);
+#pragma unroll
+                for (int m = PREP_MAX_TAPS - 2; m > 0; --m) back[n][m][ch] = back[n][m - 1][ch];
+                back[n][0][ch] = now[ch];
+            }
+        }
+        float inv = 1.0f;
+        if (normed) inv = scale / sqrtf(warp_sum(ss) + 1e-6f);
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+            if (128 * n + 4 * lane < len)
+                st4(dst + (size_t)t * dst_ld + 128 * n + 4 * lane, make_float4(y[n][0] * inv, y[n][1] * inv, y[n][2] * inv, y[n][3] * inv));
+    }
+}
+
+template <typename TA>
+static int launch_delta_prep_vec(const void* x, int ld, const void* taps, int taps_dtype, int K, const float* state, long long state_stride,
+                                 int conv_off, const int* tok_seg, const int* cu_q, const int* seg_slot, float* q32, float* k32, float* v32, float* a,
+                                 const void* A_log, const void* dt_bias, int vec_dtype, float* b, int T, int H, int G, int D, int V, float q_scale,
+                                 int DA, cudaStream_t st) {
+    const bool many = T >= 1024;                          // runs of tokens only where there are warps enough all the same
+    const int tok = many ? 8 : 1;
+    const long long tasks = (long long)((T + tok - 1) / tok) * (2 * G + H);
+    const int conv_ctas = (int)((tasks + 7) / 8);
+    auto ctas = [](long long n) { return (int)(n < 2048 ? n : 2048); };
+    const int decay_ctas = ctas(((long long)T * H * DA + 1023) / 1024), beta_ctas = ctas(((long long)T * H + 1023) / 1024);
+    const bool wide = D > 128 || V > 128;
+    auto kernel = many ? (wide ? delta_prep_vec_kernel<TA, 2, 8> : delta_prep_vec_kernel<TA, 1, 8>)
+                       : (wide ? delta_prep_vec_kernel<TA, 2, 1> : delta_prep_vec_kernel<TA, 1, 1>);
+    return rb_launch_pdl(kernel, dim3(conv_ctas + decay_ctas + beta_ctas), dim3(256), 0, st, (const TA*)x, ld, taps, taps_dtype, K, state, state_stride,
+                         conv_off, tok_seg, cu_q, seg_slot, q32, k32, v32, a, A_log, dt_bias, vec_dtype, b, T, H, G, D, V, q_scale, DA, conv_ctas,
+                         decay_ctas);
+}
+
 RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dtype, int K, const float* state,
                             long long state_stride, int conv_off, const int* tok_seg, const int* cu_q, const int* seg_slot,
                             float* q32, float* k32, float* v32, float* a, const void* A_log, const void* dt_bias,
@@ -660,6 +846,11 @@ RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dt
     if (T <= 0) return 0;
     if (K < 1) return (int)cudaErrorInvalidValue;
     const int DA = head_decay ? 1 : D;
+    if (K <= PREP_MAX_TAPS && D % 4 == 0 && V % 4 == 0 && D <= 256 && V <= 256 && ld % 4 == 0 && fours(x, act_dtype) && fours(q32) && fours(k32) &&
+        fours(v32) && fours(a) && fours(dt_bias, vec_dtype))
+        return (act_dtype == RB_F32 ? launch_delta_prep_vec<float> : launch_delta_prep_vec<bf16>)(
+            x, ld, taps, taps_dtype, K, state, state_stride, conv_off, tok_seg, cu_q, seg_slot, q32, k32, v32, a, A_log, dt_bias, vec_dtype, b, T, H, G,
+            D, V, q_scale, DA, st);
     dim3 grid(T, 2 * G + 2 * H + 1);
     if (act_dtype == RB_F32)
         rb_launch_pdl(delta_prep_kernel<float>, dim3(grid), dim3(128), 0, st, (const float*)x, ld, taps, taps_dtype, K, state, state_stride, conv_off,
@@ -1081,10 +1272,58 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const TA* __r
     }
 }
 
+// Four values a lane, all of a row's reads in flight together.  2,048 tokens of 16 heads of 128: HNG_NEW us (element by element: 17.7).
+template <typename TA, int NV>
+__global__ void __launch_bounds__(256)
+head_norm_gate_vec_kernel(const float* __restrict__ o, const TA* __restrict__ gate, int gate_ld,
+                          const void* __restrict__ w, int w_dtype, int w_mode, int gate_act, float eps,
+                          TA* __restrict__ out, int rows, int H, int V) {
+    pdl_wait();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const int t = row / H, h = row - t * H;
+    const float* x = o + (size_t)row * V + 4 * lane;
+    const TA* g = gate + (size_t)t * gate_ld + (size_t)h * V + 4 * lane;
+    float4 xv[NV], gv[NV];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const bool live = 128 * n + 4 * lane < V;
+        xv[n] = live ? ld4(x + 128 * n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        gv[n] = live ? ld4(g + 128 * n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) ss = fmaf(xv[n].x, xv[n].x, fmaf(xv[n].y, xv[n].y, fmaf(xv[n].z, xv[n].z, fmaf(xv[n].w, xv[n].w, ss))));
+    ss = warp_sum(ss);
+    const float rstd = 1.0f / sqrtf(ss / (float)V + eps);
+    auto gated = [&](float v, float u) { return v * (gate_act == 0 ? u / (1.0f + expf(-u)) : 1.0f / (1.0f + expf(-u))); };
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = 128 * n + 4 * lane;
+        if (i >= V) continue;
+        float4 y = make_float4(xv[n].x * rstd, xv[n].y * rstd, xv[n].z * rstd, xv[n].w * rstd);
+        if (w_mode != 0) {
+            const float4 k = ld4(w, w_dtype, (w_mode == 2 ? (size_t)h * V : 0) + i);
+            y.x *= k.x; y.y *= k.y; y.z *= k.z; y.w *= k.w;
+        }
+        st4(out + (size_t)row * V + i, make_float4(gated(y.x, gv[n].x), gated(y.y, gv[n].y), gated(y.z, gv[n].z), gated(y.w, gv[n].w)));
+    }
+}
+
+template <typename TA>
+static int launch_head_norm_gate_vec(const float* o, const void* gate, int gate_ld, const void* w, int w_dtype, int w_mode, int gate_act, float eps,
+                                     void* out, int rows, int H, int V, cudaStream_t st) {
+    auto kernel = V <= 128 ? head_norm_gate_vec_kernel<TA, 1> : head_norm_gate_vec_kernel<TA, 2>;
+    return rb_launch_pdl(kernel, dim3((rows + 7) / 8), dim3(256), 0, st, o, (const TA*)gate, gate_ld, w, w_dtype, w_mode, gate_act, eps, (TA*)out, rows, H, V);
+}
+
 RB_EXPORT int rb_head_norm_gate(const float* o, const void* gate, int gate_ld, const void* w, int w_dtype, int w_mode,
                                 int gate_act, float eps, void* out, int act_dtype, int T, int H, int V, cudaStream_t st) {
     const int rows = T * H;
     if (rows <= 0) return 0;
+    if (V % 4 == 0 && V <= 256 && gate_ld % 4 == 0 && fours(o) && fours(gate, act_dtype) && fours(out, act_dtype) && (w_mode == 0 || fours(w, w_dtype)))
+        return (act_dtype == RB_F32 ? launch_head_norm_gate_vec<float> : launch_head_norm_gate_vec<bf16>)(o, gate, gate_ld, w, w_dtype, w_mode, gate_act,
+                                                                                                          eps, out, rows, H, V, st);
     const int blocks = (rows + 3) / 4;
     if (act_dtype == RB_F32)
         rb_launch_pdl(head_norm_gate_kernel<float>, dim3(blocks), dim3(128), 0, st, o, (const float*)gate, gate_ld, w, w_dtype, w_mode, gate_act, eps,

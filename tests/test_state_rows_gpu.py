@@ -1,0 +1,84 @@
+"""The row kernels around a scan, four elements a lane, against the element-by-element kernels that take everything else.  The
+latter are reached through operands that lie off the addresses the former need."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def _ops():
+    from return_b200.ext import ops
+    return ops
+
+
+def off_by_one(x):
+    """The same numbers one element further on in a wider buffer."""
+    wide = torch.zeros(x.shape[0], x.shape[1] + 3, dtype=x.dtype, device=x.device)
+    wide[:, 1:1 + x.shape[1]] = x
+    return wide[:, 1:1 + x.shape[1]]
+
+
+# sums over a head in two orders and a rounding or two of the result
+def same(a, b, dt):
+    tol = 2.0 ** -17 if dt == torch.float32 else 2.0 ** -7
+    return torch.allclose(a.float(), b.float(), rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,D", [(1, 8), (3, 40), (16, 128), (2, 256)])
+def test_rotary_to_f32(dt, heads, D):
+    ops = _ops()
+    T, HD = 37, heads * D
+    x = torch.randn(T, 2 * HD, device=DEV).to(dt)
+    ang = torch.rand(50, D // 2, device=DEV) * 6
+    pos = torch.randint(0, 50, (T,), dtype=torch.int32, device=DEV)
+    outs = []
+    for form in (lambda y: y, off_by_one):
+        q, k = torch.empty(T, HD, device=DEV), torch.empty(T, HD, device=DEV)
+        ops.rotary_to_f32(form(x), 0, HD, ang.cos().contiguous(), ang.sin().contiguous(), D, pos, q, k, heads, D, 1.0, D ** -0.5)
+        outs.append((q, k))
+    assert same(outs[0][0], outs[1][0], torch.float32) and same(outs[0][1], outs[1][1], torch.float32)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,V", [(1, 4), (5, 60), (16, 128), (3, 132), (2, 256)])
+@pytest.mark.parametrize("mode,act", [(0, 0), (1, 1), (2, 0)])
+def test_head_norm_gate(dt, H, V, mode, act):
+    ops = _ops()
+    T = 19
+    o, gate = torch.randn(T, H * V, device=DEV), torch.randn(T, H * V, device=DEV).to(dt)
+    w = (None, torch.rand(V, device=DEV), torch.rand(H * V, device=DEV).to(dt))[mode]
+    outs = []
+    for form in (lambda y: y, off_by_one):
+        out = torch.empty(T, H * V, device=DEV, dtype=dt)
+        ops.head_norm_gate(o, form(gate), w, mode, act, 1e-5, out, H, V)
+        outs.append(out)
+    assert same(outs[0], outs[1], dt)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens", [[1, 1, 5, 2], [3, 1030], [9] * 120])
+@pytest.mark.parametrize("H,G,D,V,K,head_decay", [(4, 2, 8, 12, 4, False), (2, 1, 128, 256, 2, True), (2, 2, 36, 132, 1, False), (1, 1, 256, 4, 3, True)])
+def test_delta_prep(dt, lens, H, G, D, V, K, head_decay):
+    """Runs of tokens that begin within a segment, at its start and over several segments, with what the state holds before them."""
+    ops = _ops()
+    T, n, C = sum(lens), len(lens), 2 * G * D + H * V
+    x, taps = torch.randn(T, C, device=DEV).to(dt), torch.randn(C, K, device=DEV).to(dt)
+    DA = 1 if head_decay else D
+    a, b = torch.randn(T, H * DA, device=DEV), torch.randn(T, H, device=DEV)
+    A_log, dt_bias = torch.randn(H, device=DEV).to(dt), torch.randn(H * DA, device=DEV).to(dt)
+    state = torch.randn(n, 1 + C * (K - 1), device=DEV)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_q=cu, seg_slot=torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV),
+                            tok_seg=torch.repeat_interleave(torch.arange(n, device=DEV), torch.tensor(lens, device=DEV)).to(torch.int32))
+    outs = []
+    for form in (lambda y: y, off_by_one):
+        out = [torch.empty(T, w, device=DEV) for w in (G * D, G * D, H * V)] + [a.clone(), b.clone()]
+        ops.delta_prep(form(x), taps, state, 1, batch, out[0], out[1], out[2], out[3], A_log, dt_bias, out[4], H, G, D, V, D ** -0.5,
+                       head_decay=head_decay)
+        outs.append(out)
+    assert all(same(p, q, torch.float32) for p, q in zip(*outs))
