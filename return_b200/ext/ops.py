@@ -816,10 +816,15 @@ def prefill_shares(tiles, heads: int, rows: int, head_dim: int):
         if share * PREFILL_KEY_TILE < PREFILL_SPLIT_MIN_KEYS or s * rows * heads * (head_dim + 2) * 4 > PREFILL_SPLIT_SCRATCH_BYTES:
             break
         counts = [-(-t // share) for t in tiles]
-        if heads * sum(counts) > 3 * sms:              # more than SMs can take in a few rounds: the CTAs' own cost grows
+        ctas = heads * sum(counts)
+        if ctas > 2 * sms:                             # more rounds: the CTAs' own cost grows, and it is long work anyway
             break
-        work = [-(-t // c) + PREFILL_CTA_TILES for z in range(max(counts)) for t, c in zip(tiles, counts) if c > z]
-        d = _launch_tiles(work, heads, sms) + PREFILL_MERGE_TILES
+        d = share + PREFILL_CTA_TILES + PREFILL_MERGE_TILES                 # all CTAs at once
+        if ctas > sms:
+            work = [-(-t // c) + PREFILL_CTA_TILES for z in range(max(counts)) for t, c in zip(tiles, counts) if c > z]
+            if max(d, heads * sum(work) / sms + PREFILL_MERGE_TILES) >= best_done:
+                continue
+            d = _launch_tiles(work, heads, sms) + PREFILL_MERGE_TILES
         if d < best_done:
             best, best_done = (s, share), d
     return best
@@ -833,9 +838,10 @@ def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=
         return held[key]
     host = batch.host
     tiles = []
+    first, length = host.seg_pos0.tolist(), host.seg_kv_len.tolist()
     for seg, row0 in host.tiles[TILES_TC5].tolist():
-        p0 = int(host.seg_pos0[seg]) + row0
-        end = min(int(host.seg_kv_len[seg]), p0 + TC5_TILE_ROWS)
+        p0 = first[seg] + row0
+        end = min(length[seg], p0 + TC5_TILE_ROWS)
         low = max(0, p0 - window + 1) if window else p0 // chunk * chunk if chunk else 0
         kept = min(-(-keep // PREFILL_KEY_TILE), low // PREFILL_KEY_TILE) if window and keep else 0
         tiles.append((end - 1) // PREFILL_KEY_TILE - low // PREFILL_KEY_TILE + 1 + kept)
