@@ -1,17 +1,25 @@
-// The experts' products of a prompt on the fifth-generation tensor cores: C[place, n] = sum_k A[place, k] W[e][n, k]
-// over the (token, expert) pairs in the order of their experts (A holds their rows in that order), bfloat16 with
-// float32 accumulation in tensor memory, operands by TMA.
+// The experts' products of a step on the fifth-generation tensor cores: C[place, n] = sum_k A[place, k] W[e][n, k] over the
+// (token, expert) pairs in the order of their experts (A holds their rows in that order), bfloat16 with float32 accumulation in
+// tensor memory, operands by TMA.  Optionally the gated unit of the experts in the epilogue: W[e] then holds F gate rows and F up
+// rows, and C[place, f] = g sigmoid(alpha g) (u + shift) of the two sums, capped (moe.cu, clamped_glu), so that the [places, 2F]
+// intermediate is neither written nor read.
 //
-// The kernel is the persistent product kernel of gemm_tc5.cu (a producer thread, an MMA thread, four epilogue warps,
-// a ring of operand stages, two accumulators in tensor memory) with another list of tiles: an expert's run of places
-// is cut into tiles of 128 rows that begin where the run begins, so a tile never mixes experts; the rows of a tile
-// behind the run's end belong to the next expert (or lie behind the matrix and come as zeros) and are computed but
-// not stored.  The weights of all experts are one matrix [E * N, K]; a tile's box of 256 weight rows begins at its
-// expert's n-th row and may reach into the next expert's rows, whose columns are not stored either.  How many tiles
-// there are follows from the router's choice, which only the device knows: every CTA works the list out from the
-// offsets of the runs, and the grid is as large as the SMs or the worst case, whichever is smaller.
+// The operands' roles are exchanged: an expert's weight rows are the M side of the MMA (256 a tile, by a pair of CTAs on
+// neighbouring SMs with the two-SM form, cta_group::2: each CTA holds 128 of them, and their accumulators lie on its 128 TMEM
+// lanes), the expert's places are the N side, of any multiple of 32 up to 256.  A run of n places is cut into as few tiles as
+// possible, all of about the same width, so what a tile computes beside its places is at most 31 columns.  (With the places as M, a
+// tile of 128 rows or a part of one: 25 % of the products of 32 experts and 8,192 pairs were of rows behind a run's end, and each CTA
+// loaded 48 KB a k block where a pair loads 32 KB a CTA.)  Each CTA of a pair brings its weight rows and half of the places.
+//
+// Producer thread, MMA thread (of the even CTA, the leader), ring of stages, two accumulators: as in the pair kernel of
+// gemm_tc5.cu.  The accumulators come out with a weight row a lane, so the epilogue turns blocks of 32 places by 32 rows round
+// through shared memory before it stores them: neighbouring lanes then hold neighbouring columns of one place.  With the gated
+// unit, gate rows lie on lanes 0-63 and their up rows on lanes 64-127: two warps exchange halves of each block and each does half
+// of the units.  How many tiles there are follows from the router's choice, which only the device knows: every CTA works the
+// list out from the offsets of the runs.
 //
 // Every mbarrier wait is bounded; a wait that gives up raises *status and the kernel still frees its tensor memory.
+// Measured (8,192 pairs on 32 experts, H = 2,048, F = 1,536): MOE_MEASURED
 #include <cuda.h>
 
 #include "tc5.cuh"
@@ -21,193 +29,358 @@ namespace {
 
 using namespace tc5;
 
-constexpr int BM = 128;
 constexpr int BK = 64;                    // bf16 elements: one 128-byte swizzle row
-constexpr int BN = 256;
-constexpr int STAGES = 4;
+constexpr int BM = 128;                   // weight rows of a CTA
+constexpr int MAX_BN = 256;               // places of a tile at most
+constexpr int BOX = 64;                   // rows of a TMA box
+constexpr int KPS = 2;                    // k blocks of 64 a stage
+constexpr int STAGES = 3;
 constexpr int THREADS = 192;              // warp 0: TMA, warp 1: MMA, warps 2..5: epilogue
 constexpr int MAX_EXPERTS = 1024;
+constexpr unsigned A_BYTES = BM * BK * 2, B_BYTES = (MAX_BN / 2) * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KPS * BLOCK_BYTES;
+constexpr unsigned EX_FLOATS = 2 * 2 * 2 * 16 * 32;       // [pair of warps][buffer][from which half][place][row]: the exchange of gate and up sums
+constexpr unsigned TURN_BYTES = 4 * 32 * 64;              // [warp][place][32 rows of bf16]: the block that is turned round
+constexpr unsigned SMEM_BYTES = STAGES * STAGE_BYTES + EX_FLOATS * 4 + TURN_BYTES + 1024;
+
+struct Unit { float limit, alpha, shift; const float* weight; const int* pair_at; };      // the gated unit, and what multiplies a place's sums first
 
 struct Tile {
+    int e;         // expert
     int m0;        // first place (row of A and of C)
-    int rows;      // places of the tile that belong to its expert
-    int w_row;     // first row of the tile in the matrix of all experts' weights
-    int n0;        // first output column
+    int rows;      // places of the tile
+    int bn;        // the MMA's N: rows rounded up to 32
+    int nt;        // tile of weight rows
 };
 
-// Tiles are numbered with the row tiles of all experts fastest, so that neighbours share a block of weights only
-// within an expert but the tokens' rows stay in L2 across the output columns.
-__device__ __forceinline__ Tile locate(const int* s_start, const int* s_off, int E, int N, int total_m, int tile) {
-    const int nt = tile / total_m, r = tile - nt * total_m;
+// Places of a tile of a run of n places, but for the last.
+__device__ __forceinline__ int run_width(int n) {
+    const int k = (n + MAX_BN - 1) / MAX_BN;
+    return k == 0 ? 32 : ((n + k - 1) / k + 31) & ~31;
+}
+
+// Tiles are numbered with the tiles of all experts' places fastest: the weights of a block of output columns are read once,
+// and the places' rows stay in L2 across the blocks.
+__device__ __forceinline__ Tile locate(const int* s_start, const int* s_off, int E, int total_m, int tile) {
+    Tile t;
+    t.nt = tile / total_m;
+    const int r = tile - t.nt * total_m;
     int lo = 0, hi = E;                                     // the last expert whose first tile is not behind r
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (s_start[mid] <= r) lo = mid; else hi = mid;
     }
-    const int mt = r - s_start[lo];
-    Tile t;
-    t.m0 = s_off[lo] + mt * BM;
-    t.rows = min(BM, s_off[lo + 1] - t.m0);
-    t.n0 = nt * BN;
-    t.w_row = lo * N + t.n0;
+    const int width = run_width(s_off[lo + 1] - s_off[lo]);
+    t.e = lo;
+    t.m0 = s_off[lo] + (r - s_start[lo]) * width;
+    t.rows = min(width, s_off[lo + 1] - t.m0);
+    t.bn = (t.rows + 31) & ~31;
     return t;
 }
 
-__device__ __forceinline__ void store_chunk(bf16* dst, const unsigned (&r)[32], int n_valid) {
-    if (n_valid == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            uint4 v;
-            __nv_bfloat162 p0 = __floats2bfloat162_rn(__uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-            __nv_bfloat162 p1 = __floats2bfloat162_rn(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-            __nv_bfloat162 p2 = __floats2bfloat162_rn(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5]));
-            __nv_bfloat162 p3 = __floats2bfloat162_rn(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7]));
-            v.x = *reinterpret_cast<unsigned*>(&p0); v.y = *reinterpret_cast<unsigned*>(&p1);
-            v.z = *reinterpret_cast<unsigned*>(&p2); v.w = *reinterpret_cast<unsigned*>(&p3);
-            *reinterpret_cast<uint4*>(dst + j) = v;
-        }
-        return;
-    }
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-        if (j < n_valid) dst[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
+__device__ __forceinline__ unsigned cluster_ctarank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned map_to_cta(unsigned smem_addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void load_pair(unsigned smem_dst, const CUtensorMap* map, int x, int y, unsigned bar_in_cluster) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(bar_in_cluster) : "memory");
+}
+__device__ __forceinline__ void mma_ss_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+}
+__device__ __forceinline__ void mma_commit_pair(unsigned bar) {          // one arrival on this barrier in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
 }
 
+// 32 places (or 16) by 32 weight rows, place j of this lane's row in v[j]: written to `turn` [place][32] and stored with
+// neighbouring lanes on neighbouring columns.  `first`: output of the first place and of this warp's first row.
+template <int N>
+__device__ __forceinline__ void turn_and_store(unsigned char* turn, const float (&v)[N], bf16* first, int ldo, int rows, int cols, bool vec, int lane) {
+    bf16* t = reinterpret_cast<bf16*>(turn);
+    __syncwarp();                                           // the block before this one has been taken
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[j * 32 + lane] = __float2bfloat16_rn(v[j]);
+    __syncwarp();
+    if (vec && cols >= 32) {                                // four lanes a place, eight places an instruction
+#pragma unroll
+        for (int j = 0; j < N; j += 8) {
+            const int p = j + (lane >> 2);
+            if (p < rows) *reinterpret_cast<uint4*>(first + (size_t)p * ldo + (lane & 3) * 8) = *reinterpret_cast<const uint4*>(t + p * 32 + (lane & 3) * 8);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (j < rows && lane < cols) first[(size_t)j * ldo + lane] = t[j * 32 + lane];
+    }
+}
+
+template <bool GATED>
 __global__ void __launch_bounds__(THREADS)
 moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const int* __restrict__ offsets, int E, bf16* __restrict__ out, int N, int K, int ldo,
-               int* __restrict__ status, int act) {
+               int* __restrict__ status, int act, int vec, Unit unit) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    constexpr unsigned A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+    float* exchange = reinterpret_cast<float*>(base + STAGES * STAGE_BYTES);
+    unsigned char* turns = base + STAGES * STAGE_BYTES + EX_FLOATS * 4;
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_slot;
     __shared__ int s_start[MAX_EXPERTS + 1], s_off[MAX_EXPERTS + 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr unsigned TMEM_COLS = 2 * BN;
-    const int nkb = (K + BK - 1) / BK;                      // k blocks past K are zero-filled by the copy
+    const unsigned rank = cluster_ctarank();                // 0: the leader
+    const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    constexpr unsigned TMEM_COLS = 2 * MAX_BN;
+    constexpr int TILE_N = GATED ? BM : 2 * BM;             // output columns of a pair's tile
+    const int nkb = (K + BK * KPS - 1) / (BK * KPS);        // stages a tile; k blocks past K are zero-filled by the copy
 
-    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), TMEM_COLS);
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
     if (tid == 0) {
         tma::prefetch_desc(&map_a);
         tma::prefetch_desc(&map_w);
 #pragma unroll
         for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
 #pragma unroll
-        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&acc_full[b]), 1); mbar_init(smem_u32(&acc_empty[b]), 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&acc_full[b]), 1); mbar_init(smem_u32(&acc_empty[b]), 8); }
         mbar_init_fence();
     }
     pdl_wait();                                             // the offsets and the rows come from the kernels before
     for (int e = tid; e <= E; e += THREADS) s_off[e] = offsets[e];
     fence_before_sync();
     __syncthreads();
-    fence_after_sync();
-    if (tid == 0) {
+    if (warp == 0) {                                        // first tile of every expert: sums over 32 experts at a time
         int run = 0;
-        for (int e = 0; e < E; ++e) {
-            s_start[e] = run;
-            run += (s_off[e + 1] - s_off[e] + BM - 1) / BM;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, n = e < E ? s_off[e + 1] - s_off[e] : 0;
+            const int own = n > 0 ? (n + run_width(n) - 1) / run_width(n) : 0;
+            int upto = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            if (e < E) s_start[e] = run + upto - own;
+            run += __shfl_sync(0xffffffffu, upto, 31);
         }
-        s_start[E] = run;
+        if (lane == 0) s_start[E] = run;
     }
     __syncthreads();
+    cluster_sync_all();                                     // both CTAs' barriers exist before either is signalled
+    fence_after_sync();
     const int total_m = s_start[E];
-    const int tiles = total_m * ((N + BN - 1) / BN);
+    const int tiles = total_m * ((N + TILE_N - 1) / TILE_N);
     const unsigned tacc = tmem_slot;
     bool ok = true;
 
     if (warp == 0) {
-        if (lane == 0) {                                    // ---- producer
-            int it = 0;                                     // k blocks issued so far, over all tiles
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-                const Tile t = locate(s_start, s_off, E, N, total_m, tile);
+        if (lane == 0) {                                    // ---- producer (both CTAs)
+            int it = 0;                                     // stages filled so far, over all tiles
+            for (int tile = pair; tile < tiles; tile += pairs) {
+                const Tile t = locate(s_start, s_off, E, total_m, tile);
+                // this CTA's two boxes of weight rows: gate and up rows of 64 outputs, or 128 rows in a run
+                const int w0 = GATED ? t.e * 2 * N + t.nt * TILE_N + (int)rank * BOX : t.e * N + t.nt * TILE_N + (int)rank * BM;
+                const int w1 = GATED ? w0 + N : w0 + BOX;
+                const int half = t.bn >> 1, m = t.m0 + (int)rank * half, boxes = (half + BOX - 1) / BOX;
+                const unsigned bytes = A_BYTES + (unsigned)boxes * (BOX * BK * 2);
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES) ok = mbar_wait(smem_u32(&empty_bar[s]), ((it / STAGES) - 1) & 1) && ok;
-                    const unsigned full = smem_u32(&full_bar[s]);
-                    mbar_arrive_expect_tx(full, STAGE_BYTES);
+                    const unsigned full_local = smem_u32(&full_bar[s]);
+                    if (rank == 0) mbar_arrive_expect_tx(full_local, 2 * KPS * bytes);
+                    const unsigned full = map_to_cta(full_local, 0);
                     const unsigned dst = smem_u32(base + (size_t)s * STAGE_BYTES);
-                    tma::load_2d(dst, &map_a, kb * BK, t.m0, full);
-                    tma::load_2d(dst + A_BYTES, &map_w, kb * BK, t.w_row, full);
+#pragma unroll
+                    for (int j = 0; j < KPS; ++j) {
+                        const unsigned d = dst + j * BLOCK_BYTES;
+                        const int x = (kb * KPS + j) * BK;
+                        load_pair(d, &map_w, x, w0, full);
+                        load_pair(d + BOX * BK * 2, &map_w, x, w1, full);
+                        for (int b = 0; b < boxes; ++b) load_pair(d + A_BYTES + b * (BOX * BK * 2), &map_a, x, m + b * BOX, full);
+                    }
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                                    // ---- MMA issuer
-            const unsigned idesc = instr_desc_bf16(BM, BN);
+        if (lane == 0 && rank == 0) {                       // ---- MMA issuer (the leader)
             int it = 0, local = 0;
-            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
+            for (int tile = pair; tile < tiles; tile += pairs, ++local) {
+                const Tile t = locate(s_start, s_off, E, total_m, tile);
+                const unsigned idesc = instr_desc_bf16(2 * BM, t.bn);
                 const int buf = local & 1;
                 if (local >= 2) ok = mbar_wait(smem_u32(&acc_empty[buf]), ((local >> 1) - 1) & 1) && ok;
                 fence_after_sync();
-                const unsigned d = tacc + buf * BN;
+                const unsigned d = tacc + buf * MAX_BN;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
                     ok = mbar_wait(smem_u32(&full_bar[s]), (it / STAGES) & 1) && ok;
                     fence_after_sync();
-                    const unsigned a = smem_u32(base + (size_t)s * STAGE_BYTES), b = a + A_BYTES;
+                    const unsigned a0 = smem_u32(base + (size_t)s * STAGE_BYTES);
 #pragma unroll
-                    for (int k16 = 0; k16 < BK / 16; ++k16)
-                        mma_ss(d, smem_desc_sw128(a, k16 * 32), smem_desc_sw128(b, k16 * 32), idesc, kb > 0 || k16 > 0);
-                    mma_commit(smem_u32(&empty_bar[s]));    // the stage is free once these MMAs have read it
+                    for (int j = 0; j < KPS; ++j) {
+                        const unsigned a = a0 + j * BLOCK_BYTES, b = a + A_BYTES;
+#pragma unroll
+                        for (int k16 = 0; k16 < BK / 16; ++k16)
+                            mma_ss_pair(d, smem_desc_sw128(a, k16 * 32), smem_desc_sw128(b, k16 * 32), idesc, kb > 0 || j > 0 || k16 > 0);
+                    }
+                    mma_commit_pair(smem_u32(&empty_bar[s]));   // the stage is free in both CTAs once these MMAs have read it
                 }
-                mma_commit(smem_u32(&acc_full[buf]));       // this tile's accumulator is complete
+                mma_commit_pair(smem_u32(&acc_full[buf]));      // both halves of this tile's accumulator are complete
             }
         }
-    } else {                                                // ---- epilogue: TMEM lanes by warp % 4
+    } else {                                                // ---- epilogue (both CTAs): TMEM lanes by warp % 4
         const int q = warp & 3;
-        int local = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
-            const Tile t = locate(s_start, s_off, E, N, total_m, tile);
+        unsigned char* turn = turns + q * 32 * 64;
+        const unsigned acc_empty_leader0 = map_to_cta(smem_u32(&acc_empty[0]), 0), acc_empty_leader1 = map_to_cta(smem_u32(&acc_empty[1]), 0);
+        int local = 0, blocks = 0;
+        for (int tile = pair; tile < tiles; tile += pairs, ++local) {
+            const Tile t = locate(s_start, s_off, E, total_m, tile);
             const int buf = local & 1;
             ok = mbar_wait(smem_u32(&acc_full[buf]), (local >> 1) & 1) && ok;
-            if (tile + (int)gridDim.x >= tiles) pdl_trigger_late();        // the last tile of this CTA
+            if (tile + pairs >= tiles) pdl_trigger_late();                 // the last tile of this CTA
             fence_after_sync();
-            const int r_local = q * 32 + lane;
+            // this warp's first output column, and how many of its 32 exist
+            const int n0 = t.nt * TILE_N + (GATED ? (int)rank * BOX + (q & 1) * 32 : (int)rank * BM + q * 32), cols = min(32, N - n0);
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
+            for (int c0 = 0; c0 < t.rows; c0 += 32, ++blocks) {
                 unsigned r[32];
-                tmem_ld32(tacc + ((unsigned)(q * 32) << 16) + buf * BN + c0, r);
+                tmem_ld32(tacc + ((unsigned)(q * 32) << 16) + buf * MAX_BN + c0, r);
                 tmem_ld_wait();
-                if (r_local >= t.rows || t.n0 + c0 >= N) continue;
-                if (act >= 0) {
+                const int left = t.rows - c0;
+                bf16* to = out + (size_t)(t.m0 + c0) * ldo + n0;
+                if (GATED) {
+                    // warps q and q + 2 hold gate and up sums of the same 32 units: the first does places 0-15 of the block, the
+                    // second 16-31.  Two buffers: who writes into one again has met the partner after it read it.
+                    const bool up = q >= 2;
+                    float* ex = exchange + ((q & 1) * 2 + (blocks & 1)) * 1024;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(rb_activate(act, __uint_as_float(r[j]), nullptr, 0, 0));
+                    for (int j = 0; j < 16; ++j) ex[(up ? 512 : 0) + j * 32 + lane] = __uint_as_float(r[up ? j : 16 + j]);
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+                    const int p0 = up ? 16 : 0;
+                    float c = 1.f;                          // lane j: what multiplies the sums of place j of the sixteen
+                    if (unit.weight != nullptr && lane < 16 && p0 + lane < left) {
+                        const int place = t.m0 + c0 + p0 + lane;
+                        c = unit.weight[unit.pair_at ? unit.pair_at[place] : place];
+                    }
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float mine = __uint_as_float(r[up ? 16 + j : j]), other = ex[(up ? 0 : 512) + j * 32 + lane];
+                        const float f = unit.weight != nullptr ? __shfl_sync(0xffffffffu, c, j) : 1.f;
+                        const float g = fminf(f * (up ? other : mine), unit.limit);
+                        const float u = fminf(fmaxf(f * (up ? mine : other), -unit.limit), unit.limit);
+                        v[j] = g / (1.0f + expf(-unit.alpha * g)) * (u + unit.shift);
+                    }
+                    if (cols > 0) turn_and_store<16>(turn, v, to + (size_t)p0 * ldo, ldo, left - p0, cols, vec, lane);
+                } else {
+                    float v[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        v[j] = __uint_as_float(r[j]);
+                        if (act >= 0) v[j] = rb_activate(act, v[j], nullptr, 0, 0);
+                    }
+                    if (cols > 0) turn_and_store<32>(turn, v, to, ldo, left, cols, vec, lane);
                 }
-                store_chunk(out + (size_t)(t.m0 + r_local) * ldo + t.n0 + c0, r, min(32, N - t.n0 - c0));
             }
             fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));         // this warp has drained its quarter
+            if (lane == 0) mbar_arrive_in_cluster(buf ? acc_empty_leader1 : acc_empty_leader0);   // this warp has drained its quarter
         }
     }
     if (!ok) atomicExch(status, 1);
+    __syncwarp();
     fence_before_sync();
-    __syncthreads();
-    if (warp == 1) tmem_dealloc(tacc, TMEM_COLS);
+    cluster_sync_all();                                     // neither CTA leaves, or gives its tensor memory back, while the other works
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tacc), "r"(TMEM_COLS) : "memory");
+}
+
+// A map of rows of 64 elements in boxes of 64 rows, for a matrix that may have more rows than an int's worth of bytes.
+template <bool GATED>
+int launch(const void* A, int lda, const void* W, const int* offsets, int E, void* out, int ldo, int places, int N, int K, int act, int* status,
+           const Unit& unit, cudaStream_t st) {
+    CUtensorMap ma, mw;
+    if (!tma::make_map_bf16(&ma, A, places, K, lda, BOX) || !tma::make_map_bf16(&mw, W, E * N * (GATED ? 2 : 1), K, K, BOX)) return (int)cudaErrorInvalidValue;
+    // pairs that the device holds at once (an SM whose neighbour is switched off takes none)
+    static PerDevice configured;
+    static int pairs_of_device[PerDevice::MAX_DEVICES] = {0};
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int rc = configured.once([&](int dev) {
+        cudaError_t e = cudaFuncSetAttribute(moe_tc5_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        int clusters = 0;
+        e = cudaOccupancyMaxActiveClusters(&clusters, moe_tc5_kernel<GATED>, &cfg);
+        if (e != cudaSuccess) return e;
+        if (clusters < 1) return cudaErrorInvalidConfiguration;
+        pairs_of_device[dev] = clusters;
+        return cudaSuccess;
+    });
+    if (rc != 0) return rc;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const long long n_tiles = (N + (GATED ? BM : 2 * BM) - 1) / (GATED ? BM : 2 * BM);
+    const long long worst = ((long long)places / 224 + E + 1) * n_tiles;     // a run's tiles are at least 225 places wide, but for the last two
+    const int resident = pairs_of_device[dev];
+    cfg.gridDim = dim3(2 * (unsigned)(worst < resident ? worst : resident));
+    cfg.stream = st;
+    cfg.numAttrs = RB_PDL_MODE == 3 ? 1 : 2;
+    const int vec = ldo % 8 == 0 && N % 8 == 0 && ((uintptr_t)out & 15) == 0;
+    return (int)cudaLaunchKernelEx(&cfg, moe_tc5_kernel<GATED>, ma, mw, offsets, E, (bf16*)out, N, K, ldo, status, act, vec, unit);
+}
+
+bool fits(const void* A, int lda, const void* W, int E, int rows, int K) {
+    return E > 0 && E <= MAX_EXPERTS && K > 0 && K % 8 == 0 && lda % 8 == 0 && ((uintptr_t)A % 16) == 0 && ((uintptr_t)W % 16) == 0 &&
+           (long long)E * rows <= 0x7fffffffLL;
 }
 
 }  // namespace
 
 // A [places, K] (the pairs' rows in the order of their experts), W [E, N, K] contiguous, offsets int32 [E + 1] on the
-// device, out [places, N] bfloat16; act: -1, or the number of an activation (rb_activate) on the float32 sums.  status: one int in device memory, set to 1 if a wait inside the kernel gave up.
+// device, out [places, N] bfloat16; act: -1, or the number of an activation (rb_activate) on the float32 sums.  status: one int in
+// device memory, set to 1 if a wait inside the kernel gave up.
 RB_EXPORT int rb_moe_tc5_gemm(const void* A, int lda, const void* W, const int* offsets, int E, void* out, int ldo, int places,
                               int N, int K, int act, int* status, cudaStream_t st) {
     if (places <= 0 || N <= 0) return 0;
-    if (act > ACT_SILU) return (int)cudaErrorInvalidValue;
-    if (E > MAX_EXPERTS || K % 8 || lda % 8 || ((uintptr_t)A % 16) || ((uintptr_t)W % 16)) return (int)cudaErrorInvalidValue;
-    if ((long long)E * N > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
-    CUtensorMap ma, mw;
-    if (!tma::make_map_bf16(&ma, A, places, K, lda, BM) || !tma::make_map_bf16(&mw, W, E * N, K, K, BN)) return (int)cudaErrorInvalidValue;
-    const size_t smem = (size_t)STAGES * (BM + BN) * BK * 2 + 1024;
-    static PerDevice configured;
-    const int rc = configured.once([&](int) {
-        return cudaFuncSetAttribute(moe_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    });
-    if (rc != 0) return rc;
-    const long long worst = ((long long)(places + BM - 1) / BM + E) * ((N + BN - 1) / BN);
-    const int num_sms = rb_num_sms();
-    if (num_sms <= 0) return (int)cudaErrorInvalidDevice;
-    dim3 grid((unsigned)(worst < num_sms ? worst : num_sms));
-    return rb_launch_pdl(moe_tc5_kernel, grid, dim3(THREADS), smem, st, ma, mw, offsets, E, (bf16*)out, N, K, ldo, status, act);
+    if (act > ACT_SILU || !fits(A, lda, W, E, N, K)) return (int)cudaErrorInvalidValue;
+    return launch<false>(A, lda, W, offsets, E, out, ldo, places, N, K, act, status, Unit{}, st);
+}
+
+// The same with the gated unit: W [E, 2F, K] (F gate rows, then F up rows), out [places, F].  limit, alpha, shift, weight, pair_at: as
+// in rb_clamped_glu.
+RB_EXPORT int rb_moe_tc5_gated(const void* A, int lda, const void* W, const int* offsets, int E, void* out, int ldo, int places, int F,
+                               int K, float limit, float alpha, float shift, const float* weight, const int* pair_at, int* status,
+                               cudaStream_t st) {
+    if (places <= 0 || F <= 0) return 0;
+    if (!fits(A, lda, W, E, 2 * F, K)) return (int)cudaErrorInvalidValue;
+    return launch<true>(A, lda, W, offsets, E, out, ldo, places, F, K, -1, status, Unit{limit, alpha, shift, weight, pair_at}, st);
 }

@@ -1855,7 +1855,8 @@ def moe_tc5_lib() -> ctypes.CDLL:
         lib = build.load("return_moe_tc5", _MOE_TC5_SOURCES, {"RB_PDL_MODE": PDL_MODE})
         P, I = c_void_p, c_int
         lib.rb_moe_tc5_gemm.argtypes = [P, I, P, P, I, P, I, I, I, I, I, P, P]
-        lib.rb_moe_tc5_gemm.restype = c_int
+        lib.rb_moe_tc5_gated.argtypes = [P, I, P, P, I, P, I, I, I, I, c_float, c_float, c_float, P, P, P, P]
+        lib.rb_moe_tc5_gemm.restype = lib.rb_moe_tc5_gated.restype = c_int
         _moe_tc5 = lib
     return _moe_tc5
 
@@ -1879,6 +1880,21 @@ def moe_tc5_gemm(x_sorted, w, offsets, out, act: Optional[str] = None) -> None:
     _tc5_launched.add(x_sorted.device)
     _check(moe_tc5_lib().rb_moe_tc5_gemm(_ptr(x_sorted), x_sorted.stride(0), _ptr(w), _ptr(offsets), E, _ptr(out), out.stride(0),
                                          places, N, K, _act_code(act), _ptr(tc5_status(x_sorted.device)), _stream()), "moe_tc5_gemm")
+
+
+def moe_tc5_gated(x_sorted, w, offsets, out, limit: float, alpha: float, shift: float = 1.0, weight=None, pair_at=None) -> None:
+    """``moe_tc5_gemm`` with the experts' gated unit as its epilogue: w [E, 2F, K] (gate rows, then up rows), out [places, F] =
+    ``clamped_glu`` of the two products' float32 sums.  ``weight``, ``pair_at``: as in ``clamped_glu``."""
+    E, N, K = w.shape
+    places = out.shape[0]
+    assert x_sorted.dtype == w.dtype == out.dtype == torch.bfloat16 and x_sorted.stride(1) == 1 and w.is_contiguous()
+    assert x_sorted.shape == (places, K) and N == 2 * out.shape[1] and out.stride(1) == 1
+    assert weight is None or (weight.dtype == torch.float32 and weight.numel() == places and weight.is_contiguous())
+    assert pair_at is None or (pair_at.dtype == torch.int32 and pair_at.numel() == places)
+    _tc5_launched.add(x_sorted.device)
+    _check(moe_tc5_lib().rb_moe_tc5_gated(_ptr(x_sorted), x_sorted.stride(0), _ptr(w), _ptr(offsets), E, _ptr(out), out.stride(0), places,
+                                          N // 2, K, float(limit), float(alpha), float(shift), _ptr(weight), _ptr(pair_at),
+                                          _ptr(tc5_status(x_sorted.device)), _stream()), "moe_tc5_gated")
 
 
 # From this many (token, expert) pairs on, a step's experts run as tiles on the tensor cores over the pairs sorted by
@@ -1909,7 +1925,6 @@ def moe_experts(x, up, down, expert_of, weight, shared, out, limit: float = floa
 
     w_in, w_out = (weight, None) if weigh_input else (None, weight)
     hidden = buf("moe.pair_act", (pairs, F))
-    gu = buf("moe.pair_gate_up", (pairs, FU)) if act is None else hidden
     y = buf("moe.pair_y", (pairs, H))
     if (x.dtype == torch.bfloat16 and pairs >= MOE_GROUPED_MIN_PAIRS and H % 8 == 0 and F % 8 == 0 and x.stride(0) % 8 == 0
             and x.data_ptr() % 16 == 0):
@@ -1920,17 +1935,20 @@ def moe_experts(x, up, down, expert_of, weight, shared, out, limit: float = floa
         if pairs >= MOE_TC5_MIN_PAIRS and E <= 1024:
             rows = buf("moe.pair_rows", (pairs, H))
             moe_gather_rows(x, pair_at, top, rows)
-            moe_tc5_gemm(rows, up, offsets, gu, act)
             if act is None:
-                clamped_glu(gu, hidden, limit, alpha, shift, w_in, pair_at)
+                moe_tc5_gated(rows, up, offsets, hidden, limit, alpha, shift, w_in, pair_at)
+            else:
+                moe_tc5_gemm(rows, up, offsets, hidden, act)
             moe_tc5_gemm(hidden, down, offsets, y)
         else:
+            gu = buf("moe.pair_gate_up", (pairs, FU)) if act is None else hidden
             moe_grouped_gemm(x, pair_at, top, up, offsets, gu, act)
             if act is None:
                 clamped_glu(gu, hidden, limit, alpha, shift, w_in, pair_at)
             moe_grouped_gemm(hidden, None, 1, down, offsets, y)
         moe_combine(y, w_out, shared, out, row_of=place_of, top=top, shared_gate=shared_gate)
         return
+    gu = buf("moe.pair_gate_up", (pairs, FU)) if act is None else hidden
     moe_pair_linear(x, top, up, expert_of, gu, act)
     if act is None:
         clamped_glu(gu, hidden, limit, alpha, shift, w_in)
