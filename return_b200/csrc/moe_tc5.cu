@@ -35,12 +35,13 @@ constexpr int MAX_BN = 256;               // places of a tile at most
 constexpr int BOX = 64;                   // rows of a TMA box
 constexpr int KPS = 2;                    // k blocks of 64 a stage
 constexpr int STAGES = 3;
-constexpr int THREADS = 192;              // warp 0: TMA, warp 1: MMA, warps 2..5: epilogue
+constexpr int SETS = 2;                   // sets of four epilogue warps: they take blocks of 32 places in turn
+constexpr int THREADS = 64 + 128 * SETS;  // warp 0: TMA, warp 1: MMA, then the epilogue
+constexpr int AHEAD = 10;                 // stages by which the weights are asked into L2 before they are loaded
 constexpr int MAX_EXPERTS = 1024;
 constexpr unsigned A_BYTES = BM * BK * 2, B_BYTES = (MAX_BN / 2) * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KPS * BLOCK_BYTES;
-constexpr unsigned EX_FLOATS = 2 * 2 * 2 * 16 * 32;       // [pair of warps][buffer][from which half][place][row]: the exchange of gate and up sums
-constexpr unsigned TURN_BYTES = 4 * 32 * 64;              // [warp][place][32 rows of bf16]: the block that is turned round
-constexpr unsigned SMEM_BYTES = STAGES * STAGE_BYTES + EX_FLOATS * 4 + TURN_BYTES + 1024;
+constexpr unsigned TURN_BYTES = 32 * 64;                  // a warp's block of 32 places by 32 rows of bf16 that is turned round, or what its partner handed it
+constexpr unsigned SMEM_BYTES = STAGES * STAGE_BYTES + 4 * SETS * TURN_BYTES + 1024;
 
 struct Unit { float limit, alpha, shift; const float* weight; const int* pair_at; };      // the gated unit, and what multiplies a place's sums first
 
@@ -98,6 +99,9 @@ __device__ __forceinline__ void load_pair(unsigned smem_dst, const CUtensorMap* 
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(bar_in_cluster) : "memory");
 }
+__device__ __forceinline__ void prefetch_box(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ void mma_ss_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
     asm volatile(
         "{\n.reg .pred p;\n"
@@ -139,8 +143,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                int* __restrict__ status, int act, int vec, Unit unit) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* exchange = reinterpret_cast<float*>(base + STAGES * STAGE_BYTES);
-    unsigned char* turns = base + STAGES * STAGE_BYTES + EX_FLOATS * 4;
+    unsigned char* turns = base + STAGES * STAGE_BYTES;
     __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_slot;
     __shared__ int s_start[MAX_EXPERTS + 1], s_off[MAX_EXPERTS + 1];
@@ -161,7 +164,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
         for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
 #pragma unroll
-        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&acc_full[b]), 1); mbar_init(smem_u32(&acc_empty[b]), 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&acc_full[b]), 1); mbar_init(smem_u32(&acc_empty[b]), 2 * 4 * SETS); }
         mbar_init_fence();
     }
     pdl_wait();                                             // the offsets and the rows come from the kernels before
@@ -195,15 +198,31 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 0) {
         if (lane == 0) {                                    // ---- producer (both CTAs)
             int it = 0;                                     // stages filled so far, over all tiles
+            // this CTA's two boxes of weight rows: gate and up rows of 64 outputs, or 128 rows in a run
+            auto first_row = [&](const Tile& t) { return GATED ? t.e * 2 * N + t.nt * TILE_N + (int)rank * BOX : t.e * N + t.nt * TILE_N + (int)rank * BM; };
+            const int second = GATED ? N : BOX;
+            // The copies of a stage wait for memory with no more than some 44 KB of an SM in flight, so weights that come from HBM
+            // are asked into L2 AHEAD stages before (and across the border to the next tile).
+            int ask_tile = pair, ask_kb = 0, ask_row = 0;
+            auto ask = [&]() {
+                if (ask_tile >= tiles) return;
+                if (ask_kb == 0) ask_row = first_row(locate(s_start, s_off, E, total_m, ask_tile));
+#pragma unroll
+                for (int j = 0; j < KPS; ++j) {
+                    prefetch_box(&map_w, (ask_kb * KPS + j) * BK, ask_row);
+                    prefetch_box(&map_w, (ask_kb * KPS + j) * BK, ask_row + second);
+                }
+                if (++ask_kb == nkb) { ask_kb = 0; ask_tile += pairs; }
+            };
+            for (int i = 0; i < AHEAD; ++i) ask();
             for (int tile = pair; tile < tiles; tile += pairs) {
                 const Tile t = locate(s_start, s_off, E, total_m, tile);
-                // this CTA's two boxes of weight rows: gate and up rows of 64 outputs, or 128 rows in a run
-                const int w0 = GATED ? t.e * 2 * N + t.nt * TILE_N + (int)rank * BOX : t.e * N + t.nt * TILE_N + (int)rank * BM;
-                const int w1 = GATED ? w0 + N : w0 + BOX;
+                const int w0 = first_row(t), w1 = w0 + second;
                 const int half = t.bn >> 1, m = t.m0 + (int)rank * half, boxes = (half + BOX - 1) / BOX;
                 const unsigned bytes = A_BYTES + (unsigned)boxes * (BOX * BK * 2);
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
+                    ask();
                     if (it >= STAGES) ok = mbar_wait(smem_u32(&empty_bar[s]), ((it / STAGES) - 1) & 1) && ok;
                     const unsigned full_local = smem_u32(&full_bar[s]);
                     if (rank == 0) mbar_arrive_expect_tx(full_local, 2 * KPS * bytes);
@@ -248,10 +267,13 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             }
         }
     } else {                                                // ---- epilogue (both CTAs): TMEM lanes by warp % 4
-        const int q = warp & 3;
-        unsigned char* turn = turns + q * 32 * 64;
+        const int q = warp & 3, set = (warp - 2) >> 2;
+        unsigned char* turn = turns + (set * 4 + q) * TURN_BYTES;
+        float* inbox = reinterpret_cast<float*>(turn);      // [16 places][32 rows]: the partner's sums of the places that this warp does
+        float* outbox = reinterpret_cast<float*>(turns + (set * 4 + (q ^ 2)) * TURN_BYTES);
+        const int meet = 1 + set * 2 + (q & 1);             // the named barrier of the two
         const unsigned acc_empty_leader0 = map_to_cta(smem_u32(&acc_empty[0]), 0), acc_empty_leader1 = map_to_cta(smem_u32(&acc_empty[1]), 0);
-        int local = 0, blocks = 0;
+        int local = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++local) {
             const Tile t = locate(s_start, s_off, E, total_m, tile);
             const int buf = local & 1;
@@ -261,7 +283,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // this warp's first output column, and how many of its 32 exist
             const int n0 = t.nt * TILE_N + (GATED ? (int)rank * BOX + (q & 1) * 32 : (int)rank * BM + q * 32), cols = min(32, N - n0);
 #pragma unroll 1
-            for (int c0 = 0; c0 < t.rows; c0 += 32, ++blocks) {
+            for (int c0 = 32 * set; c0 < t.rows; c0 += 32 * SETS) {
                 unsigned r[32];
                 tmem_ld32(tacc + ((unsigned)(q * 32) << 16) + buf * MAX_BN + c0, r);
                 tmem_ld_wait();
@@ -269,26 +291,26 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 bf16* to = out + (size_t)(t.m0 + c0) * ldo + n0;
                 if (GATED) {
                     // warps q and q + 2 hold gate and up sums of the same 32 units: the first does places 0-15 of the block, the
-                    // second 16-31.  Two buffers: who writes into one again has met the partner after it read it.
+                    // second 16-31; each hands the other its sums of the places that are not its own.
                     const bool up = q >= 2;
-                    float* ex = exchange + ((q & 1) * 2 + (blocks & 1)) * 1024;
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) ex[(up ? 512 : 0) + j * 32 + lane] = __uint_as_float(r[up ? j : 16 + j]);
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
                     const int p0 = up ? 16 : 0;
                     float c = 1.f;                          // lane j: what multiplies the sums of place j of the sixteen
                     if (unit.weight != nullptr && lane < 16 && p0 + lane < left) {
                         const int place = t.m0 + c0 + p0 + lane;
                         c = unit.weight[unit.pair_at ? unit.pair_at[place] : place];
                     }
+                    asm volatile("bar.sync %0, 64;" ::"r"(meet) : "memory");         // the partner is done with its inbox
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) outbox[j * 32 + lane] = __uint_as_float(r[up ? j : 16 + j]);
+                    asm volatile("bar.sync %0, 64;" ::"r"(meet) : "memory");
                     float v[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        const float mine = __uint_as_float(r[up ? 16 + j : j]), other = ex[(up ? 0 : 512) + j * 32 + lane];
+                        const float mine = __uint_as_float(r[up ? 16 + j : j]), other = inbox[j * 32 + lane];
                         const float f = unit.weight != nullptr ? __shfl_sync(0xffffffffu, c, j) : 1.f;
                         const float g = fminf(f * (up ? other : mine), unit.limit);
                         const float u = fminf(fmaxf(f * (up ? mine : other), -unit.limit), unit.limit);
-                        v[j] = g / (1.0f + expf(-unit.alpha * g)) * (u + unit.shift);
+                        v[j] = __fdividef(g, 1.0f + __expf(-unit.alpha * g)) * (u + unit.shift);
                     }
                     if (cols > 0) turn_and_store<16>(turn, v, to + (size_t)p0 * ldo, ldo, left - p0, cols, vec, lane);
                 } else {
