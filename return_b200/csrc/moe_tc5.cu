@@ -19,7 +19,10 @@
 // list out from the offsets of the runs.
 //
 // Every mbarrier wait is bounded; a wait that gives up raises *status and the kernel still frees its tensor memory.
-// Measured (8,192 pairs on 32 experts, H = 2,048, F = 1,536): MOE_MEASURED
+// Bound by the weights' and rows' way in: a pair's tile of 256 rows by 131 places loads half as many bytes an MMA again as one by 256,
+// and the weights (402 + 201 MB below) come from HBM.  Measured (8,192 pairs on 32 experts, H = 2,048, F = 1,536): MOE_MEASURED
+// Boxes of 64 places instead of 32 took 8 % longer; asking the weights into L2 4 / 10 / 20 stages ahead, by TMA or by a warp of
+// prefetches, 3 / 9 / 20 % and 2 / 6 / 28 % longer.
 #include <cuda.h>
 
 #include "tc5.cuh"
@@ -32,12 +35,12 @@ using namespace tc5;
 constexpr int BK = 64;                    // bf16 elements: one 128-byte swizzle row
 constexpr int BM = 128;                   // weight rows of a CTA
 constexpr int MAX_BN = 256;               // places of a tile at most
-constexpr int BOX = 64;                   // rows of a TMA box
+constexpr int BOX = 64;                   // weight rows of a TMA box
+constexpr int PBOX = 32;                  // places of a TMA box
 constexpr int KPS = 2;                    // k blocks of 64 a stage
 constexpr int STAGES = 3;
 constexpr int SETS = 2;                   // sets of four epilogue warps: they take blocks of 32 places in turn
 constexpr int THREADS = 64 + 128 * SETS;  // warp 0: TMA, warp 1: MMA, then the epilogue
-constexpr int AHEAD = 10;                 // stages by which the weights are asked into L2 before they are loaded
 constexpr int MAX_EXPERTS = 1024;
 constexpr unsigned A_BYTES = BM * BK * 2, B_BYTES = (MAX_BN / 2) * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES, STAGE_BYTES = KPS * BLOCK_BYTES;
 constexpr unsigned TURN_BYTES = 32 * 64;                  // a warp's block of 32 places by 32 rows of bf16 that is turned round, or what its partner handed it
@@ -98,9 +101,6 @@ __device__ __forceinline__ void load_pair(unsigned smem_dst, const CUtensorMap* 
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(smem_dst), "l"(map), "r"(x), "r"(y), "r"(bar_in_cluster) : "memory");
-}
-__device__ __forceinline__ void prefetch_box(const CUtensorMap* map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void mma_ss_pair(unsigned d_tmem, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
     asm volatile(
@@ -195,34 +195,20 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const unsigned tacc = tmem_slot;
     bool ok = true;
 
+    // this CTA's two boxes of weight rows: gate and up rows of 64 outputs, or 128 rows in a run
+    auto first_row = [&](const Tile& t) { return GATED ? t.e * 2 * N + t.nt * TILE_N + (int)rank * BOX : t.e * N + t.nt * TILE_N + (int)rank * BM; };
+    const int second = GATED ? N : BOX;
+
     if (warp == 0) {
         if (lane == 0) {                                    // ---- producer (both CTAs)
             int it = 0;                                     // stages filled so far, over all tiles
-            // this CTA's two boxes of weight rows: gate and up rows of 64 outputs, or 128 rows in a run
-            auto first_row = [&](const Tile& t) { return GATED ? t.e * 2 * N + t.nt * TILE_N + (int)rank * BOX : t.e * N + t.nt * TILE_N + (int)rank * BM; };
-            const int second = GATED ? N : BOX;
-            // The copies of a stage wait for memory with no more than some 44 KB of an SM in flight, so weights that come from HBM
-            // are asked into L2 AHEAD stages before (and across the border to the next tile).
-            int ask_tile = pair, ask_kb = 0, ask_row = 0;
-            auto ask = [&]() {
-                if (ask_tile >= tiles) return;
-                if (ask_kb == 0) ask_row = first_row(locate(s_start, s_off, E, total_m, ask_tile));
-#pragma unroll
-                for (int j = 0; j < KPS; ++j) {
-                    prefetch_box(&map_w, (ask_kb * KPS + j) * BK, ask_row);
-                    prefetch_box(&map_w, (ask_kb * KPS + j) * BK, ask_row + second);
-                }
-                if (++ask_kb == nkb) { ask_kb = 0; ask_tile += pairs; }
-            };
-            for (int i = 0; i < AHEAD; ++i) ask();
             for (int tile = pair; tile < tiles; tile += pairs) {
                 const Tile t = locate(s_start, s_off, E, total_m, tile);
                 const int w0 = first_row(t), w1 = w0 + second;
-                const int half = t.bn >> 1, m = t.m0 + (int)rank * half, boxes = (half + BOX - 1) / BOX;
-                const unsigned bytes = A_BYTES + (unsigned)boxes * (BOX * BK * 2);
+                const int half = t.bn >> 1, m = t.m0 + (int)rank * half, boxes = (half + PBOX - 1) / PBOX;
+                const unsigned bytes = A_BYTES + (unsigned)boxes * (PBOX * BK * 2);
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    ask();
                     if (it >= STAGES) ok = mbar_wait(smem_u32(&empty_bar[s]), ((it / STAGES) - 1) & 1) && ok;
                     const unsigned full_local = smem_u32(&full_bar[s]);
                     if (rank == 0) mbar_arrive_expect_tx(full_local, 2 * KPS * bytes);
@@ -234,7 +220,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         const int x = (kb * KPS + j) * BK;
                         load_pair(d, &map_w, x, w0, full);
                         load_pair(d + BOX * BK * 2, &map_w, x, w1, full);
-                        for (int b = 0; b < boxes; ++b) load_pair(d + A_BYTES + b * (BOX * BK * 2), &map_a, x, m + b * BOX, full);
+                        for (int b = 0; b < boxes; ++b) load_pair(d + A_BYTES + b * (PBOX * BK * 2), &map_a, x, m + b * PBOX, full);
                     }
                 }
             }
@@ -340,7 +326,7 @@ template <bool GATED>
 int launch(const void* A, int lda, const void* W, const int* offsets, int E, void* out, int ldo, int places, int N, int K, int act, int* status,
            const Unit& unit, cudaStream_t st) {
     CUtensorMap ma, mw;
-    if (!tma::make_map_bf16(&ma, A, places, K, lda, BOX) || !tma::make_map_bf16(&mw, W, E * N * (GATED ? 2 : 1), K, K, BOX)) return (int)cudaErrorInvalidValue;
+    if (!tma::make_map_bf16(&ma, A, places, K, lda, PBOX) || !tma::make_map_bf16(&mw, W, E * N * (GATED ? 2 : 1), K, K, BOX)) return (int)cudaErrorInvalidValue;
     // pairs that the device holds at once (an SM whose neighbour is switched off takes none)
     static PerDevice configured;
     static int pairs_of_device[PerDevice::MAX_DEVICES] = {0};
