@@ -1900,9 +1900,17 @@ def moe_tc5_gated(x_sorted, w, offsets, out, limit: float, alpha: float, shift: 
 # From this many (token, expert) pairs on, a step's experts run as tiles on the tensor cores over the pairs sorted by
 # expert; below, every pair streams its expert's weights (a step of decoded tokens: few pairs, most on experts of their own).
 MOE_GROUPED_MIN_PAIRS = 64
-# From this many pairs on the tiles are those of the tcgen05 kernel (128 places x 256 columns, operands by TMA, the
-# tokens' rows gathered into the order of the places first); between the two, mma.sync tiles of 64 x 128.
-MOE_TC5_MIN_PAIRS = 1024
+# From this many pairs on the tiles are those of the tcgen05 kernel (operands by TMA, the tokens' rows gathered into the order of the
+# places first); with so much weight to stream already from MOE_GROUPED_MIN_PAIRS on.  Else mma.sync tiles of 64 x 128.  Measured,
+# us for all of ``moe_experts``, mma.sync / tcgen05: 32 experts of 1,536 x 2,048: 80 pairs 163 / 122, 400 194 / 134, 1,024 210 / 138, 8,192
+# 788 / 224; 64 experts of 768 x 1,024: 400 112 / 83; 16 such: 80 pairs 53 / 56, 200 68 / 60.
+MOE_TC5_MIN_PAIRS = 128
+MOE_TC5_MIN_WEIGHTS = 1 << 26
+
+
+def moe_on_tc5(pairs: int, experts: int, hidden: int, inner: int) -> bool:
+    """Whether a step's sorted pairs go through the tcgen05 kernel."""
+    return experts <= 1024 and (pairs >= MOE_TC5_MIN_PAIRS or experts * hidden * inner >= MOE_TC5_MIN_WEIGHTS)
 
 
 def moe_experts(x, up, down, expert_of, weight, shared, out, limit: float = float("inf"), alpha: float = 1.0, ctx=None,
@@ -1932,7 +1940,7 @@ def moe_experts(x, up, down, expert_of, weight, shared, out, limit: float = floa
         pair_at = buf("moe.pair_at", (pairs,), torch.int32)
         place_of = buf("moe.place_of", (pairs,), torch.int32)
         moe_sort(expert_of, E, offsets, pair_at, place_of)
-        if pairs >= MOE_TC5_MIN_PAIRS and E <= 1024:
+        if moe_on_tc5(pairs, E, H, F):
             rows = buf("moe.pair_rows", (pairs, H))
             moe_gather_rows(x, pair_at, top, rows)
             if act is None:

@@ -66,6 +66,12 @@ def test_prefill_key_shares():
             assert got == len(walked)
 
 
+def test_experts_dispatch():
+    from return_b200.ext import ops
+    assert ops.moe_on_tc5(128, 16, 1024, 768) and not ops.moe_on_tc5(127, 16, 1024, 768)        # little weight: from 128 pairs on
+    assert ops.moe_on_tc5(64, 32, 2048, 1536) and not ops.moe_on_tc5(8192, 1025, 2048, 1536)    # much: always; at most 1,024 experts
+
+
 def test_decode_key_splits():
     from return_b200.ext import ops
     for base in (1, 8, 64, 296, 512, 2000):
