@@ -837,9 +837,14 @@ def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=
     if held is not None and key in held:
         return held[key]
     host = batch.host
+    blocks, length = host.tiles[TILES_TC5], host.seg_kv_len
+    if not hasattr(host, "seg_pos0"):                  # a caller's own tables, without positions: every block in shares alike
+        longest = int(length[blocks[:, 0]].max())
+        bound = keys_seen(window, keep) or chunk
+        return prefill_splits(blocks.shape[0] * num_heads, min(longest, int(bound) + TC5_TILE_ROWS) if bound else longest), 0
     tiles = []
-    first, length = host.seg_pos0.tolist(), host.seg_kv_len.tolist()
-    for seg, row0 in host.tiles[TILES_TC5].tolist():
+    first, length = host.seg_pos0.tolist(), length.tolist()
+    for seg, row0 in blocks.tolist():
         p0 = first[seg] + row0
         end = min(length[seg], p0 + TC5_TILE_ROWS)
         low = max(0, p0 - window + 1) if window else p0 // chunk * chunk if chunk else 0
