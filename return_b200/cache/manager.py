@@ -21,7 +21,6 @@ for other architectures, ``LinearStateCache`` slots of fixed size per resident s
 """
 from __future__ import annotations
 
-from array import array
 from dataclasses import dataclass, field
 from typing import Callable, Dict, Hashable, List, Optional, Sequence
 
@@ -86,7 +85,6 @@ class _RequestState:
     slot: int
     length: int = 0                                     # tokens whose keys are (or were) cached
     blocks: List[List[int]] = field(default_factory=list)   # per group: page id per block, -1 = released
-    packed: List[array] = field(default_factory=list)       # the same as C ints, which a step's tables are copied from
 
 
 class CacheManager:
@@ -131,7 +129,7 @@ class CacheManager:
         if not self._free_slots:
             raise KVCapacityError(f"all {self.max_requests} request slots are in use")
         slot = self._free_slots.pop()
-        self._req[rid] = _RequestState(slot=slot, blocks=[[] for _ in self.groups], packed=[array("i") for _ in self.groups])
+        self._req[rid] = _RequestState(slot=slot, blocks=[[] for _ in self.groups])
         for hook in self.on_slot_taken:
             hook(slot)
         return slot
@@ -150,10 +148,6 @@ class CacheManager:
 
     def block_table(self, rid, group: int) -> List[int]:
         return self._req[rid].blocks[group]
-
-    def packed_block_table(self, rid, group: int) -> array:
-        """``block_table`` as C ints; to be copied, not kept."""
-        return self._req[rid].packed[group]
 
     def live(self) -> List[Hashable]:
         return list(self._req)
@@ -205,17 +199,15 @@ class CacheManager:
                      for g, need, pool in zip(self.groups, self.pages_needed(rid, n_tokens), self.pools)
                      if need > pool.num_free]
             raise KVCapacityError(f"request {rid!r}: pages (group, needed, free) {short}")
-        for g, pool, blocks, packed in zip(self.groups, self.pools, st.blocks, st.packed):
+        for g, pool, blocks in zip(self.groups, self.pools, st.blocks):
             gone = self._passed_blocks(g, blocks, st.length)
             if gone:
                 pool.give_back([blocks[b] for b in gone])
                 for b in gone:
-                    blocks[b] = packed[b] = -1
+                    blocks[b] = -1
             end_blocks = (st.length + n_tokens + g.page_size - 1) // g.page_size
             if end_blocks > len(blocks):
-                pages = pool.take(end_blocks - len(blocks))
-                blocks.extend(pages)
-                packed.extend(pages)
+                blocks.extend(pool.take(end_blocks - len(blocks)))
         old = st.length
         st.length += n_tokens
         return old
@@ -229,12 +221,12 @@ class CacheManager:
             raise ValueError(f"request {rid!r} holds {st.length} tokens; cannot truncate to {length}")
         if length < st.length and not self.truncatable:
             raise ValueError("per-request state depends on the tokens that were run: nothing can be taken back")
-        for g, pool, blocks, packed in zip(self.groups, self.pools, st.blocks, st.packed):
+        for g, pool, blocks in zip(self.groups, self.pools, st.blocks):
             keep = (length + g.page_size - 1) // g.page_size
             gone = [p for p in blocks[keep:] if p >= 0]
             if gone:
                 pool.give_back(gone)
-            del blocks[keep:], packed[keep:]
+            del blocks[keep:]
         st.length = length
 
     # ------------------------------------------------------------------ accounting, for tests and stats
@@ -247,7 +239,6 @@ class CacheManager:
             owned: List[int] = []
             for st in self._req.values():
                 owned.extend(p for p in st.blocks[gi] if p >= 0)
-                assert list(st.packed[gi]) == st.blocks[gi], f"group {gi}: a block table and its packed form disagree"
             assert len(owned) == len(set(owned)), f"group {gi}: a page is held by two block tables"
             assert sorted(owned) == pool.held_pages(), f"group {gi}: held pages and block tables disagree"
             free = list(pool._free)

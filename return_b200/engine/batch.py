@@ -62,39 +62,39 @@ def build_host_batch(entries: Sequence[StepEntry], manager, vocab_size: Optional
     rids = [e.rid for e in entries]
     if len(set(rids)) != n:
         raise ValueError("a request appears once in a step")
-    for e, L in zip(entries, lens):
-        if e.start < 0 or e.start + L != manager.length(e.rid):
-            raise ValueError(f"entry of request {e.rid!r}: cache room was not made for these tokens")
+    T = sum(lens)
+    tokens = np.empty(T, np.int32)
+    pos = np.empty(T, np.int32)
+    tok_seg = np.empty(T, np.int32)
     cu_q = np.zeros(n + 1, np.int32)
-    np.cumsum(lens, out=cu_q[1:])
-    T = int(cu_q[-1])
-    rows = cu_q[:-1].tolist()
-    wide = np.empty(T, np.int64)             # an id that does not fit 32 bits is refused below, not cut
+    seg_slot = np.empty(n, np.int32)
+    seg_pos0 = np.empty(n, np.int32)
+    seg_kv_len = np.empty(n, np.int32)
     want_rows: List[int] = []
     decode_segs: List[int] = []
     multi: List[int] = []
-    for i, (e, L, row) in enumerate(zip(entries, lens, rows)):
-        if L == 1:
-            wide[row] = e.tokens[0]
-            decode_segs.append(i)
-        else:
-            wide[row:row + L] = np.asarray(e.tokens, dtype=np.int64)
-            multi.append(i)
+    row = 0
+    for i, e in enumerate(entries):
+        L = lens[i]
+        if e.start < 0 or e.start + L != manager.length(e.rid):
+            raise ValueError(f"entry of request {e.rid!r}: cache room was not made for these tokens")
+        tokens[row:row + L] = np.asarray(e.tokens, dtype=np.int64)
+        pos[row:row + L] = np.arange(e.start, e.start + L)
+        tok_seg[row:row + L] = i
+        cu_q[i + 1] = row + L
+        seg_slot[i] = manager.slot(e.rid)
+        seg_pos0[i] = e.start
+        seg_kv_len[i] = e.start + L
         for w in e.want:
             if not (0 <= w < L):
                 raise ValueError(f"want index {w} is outside the entry's {L} tokens")
             want_rows.append(row + w)
-    tokens = wide.astype(np.int32)
-    seg_slot = np.array([manager.slot(r) for r in rids], np.int32)
-    seg_pos0 = np.array([e.start for e in entries], np.int32)
-    seg_kv_len = seg_pos0 + np.array(lens, np.int32)
-    tok_seg = np.repeat(np.arange(n, dtype=np.int32), lens)
-    pos = np.arange(T, dtype=np.int32) + (seg_pos0 - cu_q[:-1])[tok_seg]
-    if vocab_size is not None and (wide.min() < 0 or wide.max() >= vocab_size):
+        (decode_segs if L == 1 else multi).append(i)
+        row += L
+    if vocab_size is not None and (tokens.min() < 0 or tokens.max() >= vocab_size):
         raise ValueError(f"token ids must lie in [0, {vocab_size})")
-    longest = int(seg_kv_len.max())
-    if max_positions is not None and longest > max_positions:
-        raise ValueError(f"a request would reach {longest} tokens; the engine was set up for {max_positions}")
+    if max_positions is not None and int(seg_kv_len.max()) > max_positions:
+        raise ValueError(f"a request would reach {int(seg_kv_len.max())} tokens; the engine was set up for {max_positions}")
     tiles = {}
     for name, tiling in (tilings or {}).items():
         blocks = [(i, r0) for i in multi for r0 in range(0, lens[i], tiling.rows)]
@@ -103,13 +103,12 @@ def build_host_batch(entries: Sequence[StepEntry], manager, vocab_size: Optional
         tiles[name] = np.asarray(blocks, np.int32).reshape(-1, 2)
     tables = []
     for g, spec in enumerate(manager.groups):
-        blocks = (longest + spec.page_size - 1) // spec.page_size
+        blocks = max((int(seg_kv_len[i]) + spec.page_size - 1) // spec.page_size for i in range(n))
         bt = np.full((n, blocks), -1, np.int32)
-        for i, rid in enumerate(rids):
-            row_blocks = manager.packed_block_table(rid, g)
+        for i, e in enumerate(entries):
+            row_blocks = manager.block_table(e.rid, g)
             k = min(len(row_blocks), blocks)
-            if k:
-                bt[i, :k] = np.frombuffer(row_blocks, np.int32, k)
+            bt[i, :k] = row_blocks[:k]
         tables.append(bt)
     return HostBatch(
         num_tokens=T, num_segments=n, num_want=len(want_rows), tokens=tokens, pos=pos, tok_seg=tok_seg,
