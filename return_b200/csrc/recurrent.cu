@@ -324,6 +324,93 @@ linear_scan_kernel(const ScanArgs a) {
     }
 }
 
+// The scan of segments of one token each (a step of decoded tokens): the state is read and written once, so what bounds it is HBM, and
+// what counts is how much of it is in flight.  A warp takes 16 columns of a head: a lane four rows of every group of eight of one
+// column, 16 bytes an access and 512 neighbouring bytes a warp's, all of a lane's 16 accesses (keys of 128) asked for before anything
+// else.  64 requests of 16 heads of 128 x 128 with a decay per key row: 25.7 us inside a layer (the walk above: 47.1; the states are
+// 134 MB both ways, 20.5 us at the measured copy rate).  Only on the bfloat16 path: its sums run in another order than the walk's.
+template <int MODE, int NG>
+__global__ void __launch_bounds__(256, NG <= 16 ? 2 : 1)
+scan_step_kernel(const ScanArgs a) {
+    __shared__ __align__(16) float sk[8 * NG], sq[8 * NG], sg[8 * NG], sw[8 * NG];
+    pdl_wait();
+    const int seg = blockIdx.z, h = blockIdx.y, t = a.cu_q[seg];
+    const int tid = threadIdx.x, lane = tid & 31, hf = lane & 1, j = blockIdx.x * 128 + (tid >> 5) * 16 + (lane >> 1);
+    const int H = a.H, D = a.D, V = a.V, kvh = h / (H / a.G), nrd = (D + 7) >> 3;
+    float* Sg = a.state + (long long)a.seg_slot[seg] * a.state_stride + a.s_off + (size_t)h * nrd * 8 * V + ((size_t)j * 8 + 4 * hf);
+    const bool col = j < V;
+    float4 S[NG];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) S[i] = col && i < nrd ? *reinterpret_cast<const float4*>(Sg + (size_t)i * V * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr bool ROW_DECAY = MODE == MODE_DELTA || MODE == MODE_BONUS, DELTA = MODE == MODE_DELTA || MODE == MODE_DELTA_HEAD;
+    const float g1 = MODE == MODE_DECAY ? a.gate_a[h] : ROW_DECAY ? 1.f : a.gate_a[(size_t)t * H + h];
+    const float step = DELTA || MODE == MODE_SSM ? a.gate_b[(size_t)t * H + h] : 1.f;
+    const float vj = col ? ld_elem(a.v, a.v_f32, (size_t)t * a.v_ld + (size_t)h * V + j) : 0.f;
+    for (int i = tid; i < 8 * NG; i += 256) {
+        const bool live = i < D;
+        sk[i] = live ? ld_elem(a.k, a.k_f32, (size_t)t * a.k_ld + (size_t)kvh * D + i) : 0.f;
+        sq[i] = live ? ld_elem(a.q, a.q_f32, (size_t)t * a.q_ld + (size_t)kvh * D + i) * a.q_scale : 0.f;
+        if (ROW_DECAY) sg[i] = live ? a.gate_a[((size_t)t * H + h) * D + i] : 1.f;
+        if (MODE == MODE_BONUS) sw[i] = live ? a.extra[(size_t)h * D + i] : 0.f;
+    }
+    __syncthreads();
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float u = vj;
+    if (DELTA) {
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            const float4 k = *reinterpret_cast<const float4*>(sk + 8 * i + 4 * hf);
+            if (ROW_DECAY) {
+                const float4 g = *reinterpret_cast<const float4*>(sg + 8 * i + 4 * hf);
+                S[i].x *= g.x; S[i].y *= g.y; S[i].z *= g.z; S[i].w *= g.w;
+            } else {
+                S[i].x *= g1; S[i].y *= g1; S[i].z *= g1; S[i].w *= g1;
+            }
+            acc.x = fmaf(S[i].x, k.x, acc.x); acc.y = fmaf(S[i].y, k.y, acc.y); acc.z = fmaf(S[i].z, k.z, acc.z); acc.w = fmaf(S[i].w, k.w, acc.w);
+        }
+        const float kv = (acc.x + acc.y) + (acc.z + acc.w);
+        u = step * (vj - (kv + __shfl_xor_sync(0xffffffffu, kv, 1)));
+        acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (MODE == MODE_SSM) {
+        u = step * vj;
+    }
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+        const float4 k = *reinterpret_cast<const float4*>(sk + 8 * i + 4 * hf), q = *reinterpret_cast<const float4*>(sq + 8 * i + 4 * hf);
+        if (MODE == MODE_BONUS) {
+            const float4 g = *reinterpret_cast<const float4*>(sg + 8 * i + 4 * hf), w = *reinterpret_cast<const float4*>(sw + 8 * i + 4 * hf);
+            acc.x = fmaf(fmaf(w.x, k.x * u, S[i].x), q.x, acc.x); acc.y = fmaf(fmaf(w.y, k.y * u, S[i].y), q.y, acc.y);
+            acc.z = fmaf(fmaf(w.z, k.z * u, S[i].z), q.z, acc.z); acc.w = fmaf(fmaf(w.w, k.w * u, S[i].w), q.w, acc.w);
+            S[i].x = fmaf(g.x, S[i].x, k.x * u); S[i].y = fmaf(g.y, S[i].y, k.y * u);
+            S[i].z = fmaf(g.z, S[i].z, k.z * u); S[i].w = fmaf(g.w, S[i].w, k.w * u);
+        } else {
+            if (DELTA) {
+                S[i].x = fmaf(k.x, u, S[i].x); S[i].y = fmaf(k.y, u, S[i].y); S[i].z = fmaf(k.z, u, S[i].z); S[i].w = fmaf(k.w, u, S[i].w);
+            } else {
+                S[i].x = fmaf(g1, S[i].x, k.x * u); S[i].y = fmaf(g1, S[i].y, k.y * u); S[i].z = fmaf(g1, S[i].z, k.z * u); S[i].w = fmaf(g1, S[i].w, k.w * u);
+            }
+            acc.x = fmaf(S[i].x, q.x, acc.x); acc.y = fmaf(S[i].y, q.y, acc.y); acc.z = fmaf(S[i].z, q.z, acc.z); acc.w = fmaf(S[i].w, q.w, acc.w);
+        }
+    }
+    pdl_trigger_late();
+    if (col) {
+#pragma unroll
+        for (int i = 0; i < NG; ++i)
+            if (i < nrd) *reinterpret_cast<float4*>(Sg + (size_t)i * V * 8) = S[i];
+    }
+    float o = (acc.x + acc.y) + (acc.z + acc.w);
+    o += __shfl_xor_sync(0xffffffffu, o, 1);
+    if (MODE == MODE_SSM) o = fmaf(a.extra[h], vj, o);
+    if (col && hf == 0) a.out[((size_t)t * H + h) * V + j] = o;
+}
+
+template <int MODE>
+static int launch_step(const ScanArgs& a, int segments, cudaStream_t st) {
+    const dim3 grid((a.V + 127) / 128, a.H, segments);
+    if (a.D <= 64) return rb_launch_pdl(scan_step_kernel<MODE, 8>, grid, dim3(256), 0, st, a);
+    return rb_launch_pdl(scan_step_kernel<MODE, 16>, grid, dim3(256), 0, st, a);
+}
+
 template <int MODE>
 static int launch_scan(const ScanArgs& a, int segments, cudaStream_t st) {
     if (segments <= 0) return 0;
@@ -344,13 +431,22 @@ RB_EXPORT int rb_linear_scan(int mode, const void* q, const void* k, const void*
                              const float* extra, float cap,
                              float q_scale, float* state, long long state_stride, int s_off, int n_off, int m_off,
                              int f_off, const int* cu_q, const int* seg_slot, float* out, int H, int G, int D, int V,
-                             int segments, int below, cudaStream_t st) {
+                             int segments, int below, int single, cudaStream_t st) {
     ScanArgs a;
     a.q = q; a.k = k; a.v = v; a.q_ld = q_ld; a.k_ld = k_ld; a.v_ld = v_ld;
     a.q_f32 = q_f32; a.k_f32 = k_f32; a.v_f32 = v_f32;
     a.gate_a = gate_a; a.gate_b = gate_b; a.extra = extra; a.cap = cap; a.q_scale = q_scale;
     a.state = state; a.state_stride = state_stride; a.s_off = s_off; a.n_off = n_off; a.m_off = m_off; a.f_off = f_off;
     a.cu_q = cu_q; a.seg_slot = seg_slot; a.out = out; a.H = H; a.G = G; a.D = D; a.V = V; a.below = below;
+    // single: every segment has one token, and its sums may run in another order.  Keys of up to 128: what a lane holds in registers.
+    const bool aligned = ((uintptr_t)state & 15) == 0 && state_stride % 4 == 0 && s_off % 4 == 0;
+    if (single && below == 0 && aligned && segments > 0 && segments <= 65535 && D > 0 && D <= 128 && V > 0 && G > 0 && H % G == 0) {
+        if (mode == MODE_DECAY) return launch_step<MODE_DECAY>(a, segments, st);
+        if (mode == MODE_DELTA && gate_b) return launch_step<MODE_DELTA>(a, segments, st);
+        if (mode == MODE_DELTA_HEAD && gate_b) return launch_step<MODE_DELTA_HEAD>(a, segments, st);
+        if (mode == MODE_BONUS && extra) return launch_step<MODE_BONUS>(a, segments, st);
+        if (mode == MODE_SSM && extra && gate_b) return launch_step<MODE_SSM>(a, segments, st);
+    }
     if (mode == MODE_DECAY) return launch_scan<MODE_DECAY>(a, segments, st);
     if (mode == MODE_MEMORY) return launch_scan<MODE_MEMORY>(a, segments, st);
     if (mode == MODE_DELTA) return launch_scan<MODE_DELTA>(a, segments, st);
@@ -713,11 +809,11 @@ delta_prep_kernel(const TA* __restrict__ x, int ld, const void* __restrict__ tap
 template <typename TA, int NV, int TOK>
 __global__ void __launch_bounds__(256)
 delta_prep_vec_kernel(const TA* __restrict__ x, int ld, const void* __restrict__ taps, int taps_dtype, int K,
-                      const float* __restrict__ state, long long state_stride, int conv_off,
+                      float* __restrict__ state, long long state_stride, int conv_off,
                       const int* __restrict__ tok_seg, const int* __restrict__ cu_q, const int* __restrict__ seg_slot,
                       float* __restrict__ q32, float* __restrict__ k32, float* __restrict__ v32,
                       float* __restrict__ a, const void* __restrict__ A_log, const void* __restrict__ dt_bias, int vec_dtype,
-                      float* __restrict__ b, int T, int H, int G, int D, int V, float q_scale, int DA, int conv_ctas, int decay_ctas) {
+                      float* __restrict__ b, int T, int H, int G, int D, int V, float q_scale, int DA, int conv_ctas, int decay_ctas, int update) {
     pdl_wait();
     const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x >= conv_ctas) {
@@ -809,6 +905,14 @@ delta_prep_vec_kernel(const TA* __restrict__ x, int ld, const void* __restrict__
                 for (int m = PREP_MAX_TAPS - 2; m > 0; --m) back[n][m][ch] = back[n][m - 1][ch];
                 back[n][0][ch] = now[ch];
             }
+            if (TOK == 1 && update && live) {             // the segment's only token: its conv state moves on by one input
+                float* at = state + (long long)seg_slot[s] * state_stride + conv_off + (size_t)(c0 + 128 * n + 4 * lane) * (K - 1);
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch)
+#pragma unroll
+                    for (int m = 0; m < PREP_MAX_TAPS - 1; ++m)
+                        if (m < K - 1) at[ch * (K - 1) + K - 2 - m] = back[n][m][ch];
+            }
         }
         float inv = 1.0f;
         if (normed) inv = scale / sqrtf(warp_sum(ss) + 1e-6f);
@@ -820,11 +924,11 @@ delta_prep_vec_kernel(const TA* __restrict__ x, int ld, const void* __restrict__
 }
 
 template <typename TA>
-static int launch_delta_prep_vec(const void* x, int ld, const void* taps, int taps_dtype, int K, const float* state, long long state_stride,
+static int launch_delta_prep_vec(const void* x, int ld, const void* taps, int taps_dtype, int K, float* state, long long state_stride,
                                  int conv_off, const int* tok_seg, const int* cu_q, const int* seg_slot, float* q32, float* k32, float* v32, float* a,
                                  const void* A_log, const void* dt_bias, int vec_dtype, float* b, int T, int H, int G, int D, int V, float q_scale,
-                                 int DA, cudaStream_t st) {
-    const bool many = T >= 1024;                          // runs of tokens only where there are warps enough all the same
+                                 int DA, int update, cudaStream_t st) {
+    const bool many = T >= 1024 && !update;               // runs of tokens only where there are warps enough all the same
     const int tok = many ? 8 : 1;
     const long long tasks = (long long)((T + tok - 1) / tok) * (2 * G + H);
     const int conv_ctas = (int)((tasks + 7) / 8);
@@ -835,14 +939,19 @@ static int launch_delta_prep_vec(const void* x, int ld, const void* taps, int ta
                        : (wide ? delta_prep_vec_kernel<TA, 2, 1> : delta_prep_vec_kernel<TA, 1, 1>);
     return rb_launch_pdl(kernel, dim3(conv_ctas + decay_ctas + beta_ctas), dim3(256), 0, st, (const TA*)x, ld, taps, taps_dtype, K, state, state_stride,
                          conv_off, tok_seg, cu_q, seg_slot, q32, k32, v32, a, A_log, dt_bias, vec_dtype, b, T, H, G, D, V, q_scale, DA, conv_ctas,
-                         decay_ctas);
+                         decay_ctas, update);
 }
 
-RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dtype, int K, const float* state,
+RB_EXPORT int rb_conv_state_update(const void* x, int ld, int K, float* state, long long state_stride, int conv_off, const int* cu_q,
+                                   const int* seg_slot, int act_dtype, int C, int segments, cudaStream_t st);
+
+// update: every segment has one token, and the conv states move on as well (else that is a launch of its own after this one, so that
+// every token reads the old states; here a state's only reader moves it on, which saves a decode step the launch).
+RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dtype, int K, float* state,
                             long long state_stride, int conv_off, const int* tok_seg, const int* cu_q, const int* seg_slot,
                             float* q32, float* k32, float* v32, float* a, const void* A_log, const void* dt_bias,
                             int vec_dtype, float* b, int act_dtype, int T, int H, int G, int D, int V, float q_scale,
-                            int head_decay, cudaStream_t st) {
+                            int head_decay, int update, cudaStream_t st) {
     if (T <= 0) return 0;
     if (K < 1) return (int)cudaErrorInvalidValue;
     const int DA = head_decay ? 1 : D;
@@ -850,7 +959,7 @@ RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dt
         fours(v32) && fours(a) && fours(dt_bias, vec_dtype))
         return (act_dtype == RB_F32 ? launch_delta_prep_vec<float> : launch_delta_prep_vec<bf16>)(
             x, ld, taps, taps_dtype, K, state, state_stride, conv_off, tok_seg, cu_q, seg_slot, q32, k32, v32, a, A_log, dt_bias, vec_dtype, b, T, H, G,
-            D, V, q_scale, DA, st);
+            D, V, q_scale, DA, update, st);
     dim3 grid(T, 2 * G + 2 * H + 1);
     if (act_dtype == RB_F32)
         rb_launch_pdl(delta_prep_kernel<float>, dim3(grid), dim3(128), 0, st, (const float*)x, ld, taps, taps_dtype, K, state, state_stride, conv_off,
@@ -858,6 +967,7 @@ RB_EXPORT int rb_delta_prep(const void* x, int ld, const void* taps, int taps_dt
     else
         rb_launch_pdl(delta_prep_kernel<bf16>, dim3(grid), dim3(128), 0, st, (const bf16*)x, ld, taps, taps_dtype, K, state, state_stride, conv_off,
             tok_seg, cu_q, seg_slot, q32, k32, v32, a, A_log, dt_bias, vec_dtype, b, H, G, D, V, q_scale, DA);
+    if (update) return rb_conv_state_update(x, ld, K, state, state_stride, conv_off, cu_q, seg_slot, act_dtype, 2 * G * D + H * V, T, st);
     return rb_launch_status();
 }
 

@@ -1200,7 +1200,7 @@ def recurrent_lib() -> ctypes.CDLL:
     if _recurrent is None:
         lib = build.load("return_recurrent", _RECURRENT_SOURCES, {"RB_PDL_MODE": PDL_MODE})
         P, I, F, L = c_void_p, c_int, c_float, ctypes.c_longlong
-        lib.rb_linear_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, F, P, L, I, I, I, I, P, P, P, I, I, I, I, I, I, P]
+        lib.rb_linear_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, F, P, L, I, I, I, I, P, P, P, I, I, I, I, I, I, I, P]
         lib.rb_chunked_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, P, L, I, P, P, P, P] + [I] * 8 + [P, P]
         lib.rb_chunked_scan_floats.argtypes, lib.rb_chunked_scan_floats.restype = [I, I, I], L
         lib.rb_token_shift_mix.argtypes = [P, I, P, I, I, P, L, I, P, P, P, P, I, I, I, P]
@@ -1215,7 +1215,7 @@ def recurrent_lib() -> ctypes.CDLL:
         lib.rb_memory_pieces_combine.restype = c_int
         lib.rb_rotary_inplace.argtypes = [P, I, P, P, I, P, I, I, I, I, P]
         lib.rb_rotary_inplace.restype = c_int
-        lib.rb_delta_prep.argtypes = [P, I, P, I, I, P, L, I, P, P, P, P, P, P, P, P, P, I, P, I, I, I, I, I, I, F, I, P]
+        lib.rb_delta_prep.argtypes = [P, I, P, I, I, P, L, I, P, P, P, P, P, P, P, P, P, I, P, I, I, I, I, I, I, F, I, I, P]
         lib.rb_gated_conv.argtypes = [P, I, P, P, P, I, I, P, L, I, P, P, P, P, P, I, I, I, P]
         lib.rb_gated_recurrence.argtypes = [P, P, I, P, P, P, I, F, P, I, P, P, L, I, P, P, P, I, I, I, I, P, P]
         lib.rb_gated_pieces_combine.argtypes = [P, P, P, L, I, P, P, I, I, P]
@@ -1246,9 +1246,10 @@ def _is_f32(t: torch.Tensor) -> int:
 
 def linear_scan(mode: int, q, k, v, gate_a, gate_b, state, offsets, batch, out, heads: int, kv_heads: int,
                 dim: int, vdim: int, q_scale: float = 1.0, cap: float = 0.0, forgot_offset: int = -1, extra=None,
-                below: int = 0) -> None:
+                below: int = 0, single: bool = False) -> None:
     """The recurrence of a mixer with a [dim, vdim] state per head, over every segment of the step, token by token
-    (``below`` > 0: over the segments of fewer tokens only).
+    (``below`` > 0: over the segments of fewer tokens only).  ``single``: every segment has one token and the order of its sums
+    may differ from that of longer ones, which lets a kernel for such steps run.
 
     q, k: [T, >= kv_heads * dim] views (float32 or bfloat16, unit stride along a row), v: [T, >= heads * vdim];
     ``state``: float32 [slots, n], the row of a segment is ``batch.seg_slot``; ``offsets`` = (S, n, m): where the
@@ -1274,7 +1275,7 @@ def linear_scan(mode: int, q, k, v, gate_a, gate_b, state, offsets, batch, out, 
         mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _is_f32(q), _is_f32(k), _is_f32(v),
         _ptr(gate_a), _ptr(gate_b), _ptr(extra), cap, q_scale, _ptr(state), state.stride(0), offsets[0], offsets[1], offsets[2],
         forgot_offset, _ptr(batch.cu_q), _ptr(batch.seg_slot), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, below,
-        _stream()), "linear_scan")
+        1 if single else 0, _stream()), "linear_scan")
 
 
 CHUNK_TOKENS = 32                          # tokens of a chunk (csrc/recurrent_chunks.cu)
@@ -1380,13 +1381,15 @@ def rotary_inplace(x, cos, sin, rot: int, pos, heads: int, dim: int) -> None:
 
 
 def delta_prep(x, taps, state, conv_off: int, batch, q32, k32, v32, a, A_log, dt_bias, b, heads: int, kv_heads: int,
-               dim: int, vdim: int, q_scale: float, head_decay: bool = False) -> None:
+               dim: int, vdim: int, q_scale: float, head_decay: bool = False, update_state: bool = False) -> None:
     """What the delta rule needs of every token: the short causal convolution and silu of the q, k, v channels of
     ``x`` (what lies before a segment comes from the request's conv state), unit q and k heads, the row decays (in
     place over ``a``) and beta (in place over ``b``).  ``head_decay``: ``a`` holds one number a token and head
-    ([T, heads], ``dt_bias`` [heads]) instead of one a key row."""
+    ([T, heads], ``dt_bias`` [heads]) instead of one a key row.  ``update_state`` (segments of one token each only): the conv
+    states move on too (``conv_state_update``)."""
     T = x.shape[0]
     K = taps.shape[1]
+    assert not update_state or batch.num_segments == T
     assert x.stride(1) == 1 and taps.is_contiguous() and taps.shape[0] == 2 * kv_heads * dim + heads * vdim
     assert a.dtype == b.dtype == torch.float32 and a.is_contiguous() and b.is_contiguous()
     assert A_log.dtype == dt_bias.dtype
@@ -1396,7 +1399,7 @@ def delta_prep(x, taps, state, conv_off: int, batch, q32, k32, v32, a, A_log, dt
         _ptr(x), x.stride(0), _ptr(taps), dtype_code(taps.dtype), K, _ptr(state), state.stride(0), conv_off,
         _ptr(batch.tok_seg), _ptr(batch.cu_q), _ptr(batch.seg_slot), _ptr(q32), _ptr(k32), _ptr(v32), _ptr(a),
         _ptr(A_log), _ptr(dt_bias), dtype_code(A_log.dtype), _ptr(b), dtype_code(x.dtype), T, heads, kv_heads, dim, vdim,
-        q_scale, 1 if head_decay else 0, _stream()), "delta_prep")
+        q_scale, 1 if head_decay else 0, 1 if update_state else 0, _stream()), "delta_prep")
 
 
 def general_delta_scan(q, k, v, decay, neg_removal, state, s_off: int, batch, out, heads: int, dim: int) -> None:

@@ -38,6 +38,10 @@ class _StateMixer(Mixer):
     def out_projection(self):
         return self.p_o
 
+    def _single(self, batch):
+        """Whether the step holds single tokens only and, on the bfloat16 path, may sum in the order of a kernel of their own."""
+        return self.env.act_dtype != torch.float32 and batch.num_tokens == batch.num_segments
+
     # A segment of at least this many tokens is cut into pieces that are scanned side by side (bfloat16 path only:
     # the sums then take another order than token by token, which the float32 path never does).
     PIECES_MIN_TOKENS = 1024
@@ -141,7 +145,8 @@ class _StateMixer(Mixer):
             return
         pieces = self._pieces(b) if self.env.act_dtype != torch.float32 else None
         if pieces is None:
-            ops.linear_scan(mode, q, k, v, decay, step, ctx.state, (0, 0, 0), b, out, self.H, groups, self.D, self.V, extra=extra)
+            ops.linear_scan(mode, q, k, v, decay, step, ctx.state, (0, 0, 0), b, out, self.H, groups, self.D, self.V, extra=extra,
+                            single=self._single(b))
             return
         virtual, seg_first, n_pieces = pieces
         dev = out.device
@@ -200,7 +205,7 @@ class Retention(_StateMixer):
             pass
         elif pieces is None:
             ops.linear_scan(ops.SCAN_DECAY, q32, k32, v, self._decay, None, ctx.state, (0, 0, 0), b, o,
-                            self.H, self.H, self.D, self.V)
+                            self.H, self.H, self.D, self.V, single=self._single(b))
         else:
             # long segments in pieces side by side: scan every piece from zero, hand the states on in order, scan again
             virtual, seg_first, n_pieces = pieces
@@ -264,13 +269,15 @@ class ChannelDelta(_StateMixer):
         q32 = ctx.buffer("channel_delta.q", (T, GD), torch.float32, dev)
         k32 = ctx.buffer("channel_delta.k", (T, GD), torch.float32, dev)
         v32 = ctx.buffer("channel_delta.v", (T, HV), torch.float32, dev)
+        alone = b.num_tokens == b.num_segments           # segments of one token: the kernel that reads their conv states moves them on
         ops.delta_prep(proj, self.p_conv, ctx.state, self.conv_off, b, q32, k32, v32, decay, self.p_A_log,
-                       self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5)
-        ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
+                       self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5, update_state=alone)
+        if not alone:
+            ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
         o = ctx.buffer("channel_delta.o", (T, HV), torch.float32, dev)
         if not self._scan_in_chunks(ops.SCAN_DELTA, q32, k32, v32, decay, beta, ctx, o, self.G):
             ops.linear_scan(ops.SCAN_DELTA, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
-                            self.H, self.G, self.D, self.V)
+                            self.H, self.G, self.D, self.V, single=self._single(b))
         mixed = ctx.buffer("channel_delta.mixed", (T, HV), x.dtype, dev)
         ops.head_norm_gate(o, gate, self.p_norm, 1, 1, s.eps, mixed, self.H, self.V)
         return self._project_out(mixed, ctx)
@@ -502,13 +509,15 @@ class GatedDelta(_StateMixer):
         q32 = ctx.buffer("gated_delta.q", (T, GD), torch.float32, dev)
         k32 = ctx.buffer("gated_delta.k", (T, GD), torch.float32, dev)
         v32 = ctx.buffer("gated_delta.v", (T, HV), torch.float32, dev)
+        alone = b.num_tokens == b.num_segments           # see ChannelDelta.forward
         ops.delta_prep(proj, self.p_conv, ctx.state, self.conv_off, b, q32, k32, v32, decay, self.p_A_log,
-                       self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5, head_decay=True)
-        ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
+                       self.p_dt_bias, beta, self.H, self.G, self.D, self.V, self.D ** -0.5, head_decay=True, update_state=alone)
+        if not alone:
+            ops.conv_state_update(proj, s.conv_taps, ctx.state, self.conv_off, b, C)      # after every token read the old one
         o = ctx.buffer("gated_delta.o", (T, HV), torch.float32, dev)
         if not self._scan_in_chunks(ops.SCAN_DELTA_HEAD, q32, k32, v32, decay, beta, ctx, o, self.G):
             ops.linear_scan(ops.SCAN_DELTA_HEAD, q32, k32, v32, decay, beta, ctx.state, (0, 0, 0), b, o,
-                            self.H, self.G, self.D, self.V)
+                            self.H, self.G, self.D, self.V, single=self._single(b))
         mixed = ctx.buffer("gated_delta.mixed", (T, HV), x.dtype, dev)
         ops.head_norm_gate(o, proj[:, C:], self.p_norm, 1, 0, s.eps, mixed, self.H, self.V)
         return self._project_out(mixed, ctx)

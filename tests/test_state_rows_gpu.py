@@ -82,3 +82,55 @@ def test_delta_prep(dt, lens, H, G, D, V, K, head_decay):
                        head_decay=head_decay)
         outs.append(out)
     assert all(same(p, q, torch.float32) for p, q in zip(*outs))
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,D,V,K", [(4, 2, 8, 12, 4), (2, 1, 128, 256, 2), (2, 2, 36, 132, 1), (1, 1, 20, 4, 3)])
+def test_delta_prep_moves_conv_states_of_single_tokens(dt, H, G, D, V, K):
+    """The same numbers as the two kernels one after the other, in both forms, with a slot of no request between."""
+    ops = _ops()
+    T, C = 7, 2 * G * D + H * V
+    x, taps = torch.randn(T, C, device=DEV).to(dt), torch.randn(C, K, device=DEV).to(dt)
+    a, b = torch.randn(T, H * D, device=DEV), torch.randn(T, H, device=DEV)
+    A_log, dt_bias = torch.randn(H, device=DEV).to(dt), torch.randn(H * D, device=DEV).to(dt)
+    state = torch.randn(T + 1, 2 + C * (K - 1), device=DEV)
+    i32 = lambda y: torch.as_tensor(y, dtype=torch.int32, device=DEV)
+    batch = SimpleNamespace(cu_q=i32(list(range(T + 1))), seg_slot=i32([7, 0, 3, 1, 6, 2, 5]), tok_seg=i32(list(range(T))), num_segments=T)
+    for form in (lambda y: y, off_by_one):
+        outs = []
+        for fused in (False, True):
+            out, st = [torch.empty(T, w, device=DEV) for w in (G * D, G * D, H * V)] + [a.clone(), b.clone()], state.clone()
+            ops.delta_prep(form(x), taps, st, 2, batch, out[0], out[1], out[2], out[3], A_log, dt_bias, out[4], H, G, D, V, D ** -0.5,
+                           update_state=fused)
+            if not fused:
+                ops.conv_state_update(form(x), K, st, 2, batch, C)
+            outs.append(out + [st])
+        assert all(torch.equal(p, q) for p, q in zip(*outs))
+
+
+@pytest.mark.parametrize("mode", ["DECAY", "DELTA", "BONUS", "SSM", "DELTA_HEAD"])
+@pytest.mark.parametrize("n,H,G,D,V,off", [(1, 2, 1, 128, 128, 0), (5, 4, 2, 24, 40, 4), (3, 2, 2, 100, 144, 0), (2, 3, 3, 64, 7, 8)])
+def test_scan_of_single_tokens(mode, n, H, G, D, V, off):
+    """The kernel for segments of one token beside the walk: the same sums of up to 128 products in another order."""
+    ops = _ops()
+    m = getattr(ops, "SCAN_" + mode)
+    normal = lambda *s: torch.randn(*s, device=DEV)
+    q, k, v = normal(n, G * D) * D ** -0.5, torch.nn.functional.normalize(normal(n, G, D), dim=-1).reshape(n, -1), normal(n, H * V).bfloat16()
+    gate_a = torch.rand({"DECAY": (H,), "DELTA": (n, H * D), "BONUS": (n, H * D)}.get(mode, (n, H)), device=DEV)
+    gate_b = torch.rand(n, H, device=DEV) if mode in ("DELTA", "DELTA_HEAD", "SSM") else None
+    extra = normal(H, D) if mode == "BONUS" else normal(H) if mode == "SSM" else None
+    state = normal(n + 1, off + (H * ((D + 7) // 8 * 8) * V + 3) // 4 * 4)
+    batch = SimpleNamespace(cu_q=torch.arange(n + 1, dtype=torch.int32, device=DEV), num_segments=n,
+                            seg_slot=torch.arange(n, 0, -1, dtype=torch.int32, device=DEV))
+    outs = []
+    for single in (False, True):
+        st, out = state.clone(), torch.empty(n, H * V, device=DEV)
+        ops.linear_scan(m, q, k, v, gate_a, gate_b, st, (off, 0, 0), batch, out, H, G, D, V, extra=extra, single=single)
+        outs.append((out, st))
+    rows = (D + 7) // 8 * 8
+    if rows != D:                                             # rows that do not exist are zero in a real state; here they hold anything
+        keep = torch.ones(H, rows // 8, V, 8, dtype=torch.bool, device=DEV)
+        keep[:, -1, :, D % 8:] = False
+        outs = [(o, s[:, off:off + keep.numel()] * keep.reshape(-1)) for o, s in outs]
+    bound = 2.0 ** -17 * (1 + float(state.abs().max()))       # 128 roundings of 2^-24 of sums of the size of the state
+    assert all((x - y).abs().max() <= bound for x, y in zip(*outs))
