@@ -16,10 +16,12 @@ from __future__ import annotations
 import ctypes
 import fcntl
 import hashlib
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -173,3 +175,55 @@ def load(name: str, sources: Sequence[str], defines: Optional[Dict[str, object]]
                 raise ExtensionError(f"cannot load {path}: {e}") from e
             _loaded[key] = lib
         return lib
+
+
+_native_calls = None                                   # the module of csrc/native_calls.c; False where it cannot be had
+
+
+def native_calls_path() -> Optional[str]:
+    """Path of the compiled ``csrc/native_calls.c``, or None without a C compiler or Python's headers."""
+    include = sysconfig.get_paths()["include"]
+    src = os.path.join(CSRC, "native_calls.c")
+    with open(src, "rb") as fh:
+        tag = hashlib.sha256(fh.read() + (sys.version + sysconfig.get_platform()).encode()).hexdigest()[:16]
+    fname = f"return_b200_native_calls-{tag}.so"
+    pre = _readable_prebuilt(fname)
+    if pre:
+        return pre
+    cc = shutil.which("cc") or shutil.which("gcc")
+    if cc is None or not os.path.isfile(os.path.join(include, "Python.h")):
+        return None
+    out = os.path.join(build_dir(), fname)
+    if not os.path.isfile(out):
+        tmp = out + f".tmp{os.getpid()}"
+        done = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, src, "-o", tmp], capture_output=True, text=True)
+        if done.returncode != 0:
+            return None
+        os.replace(tmp, out)
+    return out
+
+
+def native_calls(lib: ctypes.CDLL) -> None:
+    """Takes the entries of a library whose ``argtypes`` are set (and which return an int) past ctypes: ``csrc/native_calls.c``.
+    Where that cannot be compiled they stay ctypes functions, which do the same."""
+    global _native_calls
+    with _lock:
+        if _native_calls is None:
+            path = native_calls_path()
+            _native_calls = False
+            if path is not None:
+                spec = importlib.util.spec_from_file_location("return_b200_native_calls", path)
+                try:
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                    _native_calls = module
+                except ImportError:
+                    pass
+    if not _native_calls:
+        return
+    kinds = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
+    for name, fn in list(vars(lib).items()):
+        if isinstance(fn, ctypes._CFuncPtr) and fn.argtypes is not None and fn.restype is ctypes.c_int and all(t in kinds for t in fn.argtypes):
+            call = _native_calls.make(ctypes.cast(fn, ctypes.c_void_p).value, "".join(kinds[t] for t in fn.argtypes), fn)
+            if call is not None:
+                setattr(lib, name, call)

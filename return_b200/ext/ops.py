@@ -37,7 +37,7 @@ def _ptr(t: Optional[torch.Tensor]):
         return None
     if not t.is_cuda:
         raise KernelError("the engine's kernels run on a CUDA device only; got a CPU tensor")
-    return t.data_ptr()              # an int: ctypes makes the pointer from it (argtypes are set)
+    return t.data_ptr()              # an int: the call makes the pointer from it (argtypes are set)
 
 
 try:                                                  # the raw handle, without building a Stream object
@@ -49,8 +49,8 @@ except AttributeError:                                # a torch without these: t
 def _stream():
     """The current stream of the current device (each launch asks: a graph capture changes it)."""
     if _raw_stream is not None:
-        return c_void_p(_raw_stream(_device_index()))
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_device_index())
+    return torch.cuda.current_stream().cuda_stream
 
 
 # kernels of this package launched by this process (a captured graph counts once, at capture)
@@ -115,6 +115,7 @@ def core() -> ctypes.CDLL:
                      "rb_softcap", "rb_activation", "rb_hyper_read_norm", "rb_hyper_write", "rb_attention_simt_mod",
                      "rb_attn_prep", "rb_attn_gate", "rb_embedding_pair", "rb_last_token"):
             getattr(lib, name).restype = c_int
+        build.native_calls(lib)
         _core = lib
     return _core
 
@@ -138,7 +139,8 @@ def build_all():
         paths.append(build.library_path(f"return_attn_tc5_d{d}", ["attention_tc5.cu"], _attn_tc5_defines(d)))
     for d in PREBUILT_HEAD_DIMS:
         paths.append(build.library_path(f"return_attn_d{d}", ["attention_mma.cu"], _attn_defines(d)))
-    return paths
+    calls = build.native_calls_path()
+    return paths + ([calls] if calls else [])
 
 
 # ------------------------------------------------------------------------------- elementwise
@@ -469,6 +471,7 @@ def tc5_lib() -> ctypes.CDLL:
         lib.rb_tc5_gemm_simple.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm_bmn.argtypes = [P, P, P, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm.restype = lib.rb_tc5_gemm_simple.restype = lib.rb_tc5_gemm_bmn.restype = c_int
+        build.native_calls(lib)
         _tc5 = lib
     return _tc5
 
@@ -672,6 +675,7 @@ def attention_lib(head_dim: int) -> ctypes.CDLL:
         lib.rb_attn_prefill.restype = lib.rb_attn_decode.restype = lib.rb_attn_head_dim.restype = c_int
         if lib.rb_attn_head_dim() != head_dim:
             raise KernelError("attention library was compiled for another head size")
+        build.native_calls(lib)
         _attn_libs[head_dim] = lib
     return lib
 
@@ -713,6 +717,7 @@ def attention_tc5_lib(head_dim: int) -> ctypes.CDLL:
         lib.rb_attn_tc5_split_floats.argtypes = [I, I, I]
         lib.rb_attn_tc5_split_floats.restype = ctypes.c_longlong
         lib.rb_attn_prefill_tc5.restype = c_int
+        build.native_calls(lib)
         _attn_tc5_libs[head_dim] = lib
     return lib
 
@@ -1103,6 +1108,7 @@ def attention_conv_lib(head_dim: int, taps: int) -> ctypes.CDLL:
         P, I, F, L = c_void_p, c_int, c_float, ctypes.c_longlong
         lib.rb_attn_conv_prep.argtypes = [P, I, P, I, P, L, I, P, P, P, P, P, I, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, F, I, P]
         lib.rb_attn_conv_prep.restype = c_int
+        build.native_calls(lib)
         _attn_conv_libs[key] = lib
     return lib
 
@@ -1148,6 +1154,7 @@ def tanh_norm_lib() -> ctypes.CDLL:
         P, I, L = c_void_p, c_int, ctypes.c_longlong
         lib.rb_tanh_joint.argtypes = [P, P, P, I, P, P, P, P, P, P, P, P, L, I, P, P, P, P, P, I, I, I, P]
         lib.rb_tanh_joint.restype = c_int
+        build.native_calls(lib)
         _tanh_norm = lib
     return _tanh_norm
 
@@ -1232,6 +1239,7 @@ def recurrent_lib() -> ctypes.CDLL:
                      "rb_head_norm_gate", "rb_add_dual_norm", "rb_scaled_sum", "rb_token_shift_mix", "rb_ssm_prep",
                      "rb_gated_part_norm"):
             getattr(lib, name).restype = c_int
+        build.native_calls(lib)
         _recurrent = lib
     return _recurrent
 
@@ -1605,6 +1613,7 @@ def latent_lib() -> ctypes.CDLL:
         for name in ("rb_latent_write", "rb_latent_attention_simt", "rb_head_gate", "rb_gemm_f32_heads",
                      "rb_latent_expand_scatter", "rb_latent_expand_query", "rb_latent_take_values"):
             getattr(lib, name).restype = c_int
+        build.native_calls(lib)
         _latent = lib
     return _latent
 
@@ -1764,6 +1773,7 @@ def moe_lib() -> ctypes.CDLL:
         for name in ("rb_moe_route", "rb_moe_pair_linear", "rb_clamped_glu", "rb_moe_combine", "rb_moe_sort",
                      "rb_moe_grouped_gemm", "rb_moe_gather_rows"):
             getattr(lib, name).restype = c_int
+        build.native_calls(lib)
         _moe = lib
     return _moe
 
@@ -1865,6 +1875,7 @@ def moe_tc5_lib() -> ctypes.CDLL:
         lib.rb_moe_tc5_gemm.argtypes = [P, I, P, P, I, P, I, I, I, I, I, P, P]
         lib.rb_moe_tc5_gated.argtypes = [P, I, P, P, I, P, I, I, I, I, c_float, c_float, c_float, P, P, P, P]
         lib.rb_moe_tc5_gemm.restype = lib.rb_moe_tc5_gated.restype = c_int
+        build.native_calls(lib)
         _moe_tc5 = lib
     return _moe_tc5
 
