@@ -203,9 +203,20 @@ def native_calls_path() -> Optional[str]:
     return out
 
 
-def native_calls(lib: ctypes.CDLL) -> None:
-    """Takes the entries of a library whose ``argtypes`` are set (and which return an int) past ctypes: ``csrc/native_calls.c``.
-    Where that cannot be compiled they stay ctypes functions, which do the same."""
+class Entries:
+    """A library's entries as attributes: those that can be called past ctypes, and the ``ctypes.CDLL``'s own for all others."""
+
+    def __init__(self, lib: ctypes.CDLL, calls: Dict[str, object]):
+        self.__dict__.update(calls)
+        self._lib = lib
+
+    def __getattr__(self, name):
+        return getattr(self.__dict__["_lib"], name)
+
+
+def native_calls(lib: ctypes.CDLL):
+    """The entries of a library whose ``argtypes`` are set (and which return an int) taken past ctypes: ``csrc/native_calls.c``.
+    ``lib`` itself stays as it is.  Where that cannot be compiled it is handed back, and does the same."""
     global _native_calls
     with _lock:
         if _native_calls is None:
@@ -220,10 +231,12 @@ def native_calls(lib: ctypes.CDLL) -> None:
                 except ImportError:
                     pass
     if not _native_calls:
-        return
+        return lib
     kinds = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
+    calls = {}
     for name, fn in list(vars(lib).items()):
         if isinstance(fn, ctypes._CFuncPtr) and fn.argtypes is not None and fn.restype is ctypes.c_int and all(t in kinds for t in fn.argtypes):
             call = _native_calls.make(ctypes.cast(fn, ctypes.c_void_p).value, "".join(kinds[t] for t in fn.argtypes), fn)
             if call is not None:
-                setattr(lib, name, call)
+                calls[name] = call
+    return Entries(lib, calls)

@@ -115,8 +115,7 @@ def core() -> ctypes.CDLL:
                      "rb_softcap", "rb_activation", "rb_hyper_read_norm", "rb_hyper_write", "rb_attention_simt_mod",
                      "rb_attn_prep", "rb_attn_gate", "rb_embedding_pair", "rb_last_token"):
             getattr(lib, name).restype = c_int
-        build.native_calls(lib)
-        _core = lib
+        _core = build.native_calls(lib)
     return _core
 
 
@@ -471,8 +470,7 @@ def tc5_lib() -> ctypes.CDLL:
         lib.rb_tc5_gemm_simple.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm_bmn.argtypes = [P, P, P, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm.restype = lib.rb_tc5_gemm_simple.restype = lib.rb_tc5_gemm_bmn.restype = c_int
-        build.native_calls(lib)
-        _tc5 = lib
+        _tc5 = build.native_calls(lib)
     return _tc5
 
 
@@ -675,8 +673,7 @@ def attention_lib(head_dim: int) -> ctypes.CDLL:
         lib.rb_attn_prefill.restype = lib.rb_attn_decode.restype = lib.rb_attn_head_dim.restype = c_int
         if lib.rb_attn_head_dim() != head_dim:
             raise KernelError("attention library was compiled for another head size")
-        build.native_calls(lib)
-        _attn_libs[head_dim] = lib
+        lib = _attn_libs[head_dim] = build.native_calls(lib)
     return lib
 
 
@@ -717,8 +714,7 @@ def attention_tc5_lib(head_dim: int) -> ctypes.CDLL:
         lib.rb_attn_tc5_split_floats.argtypes = [I, I, I]
         lib.rb_attn_tc5_split_floats.restype = ctypes.c_longlong
         lib.rb_attn_prefill_tc5.restype = c_int
-        build.native_calls(lib)
-        _attn_tc5_libs[head_dim] = lib
+        lib = _attn_tc5_libs[head_dim] = build.native_calls(lib)
     return lib
 
 
@@ -1111,8 +1107,7 @@ def attention_conv_lib(head_dim: int, taps: int) -> ctypes.CDLL:
         P, I, F, L = c_void_p, c_int, c_float, ctypes.c_longlong
         lib.rb_attn_conv_prep.argtypes = [P, I, P, I, P, L, I, P, P, P, P, P, I, I, P, P, P, I, I, I, I, I, I, I, I, I, I, F, F, I, P]
         lib.rb_attn_conv_prep.restype = c_int
-        build.native_calls(lib)
-        _attn_conv_libs[key] = lib
+        lib = _attn_conv_libs[key] = build.native_calls(lib)
     return lib
 
 
@@ -1157,8 +1152,7 @@ def tanh_norm_lib() -> ctypes.CDLL:
         P, I, L = c_void_p, c_int, ctypes.c_longlong
         lib.rb_tanh_joint.argtypes = [P, P, P, I, P, P, P, P, P, P, P, P, L, I, P, P, P, P, P, I, I, I, P]
         lib.rb_tanh_joint.restype = c_int
-        build.native_calls(lib)
-        _tanh_norm = lib
+        _tanh_norm = build.native_calls(lib)
     return _tanh_norm
 
 
@@ -1242,8 +1236,7 @@ def recurrent_lib() -> ctypes.CDLL:
                      "rb_head_norm_gate", "rb_add_dual_norm", "rb_scaled_sum", "rb_token_shift_mix", "rb_ssm_prep",
                      "rb_gated_part_norm"):
             getattr(lib, name).restype = c_int
-        build.native_calls(lib)
-        _recurrent = lib
+        _recurrent = build.native_calls(lib)
     return _recurrent
 
 
@@ -1616,8 +1609,7 @@ def latent_lib() -> ctypes.CDLL:
         for name in ("rb_latent_write", "rb_latent_attention_simt", "rb_head_gate", "rb_gemm_f32_heads",
                      "rb_latent_expand_scatter", "rb_latent_expand_query", "rb_latent_take_values"):
             getattr(lib, name).restype = c_int
-        build.native_calls(lib)
-        _latent = lib
+        _latent = build.native_calls(lib)
     return _latent
 
 
@@ -1776,8 +1768,7 @@ def moe_lib() -> ctypes.CDLL:
         for name in ("rb_moe_route", "rb_moe_pair_linear", "rb_clamped_glu", "rb_moe_combine", "rb_moe_sort",
                      "rb_moe_grouped_gemm", "rb_moe_gather_rows"):
             getattr(lib, name).restype = c_int
-        build.native_calls(lib)
-        _moe = lib
+        _moe = build.native_calls(lib)
     return _moe
 
 
@@ -1878,8 +1869,7 @@ def moe_tc5_lib() -> ctypes.CDLL:
         lib.rb_moe_tc5_gemm.argtypes = [P, I, P, P, I, P, I, I, I, I, I, P, P]
         lib.rb_moe_tc5_gated.argtypes = [P, I, P, P, I, P, I, I, I, I, c_float, c_float, c_float, P, P, P, P]
         lib.rb_moe_tc5_gemm.restype = lib.rb_moe_tc5_gated.restype = c_int
-        build.native_calls(lib)
-        _moe_tc5 = lib
+        _moe_tc5 = build.native_calls(lib)
     return _moe_tc5
 
 

@@ -24,7 +24,8 @@ def test_same_arguments(tmp_path, types):
     subprocess.run([shutil.which("cc") or "gcc", "-O1", "-shared", "-fPIC", str(src), "-o", str(out)], check=True)
     lib, plain = ctypes.CDLL(str(out)), ctypes.CDLL(str(out))
     lib.rb_entry.argtypes = plain.rb_entry.argtypes = types
-    build.native_calls(lib)
+    raw, lib = lib, build.native_calls(lib)
+    raw.rb_entry.argtypes = types                             # another thread that loads the same library declares its entries again
     small = types.count(F) <= 8 and len(types) - types.count(F) <= 48
     assert (type(lib.rb_entry).__name__ == "Call") == small
     seen = set()
