@@ -531,6 +531,11 @@ def step_kernel_times(fn, steps: int) -> Dict[str, float]:
     return dict(out)
 
 
+# What the names of a mixer's scan and of the experts' products for decoded tokens contain, whichever of their kernels a step's sizes pick.
+SCAN_KERNELS = ("linear_scan", "scan_step", "chunk_prep", "chunk_serial")
+DECODED_EXPERT_KERNELS = ("moe_pair_linear", "moe_grouped_gemm", "moe_tc5")
+
+
 def _kernel_ms(times: Dict[str, float], *needles: str) -> float:
     return sum(ms for name, ms in times.items() if any(n in name for n in needles))
 
@@ -594,8 +599,8 @@ def compare_designs(size: str, tokens: int, batch: int, steps: int, warmup: int,
     scan_flops = tokens * D * (4.0 * n_ret * H * 128 + 6.0 * n_delta * H * 128 + 4.0 * n_both * (H // 2) * 256)
     kv_bytes = lambda layers: 2 * 2 * G * D * tokens * batch * layers
     attn_flops = lambda layers: 4.0 * tokens * tokens * H * D / 2 * layers
-    scan_dec = _kernel_ms(new["decode_kernels"], "linear_scan")
-    scan_pf = _kernel_ms(new["prefill_kernels"], "linear_scan")
+    scan_dec = _kernel_ms(new["decode_kernels"], *SCAN_KERNELS)
+    scan_pf = _kernel_ms(new["prefill_kernels"], *SCAN_KERNELS)
     att_dec_new = _kernel_ms(new["decode_kernels"], "attn_decode", "attn_combine")
     att_dec_old = _kernel_ms(old["decode_kernels"], "attn_decode", "attn_combine")
     att_pf_new = _kernel_ms(new["prefill_kernels"], "attn_prefill", "attention_tc5", "tc5_merge")
@@ -697,8 +702,8 @@ def compare_gonozen(size: str, tokens: int, batch: int, steps: int, warmup: int,
                             "of_bf16_peak": frac(moe_flops, _kernel_ms(k_new, "moe_grouped_gemm", "moe_tc5"), bf16_tflops * 1e12)},
         "prefill_dense_feed_forward_qwen3": {"ms": round(ff_old_pf, 4), "of_bf16_peak": frac(dense_flops, ff_old_pf, bf16_tflops * 1e12),
                                              "note": "the three largest kernels of the step beside the attention: the gated product and the down projection among them"},
-        "decode_experts": {"ms": round(_kernel_ms(d_new, "moe_pair_linear", "moe_grouped_gemm"), 4),
-                           "of_hbm": frac(moe_bytes, _kernel_ms(d_new, "moe_pair_linear", "moe_grouped_gemm"), hbm_gbs * 1e9)},
+        "decode_experts": {"ms": round(_kernel_ms(d_new, *DECODED_EXPERT_KERNELS), 4),
+                           "of_hbm": frac(moe_bytes, _kernel_ms(d_new, *DECODED_EXPERT_KERNELS), hbm_gbs * 1e9)},
         "decode_weight_streaming_qwen3": {"ms": round(_kernel_ms(d_old, "gemm_skinny"), 4),
                                           "of_hbm": frac(dense_bytes + L * 2.0 * W * (H + 2 * G + H) * D, _kernel_ms(d_old, "gemm_skinny"), hbm_gbs * 1e9)},
     }
@@ -766,16 +771,16 @@ def compare_nozizen(size: str, tokens: int, batch: int, steps: int, warmup: int,
     k_new, k_old, d_new, d_old = new["prefill_kernels"], old["prefill_kernels"], new["decode_kernels"], old["decode_kernels"]
     att_pf, att_dec = ("attn_prefill", "attention_tc5", "merge_key_splits", "tc5_merge"), ("attn_decode", "attn_combine")
     hyper = ("hyper_read_norm", "hyper_write")
-    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), ("moe_pair_linear", "moe_grouped_gemm")
+    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), DECODED_EXPERT_KERNELS
     small = ("token_shift_mix", "ssm_prep", "conv_state_update", "gated_part_norm", "head_norm_gate", "activation_kernel",
              "clamped_glu", "moe_combine", "moe_route", "moe_sort", "moe_gather")
     hbm, peak = hbm_gbs * 1e9, bf16_tflops * 1e12
     row = lambda times, names, work, roof, key: {"ms": round(_kernel_ms(times, *names), 4), key: frac(work, _kernel_ms(times, *names), roof)}
     kernels = {
-        "decode_scan_nozizen": row(d_new, ("linear_scan",), 2.0 * state_bytes_new * batch, hbm, "of_hbm"),
-        "decode_scan_pisatar": row(d_old, ("linear_scan",), 2.0 * state_bytes_old * batch, hbm, "of_hbm"),
-        "prefill_scan_nozizen": row(k_new, ("linear_scan",), scan_flops_new, peak, "of_bf16_peak"),
-        "prefill_scan_pisatar": row(k_old, ("linear_scan",), scan_flops_old, peak, "of_bf16_peak"),
+        "decode_scan_nozizen": row(d_new, SCAN_KERNELS, 2.0 * state_bytes_new * batch, hbm, "of_hbm"),
+        "decode_scan_pisatar": row(d_old, SCAN_KERNELS, 2.0 * state_bytes_old * batch, hbm, "of_hbm"),
+        "prefill_scan_nozizen": row(k_new, SCAN_KERNELS, scan_flops_new, peak, "of_bf16_peak"),
+        "prefill_scan_pisatar": row(k_old, SCAN_KERNELS, scan_flops_old, peak, "of_bf16_peak"),
         "decode_attention_nozizen": row(d_new, att_dec, 2.0 * 2 * G * D * seen * batch * n_att, hbm, "of_hbm"),
         "decode_attention_pisatar": row(d_old, att_dec, 2.0 * 2 * G * D * tokens * batch * o_both, hbm, "of_hbm"),
         "prefill_attention_nozizen": row(k_new, att_pf, 4.0 * band * H * D * n_att, peak, "of_bf16_peak"),
@@ -870,16 +875,16 @@ def compare_duvadra(size: str, tokens: int, batch: int, steps: int, warmup: int,
     frac = lambda work, ms, peak: round(work / (ms * 1e-3) / peak, 4) if ms > 0 else None
     k_new, k_old, d_new, d_old = new["prefill_kernels"], old["prefill_kernels"], new["decode_kernels"], old["decode_kernels"]
     att_dec = ("attn_decode", "attn_combine")
-    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), ("moe_pair_linear", "moe_grouped_gemm")
+    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), DECODED_EXPERT_KERNELS
     small = ("attn_prep", "attn_gate", "gated_conv", "conv_state_update", "delta_prep", "head_norm_gate", "scaled_sum",
              "clamped_glu", "moe_combine", "moe_route", "moe_sort", "moe_gather", "embedding_pair", "last_token")
     hbm, peak = hbm_gbs * 1e9, bf16_tflops * 1e12
     row = lambda times, names, work, roof, key: {"ms": round(_kernel_ms(times, *names), 4), key: frac(work, _kernel_ms(times, *names), roof)}
     kernels = {
-        "decode_scan_duvadra": row(d_new, ("linear_scan",), 2.0 * 4 * D * D * H * n_delta * batch, hbm, "of_hbm"),
-        "decode_scan_nozizen": row(d_old, ("linear_scan",), 2.0 * 4 * D * D * H * o_state * batch, hbm, "of_hbm"),
-        "prefill_scan_duvadra": row(k_new, ("linear_scan",), 6.0 * tokens * D * D * H * n_delta, peak, "of_bf16_peak"),
-        "prefill_scan_nozizen": row(k_old, ("linear_scan",), 4.0 * tokens * D * D * H * o_state, peak, "of_bf16_peak"),
+        "decode_scan_duvadra": row(d_new, SCAN_KERNELS, 2.0 * 4 * D * D * H * n_delta * batch, hbm, "of_hbm"),
+        "decode_scan_nozizen": row(d_old, SCAN_KERNELS, 2.0 * 4 * D * D * H * o_state * batch, hbm, "of_hbm"),
+        "prefill_scan_duvadra": row(k_new, SCAN_KERNELS, 6.0 * tokens * D * D * H * n_delta, peak, "of_bf16_peak"),
+        "prefill_scan_nozizen": row(k_old, SCAN_KERNELS, 4.0 * tokens * D * D * H * o_state, peak, "of_bf16_peak"),
         "decode_recurrence_duvadra": row(d_new, ("gated_recurrence",), n_lru * batch * W * (2.0 * 4 + 2 + 8 + 2 + 2), hbm, "of_hbm"),
         "prefill_recurrence_duvadra": row(k_new, ("gated_recurrence", "gated_pieces_combine"), n_lru * tokens * W * (2.0 + 8 + 2 + 2), hbm, "of_hbm"),
         "decode_attention_duvadra": row(d_new, att_dec, 2.0 * 2 * G * D * batch * (tokens * n_blocks + seen * (n_lru + n_delta)), hbm, "of_hbm"),
@@ -961,7 +966,7 @@ def compare_losorax(size: str, tokens: int, batch: int, steps: int, warmup: int,
     k_new, k_old, d_new, d_old = new["prefill_kernels"], old["prefill_kernels"], new["decode_kernels"], old["decode_kernels"]
     att_dec = ("attn_decode", "attn_combine")
     att_pf = ("attn_prefill_kernel", "attn_prefill_tc5_kernel<true>")
-    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), ("moe_pair_linear", "moe_grouped_gemm")
+    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), DECODED_EXPERT_KERNELS
     moe_small = ("clamped_glu", "moe_combine", "moe_route", "moe_sort", "moe_gather")
     hbm, peak = hbm_gbs * 1e9, bf16_tflops * 1e12
     row = lambda times, names, work, roof, key: {"ms": round(_kernel_ms(times, *names), 4), key: frac(work, _kernel_ms(times, *names), roof)}
@@ -971,9 +976,9 @@ def compare_losorax(size: str, tokens: int, batch: int, steps: int, warmup: int,
     prep_old = 2.0 * D * ((o_blocks + o_windows) * 2 * H + (o_blocks / 2 + o_delta) * 4 * G + (o_windows - o_delta) * 3 * G)
     kernels = {
         "decode_scan_losorax": row(d_new, ("general_delta_scan",), 2.0 * 4 * D * D * H * n_delta * batch, hbm, "of_hbm"),
-        "decode_scan_duvadra": row(d_old, ("linear_scan",), 2.0 * 4 * D * D * H * o_delta * batch, hbm, "of_hbm"),
+        "decode_scan_duvadra": row(d_old, SCAN_KERNELS, 2.0 * 4 * D * D * H * o_delta * batch, hbm, "of_hbm"),
         "prefill_scan_losorax": row(k_new, ("general_delta_scan",), 6.0 * tokens * D * D * H * n_delta, peak, "of_bf16_peak"),
-        "prefill_scan_duvadra": row(k_old, ("linear_scan",), 6.0 * tokens * D * D * H * o_delta, peak, "of_bf16_peak"),
+        "prefill_scan_duvadra": row(k_old, SCAN_KERNELS, 6.0 * tokens * D * D * H * o_delta, peak, "of_bf16_peak"),
         "decode_attention_losorax": row(d_new, att_dec, 2.0 * 2 * G * D * batch * tokens * n_att, hbm, "of_hbm"),
         "decode_attention_duvadra": row(d_old, att_dec, 2.0 * 2 * G * D * batch * (tokens * o_blocks + min(tokens, window) * o_windows), hbm, "of_hbm"),
         "prefill_attention_losorax": row(k_new, att_pf, 4.0 * tokens * tokens / 2 * H * D * n_att, peak, "of_bf16_peak"),
@@ -1059,7 +1064,7 @@ def compare_sizudra(size: str, tokens: int, batch: int, steps: int, warmup: int,
     row = lambda times, names, work, roof, key: {"ms": round(_kernel_ms(times, *names), 4), key: frac(work, _kernel_ms(times, *names), roof)}
     k_new, k_q, k_g = new["prefill_kernels"], qwen["prefill_kernels"], gon["prefill_kernels"]
     d_new, d_q, d_g = new["decode_kernels"], qwen["decode_kernels"], gon["decode_kernels"]
-    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), ("moe_pair_linear", "moe_grouped_gemm")
+    moe_pf, moe_dec = ("moe_grouped_gemm", "moe_tc5"), DECODED_EXPERT_KERNELS
     kv_bytes = 2.0 * 2 * G * D * batch
     rows_bytes = 2.0 * D * 2 * (H + 2 * G) * tokens                   # a layer's projections read, queries and pages written
     joint_bytes = 2.0 * L * tokens * W * (2 * 4 + 2 + 2)
