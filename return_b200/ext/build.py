@@ -181,11 +181,14 @@ _native_calls = None                                   # the module of csrc/nati
 
 
 def native_calls_path() -> Optional[str]:
-    """Path of the compiled ``csrc/native_calls.c``, or None without a C compiler or Python's headers."""
+    """Path of the compiled ``csrc/native_calls.c``, or None without its source, a C compiler, Python's headers or a folder to write to."""
     include = sysconfig.get_paths()["include"]
     src = os.path.join(CSRC, "native_calls.c")
-    with open(src, "rb") as fh:
-        tag = hashlib.sha256(fh.read() + (sys.version + sysconfig.get_platform()).encode()).hexdigest()[:16]
+    try:
+        with open(src, "rb") as fh:
+            tag = hashlib.sha256(fh.read() + (sys.version + sysconfig.get_platform()).encode()).hexdigest()[:16]
+    except OSError:
+        return None
     fname = f"return_b200_native_calls-{tag}.so"
     pre = _readable_prebuilt(fname)
     if pre:
@@ -193,13 +196,16 @@ def native_calls_path() -> Optional[str]:
     cc = shutil.which("cc") or shutil.which("gcc")
     if cc is None or not os.path.isfile(os.path.join(include, "Python.h")):
         return None
-    out = os.path.join(build_dir(), fname)
-    if not os.path.isfile(out):
-        tmp = out + f".tmp{os.getpid()}"
-        done = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, src, "-o", tmp], capture_output=True, text=True)
-        if done.returncode != 0:
-            return None
-        os.replace(tmp, out)
+    try:
+        out = os.path.join(build_dir(), fname)
+        if not os.path.isfile(out):
+            tmp = out + f".tmp{os.getpid()}-{threading.get_ident()}"
+            done = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, src, "-o", tmp], capture_output=True, text=True)
+            if done.returncode != 0:
+                return None
+            os.replace(tmp, out)
+    except (ExtensionError, OSError):
+        return None
     return out
 
 

@@ -39,3 +39,26 @@ def test_same_arguments(tmp_path, types):
             lib.rb_entry(*args[:-1])
         with pytest.raises(ctypes.ArgumentError):
             lib.rb_entry(*args[:-1], "x" if types[-1] is not P else 1.0)
+
+
+@pytest.mark.parametrize("missing", ["folder", "compiler", "source", "disk"])
+def test_libraries_load_without_native_calls(monkeypatch, tmp_path, missing):
+    """Where the module cannot be had, a library that is there already is called through ctypes as before."""
+    monkeypatch.setattr(build, "_native_calls", None)
+    monkeypatch.setattr(build, "_readable_prebuilt", lambda name: None)
+    monkeypatch.setenv("RETURN_B200_BUILD_DIR", str(tmp_path))
+
+    def refuse(*a, **k):
+        raise build.ExtensionError("no writable build folder") if missing == "folder" else OSError("no room")
+
+    if missing == "folder":
+        monkeypatch.setattr(build, "build_dir", refuse)
+    elif missing == "compiler":
+        monkeypatch.setattr(shutil, "which", lambda name: None)
+    elif missing == "source":
+        monkeypatch.setattr(build, "CSRC", str(tmp_path))
+    else:
+        monkeypatch.setattr(build.subprocess, "run", refuse)
+    lib = ctypes.CDLL(None)
+    assert build.native_calls_path() is None
+    assert build.native_calls(lib) is lib
