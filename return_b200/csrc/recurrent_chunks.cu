@@ -10,7 +10,8 @@
 //
 // `chunk_prep_kernel` works out k * P, q * P, k * P_32 / P_t, T, M and P_32 for all chunks and heads side by side and leaves them in the
 // order in which the second kernel's matrix instructions want them.  `chunk_serial_kernel` walks the chunks of a segment in order,
-// a CTA per 16 value columns of a head; the state stays in registers and S0 goes through matrix instructions.
+// a CTA per 16 value columns of a head, for the long segments only: a CTA takes an SM's shared memory, so one that finds nothing to do
+// still holds up those behind it.  The state stays in registers and S0 goes through matrix instructions.
 //
 // All arithmetic keeps float32's precision.  The products run as bfloat16 matrix instructions on operands split into three
 // bfloat16 parts (x = h + m + l, 24 bits), six of the nine products (hh, hm, mh, hl, lh, mm; the rest is below 2^-24), the five small
@@ -43,6 +44,7 @@ struct ChunkArgs {
     int* status;                                        // set to 1 if a wait gave up
     int H, G, D, V, segments;
     int min_tokens;                                     // segments of fewer tokens are none of these kernels' business
+    int longs;                                          // how many segments are long (at most)
     int first, count;                                   // the window: these chunks of all segments' chunks, counted in order
 };
 
@@ -60,38 +62,71 @@ __device__ __forceinline__ float ld_elem(const void* p, int f32, size_t i) {
     return f32 ? ((const float*)p)[i] : __bfloat162float(((const bf16*)p)[i]);
 }
 
-// Chunks of the segments in front of `seg` (seg = segments: of all), by one warp.
-__device__ __forceinline__ int chunks_before(const ChunkArgs& a, int seg, int lane) {
-    int n = 0;
-    for (int s = lane; s < seg; s += 32) {
-        const int len = a.cu_q[s + 1] - a.cu_q[s];
-        if (len >= a.min_tokens) n += (len + CT - 1) / CT;
+// Chunks of segments base + 32 u + lane (0: a segment that is none of these kernels' business), and where these begin and end, all
+// looked up together.
+struct Found { int own[4], begin[4], end[4]; };
+__device__ __forceinline__ Found own_chunks(const ChunkArgs& a, int base, int lane) {
+    Found f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int s = base + 32 * u + lane;
+        f.begin[u] = s < a.segments ? a.cu_q[s] : 0;
+        f.end[u] = s < a.segments ? a.cu_q[s + 1] : 0;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
-    return n;
+    for (int u = 0; u < 4; ++u) {
+        const int len = f.end[u] - f.begin[u];
+        f.own[u] = len >= a.min_tokens ? (len + CT - 1) / CT : 0;
+    }
+    return f;
+}
+struct Place { int seg, chunk, begin, end; };            // a segment (-1: none), a chunk or a number of chunks, the segment's tokens
+
+// The `which`-th long segment and how many chunks lie in front of it, by one warp.
+__device__ __forceinline__ Place find_segment(const ChunkArgs& a, int which, int lane) {
+    Place p = {-1, 0, 0, 0};
+    for (int base = 0; base < a.segments && p.seg < 0; base += 128) {
+        const Found f = own_chunks(a, base, lane);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const unsigned there = __ballot_sync(0xffffffffu, f.own[u] > 0);
+            const bool here = p.seg < 0 && which < __popc(there);
+            const bool it = here && f.own[u] > 0 && __popc(there & ((1u << lane) - 1u)) == which;
+            const int at = here ? __ffs(__ballot_sync(0xffffffffu, it)) - 1 : 0;
+            if (p.seg < 0) p.chunk += __reduce_add_sync(0xffffffffu, !here || lane < at ? f.own[u] : 0);
+            if (here) {
+                p.seg = base + 32 * u + at;
+                p.begin = __shfl_sync(0xffffffffu, f.begin[u], at);
+                p.end = __shfl_sync(0xffffffffu, f.end[u], at);
+            }
+            which -= __popc(there);
+        }
+    }
+    return p;
 }
 
-// The segment that chunk `c` belongs to and the chunk's number in it, by one warp; segment -1 if there is no such chunk.
-__device__ __forceinline__ int2 find_chunk(const ChunkArgs& a, int c, int lane) {
-    for (int base = 0; base < a.segments; base += 32) {
-        const int s = base + lane;
-        const int len = s < a.segments ? a.cu_q[s + 1] - a.cu_q[s] : 0;
-        const int own = len >= a.min_tokens ? (len + CT - 1) / CT : 0;
-        int upto = own;                                  // inclusive sums over the lanes
+// The segment that chunk `c` belongs to and the chunk's number in it, by one warp.
+__device__ __forceinline__ Place find_chunk(const ChunkArgs& a, int c, int lane) {
+    for (int base = 0; base < a.segments; base += 128) {
+        const Found f = own_chunks(a, base, lane);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o);
-            if (lane >= o) upto += v;
+        for (int u = 0; u < 4; ++u) {
+            const int all = __reduce_add_sync(0xffffffffu, f.own[u]);
+            if (c < all) {
+                int upto = f.own[u];                     // inclusive sums over the lanes
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                    if (lane >= o) upto += v;
+                }
+                const int at = __ffs(__ballot_sync(0xffffffffu, c < upto)) - 1;
+                return {base + 32 * u + at, c - __shfl_sync(0xffffffffu, upto - f.own[u], at), __shfl_sync(0xffffffffu, f.begin[u], at),
+                        __shfl_sync(0xffffffffu, f.end[u], at)};
+            }
+            c -= all;
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, c < upto);
-        if (hit) {
-            const int at = __ffs(hit) - 1;
-            return make_int2(base + at, c - __shfl_sync(0xffffffffu, upto - own, at));
-        }
-        c -= __shfl_sync(0xffffffffu, upto, 31);
     }
-    return make_int2(-1, 0);
+    return {-1, 0, 0, 0};
 }
 
 // ---------------------------------------------------------------- float32 products by three bfloat16 parts
@@ -248,19 +283,18 @@ chunk_prep_kernel(const ChunkArgs a) {
     __shared__ double bd[4][DP];                         // decays of the whole blocks: products are rounded once, where they are used
     __shared__ __align__(16) float Am[CT][CT + 4], Mm[CT][CT + 4], Tm[CT][CT + 4];
     __shared__ float beta[CT];
-    __shared__ int2 which;
+    __shared__ Place which;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.y;
     pdl_wait();
     if (warp == 0) {
-        const int2 w = find_chunk(a, a.first + blockIdx.x, lane);
+        const Place w = find_chunk(a, a.first + blockIdx.x, lane);
         if (lane == 0) which = w;
     }
     for (int e = tid; e < CT * CT; e += THREADS) Am[e / CT][e % CT] = Mm[e / CT][e % CT] = 0.f;
     __syncthreads();
-    const int seg = which.x;
-    if (seg < 0) return;
-    const int t0 = a.cu_q[seg] + which.y * CT, n = min(CT, a.cu_q[seg + 1] - t0);
+    if (which.seg < 0) return;
+    const int t0 = which.begin + which.chunk * CT, n = min(CT, which.end - t0);
     const int H = a.H, D = a.D, kvh = h / (H / a.G);
     load_rows<DP>(Ks, a.k, a.k_f32, t0, n, a.k_ld, kvh * D, D, 1.f, 0.f);
     load_rows<DP>(Qs, a.q, a.q_f32, t0, n, a.q_ld, kvh * D, D, a.q_scale, 0.f);
@@ -503,22 +537,22 @@ chunk_serial_kernel(const ChunkArgs a) {
     unsigned* Rp = Sp + KT * 384;                        // [2][3][lane][4]
     unsigned* Up = Rp + 2 * 384;                         // [chunk % 2][2][3][lane][4]
     __shared__ __align__(8) unsigned long long full[STAGES];
-    __shared__ int before;
+    __shared__ Place which;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int seg = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * COLS;
+    const int h = blockIdx.y, j0 = blockIdx.x * COLS;
     pdl_wait();
-    const int t_first = a.cu_q[seg], t_end = a.cu_q[seg + 1];
-    if (t_end - t_first < a.min_tokens) return;
     if (warp == 0) {
-        const int n = chunks_before(a, seg, lane);
+        const Place w = find_segment(a, blockIdx.z, lane);
         if (lane == 0) {
-            before = n;
+            which = w;
 #pragma unroll
             for (int i = 0; i < STAGES; ++i) tc5::mbar_init(tc5::smem_u32(&full[i]), 1);
             tc5::mbar_init_fence();
         }
     }
     __syncthreads();
+    const int seg = which.seg, before = which.chunk, t_first = which.begin, t_end = which.end;
+    if (seg < 0) return;
     // this segment's chunks that lie in the window
     const int c_begin = max(0, a.first - before);
     const int c_end = min((t_end - t_first + CT - 1) / CT, a.first + a.count - before);
@@ -716,7 +750,7 @@ int launch_chunks(const ChunkArgs& a, cudaStream_t st) {
     if (rc) return rc;
     rc = rb_launch_pdl(chunk_prep_kernel<MODE, DP>, dim3(a.count, a.H), dim3(THREADS), prep_bytes, st, a);
     if (rc) return rc;
-    return rb_launch_pdl(chunk_serial_kernel<MODE, DP>, dim3((a.V + COLS - 1) / COLS, a.H, a.segments), dim3(32 * serial_warps<DP>()), serial_bytes, st, a);
+    return rb_launch_pdl(chunk_serial_kernel<MODE, DP>, dim3((a.V + COLS - 1) / COLS, a.H, a.longs), dim3(32 * serial_warps<DP>()), serial_bytes, st, a);
 }
 
 template <int MODE>
@@ -735,22 +769,22 @@ RB_EXPORT long long rb_chunked_scan_floats(int mode, int H, int D) {
     return (long long)H * (delta ? Layout<128>::DELTA : Layout<128>::PLAIN);
 }
 
-// The segments of at least `min_tokens` tokens; `first` and `count`: which of their chunks, counted over all such segments in
+// The segments of at least `min_tokens` tokens, of which there are `longs` at most; `first` and `count`: which of their chunks, counted over all such segments in
 // order.  A caller with less scratch than all chunks need goes through them window by window, in order.
 RB_EXPORT int rb_chunked_scan(int mode, const void* q, const void* k, const void* v, int q_ld, int k_ld, int v_ld, int q_f32, int k_f32,
                               int v_f32, const float* gate_a, const float* gate_b, const float* extra, float q_scale, float* state,
                               long long state_stride, int s_off, const int* cu_q, const int* seg_slot, float* scratch, float* out, int H,
-                              int G, int D, int V, int segments, int min_tokens, int first, int count, int* status, cudaStream_t st) {
+                              int G, int D, int V, int segments, int min_tokens, int longs, int first, int count, int* status, cudaStream_t st) {
     if (segments <= 0 || count <= 0) return 0;
     if (rb_chunked_scan_floats(mode, H, D) == 0 || V <= 0 || G <= 0 || H % G || min_tokens < 1 || first < 0) return (int)cudaErrorInvalidValue;
-    if (((uintptr_t)scratch & 15) || segments > 65535) return (int)cudaErrorInvalidValue;
+    if (((uintptr_t)scratch & 15) || longs < 1 || longs > 65535) return (int)cudaErrorInvalidValue;
     ChunkArgs a;
     a.q = q; a.k = k; a.v = v; a.q_ld = q_ld; a.k_ld = k_ld; a.v_ld = v_ld;
     a.q_f32 = q_f32; a.k_f32 = k_f32; a.v_f32 = v_f32;
     a.gate_a = gate_a; a.gate_b = gate_b; a.extra = extra; a.q_scale = q_scale;
     a.state = state; a.state_stride = state_stride; a.s_off = s_off; a.cu_q = cu_q; a.seg_slot = seg_slot;
     a.scratch = scratch; a.out = out; a.status = status; a.H = H; a.G = G; a.D = D; a.V = V; a.segments = segments;
-    a.min_tokens = min_tokens; a.first = first; a.count = count;
+    a.min_tokens = min_tokens; a.longs = longs; a.first = first; a.count = count;
     if (mode == CHUNK_DECAY) return launch_mode<CHUNK_DECAY>(a, st);
     if (mode == CHUNK_DELTA) return gate_b ? launch_mode<CHUNK_DELTA>(a, st) : (int)cudaErrorInvalidValue;
     if (mode == CHUNK_DELTA_HEAD) return gate_b ? launch_mode<CHUNK_DELTA_HEAD>(a, st) : (int)cudaErrorInvalidValue;

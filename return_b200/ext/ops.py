@@ -1205,7 +1205,7 @@ def recurrent_lib() -> ctypes.CDLL:
         lib = build.load("return_recurrent", _RECURRENT_SOURCES, {"RB_PDL_MODE": PDL_MODE})
         P, I, F, L = c_void_p, c_int, c_float, ctypes.c_longlong
         lib.rb_linear_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, F, P, L, I, I, I, I, P, P, P, I, I, I, I, I, I, I, P]
-        lib.rb_chunked_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, P, L, I, P, P, P, P] + [I] * 8 + [P, P]
+        lib.rb_chunked_scan.argtypes = [I, P, P, P, I, I, I, I, I, I, P, P, P, F, P, L, I, P, P, P, P] + [I] * 9 + [P, P]
         lib.rb_chunked_scan_floats.argtypes, lib.rb_chunked_scan_floats.restype = [I, I, I], L
         lib.rb_token_shift_mix.argtypes = [P, I, P, I, I, P, L, I, P, P, P, P, I, I, I, P]
         lib.rb_ssm_prep.argtypes = [P, I, I, I, P, P, I, I, P, L, I, P, P, P, P, I, I, P, P, I, P, P, I, I, P]
@@ -1294,9 +1294,10 @@ def chunked_scan_ok(mode: int, heads: int, dim: int) -> bool:
 
 
 def chunked_scan(mode: int, q, k, v, gate_a, gate_b, state, s_off: int, batch, chunks: int, min_tokens: int, out, heads: int,
-                 kv_heads: int, dim: int, vdim: int, extra=None, buffer=None) -> None:
+                 kv_heads: int, dim: int, vdim: int, extra=None, buffer=None, longs: Optional[int] = None) -> None:
     """``linear_scan`` for the segments of at least ``min_tokens`` tokens, 32 tokens at a time (every mode but SCAN_MEMORY, keys up
-    to 128).  ``chunks``: how many chunks of 32 these segments have between them.  ``buffer(name, shape, dtype, device)`` gives
+    to 128).  ``chunks``: how many chunks of 32 these segments have between them; ``longs``: how many
+    such segments there are (None: the step's segments at most).  ``buffer(name, shape, dtype, device)`` gives
     the scratch."""
     assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
     assert out.dtype == torch.float32 and out.is_contiguous() and out.shape[1] == heads * vdim
@@ -1317,7 +1318,7 @@ def chunked_scan(mode: int, q, k, v, gate_a, gate_b, state, s_off: int, batch, c
         _check(lib.rb_chunked_scan(
             mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _is_f32(q), _is_f32(k), _is_f32(v),
             _ptr(gate_a), _ptr(gate_b), _ptr(extra), 1.0, _ptr(state), state.stride(0), s_off, _ptr(batch.cu_q), _ptr(batch.seg_slot),
-            _ptr(scratch), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, min_tokens, first, min(window, chunks - first),
+            _ptr(scratch), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, min_tokens, batch.num_segments if longs is None else longs, first, min(window, chunks - first),
             _ptr(tc5_status(out.device)), _stream()), "chunked_scan", 2)
 
 

@@ -108,3 +108,39 @@ def test_chunked_scan(mode, lens, H, G, D, V, decay, form, monkeypatch):
             off = lambda z: float((z.double() - w).norm() / w.norm())
             # sums of up to 128 + 32 terms rounded to 24 bits, in other orders: a few 2^-24 either way
             assert off(x) < 2.0 * off(y) + 2.0 ** -22, (i, off(x), off(y))
+
+
+@pytest.mark.parametrize("lens", [[1] * 131 + [70, 1, 64, 3, 200], [100] + [1] * 40 + [65], [64] * 37 + [1] * 95 + [97]])
+def test_long_segments_are_found(lens):
+    """The grid of the second kernel covers the long segments alone, wherever they stand among the others; a grid that covers more
+    gives the same, in windows that begin within a segment too."""
+    ops = _ops()
+    H, D, V, T, n = 2, 64, 24, sum(lens), len(lens)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    normal = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    q, k, v, state = normal(T, H * D) * D ** -0.5, normal(T, H * D) * D ** -0.5, normal(T, H * V), normal(n, H * D * V)
+    gate = torch.rand(H, generator=gen, device=DEV)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_q=cu, num_segments=n, seg_slot=torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV))
+    longs, chunks = sum(x >= 64 for x in lens), sum((x + 31) // 32 for x in lens if x >= 64)
+    outs = []
+    for grid, scratch in ((longs, 64 << 20), (None, 64 << 20), (longs, 5 * 4 * ops.recurrent_lib().rb_chunked_scan_floats(ops.SCAN_DECAY, H, D))):
+        st, out = state.clone(), torch.zeros(T, H * V, device=DEV)
+        old, ops.CHUNK_SCRATCH_BYTES = ops.CHUNK_SCRATCH_BYTES, scratch
+        try:
+            ops.chunked_scan(ops.SCAN_DECAY, q, k, v, gate, None, st, 0, batch, chunks, 64, out, H, H, D, V, longs=grid)
+        finally:
+            ops.CHUNK_SCRATCH_BYTES = old
+        outs.append((out, st))
+    ops.check_status(DEV)
+    for out, st in outs[1:]:
+        assert torch.equal(out, outs[0][0]) and torch.equal(st, outs[0][1])
+    walked, st = torch.zeros(T, H * V, device=DEV), state.clone()
+    ops.linear_scan(ops.SCAN_DECAY, q, k, v, gate, None, st, (0, 0, 0), batch, walked, H, H, D, V)
+    for i, (a, b) in enumerate(zip(cu[:-1].tolist(), cu[1:].tolist())):
+        slot = n - 1 - i
+        if b - a < 64:                                         # left alone
+            assert not outs[0][0][a:b].any() and torch.equal(outs[0][1][slot], state[slot])
+        else:                                                  # the same sums of up to 64 + 32 terms in another order
+            assert torch.allclose(outs[0][0][a:b], walked[a:b], rtol=2.0 ** -18, atol=2.0 ** -18 * float(walked.abs().max()))
+            assert torch.allclose(outs[0][1][slot], st[slot], rtol=2.0 ** -18, atol=2.0 ** -18 * float(st.abs().max()))

@@ -66,6 +66,44 @@ def test_prefill_key_shares():
             assert got == len(walked)
 
 
+def _state_mixer(H, D, V, dtype):
+    from types import SimpleNamespace
+    from return_b200.parts.recurrent import _StateMixer
+    m = object.__new__(_StateMixer)
+    m.H, m.D, m.V, m.env = H, D, V, SimpleNamespace(act_dtype=dtype, device="cpu")
+    return m
+
+
+def _scan_batch(lens):
+    from types import SimpleNamespace
+
+    import numpy as np
+    cu = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    host = SimpleNamespace(cu_q=cu, num_multi=sum(n > 1 for n in lens))
+    return SimpleNamespace(host=host, scratch={}, num_segments=len(lens), num_tokens=int(cu[-1]))
+
+
+def test_chunked_scan_is_launched_for_the_long_segments_alone(monkeypatch):
+    """The scan in chunks takes an SM a CTA: decoded tokens beside a portion must not add CTAs to it."""
+    from types import SimpleNamespace
+
+    import torch
+    from return_b200.ext import ops
+    seen = []
+    monkeypatch.setattr(ops, "chunked_scan_ok", lambda mode, heads, dim: True)
+    monkeypatch.setattr(ops, "chunked_scan", lambda mode, *a, **k: seen.append(("chunks", a[8], k["longs"])))
+    monkeypatch.setattr(ops, "linear_scan", lambda mode, *a, **k: seen.append(("walk", k["below"])))
+    m = _state_mixer(16, 128, 128, torch.bfloat16)
+    least = m.CHUNKED_MIN_TOKENS
+    for lens, want in (([1] * 64 + [200], [("chunks", 7, 1), ("walk", least)]), ([300, 1, least, least - 1], [("chunks", 10 + least // 32, 2), ("walk", least)]),
+                       ([least], [("chunks", least // 32, 1)]), ([1, least - 1], [])):
+        seen.clear()
+        batch = _scan_batch(lens)
+        ctx = SimpleNamespace(batch=batch, state=None, buffer=None)
+        assert m._scan_in_chunks(ops.SCAN_DELTA, None, None, None, None, None, ctx, None, 4) == bool(want)
+        assert seen == want
+
+
 def test_experts_dispatch():
     from return_b200.ext import ops
     assert ops.moe_on_tc5(128, 16, 1024, 768) and not ops.moe_on_tc5(127, 16, 1024, 768)        # little weight: from 128 pairs on
