@@ -324,7 +324,8 @@ linear_scan_kernel(const ScanArgs a) {
     }
 }
 
-// The scan of segments of one token each (a step of decoded tokens): the state is read and written once, so what bounds it is HBM, and
+// The scan of segments of one token each (a step of decoded tokens, or the decoded tokens beside portions that run in chunks, so that a
+// decoded token gets the same bits in both): the state is read and written once, so what bounds it is HBM, and
 // what counts is how much of it is in flight.  A warp takes 16 columns of a head: a lane four rows of every group of eight of one
 // column, 16 bytes an access and 512 neighbouring bytes a warp's, all of a lane's 16 accesses (keys of 128) asked for before anything
 // else.  64 requests of 16 heads of 128 x 128 with a decay per key row: 25.7 us inside a layer (the walk above: 47.1; the states are
@@ -335,6 +336,7 @@ scan_step_kernel(const ScanArgs a) {
     __shared__ __align__(16) float sk[8 * NG], sq[8 * NG], sg[8 * NG], sw[8 * NG];
     pdl_wait();
     const int seg = blockIdx.z, h = blockIdx.y, t = a.cu_q[seg];
+    if (a.below > 0 && a.cu_q[seg + 1] - t >= a.below) return;         // recurrent_chunks.cu takes it
     const int tid = threadIdx.x, lane = tid & 31, hf = lane & 1, j = blockIdx.x * 128 + (tid >> 5) * 16 + (lane >> 1);
     const int H = a.H, D = a.D, V = a.V, kvh = h / (H / a.G), nrd = (D + 7) >> 3;
     float* Sg = a.state + (long long)a.seg_slot[seg] * a.state_stride + a.s_off + (size_t)h * nrd * 8 * V + ((size_t)j * 8 + 4 * hf);
@@ -438,9 +440,9 @@ RB_EXPORT int rb_linear_scan(int mode, const void* q, const void* k, const void*
     a.gate_a = gate_a; a.gate_b = gate_b; a.extra = extra; a.cap = cap; a.q_scale = q_scale;
     a.state = state; a.state_stride = state_stride; a.s_off = s_off; a.n_off = n_off; a.m_off = m_off; a.f_off = f_off;
     a.cu_q = cu_q; a.seg_slot = seg_slot; a.out = out; a.H = H; a.G = G; a.D = D; a.V = V; a.below = below;
-    // single: every segment has one token, and its sums may run in another order.  Keys of up to 128: what a lane holds in registers.
+    // single: every segment (of fewer than `below` tokens) has one token, and its sums may run in another order.  Keys of up to 128: what a lane holds in registers.
     const bool aligned = ((uintptr_t)state & 15) == 0 && state_stride % 4 == 0 && s_off % 4 == 0;
-    if (single && below == 0 && aligned && segments > 0 && segments <= 65535 && D > 0 && D <= 128 && V > 0 && G > 0 && H % G == 0) {
+    if (single && aligned && segments > 0 && segments <= 65535 && D > 0 && D <= 128 && V > 0 && G > 0 && H % G == 0) {
         if (mode == MODE_DECAY) return launch_step<MODE_DECAY>(a, segments, st);
         if (mode == MODE_DELTA && gate_b) return launch_step<MODE_DELTA>(a, segments, st);
         if (mode == MODE_DELTA_HEAD && gate_b) return launch_step<MODE_DELTA_HEAD>(a, segments, st);

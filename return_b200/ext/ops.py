@@ -1252,8 +1252,8 @@ def linear_scan(mode: int, q, k, v, gate_a, gate_b, state, offsets, batch, out, 
                 dim: int, vdim: int, q_scale: float = 1.0, cap: float = 0.0, forgot_offset: int = -1, extra=None,
                 below: int = 0, single: bool = False) -> None:
     """The recurrence of a mixer with a [dim, vdim] state per head, over every segment of the step, token by token
-    (``below`` > 0: over the segments of fewer tokens only).  ``single``: every segment has one token and the order of its sums
-    may differ from that of longer ones, which lets a kernel for such steps run.
+    (``below`` > 0: over the segments of fewer tokens only).  ``single``: every one of these segments has one token and the
+    order of its sums may differ from that of longer ones, which lets a kernel for single tokens run.
 
     q, k: [T, >= kv_heads * dim] views (float32 or bfloat16, unit stride along a row), v: [T, >= heads * vdim];
     ``state``: float32 [slots, n], the row of a segment is ``batch.seg_slot``; ``offsets`` = (S, n, m): where the

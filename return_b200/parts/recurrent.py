@@ -98,8 +98,8 @@ class _StateMixer(Mixer):
     CHUNKED_MIN_KEYS = 48
 
     def _chunks(self, mode, batch):
-        """None, or (chunks of the step's long segments, how many these are, whether there are short ones beside them).  Worked out
-        once per step and kind of scan."""
+        """None, or (chunks of the step's long segments, how many these are, how many tokens the longest of the others has: 0 if there
+        are none).  Worked out once per step and kind of scan."""
         host = getattr(batch, "host", None)
         if self.env.act_dtype == torch.float32 or host is None or not getattr(host, "num_multi", 0):
             return None
@@ -110,7 +110,7 @@ class _StateMixer(Mixer):
             return memo[key]
         lens = np.diff(host.cu_q).astype(np.int64)
         long = lens >= self.CHUNKED_MIN_TOKENS
-        plan = (int(((lens[long] + ops.CHUNK_TOKENS - 1) // ops.CHUNK_TOKENS).sum()), int(long.sum()), bool((~long).any())) if long.any() else None
+        plan = (int(((lens[long] + ops.CHUNK_TOKENS - 1) // ops.CHUNK_TOKENS).sum()), int(long.sum()), int(lens[~long].max(initial=0))) if long.any() else None
         if plan is not None and not ops.chunked_scan_ok(mode, self.H, self.D):
             plan = None
         counts = self._piece_counts(lens) if linear and plan is not None else None
@@ -127,12 +127,12 @@ class _StateMixer(Mixer):
         plan = self._chunks(mode, b)
         if plan is None:
             return False
-        chunks, longs, others = plan
+        chunks, longs, longest_other = plan
         ops.chunked_scan(mode, q, k, v, gate_a, gate_b, ctx.state, 0, b, chunks, self.CHUNKED_MIN_TOKENS, out, self.H, groups,
                          self.D, self.V, extra=extra, buffer=ctx.buffer, longs=longs)
-        if others:
+        if longest_other:                                   # decoded tokens beside the portions go through the kernel of a decode step
             ops.linear_scan(mode, q, k, v, gate_a, gate_b, ctx.state, (0, 0, 0), b, out, self.H, groups, self.D, self.V, extra=extra,
-                            below=self.CHUNKED_MIN_TOKENS)
+                            below=self.CHUNKED_MIN_TOKENS, single=longest_other == 1)
         return True
 
     def _scan(self, mode, q, k, v, decay, step, ctx, out, groups, extra, by_row):

@@ -92,10 +92,10 @@ def test_chunked_scan_is_launched_for_the_long_segments_alone(monkeypatch):
     seen = []
     monkeypatch.setattr(ops, "chunked_scan_ok", lambda mode, heads, dim: True)
     monkeypatch.setattr(ops, "chunked_scan", lambda mode, *a, **k: seen.append(("chunks", a[8], k["longs"])))
-    monkeypatch.setattr(ops, "linear_scan", lambda mode, *a, **k: seen.append(("walk", k["below"])))
+    monkeypatch.setattr(ops, "linear_scan", lambda mode, *a, **k: seen.append(("singles" if k["single"] else "walk", k["below"])))
     m = _state_mixer(16, 128, 128, torch.bfloat16)
     least = m.CHUNKED_MIN_TOKENS
-    for lens, want in (([1] * 64 + [200], [("chunks", 7, 1), ("walk", least)]), ([300, 1, least, least - 1], [("chunks", 10 + least // 32, 2), ("walk", least)]),
+    for lens, want in (([1] * 64 + [200], [("chunks", 7, 1), ("singles", least)]), ([300, 1, least, least - 1], [("chunks", 10 + least // 32, 2), ("walk", least)]),
                        ([least], [("chunks", least // 32, 1)]), ([1, least - 1], [])):
         seen.clear()
         batch = _scan_batch(lens)

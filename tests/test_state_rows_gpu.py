@@ -134,3 +134,37 @@ def test_scan_of_single_tokens(mode, n, H, G, D, V, off):
         outs = [(o, s[:, off:off + keep.numel()] * keep.reshape(-1)) for o, s in outs]
     bound = 2.0 ** -17 * (1 + float(state.abs().max()))       # 128 roundings of 2^-24 of sums of the size of the state
     assert all((x - y).abs().max() <= bound for x, y in zip(*outs))
+
+
+@pytest.mark.parametrize("mode", ["DECAY", "DELTA", "BONUS", "SSM", "DELTA_HEAD"])
+def test_single_tokens_beside_long_segments_get_the_same_bits(mode):
+    """A decoded token's output and state do not depend on whether a long portion shares its step."""
+    ops = _ops()
+    m, H, G, D, V = getattr(ops, "SCAN_" + mode), 4, 2, 72, 40
+    lens = [1, 1, 130, 1, 64, 1]
+    T, n = sum(lens), len(lens)
+    normal = lambda *s: torch.randn(*s, device=DEV)
+    q, k, v = normal(T, G * D) * D ** -0.5, torch.nn.functional.normalize(normal(T, G, D), dim=-1).reshape(T, -1), normal(T, H * V).bfloat16()
+    gate_a = torch.rand({"DECAY": (H,), "DELTA": (T, H * D), "BONUS": (T, H * D)}.get(mode, (T, H)), device=DEV)
+    gate_b = torch.rand(T, H, device=DEV) if mode in ("DELTA", "DELTA_HEAD", "SSM") else None
+    extra = normal(H, D) if mode == "BONUS" else normal(H) if mode == "SSM" else None
+    state = normal(n, H * D * V)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    slots = torch.arange(n - 1, -1, -1, dtype=torch.int32, device=DEV)
+
+    def run(tokens, cu, slots, below):
+        st, out = state.clone(), torch.full((len(tokens), H * V), 7.0, device=DEV)
+        pick = lambda x: None if x is None else x[tokens].contiguous()
+        batch = SimpleNamespace(cu_q=cu, seg_slot=slots, num_segments=len(slots))
+        ops.linear_scan(m, pick(q), pick(k), pick(v), gate_a if mode == "DECAY" else pick(gate_a), pick(gate_b), st, (0, 0, 0), batch, out,
+                        H, G, D, V, extra=extra, below=below, single=True)
+        return out, st
+
+    alone = [i for i, x in enumerate(lens) if x == 1]
+    rows = cu[:-1][alone].long()
+    out, st = run(torch.arange(T, device=DEV), cu, slots, 64)
+    one, st1 = run(rows, torch.arange(len(alone) + 1, dtype=torch.int32, device=DEV), slots[alone], 0)
+    assert torch.equal(out[rows], one) and torch.equal(st, st1)
+    others = torch.ones(T, dtype=torch.bool, device=DEV)
+    others[rows] = False
+    assert (out[others] == 7.0).all()                          # long segments are left alone, their states too (st1 has the old ones)
