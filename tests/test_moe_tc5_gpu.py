@@ -51,3 +51,23 @@ def test_moe_tc5_gated(runs, F, K, weighed):
     g, u = s[:, :F].clamp(max=1.5), s[:, F:].clamp(-1.5, 1.5)
     want = g * torch.sigmoid(1.702 * g) * (u + 1.0)
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -12).all()
+
+
+def test_moe_tc5_gated_unit_keeps_float32():
+    """The unit alone, of sums that are exact: rounded to bfloat16 it is the rounded 64-bit value but where that lies next to the middle
+    between two bfloat16 numbers.  Four float32 roundings of 2^-24 against a spacing of 2^-8 to 2^-7: one in some 4,000 at most; an exponential
+    that loses bits with the size of its argument would miss thirty times as many."""
+    from return_b200.ext import ops
+    F, K = 1024, 64
+    g = torch.Generator(device=DEV).manual_seed(0)
+    gate = (torch.rand(F, K, generator=g, device=DEV) * 67 - 60).bfloat16()
+    up = torch.randn(F, K, generator=g, device=DEV).bfloat16()
+    x, w = torch.eye(K, device=DEV).bfloat16(), torch.cat([gate, up])[None].contiguous()            # place k takes column k
+    out = torch.empty(K, F, dtype=torch.bfloat16, device=DEV)
+    ops.moe_tc5_gated(x, w, torch.tensor([0, K], dtype=torch.int32, device=DEV), out, 7.0, 1.0, 1.0)
+    ops.check_status(DEV)
+    a, b = gate.T.double().clamp(max=7.0), up.T.double().clamp(-7.0, 7.0)
+    want = a * torch.sigmoid(a) * (b + 1.0)
+    missed = (out != want.to(torch.bfloat16)).double().mean().item()
+    assert missed <= 1.0 / 4000, missed
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs()).all()
