@@ -20,9 +20,10 @@
 //
 // Every mbarrier wait is bounded; a wait that gives up raises *status and the kernel still frees its tensor memory.
 // Bound by the weights' and rows' way in: a pair's tile of 256 rows by 131 places loads half as many bytes an MMA again as one by 256,
-// and the weights (402 + 201 MB below) come from HBM.  Measured (8,192 pairs on 32 experts, H = 2,048, F = 1,536): 133 us gated and 79 us
-// down (the kernel with places as M, and a pass for the units: 199 and 22 us together); 400 pairs: 134 us for everything where mma.sync tiles
-// took 194.
+// and the weights (402 + 201 MB below) come from HBM.  Measured (8,192 pairs on 32 experts, H = 2,048, F = 1,536): 131 us gated and 59-70 us
+// down (the kernel with places as M, and a pass for the units: 199 and 22 us together).  With few and small tiles what counts is the set-up (the
+// pair's barrier stands in front of the wait for the kernels before this one) and the last tile's epilogue, which nothing hides: 1,024 pairs on 16 experts
+// of 1,024 x 768 take 57 us with everything around them, 61 before those two were looked at, 55 with places as M; 8,160 pairs 111, 118, 109.
 // Boxes of 64 places instead of 32 took 8 % longer; asking the weights into L2 4 / 10 / 20 stages ahead, by TMA or by a warp of
 // prefetches, 3 / 9 / 20 % and 2 / 6 / 28 % longer.
 #include <cuda.h>
@@ -138,6 +139,12 @@ __device__ __forceinline__ void turn_and_store(unsigned char* turn, const float 
     }
 }
 
+template <int ACT>
+__device__ __forceinline__ void activate_all(float (&v)[32]) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = rb_activate(ACT, v[j], nullptr, 0, 0);
+}
+
 // g sigmoid(alpha g) (u + shift) of the capped sums.  The quotient by 1 + exp(-alpha g) is a product with its reciprocal, put right by what
 // is left over (one step of Newton's method): off by no more than a rounding or two, for a fraction of a rounded division's instructions.
 __device__ __forceinline__ float gated(float g, float u, const Unit& unit) {
@@ -181,9 +188,11 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(&acc_full[b]), 1); mbar_init(smem_u32(&acc_empty[b]), 2 * 4 * SETS); }
         mbar_init_fence();
     }
+    fence_before_sync();
+    cluster_sync_all();                                     // both CTAs' barriers exist before either is signalled
+    fence_after_sync();
     pdl_wait();                                             // the offsets and the rows come from the kernels before
     for (int e = tid; e <= E; e += THREADS) s_off[e] = offsets[e];
-    fence_before_sync();
     __syncthreads();
     if (warp == 0) {                                        // first tile of every expert: sums over 32 experts at a time
         int run = 0;
@@ -202,8 +211,6 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (lane == 0) s_start[E] = run;
     }
     __syncthreads();
-    cluster_sync_all();                                     // both CTAs' barriers exist before either is signalled
-    fence_after_sync();
     const int total_m = s_start[E];
     const int tiles = total_m * ((N + TILE_N - 1) / TILE_N);
     const unsigned tacc = tmem_slot;
@@ -294,10 +301,11 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     // second 16-31; each hands the other its sums of the places that are not its own.
                     const bool up = q >= 2;
                     const int p0 = up ? 16 : 0;
-                    float c = 1.f;                          // lane j: what multiplies the sums of place j of the sixteen
-                    if (unit.weight != nullptr && lane < 16 && p0 + lane < left) {
-                        const int place = t.m0 + c0 + p0 + lane;
-                        c = unit.weight[unit.pair_at ? unit.pair_at[place] : place];
+                    if (unit.weight != nullptr) {           // lane j: what multiplies the sums of place j of the block
+                        const int place = t.m0 + c0 + lane;
+                        const float c = lane < left ? unit.weight[unit.pair_at ? unit.pair_at[place] : place] : 1.f;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__shfl_sync(0xffffffffu, c, j) * __uint_as_float(r[j]));
                     }
                     asm volatile("bar.sync %0, 64;" ::"r"(meet) : "memory");         // the partner is done with its inbox
 #pragma unroll
@@ -307,17 +315,19 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const float mine = __uint_as_float(r[up ? 16 + j : j]), other = inbox[j * 32 + lane];
-                        const float f = unit.weight != nullptr ? __shfl_sync(0xffffffffu, c, j) : 1.f;
-                        v[j] = gated(f * (up ? other : mine), f * (up ? mine : other), unit);
+                        v[j] = gated(up ? other : mine, up ? mine : other, unit);
                     }
                     if (cols > 0) turn_and_store<16>(turn, v, to + (size_t)p0 * ldo, ldo, left - p0, cols, vec, lane);
                 } else {
                     float v[32];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        v[j] = __uint_as_float(r[j]);
-                        if (act >= 0) v[j] = rb_activate(act, v[j], nullptr, 0, 0);
-                    }
+                    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+                    // one look at which activation it is: a look a sum put the code of all four between any two sums, and fetching it
+                    // cost 0.7 us a block even where there was none
+                    if (act == ACT_RELU2) activate_all<ACT_RELU2>(v);
+                    else if (act == ACT_TANH) activate_all<ACT_TANH>(v);
+                    else if (act == ACT_GELU_TANH) activate_all<ACT_GELU_TANH>(v);
+                    else if (act == ACT_SILU) activate_all<ACT_SILU>(v);
                     if (cols > 0) turn_and_store<32>(turn, v, to, ldo, left, cols, vec, lane);
                 }
             }
@@ -333,7 +343,6 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tacc), "r"(TMEM_COLS) : "memory");
 }
 
-// A map of rows of 64 elements in boxes of 64 rows, for a matrix that may have more rows than an int's worth of bytes.
 template <bool GATED>
 int launch(const void* A, int lda, const void* W, const int* offsets, int E, void* out, int ldo, int places, int N, int K, int act, int* status,
            const Unit& unit, cudaStream_t st) {
@@ -369,7 +378,7 @@ int launch(const void* A, int lda, const void* W, const int* offsets, int E, voi
     int dev = 0;
     cudaGetDevice(&dev);
     const long long n_tiles = (N + (GATED ? BM : 2 * BM) - 1) / (GATED ? BM : 2 * BM);
-    const long long worst = ((long long)places / 224 + E + 1) * n_tiles;     // a run's tiles are at least 225 places wide, but for the last two
+    const long long worst = ((long long)places / MAX_BN + E) * n_tiles;      // a run of n places has ceil(n / MAX_BN) tiles at most, none if it is empty
     const int resident = pairs_of_device[dev];
     cfg.gridDim = dim3(2 * (unsigned)(worst < resident ? worst : resident));
     cfg.stream = st;
