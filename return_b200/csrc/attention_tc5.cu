@@ -53,6 +53,8 @@
 // Measured (16 heads; 512 rows behind 7,680 keys, a prompt of 200, 61 rows behind 1,500): 65 us; every block in two
 // shares alike 86, one CTA a block 148.
 // *status is raised if a wait gave up.
+#include <initializer_list>
+
 #include "tc5.cuh"
 
 #ifndef HEAD_DIM
@@ -180,7 +182,8 @@ __device__ __forceinline__ int shares_of(int nt, int n_split, int share) {
     return share > 0 ? min(n_split, max(1, (nt + share - 1) / share)) : n_split;
 }
 
-template <bool MOD>
+// SPLIT: the keys of some block are split (an unsplit launch, which may be a few microseconds long, is spared fetching that code).
+template <bool MOD, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restrict__ kpool,
                         const bf16* __restrict__ vpool, const int* __restrict__ tiles,
@@ -225,9 +228,9 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     int na = min(p_last, p0 + QM - 1) / KN - jt_first + 1;
     int nb = m_rows > QM ? p_last / KN - jt_first + 1 : 0;
     int nt = max(na, nb);
-    const int n_split = shares_of(nt, gridDim.z, share), split = blockIdx.z;
+    const int n_split = SPLIT ? shares_of(nt, gridDim.z, share) : 1, split = SPLIT ? blockIdx.z : 0;
     if (split >= n_split) return;                         // a short block: fewer CTAs than the longest
-    if (n_split > 1) {                                    // this CTA's share of the block's key tiles; it may be empty
+    if (SPLIT && n_split > 1) {                                    // this CTA's share of the block's key tiles; it may be empty
         const int per = (nt + n_split - 1) / n_split;
         const int t0 = split * per;
         const int len = max(0, min(nt, t0 + per) - t0);
@@ -242,22 +245,13 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     const unsigned bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * i; };
 
-    // The rows go to shared memory and back a whole row by neighbouring lanes, so that an instruction touches whole lines (a lane
-    // a row, 16 bytes at a time, took 4.4 us for the queries and 1.5 us for the outputs of a CTA, whose key tiles take 1.1 us
-    // each; a prompt of 2,048 tokens, 32 heads of 128: 58.6 -> 52.3 us).
+    // Query rows of two lines go to shared memory a whole row by neighbouring lanes (a lane a row, 16 bytes at a time, asked for 32
+    // lines an instruction: 4.4 us of a CTA whose key tiles take 1.1 us each), and partial results of a split leave it likewise.  In a
+    // loop, behind the set-up, without a copy for rows that do not exist and with finished rows stored by the lanes that hold them: unrolled in
+    // front of the set-up, with finished rows turned round as well, a short prompt, which runs that code once, waited a microsecond longer for it.
+    // 50 tokens of 32 heads of 128: 6.2 us (unrolled 7.8, a lane a row 6.4); 2,048 tokens: 50-51 us (51, 57).
     constexpr int LPR = D / 8, RPI = 32 / LPR;            // lanes a row of 16-byte pieces, rows an instruction
     const int rsel = lane / LPR, sub = lane % LPR;
-    if (warp < 2 * 4) {
-        const int qt = warp >> 2;
-        const unsigned tile = smem_u32(sQ) + qt * Q_BYTES + (unsigned)(sub >> 3) * (QM * 128);
-#pragma unroll
-        for (int i = 0; i < 32 / RPI; ++i) {
-            const int r = (warp & 3) * 32 + i * RPI + rsel, grow = qt * QM + r;
-            const bool there = grow < m_rows;             // rows that do not exist are zero
-            cp_async16(tile + sw128_offset(r, sub & 7), there ? q + (size_t)(q_begin + row0 + grow) * ld + (size_t)h * D + sub * 8 : q, there);
-        }
-        cp_async_commit();
-    }
     if (warp == W_MMA) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
     if (tid == 0) {
         for (int i = 0; i < N_BARS; ++i)
@@ -267,6 +261,17 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
+    if (D > 64 && warp < 2 * 4 && (warp >> 2) * QM < m_rows) {      // a tile without rows has no products either
+        unsigned char* tile = sQ + (warp >> 2) * Q_BYTES + (unsigned)(sub >> 3) * (QM * 128);
+#pragma unroll 1
+        for (int i = 0; i < 32 / RPI; ++i) {
+            const int row = (warp & 3) * 32 + i * RPI + rsel, in_cta = (warp >> 2) * QM + row;
+            unsigned char* to = tile + sw128_offset(row, sub & 7);
+            if (in_cta < m_rows) cp_async16(smem_u32(to), q + (size_t)(q_begin + row0 + in_cta) * ld + (size_t)h * D + sub * 8, true);
+            else *reinterpret_cast<uint4*>(to) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        cp_async_commit();
+    }
     const unsigned tmem = *tmem_slot;
     bool ok = true;
 
@@ -293,7 +298,17 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
         const float* bias_row = (MOD && sm.bias) ? sm.bias + (size_t)h * sm.bias_n : nullptr;
         const float bias_last_l = (MOD && sm.bias) ? bias_row[sm.bias_n - 1] * LOG2E : 0.f;
         unsigned char* myPs = sP + qt * 2 * P_BYTES;           // this query tile's two P buffers
-        cp_async_wait<0>();                                  // the query rows, asked for before anything else
+        if (D == 64) {                                       // a row is one line: a lane a row
+            const bf16* qrow = q + (size_t)(q_begin + row0 + grow) * ld + (size_t)h * D;
+#pragma unroll
+            for (int c = 0; c < D / 8; ++c) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (row_valid) v = *reinterpret_cast<const uint4*>(qrow + c * 8);
+                *reinterpret_cast<uint4*>(sQ + qt * Q_BYTES + (c >> 3) * (QM * 128) + sw128_offset(r, c & 7)) = v;
+            }
+        } else {
+            cp_async_wait<0>();
+        }
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_Q_READY));
@@ -452,10 +467,10 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
             fence_after_sync();
         }
         const size_t token0 = (size_t)(q_begin + row0 + qt * QM);     // the query tile's first row
-        // Finished rows pass through the tile's P buffers, which no MMA reads any more, 16-byte piece p of row r at p ^ (r % 8).
-        auto row_at = [&](int row, int piece, int pieces) { return reinterpret_cast<uint4*>(myPs + row * (pieces * 16) + ((piece ^ (row & 7)) << 4)); };
-        if (n_split > 1) {
-            // one of several CTAs over this row's keys: O as it stands, with the reference maximum and the sum
+        if (SPLIT && n_split > 1) {
+            // one of several CTAs over this row's keys: O as it stands, with the reference maximum and the sum.  It passes through the
+            // tile's P buffers, which no MMA reads any more: 16-byte piece p of row r at p ^ (r % 8).
+            auto row_at = [&](int row, int piece) { return reinterpret_cast<uint4*>(myPs + row * 128 + ((piece ^ (row & 7)) << 4)); };
             if (row_valid) {
                 const size_t slot = ((size_t)split * total_rows + token0 + r) * Hq + h;
                 part_ml[2 * slot] = n_mine > 0 ? m_ref : -INFINITY;
@@ -469,42 +484,38 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
                     tmem_ld_wait();
                     __syncwarp();                            // the columns before these have been taken
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) *row_at(r, i, 8) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+                    for (int i = 0; i < 8; ++i) *row_at(r, i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int rr = (warp & 3) * 32 + i * 4 + (lane >> 3);
                         if (qt * QM + rr < m_rows)
-                            *reinterpret_cast<uint4*>(part_o + (((size_t)split * total_rows + token0 + rr) * Hq + h) * D + c0 + (lane & 7) * 4) = *row_at(rr, lane & 7, 8);
+                            *reinterpret_cast<uint4*>(part_o + (((size_t)split * total_rows + token0 + rr) * Hq + h) * D + c0 + (lane & 7) * 4) = *row_at(rr, lane & 7);
                     }
                 }
             }
         } else if (n_mine > 0) {
             // a sink: a term of the denominator that has no key and no value, not scaled
             const float inv = 1.f / (sink != nullptr ? l_run + exp2f(sink[h] * LOG2E - m_ref) : l_run);
+            bf16* orow = out + (token0 + r) * ((size_t)Hq * D) + (size_t)h * D;
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 32) {
                 unsigned o[32];
                 tmem_ld32(o_addr + c0, o);
                 tmem_ld_wait();
+                if (row_valid) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint4 v;
-                    __nv_bfloat162 a0 = __floats2bfloat162_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                    __nv_bfloat162 a1 = __floats2bfloat162_rn(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                    __nv_bfloat162 a2 = __floats2bfloat162_rn(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                    __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                    v.x = *reinterpret_cast<unsigned*>(&a0); v.y = *reinterpret_cast<unsigned*>(&a1);
-                    v.z = *reinterpret_cast<unsigned*>(&a2); v.w = *reinterpret_cast<unsigned*>(&a3);
-                    *row_at(r, (c0 + i) >> 3, LPR) = v;
+                    for (int i = 0; i < 32; i += 8) {
+                        uint4 v;
+                        __nv_bfloat162 a0 = __floats2bfloat162_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                        __nv_bfloat162 a1 = __floats2bfloat162_rn(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                        __nv_bfloat162 a2 = __floats2bfloat162_rn(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                        __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                        v.x = *reinterpret_cast<unsigned*>(&a0); v.y = *reinterpret_cast<unsigned*>(&a1);
+                        v.z = *reinterpret_cast<unsigned*>(&a2); v.w = *reinterpret_cast<unsigned*>(&a3);
+                        *reinterpret_cast<uint4*>(orow + c0 + i) = v;
+                    }
                 }
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 32 / RPI; ++i) {
-                const int rr = (warp & 3) * 32 + i * RPI + rsel;
-                if (qt * QM + rr < m_rows)
-                    *reinterpret_cast<uint4*>(out + (token0 + rr) * ((size_t)Hq * D) + (size_t)h * D + sub * 8) = *row_at(rr, sub, LPR);
             }
         }
     } else if (warp == W_MMA || warp == W_MMA_B) {
@@ -715,8 +726,10 @@ RB_EXPORT int rb_attn_prefill_tc5_mod(const void* q, int ld, const void* kpool, 
     if ((window > 0 && chunk > 0) || keep < 0 || (keep > 0 && window <= 0) || share < 0) return (int)cudaErrorInvalidValue;
     static PerDevice configured;
     const int rc = configured.once([](int) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {attn_prefill_tc5_kernel<false, false>, attn_prefill_tc5_kernel<false, true>, attn_prefill_tc5_kernel<true, false>,
+                            attn_prefill_tc5_kernel<true, true>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         return e;
     });
     if (rc != 0) return rc;
@@ -725,14 +738,12 @@ RB_EXPORT int rb_attn_prefill_tc5_mod(const void* q, int ld, const void* kpool, 
     dim3 grid(Hq, n_tiles, n_split);
     ScoreMod sm;
     sm.scale = scale; sm.softcap = softcap; sm.slopes = slopes; sm.chunk = chunk; sm.bias = bias; sm.bias_n = bias ? bias_n : 0; sm.keep = keep;
-    if (chunk > 0 || softcap > 0.f || slopes != nullptr || bias != nullptr || keep > 0)
-        attn_prefill_tc5_kernel<true><<<grid, THREADS, SMEM_BYTES, st>>>(
-            (const bf16*)q, ld, (const bf16*)kpool, (const bf16*)vpool, tiles, cu_q, seg_pos0, block_table, bt_stride,
-            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm, share);
-    else
-        attn_prefill_tc5_kernel<false><<<grid, THREADS, SMEM_BYTES, st>>>(
-            (const bf16*)q, ld, (const bf16*)kpool, (const bf16*)vpool, tiles, cu_q, seg_pos0, block_table, bt_stride,
-            page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm, share);
+    const bool mod = chunk > 0 || softcap > 0.f || slopes != nullptr || bias != nullptr || keep > 0;
+    auto kernel = mod ? (n_split > 1 ? attn_prefill_tc5_kernel<true, true> : attn_prefill_tc5_kernel<true, false>)
+                      : (n_split > 1 ? attn_prefill_tc5_kernel<false, true> : attn_prefill_tc5_kernel<false, false>);
+    kernel<<<grid, THREADS, SMEM_BYTES, st>>>(
+        (const bf16*)q, ld, (const bf16*)kpool, (const bf16*)vpool, tiles, cu_q, seg_pos0, block_table, bt_stride,
+        page_size, (bf16*)out, Hq, Hkv, scale * LOG2E, window, part_o, part_ml, total_rows, status, sink, sm, share);
     if (n_split > 1) {
         dim3 mgrid(Hq, n_tiles, NQ * QM / 8);
         merge_key_splits_kernel<<<mgrid, 256, 0, st>>>(part_o, part_ml, tiles, cu_q, seg_pos0, n_split, share, window, chunk, keep, total_rows, Hq,
