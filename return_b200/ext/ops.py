@@ -9,7 +9,6 @@ library (rollout/monkey_patch/qwen3.py:21-22,29-31,56).
 from __future__ import annotations
 
 import ctypes
-import heapq
 from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
@@ -776,42 +775,35 @@ def prefill_splits(n_ctas: int, longest_context: int) -> int:
 
 PREFILL_KEY_TILE = 64              # keys of a tile of the tcgen05 prefill attention kernel
 # What a CTA costs beside its key tiles (query rows in, tensor memory, the first scores, rows out) and what the merge of a split
-# costs, in key tiles of 1.1 us: measured 9 us and 4 us.
-PREFILL_CTA_TILES, PREFILL_MERGE_TILES = 8, 4
-PREFILL_SHARES_SLACK = 1.15          # over the average load; 400 random steps: at most 7 % worse a choice, 0.03 % on average (1.3: 19 and 0.5)
+# costs, in key tiles; the part of an average CTA that the last round of a launch runs on for, behind the SMs' average load; how
+# long a CTA has to be beside the longest to count as one that fills a round, and what those take of the longest on average; and how many
+# CTAs an SM there may be at most.  Fitted to 330 random steps (1 to 6 requests of up to 6,200 new tokens behind up to 10,500 cached ones,
+# 4 to 32 heads of 64 and 128), every split of each timed: the choice takes 0.4 % longer than the best split on average and 15 % at worst,
+# which is what a walk through the launch's CTAs gave (0.4 % and 14 %); unsplit 44 % and 6.8 times.  CTAs that find no share left to
+# take cost too little to count.
+PREFILL_CTA_TILES, PREFILL_MERGE_TILES, PREFILL_LAST_ROUND, PREFILL_LONG, PREFILL_ROUND, PREFILL_CTAS_PER_SM = 4, 6, 0.5, 0.75, 0.85, 2
 PREFILL_SPLIT_SCRATCH_BYTES = 64 << 20
-
-
-def _launch_tiles(work, heads: int, sms: int) -> int:
-    """When a launch is done whose CTAs, ``heads`` alike of every length in ``work`` in this order, go one by one to the SM that
-    is free first."""
-    free = [(0, sms)]                                  # (time, SMs that are free then), a heap
-    done = 0
-    for length in work:
-        need = heads
-        while need:
-            at, n = heapq.heappop(free)
-            took = min(n, need)
-            if n > took:
-                heapq.heappush(free, (at, n - took))
-            heapq.heappush(free, (at + length, took))
-            done = max(done, at + length)
-            need -= took
-    return done
 
 
 def prefill_shares(tiles, heads: int, rows: int, head_dim: int):
     """(CTAs that the longest block's keys are split over, key tiles of a CTA's share or 0 for no split) for blocks that walk
     ``tiles`` key tiles each, all ``heads`` alike, ``rows`` query rows in all.  Among splits of the longest block into s shares (of
     PREFILL_SPLIT_MIN_KEYS keys at least), with every other block cut into shares of about that size, the one whose launch is done
-    first (``_launch_tiles``; the kernel starts first shares of all blocks first, then second ones, ...).  The partial results of a
-    split stay under PREFILL_SPLIT_SCRATCH_BYTES."""
-    n, total, sms, longest = len(tiles), sum(tiles), num_sms(), max(tiles)
-    if n > 256:                                        # many blocks: whatever is uneven is short beside the rest
+    first.  A new step pays for this in host time, so it is a few sums over the blocks (4 to 40 us) and no walk through the launch (0.1 to
+    1 ms).  The partial results of a split stay under PREFILL_SPLIT_SCRATCH_BYTES."""
+    n, total, sms, longest = len(tiles), heads * sum(tiles), num_sms(), max(tiles)
+    if heads * n > PREFILL_CTAS_PER_SM * sms:          # more rounds: the CTAs' own cost grows, and it is long work anyway
         return 1, 0
-    at_once = longest + PREFILL_CTA_TILES
-    best, best_done = (1, 0), at_once if heads * n <= sms else _launch_tiles([t + PREFILL_CTA_TILES for t in tiles], heads, sms)
-    if best_done <= 1.25 * heads * (total + n * PREFILL_CTA_TILES) / sms:            # the blocks keep the SMs busy as they are
+
+    def done(ctas, long, top):
+        load = (total + ctas * PREFILL_CTA_TILES) / sms
+        if ctas <= sms:                                # one round
+            return max(top + PREFILL_CTA_TILES, load)
+        return max(top + PREFILL_CTA_TILES, load + PREFILL_LAST_ROUND * (total / ctas + PREFILL_CTA_TILES),
+                   -(-long // sms) * (PREFILL_ROUND * top + PREFILL_CTA_TILES))
+
+    best, best_done = (1, 0), done(heads * n, heads * sum([t >= PREFILL_LONG * longest for t in tiles]), longest)
+    if best_done <= 1.25 * (total + heads * n * PREFILL_CTA_TILES) / sms:            # the blocks keep the SMs busy as they are
         return best
     for s in (2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 32, 48, 64):
         share = -(-longest // s)
@@ -819,16 +811,10 @@ def prefill_shares(tiles, heads: int, rows: int, head_dim: int):
             break
         counts = [-(-t // share) for t in tiles]
         ctas = heads * sum(counts)
-        if ctas > 2 * sms:                             # more rounds: the CTAs' own cost grows, and it is long work anyway
+        if ctas > PREFILL_CTAS_PER_SM * sms:
             break
-        d = share + PREFILL_CTA_TILES + PREFILL_MERGE_TILES                 # all CTAs at once
-        if ctas > sms:
-            # the SMs' average load, which a launch of one round and a bit exceeds by a good part: where that cannot win, the
-            # walk through the launch (20 us of the host) is not worth it
-            if PREFILL_SHARES_SLACK * ((heads * total + ctas * PREFILL_CTA_TILES) / sms + PREFILL_MERGE_TILES) >= best_done:
-                continue
-            lengths = [-(-t // c) + PREFILL_CTA_TILES for t, c in zip(tiles, counts)]
-            d = _launch_tiles([t for z in range(max(counts)) for t, c in zip(lengths, counts) if c > z], heads, sms) + PREFILL_MERGE_TILES
+        long = heads * sum([c for t, c in zip(tiles, counts) if -(-t // c) >= PREFILL_LONG * share]) if ctas > sms else 0
+        d = done(ctas, long, share) + PREFILL_MERGE_TILES
         if d < best_done:
             best, best_done = (s, share), d
     return best
@@ -846,6 +832,8 @@ def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=
         longest = int(length[blocks[:, 0]].max())
         bound = keys_seen(window, keep) or chunk
         return prefill_splits(blocks.shape[0] * num_heads, min(longest, int(bound) + TC5_TILE_ROWS) if bound else longest), 0
+    if num_heads * blocks.shape[0] > PREFILL_CTAS_PER_SM * num_sms():  # (``prefill_shares`` says so too) no look at the blocks is needed
+        return 1, 0
     tiles = []
     first, length = host.seg_pos0.tolist(), length.tolist()
     for seg, row0 in blocks.tolist():

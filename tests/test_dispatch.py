@@ -66,6 +66,26 @@ def test_prefill_key_shares():
             assert got == len(walked)
 
 
+def test_prefill_key_shares_cost_little():
+    """A new step pays for the choice in host time: a few sums a candidate, however many blocks there are and however uneven."""
+    import random
+    import sys
+
+    from return_b200.ext import ops
+    ops.num_sms()
+    rng = random.Random(0)
+    for n, heads in ((4, 16), (12, 4), (16, 4), (64, 4), (128, 32), (256, 32)):
+        for _ in range(20):
+            tiles = sorted((int(2 ** rng.uniform(0, 9)) for _ in range(n)), reverse=True)
+            calls = []
+            sys.setprofile(lambda frame, event, arg: calls.append(event) if event in ("call", "c_call") else None)
+            try:
+                ops.prefill_shares(tiles, heads, 64 * n, 128)
+            finally:
+                sys.setprofile(None)
+            assert len(calls) <= 120, (n, heads, len(calls))
+
+
 def _state_mixer(H, D, V, dtype):
     from types import SimpleNamespace
     from return_b200.parts.recurrent import _StateMixer
