@@ -87,13 +87,15 @@ class _StateMixer(Mixer):
 
     # A segment of at least this many tokens goes through the scan 32 tokens at a time (bfloat16 path only: the sums then take
     # another order than token by token, which the float32 path never does).  Measured with 16 heads of 128 x 128 (delta rule with
-    # a decay per key row / fixed decay, us): 64 tokens 35 / 23 token by token, 31 / 27 in chunks (and a launch more); 96 tokens 49 / 31 and 33 / 28; 256 tokens 119 / 71 and 47 / 40;
-    # 2,048 tokens 900 / 515 and 219 / 150.
+    # a decay per key row / fixed decay, us): 64 tokens 35 / 23 token by token, 31 / 27 in chunks (and a launch more); 96 tokens 49 / 31
+    # and 33 / 28; 256 tokens 119 / 71 and 47 / 40; 2,048 tokens 900 / 515 and 219 / 150.  With 64 decoded tokens beside it a whole layer takes
+    # 150 / 107 with a portion of 100 token by token, 96 / 74 in chunks.
     CHUNKED_MIN_TOKENS = 96
-    # Where a segment can be cut into pieces that are scanned side by side instead, that wins with many pieces: k pieces of a
-    # segment of n tokens take 2 n / k tokens' time (0.25 us each) and 20 us, chunks n / 32 times 1.6 us, so the two meet at
-    # k = 10 (16 heads of 128 values give 4 pieces, 8 heads 9, 4 heads 16); and with few key rows, because a chunk's matrices
-    # are padded to 64 while a token's time falls with them.
+    # Where a segment can be cut into pieces that are scanned side by side instead, that wins with many of them: pieces divide the
+    # token-by-token time and chunks do not.  Measured on a whole retention (2 to 32 heads, keys of 16 to 128, values of 64 to 256,
+    # 1,024 to 4,096 tokens): 4 pieces take 1.65 to 2.9 times as long as chunks, 8 and 9 pieces 1.08 to 1.73 times, 16 to 32 pieces 0.41 to 1.07
+    # times; between 9 and 16 the two meet.  Keys below 48 keep the pieces wherever there are any, which is no gain (4 pieces of 16 heads of 32 x 128 and
+    # 2,048 tokens: 268 us, chunks 132); portions that are not cut go in chunks whatever their keys.
     CHUNKED_MAX_PIECES = 12
     CHUNKED_MIN_KEYS = 48
 

@@ -124,6 +124,24 @@ def test_chunked_scan_is_launched_for_the_long_segments_alone(monkeypatch):
         assert seen == want
 
 
+def test_which_scan_a_portion_takes(monkeypatch):
+    """Chunks from CHUNKED_MIN_TOKENS on, but where a linear scan can be cut into many pieces, or into any with few key rows."""
+    import torch
+    from return_b200.ext import ops
+    monkeypatch.setattr(ops, "num_sms", lambda: 148)
+    monkeypatch.setattr(ops, "chunked_scan_ok", lambda mode, heads, dim: mode != ops.SCAN_MEMORY and dim <= 128)
+    for H, D, V, mode, lens, pieces, chunks in (
+            (2, 24, 40, ops.SCAN_DECAY, [992], None, 31), (2, 24, 40, ops.SCAN_DECAY, [1, 1190], [1, 9], None), (2, 64, 40, ops.SCAN_DECAY, [1190], [9], 38),
+            (2, 64, 40, ops.SCAN_SSM, [2048], [16], None), (2, 64, 40, ops.SCAN_DELTA, [2048], [16], 64), (2, 24, 40, ops.SCAN_DELTA_HEAD, [1190], [9], 38),
+            (16, 128, 128, ops.SCAN_BONUS, [2048], [4], 64), (16, 32, 128, ops.SCAN_BONUS, [2048], [4], None), (16, 32, 256, ops.SCAN_BONUS, [2048], None, 64),
+            (16, 128, 128, ops.SCAN_DECAY, [95, 1], None, None), (16, 128, 128, ops.SCAN_DECAY, [96, 1], None, 3), (4, 200, 64, ops.SCAN_DECAY, [500], None, None)):
+        m, batch = _state_mixer(H, D, V, torch.bfloat16), _scan_batch(lens)
+        plan = m._chunks(mode, batch)
+        assert (plan and plan[0]) == chunks, (H, D, V, mode, lens, plan)
+        assert m._piece_counts(batch.host.cu_q[1:] - batch.host.cu_q[:-1]) == pieces
+        assert _state_mixer(H, D, V, torch.float32)._chunks(mode, _scan_batch(lens)) is None
+
+
 def test_experts_dispatch():
     from return_b200.ext import ops
     assert ops.moe_on_tc5(128, 16, 1024, 768) and not ops.moe_on_tc5(127, 16, 1024, 768)        # little weight: from 128 pairs on

@@ -682,6 +682,7 @@ def test_a_long_prompt_scanned_in_pieces_side_by_side(tmp_path_factory, monkeypa
     decoded afterwards start from, and a short request in the same step must all be right; the decays are slow, so a
     state handed on wrongly would show to the end.  The float32 path never cuts."""
     from return_b200.ext import ops
+    from return_b200.parts.recurrent import _StateMixer
     raw = config([wkv_layer(heads=2, dim=24, rank=4, mlp=None), ssm_layer(heads=3, vdim=16, state=24, groups=1, conv=3, norm_groups=1, mlp=None),
                   wkv_layer(heads=1, dim=40, rank=2, mlp=dense(32)), ssm_layer(heads=2, vdim=40, state=8, groups=2, conv=2, norm_groups=2, mlp=None)],
                  width=32, streams=2)
@@ -703,9 +704,16 @@ def test_a_long_prompt_scanned_in_pieces_side_by_side(tmp_path_factory, monkeypa
     assert calls == [True, False, True, False]                       # once a layer, in the step that holds the long portion
     assert_close(got["r0"][:1298], plain_rows(entry, long_ids)[:1298], "bfloat16", "long")
     assert_close(got["r1"], plain_rows(entry, short_ids), "bfloat16", "short")
-    one = run_trace(entry[0], "bfloat16", tail_decoded({"r0": long_ids[:1000]}, tail=8))
-    assert len(calls) == 4                                           # a portion of 992 tokens is walked in one go
-    assert_close(got["r0"][:1000], one["r0"], "bfloat16", "pieces against one walk")
+    # a portion of 992 tokens is not cut: it goes in chunks, or with these held off token by token
+    chunked, in_chunks = [], ops.chunked_scan
+    monkeypatch.setattr(ops, "chunked_scan", lambda *a, **k: (chunked.append(a[0]), in_chunks(*a, **k))[1])
+    for layers in (4, 0):
+        chunked.clear()
+        if not layers:
+            monkeypatch.setattr(_StateMixer, "CHUNKED_MIN_TOKENS", 1 << 30)
+        one = run_trace(entry[0], "bfloat16", tail_decoded({"r0": long_ids[:1000]}, tail=8))
+        assert len(calls) == 4 and len(chunked) == layers
+        assert_close(got["r0"][:1000], one["r0"], "bfloat16", "pieces against one walk" if not layers else "pieces against chunks")
     exact = run_trace(entry[0], "float32", steps)
     assert len(calls) == 4
     assert_close(exact["r0"][:1298], plain_rows(entry, long_ids)[:1298], "float32", "long")

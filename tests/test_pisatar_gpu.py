@@ -274,11 +274,16 @@ def test_long_decoding(tmp_path_factory, dtype, graph):
         assert_close(got[rid], plain_rows(entry, ids)[2:], dtype, rid)
 
 
-def test_a_long_prompt_scanned_in_pieces_side_by_side(tmp_path_factory):
+def test_a_long_prompt_scanned_in_pieces_side_by_side(tmp_path_factory, monkeypatch):
     """On the bfloat16 path a retention and a matrix memory cut a portion of 1,024 tokens or more into pieces that are
     scanned at the same time, hand the states from piece to piece and scan again.  The outputs of every piece, the state that the tokens
     decoded afterwards start from, and a short request in the same step must all be right; the decays are slow, so a
     state handed on wrongly would show to the end."""
+    from return_b200.ext import ops
+    from return_b200.parts.recurrent import _StateMixer
+    used = []
+    for name in ("chunked_scan", "scan_pieces_combine", "memory_pieces_combine"):
+        monkeypatch.setattr(ops, name, lambda *a, _f=getattr(ops, name), _n=name, **k: (used.append(_n), _f(*a, **k))[1])
     raw = config([retention_layer(heads=2, dim=24, vdim=40, rot=16, decay=[0.999, 0.9995]),
                   parallel_layer(heads=2, kv_heads=1, dim=16, vdim=16, rot=8, mem=(2, 16, 24), scales=(0.3, 1.0), cap=6.0),
                   retention_layer(heads=3, dim=16, vdim=16, rot=8, decay=[0.99, 0.999, 0.9999], ff=0)], width=32)
@@ -297,9 +302,16 @@ def test_a_long_prompt_scanned_in_pieces_side_by_side(tmp_path_factory):
     got = run_trace(entry[0], "bfloat16", steps)
     assert_close(got["r0"][:1298], plain_rows(entry, long_ids)[:1298], "bfloat16", "long")
     assert_close(got["r1"], plain_rows(entry, short_ids), "bfloat16", "short")
-    # the walk token by token and the walk in pieces agree to rounding
-    one = run_trace(entry[0], "bfloat16", tail_decoded({"r0": long_ids[:1000]}, tail=8))
-    assert_close(got["r0"][:1000], one["r0"], "bfloat16", "pieces against one walk")
+    assert used[-3:] == ["scan_pieces_combine", "memory_pieces_combine", "scan_pieces_combine"]     # a layer each, in the long portion's step
+    # the walk token by token, the walk in chunks and the walk in pieces agree to rounding: a portion of 992 tokens is not cut into
+    # pieces, and goes through the retentions in chunks unless these are held off
+    for chunks in (True, False):
+        used.clear()
+        if not chunks:
+            monkeypatch.setattr(_StateMixer, "CHUNKED_MIN_TOKENS", 1 << 30)
+        one = run_trace(entry[0], "bfloat16", tail_decoded({"r0": long_ids[:1000]}, tail=8))
+        assert used == ["chunked_scan"] * (2 if chunks else 0)
+        assert_close(got["r0"][:1000], one["r0"], "bfloat16", "pieces against one walk" if not chunks else "pieces against chunks")
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
