@@ -238,16 +238,25 @@ def kernel_attention_prefill(batch=1, ctx=2048, q_len=2048, heads=32, kv_heads=8
     """The prefill attention kernel alone: device time and TFLOP/s over the visible keys.
     ``window``, ``keep``, ``softcap``: the score options of ``ops.paged_attention`` (0: none).
     ``impl`` 0: the tcgen05 kernel (head sizes 64 and 128); 1: the mma.sync kernel.
-    ``splits``: ways the tcgen05 kernel splits the keys (0: the engine's choice for this many CTAs)."""
+    ``splits``: ways the tcgen05 kernel splits every block's keys (0: the engine's choice, which may give each block as many shares
+    as its context has)."""
+    import numpy as np
+
     from .ext import ops
     dev = torch.device("cuda:0")
     qkv, k_pool, v_pool, bt, cu_q, seg_pos0, _ = _paged_case(batch, ctx, q_len, heads, kv_heads, head_dim, page, dev)
     out = torch.empty((batch * q_len, heads * head_dim), dtype=torch.bfloat16, device=dev)
     rows = 64 if impl else ops.TC5_TILE_ROWS
-    tiles = torch.tensor([(i, r) for i in range(batch) for r in range(0, q_len, rows)], dtype=torch.int32, device=dev)
+    blocks = [(i, r) for i in range(batch) for r in range(0, q_len, rows)]
+    if not impl:
+        blocks.sort(key=lambda b: -b[1])               # the engine's order: the longest contexts first
+    tiles = torch.tensor(blocks, dtype=torch.int32, device=dev)
     kernel = ops.attention_prefill_mma if impl else ops.attention_prefill_tc5
-    splits = splits or ops.prefill_splits(int(tiles.shape[0]) * heads, ctx)
-    more = {} if impl else {"num_splits": splits, "held": {}}
+    share = 0
+    if not splits:
+        first, length = np.full(batch, ctx - q_len), np.full(batch, ctx)
+        splits, share = ops.prefill_block_shares(np.asarray(blocks), first, length, batch * q_len, heads, head_dim, window, 0, keep)
+    more = {} if impl else {"num_splits": splits, "share": share, "held": {}}
     fn = lambda: kernel(qkv, k_pool, v_pool, tiles, cu_q, seg_pos0, bt, page, out, heads,
                         kv_heads, head_dim, head_dim ** -0.5, window, softcap=softcap, keep=keep, **more)
     ms = _time_kernels([fn], iters, warmup)
@@ -256,7 +265,7 @@ def kernel_attention_prefill(batch=1, ctx=2048, q_len=2048, heads=32, kv_heads=8
         pairs = sum(min(p + 1, window + min(keep, max(0, p + 1 - window))) for p in range(ctx - q_len, ctx))
     flops = 4.0 * batch * heads * head_dim * pairs
     return {"kernel": "attention_prefill_mma" if impl else "attention_prefill_tc5", "batch": batch, "ctx": ctx, "q_len": q_len, "splits": 1 if impl else splits,
-            "ctas": int(tiles.shape[0]) * heads, "ms": ms, "TFLOPs": flops / ms / 1e9}
+            "share": 0 if impl else share, "ctas": int(tiles.shape[0]) * heads, "ms": ms, "TFLOPs": flops / ms / 1e9}
 
 
 def kernel_gemm(M=8, N=4096, K=4096, iters=10, warmup=3, out_f32=0, impl=0) -> Dict[str, float]:

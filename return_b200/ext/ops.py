@@ -820,29 +820,34 @@ def prefill_shares(tiles, heads: int, rows: int, head_dim: int):
     return best
 
 
-def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=0):
-    """``prefill_shares`` of this step's blocks, worked out once per step and kind of layer."""
-    held = getattr(batch, "scratch", None)
-    key = ("attention.prefill_shares", num_heads, head_dim, window, chunk, keep)
-    if held is not None and key in held:
-        return held[key]
-    host = batch.host
-    blocks, length = host.tiles[TILES_TC5], host.seg_kv_len
-    if not hasattr(host, "seg_pos0"):                  # a caller's own tables, without positions: every block in shares alike
-        longest = int(length[blocks[:, 0]].max())
-        bound = keys_seen(window, keep) or chunk
-        return prefill_splits(blocks.shape[0] * num_heads, min(longest, int(bound) + TC5_TILE_ROWS) if bound else longest), 0
-    if num_heads * blocks.shape[0] > PREFILL_CTAS_PER_SM * num_sms():  # (``prefill_shares`` says so too) no look at the blocks is needed
+def prefill_block_shares(blocks, seg_pos0, seg_kv_len, rows: int, heads: int, head_dim: int, window=None, chunk=None, keep=0):
+    """``prefill_shares`` of blocks [n, 2] = (segment, first row) of up to TC5_TILE_ROWS query rows (numpy arrays)."""
+    if heads * blocks.shape[0] > PREFILL_CTAS_PER_SM * num_sms():        # (``prefill_shares`` says so too) no look at the blocks is needed
         return 1, 0
     tiles = []
-    first, length = host.seg_pos0.tolist(), length.tolist()
+    first, length = seg_pos0.tolist(), seg_kv_len.tolist()
     for seg, row0 in blocks.tolist():
         p0 = first[seg] + row0
         end = min(length[seg], p0 + TC5_TILE_ROWS)
         low = max(0, p0 - window + 1) if window else p0 // chunk * chunk if chunk else 0
         kept = min(-(-keep // PREFILL_KEY_TILE), low // PREFILL_KEY_TILE) if window and keep else 0
         tiles.append((end - 1) // PREFILL_KEY_TILE - low // PREFILL_KEY_TILE + 1 + kept)
-    shares = prefill_shares(tiles, num_heads, host.num_tokens, head_dim)
+    return prefill_shares(tiles, heads, rows, head_dim)
+
+
+def prefill_shares_of(batch, num_heads, head_dim, window=None, chunk=None, keep=0):
+    """``prefill_block_shares`` of this step's blocks, worked out once per step and kind of layer."""
+    held = getattr(batch, "scratch", None)
+    key = ("attention.prefill_shares", num_heads, head_dim, window, chunk, keep)
+    if held is not None and key in held:
+        return held[key]
+    host = batch.host
+    blocks = host.tiles[TILES_TC5]
+    if not hasattr(host, "seg_pos0"):                  # a caller's own tables, without positions: every block in shares alike
+        longest = int(host.seg_kv_len[blocks[:, 0]].max())
+        bound = keys_seen(window, keep) or chunk
+        return prefill_splits(blocks.shape[0] * num_heads, min(longest, int(bound) + TC5_TILE_ROWS) if bound else longest), 0
+    shares = prefill_block_shares(blocks, host.seg_pos0, host.seg_kv_len, host.num_tokens, num_heads, head_dim, window, chunk, keep)
     if held is not None:
         held[key] = shares
     return shares
