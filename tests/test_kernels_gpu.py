@@ -346,6 +346,51 @@ def test_attention_prefill_tc5_shares(D, window, keep, softcap, share):
     assert torch.allclose(outs[1].float(), outs[0].float(), atol=2.0 ** -6, rtol=2.0 ** -6)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("chunk,window,keep,scores", [(96, 0, 0, ""), (256, 0, 0, "slopes"), (640, 0, 0, "bias"), (0, 0, 0, "slopes"), (0, 200, 65, "bias"), (0, 0, 0, "")])
+@pytest.mark.parametrize("share", [1, 3])
+def test_attention_prefill_tc5_shares_with_score_options(D, chunk, window, keep, scores, share):
+    """A sink, which a block of one share adds itself and the merge adds for the others, in launches that hold both kinds; blocks that
+    begin on both sides of a position block's edge; penalties and biases.  Partial results that a launch does not write are NaN."""
+    ops = _ops()
+    Hq, Hkv, P = 4, 2, 16
+    kv_lens, q_lens = [2, 64, 98, 700, 1000, 600], [2, 64, 5, 300, 70, 257]        # first positions 0, 0, 93, 400, 930, 343
+    pg = Paged(kv_lens, q_lens, Hq, Hkv, D, P, torch.bfloat16, seed=D + chunk)
+    g = torch.Generator().manual_seed(D)
+    sink = torch.randn(Hq, generator=g).to(DEV)
+    slopes = torch.rand(Hq, generator=g).mul(0.05).to(DEV) if scores == "slopes" else None
+    bias = torch.randn(Hq, 50, generator=g).to(DEV) if scores == "bias" else None
+    tiles = torch.tensor([(i, r0) for i, ql in enumerate(q_lens) for r0 in range(0, ql, ops.TC5_TILE_ROWS)], dtype=torch.int32, device=DEV)
+    outs = []
+    for splits, per in ((1, 0), (5, share)):
+        held = {}
+        for _ in range(2):
+            for name, t in held.items():
+                t.fill_(float("nan"))
+            outs.append(torch.full((sum(q_lens), Hq * D), float("nan"), device=DEV, dtype=torch.bfloat16))
+            ops.attention_prefill_tc5(pg.qkv, pg.kpool, pg.vpool, tiles, pg.cu_q, pg.seg_pos0, pg.bt, P, outs[-1], Hq, Hkv, D, D ** -0.5,
+                                      window, num_splits=splits, held=held, sink=sink, chunk=chunk, slopes=slopes, bias=bias, keep=keep, share=per)
+        assert torch.equal(outs[-1], outs[-2])
+    ops.check_status(DEV)
+    # probabilities are rounded to bfloat16 against another reference maximum, at most 2^-8 of a value either way
+    assert torch.allclose(outs[-1].float(), outs[0].float(), atol=2.0 ** -6, rtol=2.0 ** -6)
+    # and both against float32: scores of visible keys, with the sink as a term of the denominator
+    q, row = pg.qkv[:, :Hq * D].float().view(-1, Hq, D), 0
+    for i, (L, ql) in enumerate(zip(kv_lens, q_lens)):
+        k, v = (x[i].to(torch.bfloat16).float().to(DEV).repeat_interleave(Hq // Hkv, 1) for x in (pg.k, pg.v))
+        p, j = torch.arange(L - ql, L, device=DEV)[:, None], torch.arange(L, device=DEV)[None]
+        seen = (j <= p) & ((j >= p // chunk * chunk) if chunk else ((j > p - window) | (j < keep)) if window else torch.ones_like(j <= p))
+        s = torch.einsum("thd,jhd->htj", q[row:row + ql], k) * D ** -0.5
+        if slopes is not None:
+            s = s - slopes[:, None, None] * (p - j)
+        if bias is not None:
+            s = s + bias[:, (p - j).clamp(0, 49)]
+        s = torch.cat([s.masked_fill(~seen, float("-inf")), sink[:, None, None].expand(-1, ql, 1)], -1)
+        want = torch.einsum("htj,jhd->thd", s.softmax(-1)[..., :-1], v).reshape(ql, -1)
+        assert torch.allclose(outs[-1][row:row + ql].float(), want, atol=3e-2, rtol=3e-2), i
+        row += ql
+
+
 def test_prefill_split_choice():
     """Keys are split only while blocks x heads leave SMs idle and every share keeps enough keys."""
     ops = _ops()

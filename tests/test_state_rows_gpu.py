@@ -85,6 +85,31 @@ def test_delta_prep(dt, lens, H, G, D, V, K, head_decay):
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,D,V,K", [(4, 2, 8, 12, 4), (2, 1, 128, 256, 2)])
+def test_delta_prep_bits_do_not_depend_on_the_step(dt, H, G, D, V, K):
+    """Steps of 1,024 tokens and more take runs of tokens a warp: the same bits as a segment alone."""
+    ops = _ops()
+    lens, C = [531, 2, 600], 2 * G * D + H * V
+    T, n = sum(lens), len(lens)
+    x, taps = torch.randn(T, C, device=DEV).to(dt), torch.randn(C, K, device=DEV).to(dt)
+    a, b = torch.randn(T, H * D, device=DEV), torch.randn(T, H, device=DEV)
+    A_log, dt_bias = torch.randn(H, device=DEV).to(dt), torch.randn(H * D, device=DEV).to(dt)
+    state = torch.randn(n, C * (K - 1), device=DEV)
+
+    def run(segs):
+        rows = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in segs]).to(DEV)
+        sizes = torch.tensor([lens[i] for i in segs], device=DEV)
+        batch = SimpleNamespace(cu_q=torch.nn.functional.pad(sizes.cumsum(0), (1, 0)).to(torch.int32), seg_slot=torch.tensor(segs, dtype=torch.int32, device=DEV),
+                                tok_seg=torch.repeat_interleave(torch.arange(len(segs), device=DEV), sizes).to(torch.int32))
+        out = [torch.empty(len(rows), w, device=DEV) for w in (G * D, G * D, H * V)] + [a[rows], b[rows]]
+        ops.delta_prep(x[rows], taps, state, 0, batch, out[0], out[1], out[2], out[3], A_log, dt_bias, out[4], H, G, D, V, D ** -0.5)
+        return out
+
+    whole, apart = run([0, 1, 2]), [run([i]) for i in range(n)]
+    assert all(torch.equal(w, torch.cat(parts)) for w, parts in zip(whole, zip(*apart)))
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,D,V,K", [(4, 2, 8, 12, 4), (2, 1, 128, 256, 2), (2, 2, 36, 132, 1), (1, 1, 20, 4, 3)])
 def test_delta_prep_moves_conv_states_of_single_tokens(dt, H, G, D, V, K):
     """The same numbers as the two kernels one after the other, in both forms, with a slot of no request between."""
