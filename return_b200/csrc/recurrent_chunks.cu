@@ -48,12 +48,13 @@ struct ChunkArgs {
     int first, count;                                   // the window: these chunks of all segments' chunks, counted in order
 };
 
-// What a chunk leaves per head, in floats: q * P, k * P_32 / P_t, M, P_32, then (delta rules) k * P, T.  Matrices lie in the order of
+// What a chunk leaves per head, in floats: q * P, k * P_32 / P_t, M, P_32, eight marks (one a warp: whether anything is not an
+// ordinary number; 32 places, so that chunks lie on 128-byte boundaries), then (delta rules) k * P, T.  Matrices lie in the order of
 // m16n8k16's second operand: [block of 16 along the sum][block of 8 along the other side][lane][4], lane l holding column l / 4
 // and rows 2 (l % 4) + {0, 1, 8, 9}.
 template <int DP> struct Layout {
     static constexpr int X = CT * DP;
-    static constexpr int Q = 0, KS = X, M = 2 * X, G = 2 * X + CT * CT, KP = G + DP, T = KP + X, DELTA = T + CT * CT, PLAIN = KP;
+    static constexpr int Q = 0, KS = X, M = 2 * X, G = 2 * X + CT * CT, MARKS = G + DP, KP = MARKS + 32, T = KP + X, DELTA = T + CT * CT, PLAIN = KP;
 };
 
 template <int MODE> constexpr bool is_delta() { return MODE == CHUNK_DELTA || MODE == CHUNK_DELTA_HEAD; }
@@ -130,6 +131,12 @@ __device__ __forceinline__ Place find_chunk(const ChunkArgs& a, int c, int lane)
 }
 
 // ---------------------------------------------------------------- float32 products by three bfloat16 parts
+// Beyond this the leading part would be an infinity.  An infinity or a NaN has no parts, and multiplied with the zeros above a
+// triangle's diagonal it would reach the tokens before its own: chunks in which one turns up end the fast way (walk_tokens).
+constexpr float LARGEST = 3.38e38f;
+__device__ __forceinline__ bool ordinary(float x) { return fabsf(x) <= LARGEST; }
+__device__ __forceinline__ bool ordinary(const float4& x) { return ordinary(x.x) && ordinary(x.y) && ordinary(x.z) && ordinary(x.w); }
+
 struct Parts { unsigned h, m, l; };      // of two neighbouring elements: the first in the low half
 
 __device__ __forceinline__ unsigned pack2(float lo, float hi) {
@@ -438,6 +445,11 @@ chunk_prep_kernel(const ChunkArgs a) {
     }
     __syncthreads();
     float* to = a.scratch + ((size_t)blockIdx.x * H + h) * (DELTA ? L::DELTA : L::PLAIN);
+    bool fine = true;
+    auto leave = [&](int at, const float4& x) {
+        *(float4*)(to + at) = x;
+        fine = fine && ordinary(x);
+    };
     // ---- T by forward substitution (warp 0; a lane a column), the writes by the others
     if (DELTA && warp == 0) {
         float T[CT];
@@ -465,10 +477,10 @@ chunk_prep_kernel(const ChunkArgs a) {
             for (int b = 0; b < nt; ++b) { d[0] *= bd[b][i]; d[1] *= bd[b][i + 1]; d[2] *= bd[b][i + 8]; d[3] *= bd[b][i + 9]; }
             const float p[4] = {(float)d[0], (float)d[1], (float)d[2], (float)d[3]};
             const float* q = Qs + (8 * nt + r) * PITCH + i;
-            *(float4*)(to + L::Q + e * 128 + lane * 4) = make_float4(q[0] * p[0], q[1] * p[1], q[8] * p[2], q[9] * p[3]);
+            leave(L::Q + e * 128 + lane * 4, make_float4(q[0] * p[0], q[1] * p[1], q[8] * p[2], q[9] * p[3]));
             if (DELTA) {
                 const float* k = Ks + (8 * nt + r) * PITCH + i;
-                *(float4*)(to + L::KP + e * 128 + lane * 4) = make_float4(k[0] * p[0], k[1] * p[1], k[8] * p[2], k[9] * p[3]);
+                leave(L::KP + e * 128 + lane * 4, make_float4(k[0] * p[0], k[1] * p[1], k[8] * p[2], k[9] * p[3]));
             }
         }
         // ... over the tokens: k * P_32 / P_t
@@ -478,21 +490,27 @@ chunk_prep_kernel(const ChunkArgs a) {
             for (int b = 2 * kt + 2; b < 4; ++b) d *= bd[b][i];
             const float p1 = (float)d, p0 = (float)(d * bd[2 * kt + 1][i]);
             const float* k = Gs + t * PITCH + i;
-            *(float4*)(to + L::KS + e * 128 + lane * 4) = make_float4(k[0] * p0, k[PITCH] * p0, k[8 * PITCH] * p1, k[9 * PITCH] * p1);
+            leave(L::KS + e * 128 + lane * 4, make_float4(k[0] * p0, k[PITCH] * p0, k[8 * PITCH] * p1, k[9 * PITCH] * p1));
         }
         if (w0 == 0) {
-            for (int i = lane; i < DP; i += 32) to[L::G + i] = (float)(bd[0][i] * bd[1][i] * bd[2][i] * bd[3][i]);
+            for (int i = lane; i < DP; i += 32) {
+                const float g = (float)(bd[0][i] * bd[1][i] * bd[2][i] * bd[3][i]);
+                to[L::G + i] = g;
+                fine = fine && ordinary(g);
+            }
         }
         for (int e = w0; e < (CT / 16) * (CT / 8); e += ws) {
             const int kt = e / (CT / 8), t = 8 * (e % (CT / 8)) + r, s = 16 * kt + c2;
-            *(float4*)(to + L::M + e * 128 + lane * 4) = make_float4(Mm[t][s], Mm[t][s + 1], Mm[t][s + 8], Mm[t][s + 9]);
+            leave(L::M + e * 128 + lane * 4, make_float4(Mm[t][s], Mm[t][s + 1], Mm[t][s + 8], Mm[t][s + 9]));
         }
     }
     if (DELTA) {
         __syncthreads();
         const int kt = warp / (CT / 8), t = 8 * (warp % (CT / 8)) + (lane >> 2), s = 16 * kt + 2 * (lane & 3);
-        *(float4*)(to + L::T + warp * 128 + lane * 4) = make_float4(Tm[t][s], Tm[t][s + 1], Tm[t][s + 8], Tm[t][s + 9]);
+        leave(L::T + warp * 128 + lane * 4, make_float4(Tm[t][s], Tm[t][s + 1], Tm[t][s + 8], Tm[t][s + 9]));
     }
+    const bool marked = __any_sync(0xffffffffu, !fine);
+    if (lane == 0) to[L::MARKS + warp] = marked ? 1.f : 0.f;
     pdl_trigger_late();
 }
 
@@ -520,6 +538,90 @@ template <int DP, bool DELTA> constexpr size_t serial_smem() {
     return (size_t)STAGES * (DELTA ? Layout<DP>::DELTA : Layout<DP>::PLAIN) * 4      // chunks
            + (size_t)(DELTA ? 2 : 1) * (DP / 16) * 512 * 4                           // parts of the sums over the key rows
            + (size_t)(DP / 16 + 2 + 4) * 384 * 4;                                    // the state, v - (k * P) S0 and U (of two chunks) in three parts
+}
+
+// Tokens t0 .. t0 + n - 1 one by one, by the CTA that keeps the state S (two rows of two columns a thread, laid out as in
+// chunk_serial_kernel): what is left of a segment from the chunk on in which an infinity or a NaN turns up, so that it reaches
+// the tokens and columns that it reaches in recurrent.cu, and no others.  `sums`: 48 floats a warp.
+template <int MODE, int DP>
+__device__ __noinline__ float4 walk_tokens(const ChunkArgs& a, int t0, int n, int h, int col, float4 S4, float* sums) {
+    constexpr bool DELTA = is_delta<MODE>(), ROWS = MODE == CHUNK_DELTA || MODE == CHUNK_BONUS;
+    constexpr int WARPS = serial_warps<DP>();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c8 = lane >> 2, i0 = 8 * warp + 2 * (lane & 3);
+    const int H = a.H, D = a.D, V = a.V, kvh = h / (H / a.G);
+    float S[4] = {S4.x, S4.y, S4.z, S4.w};
+    const bool ok[2] = {col < V, col + 8 < V}, row[2] = {i0 < D, i0 + 1 < D};
+    auto quad = [](float x) {
+        x += __shfl_xor_sync(0xffffffffu, x, 1);
+        return x + __shfl_xor_sync(0xffffffffu, x, 2);
+    };
+    // the sums over a column's rows: this warp's, left in shared memory; then (behind a barrier) all warps'
+    auto put_sums = [&](float* to, float x, float y) {
+        x = quad(x);
+        y = quad(y);
+        if ((lane & 3) == 0) { to[warp * 16 + c8] = x; to[warp * 16 + 8 + c8] = y; }
+    };
+    auto all_of = [&](const float* from, int c) {
+        float x = 0.f;
+        for (int w = 0; w < WARPS; ++w) x += from[w * 16 + 8 * c + c8];
+        return x;
+    };
+    __syncthreads();                                     // nobody reads what lay here before
+    for (int i = 0; i < n; ++i) {
+        const size_t t = (size_t)(t0 + i);
+        float k[2], q[2], g[2], w[2], v[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            k[r] = row[r] ? ld_elem(a.k, a.k_f32, t * a.k_ld + (size_t)kvh * D + i0 + r) : 0.f;
+            q[r] = row[r] ? ld_elem(a.q, a.q_f32, t * a.q_ld + (size_t)kvh * D + i0 + r) * a.q_scale : 0.f;
+            g[r] = !row[r] ? 1.f : MODE == CHUNK_DECAY ? a.gate_a[h] : ROWS ? a.gate_a[(t * H + h) * D + i0 + r] : a.gate_a[t * H + h];
+            w[r] = MODE == CHUNK_BONUS && row[r] ? a.extra[(size_t)h * D + i0 + r] : 0.f;
+            v[r] = ok[r] ? ld_elem(a.v, a.v_f32, t * a.v_ld + (size_t)h * V + col + 8 * r) : 0.f;
+        }
+        float u[2] = {v[0], v[1]}, o[2] = {0.f, 0.f};
+        if (DELTA) {
+            float p[2] = {0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    S[2 * c + r] *= g[r];
+                    if (row[r]) p[c] = fmaf(S[2 * c + r], k[r], p[c]);
+                }
+            put_sums(sums, p[0], p[1]);
+            __syncthreads();
+            const float beta = a.gate_b[t * H + h];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) u[c] = beta * (v[c] - all_of(sums, c));
+        } else if (MODE == CHUNK_SSM) {
+            const float step = a.gate_b[t * H + h];
+            u[0] *= step;
+            u[1] *= step;
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                if (!row[r]) continue;
+                float& s = S[2 * c + r];
+                if (MODE == CHUNK_BONUS) o[c] = fmaf(fmaf(w[r], k[r] * u[c], s), q[r], o[c]);
+                s = DELTA ? fmaf(k[r], u[c], s) : fmaf(g[r], s, k[r] * u[c]);
+                if (MODE != CHUNK_BONUS) o[c] = fmaf(s, q[r], o[c]);
+            }
+        float* mine = sums + (1 + (i & 1)) * 16 * WARPS;
+        put_sums(mine, o[0], o[1]);
+        __syncthreads();
+        if (warp == 0 && (lane & 3) == 0) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float x = all_of(mine, c);
+                if (MODE == CHUNK_SSM) x = fmaf(a.extra[h], v[c], x);
+                if (ok[c]) a.out[(t * H + h) * V + col + 8 * c] = x;
+            }
+        }
+    }
+    __syncthreads();
+    return make_float4(S[0], S[1], S[2], S[3]);
 }
 
 template <int MODE, int DP>
@@ -639,11 +741,18 @@ chunk_serial_kernel(const ChunkArgs a) {
     };
     bool ok = true;
 
-    for (int c = 0; c < chunks; ++c) {
+    int c = 0;
+    for (; c < chunks; ++c) {
         ok = tc5::mbar_wait(tc5::smem_u32(&full[c % STAGES]), (c / STAGES) & 1) && ok;
         __syncthreads();                                 // the state's parts are there; nobody is in chunk c - 1
         fetch(c + 2);
         const float* X = stages + (c % STAGES) * PER;
+        const float4 mark0 = *reinterpret_cast<const float4*>(X + L::MARKS), mark1 = *reinterpret_cast<const float4*>(X + L::MARKS + 4);
+        bool odd = (mark0.x + mark0.y) + (mark0.z + mark0.w) + ((mark1.x + mark1.y) + (mark1.z + mark1.w)) != 0.f;
+        if (!DELTA) {                                    // (the delta rules' U shows it)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) odd = odd || !ordinary(S[i]);
+        }
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -671,10 +780,13 @@ chunk_serial_kernel(const ChunkArgs a) {
                                                         big[nt][3] + small[nt][3]);
         }
         if (!DELTA && right) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) odd = odd || !ordinary(v[i]);
             if (PAIRED) put_half(Up + (c & 1) * 768, rb, rc, rc ? v[2] : v[0], rc ? v[3] : v[1]);
             else put(Up + (c & 1) * 768, rb, v);
         }
-        __syncthreads();
+        if (DELTA) __syncthreads();
+        else odd = __syncthreads_or(odd);
         if (output) {
             if (c > 0) finish(c - 1);
             const float* from = part + (DELTA ? KT * 512 : 0) + ob * 128 + lane * 4;
@@ -717,9 +829,12 @@ chunk_serial_kernel(const ChunkArgs a) {
                 two_blocks(x, X + L::T + warp * 128, 512, lane);
                 mma6_alone(u, Rp, x, (warp >> 1) + 1, lane);
                 put(Up + (c & 1) * 768, warp, u);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) odd = odd || !ordinary(u[i]);
             }
+            odd = __syncthreads_or(odd);
         }
-        if (DELTA) __syncthreads();
+        if (odd) break;                                  // (all threads alike) the state is still the one before this chunk
         // ---- the state behind the chunk, eight rows; it is added to on the CUDA cores, which round to nearest
         {
             const float2 g = *(const float2*)(X + L::G + 8 * warp + 2 * (lane & 3));
@@ -732,7 +847,15 @@ chunk_serial_kernel(const ChunkArgs a) {
             put(Sp, warp, S);
         }
     }
-    if (output) finish(chunks - 1);
+    if (c == chunks) {
+        if (output) finish(chunks - 1);
+    } else {
+        for (int d = c + 1; d < min(c + 3, chunks); ++d)               // copies on their way
+            ok = tc5::mbar_wait(tc5::smem_u32(&full[d % STAGES]), (d / STAGES) & 1) && ok;
+        const int t0 = t_first + (c_begin + c) * CT;
+        const float4 s4 = walk_tokens<MODE, DP>(a, t0, min(t_end, t_first + c_end * CT) - t0, h, col, make_float4(S[0], S[1], S[2], S[3]), part);
+        S[0] = s4.x; S[1] = s4.y; S[2] = s4.z; S[3] = s4.w;
+    }
     if (!ok) atomicExch(a.status, 1);
     pdl_trigger_late();
     if (in0) { home[0] = S[0]; home[1] = S[1]; }

@@ -144,3 +144,65 @@ def test_long_segments_are_found(lens):
         else:                                                  # the same sums of up to 64 + 32 terms in another order
             assert torch.allclose(outs[0][0][a:b], walked[a:b], rtol=2.0 ** -18, atol=2.0 ** -18 * float(walked.abs().max()))
             assert torch.allclose(outs[0][1][slot], st[slot], rtol=2.0 ** -18, atol=2.0 ** -18 * float(st.abs().max()))
+
+
+@pytest.mark.parametrize("mode", ["DECAY", "DELTA", "BONUS", "SSM", "DELTA_HEAD"])
+@pytest.mark.parametrize("D,V", [(24, 40), (128, 16)])
+@pytest.mark.parametrize("where,what", [("v", "inf"), ("v", "nan"), ("v", "3.4e38"), ("k", "nan"), ("k", "inf"), ("q", "nan"), ("gate_a", "nan"),
+                                        ("gate_b", "inf"), ("state", "-inf"), ("state", "nan")])
+def test_infinities_and_nans_reach_what_they_reach_token_by_token(mode, D, V, where, what):
+    """An infinity, a NaN or a number beyond bfloat16's largest, in one token and head: no token before it, no other head or request
+    and (in a value or a state) no other column sees it, and the tokens behind it hold infinities and NaNs where the walk has them."""
+    ops = _ops()
+    m, x = getattr(ops, "SCAN_" + mode), float(what)
+    delta = mode.startswith("DELTA")
+    if where == "gate_b" and not (delta or mode == "SSM") or where == "gate_a" and mode == "DECAY":
+        pytest.skip("no such operand")
+    lens, H, G, at = [70, 100, 40], 4, 2, 70 + 43                # the 12th token of the second segment's second chunk
+    T, n = sum(lens), len(lens)
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    normal = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    q, k, v = normal(T, G * D) * D ** -0.5, torch.nn.functional.normalize(normal(T, G, D), dim=-1).reshape(T, -1), normal(T, H * V)
+    shape = {"DECAY": (H,), "DELTA": (T, H * D), "BONUS": (T, H * D)}.get(mode, (T, H))
+    gate_a = torch.rand(*shape, generator=gen, device=DEV)
+    gate_b = torch.rand(T, H, generator=gen, device=DEV) if delta or mode == "SSM" else None
+    extra = normal(H, D) if mode == "BONUS" else normal(H) if mode == "SSM" else None
+    state = normal(n, H * D * V) * 0.3
+    head = 3                                                     # the head of values, gates and state; its queries and keys are the second group's
+    if where == "v":
+        v[at, head * V + 5] = x
+    elif where == "state":
+        state[1, head * D * V + (0 * V + 5) * 8 + 2] = x         # a row of column 5
+    elif where in ("k", "q"):
+        {"k": k, "q": q}[where][at, 1 * D + 9] = x
+    elif where == "gate_b":
+        gate_b[at, head] = x
+    else:
+        gate_a[at, head * (gate_a.shape[1] // H)] = x
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    batch = SimpleNamespace(cu_q=cu, num_segments=n, seg_slot=torch.arange(n, dtype=torch.int32, device=DEV))
+    outs = []
+    for chunks in (False, True):
+        st, out = state.clone(), torch.zeros(T, H * V, device=DEV)
+        if chunks:
+            ops.chunked_scan(m, q, k, v, gate_a, gate_b, st, 0, batch, 9, 1, out, H, G, D, V, extra=extra, longs=n)
+        else:
+            ops.linear_scan(m, q, k, v, gate_a, gate_b, st, (0, 0, 0), batch, out, H, G, D, V, extra=extra)
+        outs.append((out, st))
+    ops.check_status(DEV)
+    # a column's sums are of terms of its own size, in another order
+    columns = [lambda y: y.view(T, H * V).amax(0).expand(T, -1), lambda y: y.view(n, H, D // 8, V, 8).amax((2, 4), keepdim=True).expand(n, H, D // 8, V, 8).reshape(n, -1)]
+    for walked, got, size in zip(outs[0], outs[1], columns):
+        plain = walked.isfinite()
+        assert torch.equal(got.isnan(), walked.isnan()) and torch.equal(got[walked.isinf()], walked[walked.isinf()])
+        bound = 2.0 ** -17 * (1.0 + size(torch.where(plain, walked.abs(), torch.zeros_like(walked))))
+        assert ((got - walked).abs() <= bound)[plain].all()
+    out = outs[1][0]
+    first = 70 if where == "state" else at
+    assert out[:first].isfinite().all() and out[170:].isfinite().all()       # the tokens before, and the third request
+    if where in ("v", "state"):
+        others = torch.ones(H * V, dtype=torch.bool, device=DEV)
+        others[head * V + 5] = False
+        assert out[:, others].isfinite().all()
+    if what != "3.4e38":
+        assert not out[first:170].isfinite().all()
