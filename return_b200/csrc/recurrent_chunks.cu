@@ -132,7 +132,7 @@ __device__ __forceinline__ Place find_chunk(const ChunkArgs& a, int c, int lane)
 
 // ---------------------------------------------------------------- float32 products by three bfloat16 parts
 // Beyond this the leading part would be an infinity.  An infinity or a NaN has no parts, and multiplied with the zeros above a
-// triangle's diagonal it would reach the tokens before its own: chunks in which one turns up end the fast way (walk_tokens).
+// triangle's diagonal it would reach the tokens before its own: chunks in which one turns up make a segment take the slow way (walk_tokens).
 constexpr float LARGEST = 3.38e38f;
 __device__ __forceinline__ bool ordinary(float x) { return fabsf(x) <= LARGEST; }
 __device__ __forceinline__ bool ordinary(const float4& x) { return ordinary(x.x) && ordinary(x.y) && ordinary(x.z) && ordinary(x.w); }
@@ -525,6 +525,8 @@ chunk_prep_kernel(const ChunkArgs a) {
 // the matrix instructions alone would be 0.75 us a chunk), 1.6 us of the others (102 us).  With cp.async by all threads in the place of the
 // bulk copies and the outputs finished in their own chunk: 187 and 128 us; with eight warps instead of sixteen and the values'
 // conversion behind their load: 167 and 184.  The first kernel takes 60 and 42 us there; token by token it was 893 and 508.
+// Whether everything was an ordinary number is looked at once, behind the last chunk: 2 % of a layer (309.6 us a delta-rule layer of 2,048 tokens,
+// 303.7 without; at every chunk's barrier 314.4).
 constexpr int STAGES = 3;
 
 __device__ __forceinline__ void bulk_copy(unsigned smem, const float* gmem, unsigned bytes, unsigned bar) {
@@ -541,7 +543,7 @@ template <int DP, bool DELTA> constexpr size_t serial_smem() {
 }
 
 // Tokens t0 .. t0 + n - 1 one by one, by the CTA that keeps the state S (two rows of two columns a thread, laid out as in
-// chunk_serial_kernel): what is left of a segment from the chunk on in which an infinity or a NaN turns up, so that it reaches
+// chunk_serial_kernel): a segment in which an infinity or a NaN turned up, once more from the state that it began with, so that it reaches
 // the tokens and columns that it reaches in recurrent.cu, and no others.  `sums`: 48 floats a warp.
 template <int MODE, int DP>
 __device__ __noinline__ float4 walk_tokens(const ChunkArgs& a, int t0, int n, int h, int col, float4 S4, float* sums) {
@@ -739,20 +741,15 @@ chunk_serial_kernel(const ChunkArgs a) {
             if (ok1) o[(size_t)H * V + 8] = own[3];
         }
     };
-    bool ok = true;
+    bool ok = true, odd = false;                         // odd: something was no ordinary number
 
-    int c = 0;
-    for (; c < chunks; ++c) {
+    for (int c = 0; c < chunks; ++c) {
         ok = tc5::mbar_wait(tc5::smem_u32(&full[c % STAGES]), (c / STAGES) & 1) && ok;
         __syncthreads();                                 // the state's parts are there; nobody is in chunk c - 1
         fetch(c + 2);
         const float* X = stages + (c % STAGES) * PER;
-        const float4 mark0 = *reinterpret_cast<const float4*>(X + L::MARKS), mark1 = *reinterpret_cast<const float4*>(X + L::MARKS + 4);
-        bool odd = (mark0.x + mark0.y) + (mark0.z + mark0.w) + ((mark1.x + mark1.y) + (mark1.z + mark1.w)) != 0.f;
-        if (!DELTA) {                                    // (the delta rules' U shows it)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) odd = odd || !ordinary(S[i]);
-        }
+        if (tid < 8) odd = odd || X[L::MARKS + tid] != 0.f;
+        if (!DELTA) odd = odd || !(ordinary(S[0]) && ordinary(S[1]) && ordinary(S[2]) && ordinary(S[3]));          // (the delta rules' U shows it)
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -780,13 +777,11 @@ chunk_serial_kernel(const ChunkArgs a) {
                                                         big[nt][3] + small[nt][3]);
         }
         if (!DELTA && right) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) odd = odd || !ordinary(v[i]);
+            odd = odd || !(ordinary(v[0]) && ordinary(v[1]) && ordinary(v[2]) && ordinary(v[3]));
             if (PAIRED) put_half(Up + (c & 1) * 768, rb, rc, rc ? v[2] : v[0], rc ? v[3] : v[1]);
             else put(Up + (c & 1) * 768, rb, v);
         }
-        if (DELTA) __syncthreads();
-        else odd = __syncthreads_or(odd);
+        __syncthreads();
         if (output) {
             if (c > 0) finish(c - 1);
             const float* from = part + (DELTA ? KT * 512 : 0) + ob * 128 + lane * 4;
@@ -829,12 +824,10 @@ chunk_serial_kernel(const ChunkArgs a) {
                 two_blocks(x, X + L::T + warp * 128, 512, lane);
                 mma6_alone(u, Rp, x, (warp >> 1) + 1, lane);
                 put(Up + (c & 1) * 768, warp, u);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) odd = odd || !ordinary(u[i]);
+                odd = odd || !(ordinary(u[0]) && ordinary(u[1]) && ordinary(u[2]) && ordinary(u[3]));
             }
-            odd = __syncthreads_or(odd);
+            __syncthreads();
         }
-        if (odd) break;                                  // (all threads alike) the state is still the one before this chunk
         // ---- the state behind the chunk, eight rows; it is added to on the CUDA cores, which round to nearest
         {
             const float2 g = *(const float2*)(X + L::G + 8 * warp + 2 * (lane & 3));
@@ -847,13 +840,12 @@ chunk_serial_kernel(const ChunkArgs a) {
             put(Sp, warp, S);
         }
     }
-    if (c == chunks) {
-        if (output) finish(chunks - 1);
-    } else {
-        for (int d = c + 1; d < min(c + 3, chunks); ++d)               // copies on their way
-            ok = tc5::mbar_wait(tc5::smem_u32(&full[d % STAGES]), (d / STAGES) & 1) && ok;
-        const int t0 = t_first + (c_begin + c) * CT;
-        const float4 s4 = walk_tokens<MODE, DP>(a, t0, min(t_end, t_first + c_end * CT) - t0, h, col, make_float4(S[0], S[1], S[2], S[3]), part);
+    if (output) finish(chunks - 1);
+    // Looked at once, behind the last chunk: the slot still holds the state before the first, and every output is written again.
+    if (__syncthreads_or(odd)) {
+        const int t0 = t_first + c_begin * CT;
+        const float4 s4 = walk_tokens<MODE, DP>(a, t0, min(t_end, t_first + c_end * CT) - t0, h, col,
+                                                make_float4(in0 ? home[0] : 0.f, in0 ? home[1] : 0.f, in1 ? home[64] : 0.f, in1 ? home[65] : 0.f), part);
         S[0] = s4.x; S[1] = s4.y; S[2] = s4.z; S[3] = s4.w;
     }
     if (!ok) atomicExch(a.status, 1);
