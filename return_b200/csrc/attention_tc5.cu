@@ -246,10 +246,10 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
     auto bar = [&](int i) { return bar0 + 8u * i; };
 
     // Query rows of two lines go to shared memory a whole row by neighbouring lanes (a lane a row, 16 bytes at a time, asked for 32
-    // lines an instruction: 4.4 us of a CTA whose key tiles take 1.1 us each), and partial results of a split leave it likewise.  In a
-    // loop, behind the set-up, without a copy for rows that do not exist and with finished rows stored by the lanes that hold them: unrolled in
-    // front of the set-up, with finished rows turned round as well, a short prompt, which runs that code once, waited a microsecond longer for it.
-    // 50 tokens of 32 heads of 128: 6.2 us (unrolled 7.8, a lane a row 6.4); 2,048 tokens: 50-51 us (51, 57).
+    // lines an instruction: 4.4 us of a CTA whose key tiles take 1.1 us each), and a full tile's finished rows and the partial results of a
+    // split leave it likewise.  In loops, behind the set-up, without a copy for rows that do not exist and with the rows of a part of a tile stored by
+    // the lanes that hold them: unrolled in front of the set-up, and with every row turned round, a short prompt, which runs that code once, waited a
+    // microsecond longer for it.  50 tokens of 32 heads of 128: 6.2-6.5 us (unrolled 7.8, a lane a row 6.4); 2,048 tokens: 49.6 us (50.7, 57.4).
     constexpr int LPR = D / 8, RPI = 32 / LPR;            // lanes a row of 16-byte pieces, rows an instruction
     const int rsel = lane / LPR, sub = lane % LPR;
     if (warp == W_MMA) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
@@ -497,7 +497,11 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
         } else if (n_mine > 0) {
             // a sink: a term of the denominator that has no key and no value, not scaled
             const float inv = 1.f / (sink != nullptr ? l_run + exp2f(sink[h] * LOG2E - m_ref) : l_run);
+            // A full tile's rows of two lines are turned round through the tile's P buffers, which no MMA reads any more (16-byte piece p of
+            // row r at p ^ (r % 8)), and leave whole, by neighbouring lanes; the rows of a part leave from the lanes that hold them.
+            const bool turned = D > 64 && full_tile;
             bf16* orow = out + (token0 + r) * ((size_t)Hq * D) + (size_t)h * D;
+            auto row_at = [&](int row, int piece) { return reinterpret_cast<uint4*>(myPs + row * (D * 2) + ((piece ^ (row & 7)) << 4)); };
 #pragma unroll 1
             for (int c0 = 0; c0 < D; c0 += 32) {
                 unsigned o[32];
@@ -513,8 +517,16 @@ attn_prefill_tc5_kernel(const bf16* __restrict__ q, int ld, const bf16* __restri
                         __nv_bfloat162 a3 = __floats2bfloat162_rn(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
                         v.x = *reinterpret_cast<unsigned*>(&a0); v.y = *reinterpret_cast<unsigned*>(&a1);
                         v.z = *reinterpret_cast<unsigned*>(&a2); v.w = *reinterpret_cast<unsigned*>(&a3);
-                        *reinterpret_cast<uint4*>(orow + c0 + i) = v;
+                        *(turned ? row_at(r, (c0 + i) >> 3) : reinterpret_cast<uint4*>(orow + c0 + i)) = v;
                     }
+                }
+            }
+            if (turned) {
+                __syncwarp();
+#pragma unroll 4
+                for (int i = 0; i < 32 / RPI; ++i) {
+                    const int rr = (warp & 3) * 32 + i * RPI + rsel;
+                    *reinterpret_cast<uint4*>(out + (token0 + rr) * ((size_t)Hq * D) + (size_t)h * D + sub * 8) = *row_at(rr, sub);
                 }
             }
         }
