@@ -89,7 +89,7 @@ def core() -> ctypes.CDLL:
         lib.rb_rmsnorm_rows_ld.argtypes = [P, I, P, I, F, F, P, I, I, I, I, P]
         lib.rb_rmsnorm_rows_ld.restype = c_int
         lib.rb_swiglu.argtypes = [P, P, I, I, I, I, I, P]
-        lib.rb_gemm_f32.argtypes = [P, P, P, I, I, I, I, I, I, I, P]
+        lib.rb_gemm_f32.argtypes = [P, P, P, I, I, I, I, I, I, I, P, P]
         lib.rb_gemm_skinny.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P]
         lib.rb_gemm_skinny.restype = c_int
         lib.rb_gemm_skinny_act.argtypes = [P, P, P, I, I, P, I, I, I, I, I, I, I, P]
@@ -307,15 +307,17 @@ def softcap(x: torch.Tensor, cap: float) -> None:
 # ------------------------------------------------------------------------------- matrix products
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int = -1) -> None:
-    """out[M, N] = x[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K).  ``kind``: 0-3 one size of tile, 4 the
-    kernel for up to 4 rows, -1 the one that suits the sizes; all give the same bits."""
+    """out[M, N] = x[M, K] @ w[N, K]^T in float32's precision (operands split into three bfloat16 parts each, tensor cores; fixed
+    order over K).  ``kind``: 0-11 one shape of tile and split, -1 the one that suits the sizes; all give the same bits."""
     M, K = x.shape
     N = w.shape[0]
     assert x.dtype == w.dtype == out.dtype == torch.float32
     assert w.shape[1] == K and out.shape == (M, N)
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
-    _check(core().rb_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                              kind, _stream()), "gemm_f32")
+    rc = core().rb_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                            kind, _ptr(tc5_status(x.device)), _stream())
+    _tc5_launched.add(x.device)
+    _check(rc, "gemm_f32")
 
 
 SKINNY_KERNEL_MAX_ROWS = 32     # what the kernel takes
@@ -571,7 +573,7 @@ def gemm_tc5_bmn(x: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int = 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[str] = None,
            bias: Optional[torch.Tensor] = None) -> None:
-    """out = x @ w^T.  float32: the engine's own FFMA kernel.  bfloat16 with up to 8 rows: the
+    """out = x @ w^T.  float32: the engine's own kernel in that precision.  bfloat16 with up to 8 rows: the
     engine's weight-streaming kernel.  bfloat16 with more rows: cuBLAS with float32 accumulation.
     The output is bfloat16 or float32 (``out``'s dtype).  ``act``: out = f(x @ w^T) for one of ``ACTIVATIONS``
     (``bias``: its bias per column): in the weight-streaming kernel's epilogue, else a launch of its own in place."""

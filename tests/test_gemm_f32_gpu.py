@@ -1,0 +1,80 @@
+"""The float32 product's shapes at the edges of its tiles, runs and groups, and what numbers without parts do."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _ops():
+    from return_b200.ext import ops
+    return ops
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (16, 129, 65), (17, 1, 511), (64, 127, 512), (65, 128, 576), (80, 256, 1024), (81, 130, 1088), (163, 384, 260),
+                                   (257, 128, 3072)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_every_shape_gives_the_same_bits(M, N, K, offset):
+    """K around whole blocks of 64, runs of two and four groups of them; M around the tiles' widths.  Three of nine products are left out (each at
+    most 2^-24 of its term), a run of 128 values is cut off and not rounded (at most 8 + 5 times 2^-23 of its terms' sizes), and
+    the sums of runs and groups round once each."""
+    ops = _ops()
+    torch.manual_seed(M * 7 + K)
+    wide = torch.randn(M + N, K + 3, device=DEV)
+    x, w = wide[:M, offset:offset + K], wide[M:, offset:offset + K]
+    if offset == 0 and K % 4 == 0:
+        x, w = x.contiguous(), w.contiguous()
+    outs = []
+    for kind in range(-1, 12):
+        outs.append(torch.full((M, N), float("nan"), device=DEV))
+        ops.gemm_f32(x, w, outs[-1], kind=kind)
+        assert torch.equal(outs[-1], outs[0]), kind
+    ops.check_status(x.device)
+    exact = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    roundings = 3 * 2.0 ** -24 + 13 * 2.0 ** -23 + (K / 128 + 4) * 2.0 ** -24
+    assert ((outs[0].double() - exact).abs() <= size * roundings).all()
+
+
+def test_error_is_below_a_chain_of_multiply_adds():
+    ops = _ops()
+    torch.manual_seed(5)
+    x, w = torch.randn(33, 1024, device=DEV), torch.randn(200, 1024, device=DEV)
+    out = torch.empty(33, 200, device=DEV)
+    ops.gemm_f32(x, w, out)
+    exact = x.double() @ w.double().T
+    acc = torch.zeros(33, 200, device=DEV)
+    for k in range(1024):                                     # float32(float64 product + sum): one rounding, as fused
+        acc = (acc.double() + x[:, k:k + 1].double() * w[:, k].double()).float()
+    assert (out.double() - exact).norm() < (acc.double() - exact).norm()
+
+
+@pytest.mark.parametrize("kind", [-1, 0, 4, 8, 11])
+def test_numbers_without_parts(kind):
+    """Infinities, NaNs and numbers next to the largest: their rows and columns hold what a chain of float32 products and sums
+    holds, and nothing else changes."""
+    ops = _ops()
+    torch.manual_seed(3)
+    M, N, K = 40, 140, 320
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    plain = torch.empty(M, N, device=DEV)
+    ops.gemm_f32(x, w, plain, kind=kind)
+    inf, big = float("inf"), 3.4e38
+    x[3, 17], x[7, 100], x[9, 5], x[11, 64] = inf, float("nan"), -inf, big
+    w[64, 3], w[139, 200], w[2, 64] = -inf, float("nan"), 0.25
+    w[5, 17] = 0.0                                            # inf * 0
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_f32(x, w, out, kind=kind)
+    rows, cols = [3, 7, 9, 11], [64, 139]
+    keep_r = [i for i in range(M) if i not in rows]
+    keep_c = [i for i in range(N) if i not in cols and i not in (2, 5)]
+    assert torch.equal(out[keep_r][:, keep_c], plain[keep_r][:, keep_c])
+    want = x.double() @ w.double().T                          # (3.4e38 times a normal weight may pass float32's range)
+    for r in rows:
+        far = want[r].abs() > 3.4028235e38
+        want[r] = torch.where(far & want[r].isfinite(), torch.copysign(torch.full_like(want[r], inf), want[r]), want[r])
+    got = out.double()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+    fine = want.isfinite()
+    assert ((got - want).abs()[fine] <= 1e-4 * want.abs()[fine] + 1e-3).all()
