@@ -439,6 +439,9 @@ def gated_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, interleave
     if interleave == 8 and x.shape[0] >= PAIR_MIN_ROWS and pair_ok(x, w, out):
         gemm_tc5(x, w, out, gated=True, pair=True, act=act)
         return
+    if interleave == 8 and w.shape[0] % 16 == 0 and out.dtype == torch.bfloat16 and rows_ok(x, w):
+        gemm_rows(x, w, out, gated=True, act=act)
+        return
     if ctx is not None:
         gu = ctx.buffer("gated_linear.gate_up", (x.shape[0], w.shape[0]), x.dtype, x.device)
     else:
@@ -448,7 +451,7 @@ def gated_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, interleave
 
 
 _tc5 = None
-_TC5_SOURCES = ["gemm_tc5.cu", "gemm_stream.cu"]
+_TC5_SOURCES = ["gemm_tc5.cu", "gemm_stream.cu", "gemm_rows.cu"]
 
 
 def _tc5_defines():
@@ -470,6 +473,8 @@ def tc5_lib() -> ctypes.CDLL:
         lib.rb_tc5_gemm_pair.restype = c_int
         lib.rb_tc5_gemm_simple.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm_bmn.argtypes = [P, P, P, I, I, I, I, I, I, I, P, P]
+        lib.rb_gemm_rows.argtypes = [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P]
+        lib.rb_gemm_rows.restype = c_int
         lib.rb_tc5_gemm.restype = lib.rb_tc5_gemm_simple.restype = lib.rb_tc5_gemm_bmn.restype = c_int
         _tc5 = build.native_calls(lib)
     return _tc5
@@ -571,10 +576,50 @@ def gemm_tc5_bmn(x: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int = 
                                      _ptr(tc5_status(x.device)), _stream()), "gemm_tc5_bmn")
 
 
+# Where the kernel for the rows of an ordinary step is the fastest way.  As kernels alone the library's are 5-25 % faster from some 30 rows on
+# (512 x 6,144 x 1,024 8.2 us against 9.9, 64 x 2,048 x 2,048 5.7 and 6.0), but a launch through torch takes the host 10 us against
+# 3 and does not overlap the kernel before it: up to this much work the step gains (a step of 512 tokens through six layers of 1,024
+# 1,038 -> 874 us; a captured one of 16 tokens 283 -> 267, of 64 387 -> 381; feed-forwards of 1,024 x 3,072 28.8 -> 19.0), above it loses
+# (600 rows of 2,048 x 6,144: 46.8 -> 53.1), and so with more weights to stream (64 tokens through layers of 4,096: 318 -> 333), but for few rows of
+# long sums: with K at least twice N the weight tiles are few, and K is cut over a cluster (64 x 4,096 x 12,288 21.7 -> 20.4).
+ROWS_MAX_WORK = 3300 << 20
+ROWS_MAX_WEIGHTS = 1 << 24
+ROWS_LONG_SUMS = 128
+
+
+def rows_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether the kernel for the rows of an ordinary step takes this product and is the fastest way."""
+    M, K = x.shape
+    N = w.shape[0]
+    if x.dtype != torch.bfloat16 or M * N * K > ROWS_MAX_WORK and not (M <= ROWS_LONG_SUMS and K >= 2 * N):
+        return False
+    return ((N * K <= ROWS_MAX_WEIGHTS or M <= ROWS_LONG_SUMS and K >= 2 * N) and K % 8 == 0
+            and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False, act: Optional[str] = None, tiles: int = -1,
+              log2_split: int = -1) -> None:
+    """out[M, N] = x[M, K] @ w[N, K]^T in bfloat16 for the rows of an ordinary step: tcgen05, weight rows as the M side, K cut over
+    the CTAs of a cluster.  ``gated``: w holds gate and up rows woven in blocks of 8, out [M, N/2] = act(gate) * up with ``act`` one of
+    ``GATES`` (None: silu); otherwise ``act``: one of ``ACTIVATIONS`` on the float32 sums.  ``tiles``, ``log2_split``: how many tiles M
+    falls into and the CTAs that share K (-1: what suits the sizes)."""
+    M, K = x.shape
+    N = w.shape[0]
+    assert x.dtype == w.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32)
+    assert w.shape[1] == K and out.shape == (M, N // 2 if gated else N)
+    assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
+    rc = tc5_lib().rb_gemm_rows(_ptr(x), _ptr(w), _ptr(out), 1 if out.dtype == torch.float32 else 0, _gated_code(gated, act or "silu"),
+                                ACTIVATIONS[act] if act is not None and not gated else -1, M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                                tiles, log2_split, _ptr(tc5_status(x.device)), _stream())
+    _tc5_launched.add(x.device)
+    _check(rc, "gemm_rows")
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[str] = None,
            bias: Optional[torch.Tensor] = None) -> None:
     """out = x @ w^T.  float32: the engine's own kernel in that precision.  bfloat16 with up to 8 rows: the
-    engine's weight-streaming kernel.  bfloat16 with more rows: cuBLAS with float32 accumulation.
+    engine's weight-streaming kernel; with more rows the tcgen05 kernel ``gemm_rows`` where that is faster (``rows_ok``), else cuBLAS;
+    float32 accumulation everywhere.
     The output is bfloat16 or float32 (``out``'s dtype).  ``act``: out = f(x @ w^T) for one of ``ACTIVATIONS``
     (``bias``: its bias per column): in the weight-streaming kernel's epilogue, else a launch of its own in place."""
     if x.dtype == torch.float32:
@@ -587,6 +632,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[st
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
     if skinny_ok(x, w):
         gemm_skinny(x, w, out, act=act, bias=bias)
+        return
+    if act != "neg_exp_exp" and rows_ok(x, w):
+        gemm_rows(x, w, out, act=act)
         return
     if out.dtype == torch.float32:
         torch.mm(x, w.t(), out_dtype=torch.float32, out=out)

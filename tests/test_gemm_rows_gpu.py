@@ -1,0 +1,80 @@
+"""The product for the rows of an ordinary step at the edges of its tiles, stages and shares of K."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _ops():
+    from return_b200.ext import ops
+    return ops
+
+
+def _inputs(M, N, K, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.empty(M, K + 8, device=DEV).normal_(generator=g).bfloat16()[:, :K]          # rows apart by more than their length
+    w = torch.empty(N, K, device=DEV).normal_(std=0.05, generator=g).bfloat16()
+    return x, w, x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+
+
+def _close(got, exact, size, K, scale=1.0):
+    """float32 sums of K products (K / 16 of them cut off), and one rounding to the output's type."""
+    unit = 2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -24
+    assert ((got.double() - exact).abs() <= scale * (exact.abs() * unit + size * (K / 16 + 4) * 2.0 ** -23)).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 16, 8), (16, 128, 64), (17, 129, 128), (33, 96, 136), (64, 257, 192), (130, 384, 320), (255, 130, 1024), (257, 200, 512),
+                                   (513, 64, 2048)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_tiles_and_shares(M, N, K, f32):
+    ops = _ops()
+    x, w, exact, size = _inputs(M, N, K, M + K)
+    wide = torch.full((M, N + 24), 7.0, device=DEV, dtype=torch.float32 if f32 else torch.bfloat16)
+    least = (M + 255) // 256
+    for tiles, ls in [(-1, -1)] + [(t, l) for t in (least, least + 1, least + 3) for l in (0, 1, 2)]:
+        for shift in (0, 1):                                  # output rows of whole 16-byte pieces, and not
+            wide.fill_(7.0)
+            out = wide[:, 8 + shift:8 + shift + N]
+            ops.gemm_rows(x, w, out, tiles=tiles, log2_split=ls)
+            _close(out, exact, size, K)
+            assert (wide[:, :8 + shift] == 7.0).all() and (wide[:, 8 + shift + N:] == 7.0).all()
+    ops.check_status(x.device)
+
+
+@pytest.mark.parametrize("gate", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("M,N,K", [(9, 32, 64), (100, 272, 320), (300, 512, 1024)])
+def test_gated_unit(M, N, K, gate):
+    ops = _ops()
+    x, w, exact, size = _inputs(M, N, K, M)
+    g, u = exact.view(M, -1, 2, 8).unbind(2)
+    a = g * torch.sigmoid(g) if gate == "silu" else torch.nn.functional.gelu(g, approximate="tanh")
+    want = (a * u).reshape(M, N // 2)
+    bound = size.view(M, -1, 2, 8).amax(2).reshape(M, N // 2) * (1 + exact.abs().view(M, -1, 2, 8).amax(2).reshape(M, N // 2))
+    for ls in (-1, 0, 2):
+        out = torch.full((M, N // 2), float("nan"), device=DEV, dtype=torch.bfloat16)
+        ops.gemm_rows(x, w, out, gated=True, act=gate, tiles=-1 if ls < 0 else (M + 255) // 256, log2_split=ls)
+        _close(out, want, bound, K, 2.5)                      # (the unit's slope is at most 1.13 times the other factor, of each of the two sums)
+    ops.check_status(x.device)
+
+
+@pytest.mark.parametrize("act", ["relu2", "tanh", "gelu_tanh", "silu"])
+def test_activation_on_the_sums(act):
+    ops = _ops()
+    x, w, exact, _ = _inputs(70, 136, 256, 4)
+    f = {"relu2": lambda v: torch.relu(v) ** 2, "tanh": torch.tanh, "silu": lambda v: v * torch.sigmoid(v),
+         "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act]
+    out = torch.empty(70, 136, device=DEV, dtype=torch.bfloat16)
+    ops.linear(x, w, out, act=act)
+    want = f(exact)
+    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+    ops.check_status(x.device)
+
+
+def test_what_the_kernel_does_not_take_goes_to_the_library():
+    ops = _ops()
+    x, w, exact, size = _inputs(40, 100, 100, 5)              # K is no multiple of eight
+    assert not ops.rows_ok(x, w)
+    out = torch.empty(40, 100, device=DEV, dtype=torch.bfloat16)
+    ops.linear(x, w, out)
+    _close(out, exact, size, 100)
