@@ -277,7 +277,7 @@ __device__ __forceinline__ void load_rows(float* to, const void* p, int f32, int
 }
 
 template <int MODE, int DP>
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(THREADS, 3)
 chunk_prep_kernel(const ChunkArgs a) {
     using L = Layout<DP>;
     constexpr bool DELTA = is_delta<MODE>();
@@ -698,30 +698,49 @@ chunk_serial_kernel(const ChunkArgs a) {
     // who takes v - (k * P) S0 or v (block rb of 8 tokens; with PAIRED column rc of the two), and who the outputs (block ob)
     const bool right = warp < WARPS / 2, output = warp >= WARPS - 4;
     const int rb = PAIRED ? warp >> 1 : warp, rc = PAIRED ? warp & 1 : 0, ob = warp - (WARPS - 4);
-    // values of a chunk, asked for a chunk ahead: tokens ta, ta + 1 of col, then of col + 8.  The loaded bits stay as they are until
-    // they are used: a conversion right behind a load would make the warp wait for it there.
-    unsigned v_next[4];
+    // Values of a chunk, asked for a chunk ahead: tokens ta, ta + 1 of col, then of col + 8, by the warps that need them (what is not
+    // there stays zero).  The loaded bits stay as they are until they are used: a conversion right behind a load would make the warp
+    // wait for it there.
+    unsigned v_next[4] = {0u, 0u, 0u, 0u};
     float step_next[2] = {0.f, 0.f};
-    auto raw = [&](size_t i) -> unsigned { return a.v_f32 ? ((const unsigned*)a.v)[i] : (unsigned)((const unsigned short*)a.v)[i]; };
-    auto values = [&](int c) {
-        const bool mine = (right || (MODE == CHUNK_SSM && output)) && c < chunks;
-        const int ta = t_first + (c_begin + c) * CT + 8 * (right ? rb : ob) + 2 * (lane & 3);
-        const bool l0 = mine && ta < t_end, l1 = mine && ta + 1 < t_end, c0 = ok0 && !(PAIRED && right && rc), c1 = ok1 && !(PAIRED && right && !rc);
-        const size_t at = (size_t)ta * a.v_ld + (size_t)h * V + col;
-        v_next[0] = l0 && c0 ? raw(at) : 0u;
-        v_next[1] = l1 && c0 ? raw(at + a.v_ld) : 0u;
-        v_next[2] = l0 && c1 ? raw(at + 8) : 0u;
-        v_next[3] = l1 && c1 ? raw(at + a.v_ld + 8) : 0u;
-        if (MODE == CHUNK_SSM && right) {
-            step_next[0] = l0 ? a.gate_b[(size_t)ta * H + h] : 0.f;
-            step_next[1] = l1 ? a.gate_b[(size_t)(ta + 1) * H + h] : 0.f;
+    const bool has_values = right || (MODE == CHUNK_SSM && output);
+    const bool c0 = ok0 && !(PAIRED && right && rc), c1 = ok1 && !(PAIRED && right && !rc);
+    int t_next = t_first + c_begin * CT + 8 * (right ? rb : ob) + 2 * (lane & 3);
+    const int t_stop = min(t_end, t_first + c_end * CT);
+    const char* v_at = (const char*)a.v + ((size_t)t_next * a.v_ld + (size_t)h * V + col) * (a.v_f32 ? 4 : 2);
+    const size_t v_row = (size_t)a.v_ld * (a.v_f32 ? 4 : 2);
+    auto values = [&]() {
+        if (!has_values) return;
+        const bool l0 = t_next < t_stop, l1 = t_next + 1 < t_stop;
+        if (a.v_f32) {
+            const unsigned* p = (const unsigned*)v_at;
+            const unsigned* n = (const unsigned*)(v_at + v_row);
+            v_next[0] = l0 && c0 ? p[0] : 0u;
+            v_next[1] = l1 && c0 ? n[0] : 0u;
+            v_next[2] = l0 && c1 ? p[8] : 0u;
+            v_next[3] = l1 && c1 ? n[8] : 0u;
+        } else {
+            const unsigned short* p = (const unsigned short*)v_at;
+            const unsigned short* n = (const unsigned short*)(v_at + v_row);
+            v_next[0] = l0 && c0 ? p[0] : 0u;
+            v_next[1] = l1 && c0 ? n[0] : 0u;
+            v_next[2] = l0 && c1 ? p[8] : 0u;
+            v_next[3] = l1 && c1 ? n[8] : 0u;
         }
+        if (MODE == CHUNK_SSM && right) {
+            step_next[0] = l0 ? a.gate_b[(size_t)t_next * H + h] : 0.f;
+            step_next[1] = l1 ? a.gate_b[(size_t)(t_next + 1) * H + h] : 0.f;
+        }
+        t_next += CT;
+        v_at += CT * v_row;
     };
-    values(0);
+    values();
     // A chunk's outputs are finished while the next one's U is made, by warps that have nothing to do with that: they keep
-    // (q * P) S0, their rows of M and (for the skip) the values.
+    // (q * P) S0, their rows of M and (for the skip) the values.  An infinity or a NaN anywhere (in the state, in U, in a value) is in some
+    // output of its column, times a zero or not, so they alone are looked at, and the marks of what the first kernel left.
     float o_sum[4], o_skip[4] = {0.f, 0.f, 0.f, 0.f};
     float4 o_m[2];
+    bool ok = true, odd = false;                         // odd: something was no ordinary number
     auto finish = [&](int c) {
         float own[4];
         mma6_alone(own, Up + (c & 1) * 768, o_m, (ob >> 1) + 1, lane);
@@ -729,6 +748,7 @@ chunk_serial_kernel(const ChunkArgs a) {
         for (int i = 0; i < 4; ++i) {
             own[i] += o_sum[i];
             if (MODE == CHUNK_SSM) own[i] = fmaf(skip, o_skip[i], own[i]);
+            odd = odd || !ordinary(own[i]);
         }
         const int ta = t_first + (c_begin + c) * CT + 8 * ob + 2 * (lane & 3);
         float* o = a.out + ((size_t)ta * H + h) * V + col;
@@ -741,22 +761,20 @@ chunk_serial_kernel(const ChunkArgs a) {
             if (ok1) o[(size_t)H * V + 8] = own[3];
         }
     };
-    bool ok = true, odd = false;                         // odd: something was no ordinary number
 
     for (int c = 0; c < chunks; ++c) {
         ok = tc5::mbar_wait(tc5::smem_u32(&full[c % STAGES]), (c / STAGES) & 1) && ok;
         __syncthreads();                                 // the state's parts are there; nobody is in chunk c - 1
         fetch(c + 2);
         const float* X = stages + (c % STAGES) * PER;
-        if (tid < 8) odd = odd || X[L::MARKS + tid] != 0.f;
-        if (!DELTA) odd = odd || !(ordinary(S[0]) && ordinary(S[1]) && ordinary(S[2]) && ordinary(S[3]));          // (the delta rules' U shows it)
+        if (warp == WARPS / 2 && lane < 8) odd = odd || X[L::MARKS + lane] != 0.f;
         float v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             v[i] = __uint_as_float(a.v_f32 ? v_next[i] : v_next[i] << 16);
             if (MODE == CHUNK_SSM && right) v[i] *= step_next[i & 1];
         }
-        values(c + 1);
+        values();
         // ---- products with the state, over 16 of the key rows
         {
             const int half = warp / KT, kt = warp % KT, nt0 = DELTA ? 0 : 2 * half;
@@ -776,23 +794,20 @@ chunk_serial_kernel(const ChunkArgs a) {
                 *(float4*)(to + nt * 128) = make_float4(big[nt][0] + small[nt][0], big[nt][1] + small[nt][1], big[nt][2] + small[nt][2],
                                                         big[nt][3] + small[nt][3]);
         }
+        if (!DELTA && output && c > 0) finish(c - 1);
         if (!DELTA && right) {
-            odd = odd || !(ordinary(v[0]) && ordinary(v[1]) && ordinary(v[2]) && ordinary(v[3]));
             if (PAIRED) put_half(Up + (c & 1) * 768, rb, rc, rc ? v[2] : v[0], rc ? v[3] : v[1]);
             else put(Up + (c & 1) * 768, rb, v);
         }
         __syncthreads();
+        float o_new[4] = {0.f, 0.f, 0.f, 0.f};
         if (output) {
-            if (c > 0) finish(c - 1);
             const float* from = part + (DELTA ? KT * 512 : 0) + ob * 128 + lane * 4;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { o_sum[i] = 0.f; o_skip[i] = v[i]; }
 #pragma unroll
             for (int w = 0; w < KT; ++w) {
                 const float4 x = *(const float4*)(from + w * 512);
-                o_sum[0] += x.x; o_sum[1] += x.y; o_sum[2] += x.z; o_sum[3] += x.w;
+                o_new[0] += x.x; o_new[1] += x.y; o_new[2] += x.z; o_new[3] += x.w;
             }
-            two_blocks(o_m, X + L::M + ob * 128, 512, lane);
         }
         if (DELTA) {
             if (right) {
@@ -824,9 +839,15 @@ chunk_serial_kernel(const ChunkArgs a) {
                 two_blocks(x, X + L::T + warp * 128, 512, lane);
                 mma6_alone(u, Rp, x, (warp >> 1) + 1, lane);
                 put(Up + (c & 1) * 768, warp, u);
-                odd = odd || !(ordinary(u[0]) && ordinary(u[1]) && ordinary(u[2]) && ordinary(u[3]));
+            } else if (output && c > 0) {
+                finish(c - 1);
             }
             __syncthreads();
+        }
+        if (output) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { o_sum[i] = o_new[i]; o_skip[i] = v[i]; }
+            two_blocks(o_m, X + L::M + ob * 128, 512, lane);
         }
         // ---- the state behind the chunk, eight rows; it is added to on the CUDA cores, which round to nearest
         {
