@@ -1,5 +1,5 @@
 // Paged causal attention on the CUDA cores, for any element type, head size, page size and
-// segment shape: the kernel of the 32-bit path, and the plain twin of the tensor-core kernels.
+// segment shape: the kernel of the 32-bit path where attention_f32.cu does not take the head size, and the plain twin of the tensor-core kernels.
 //
 // A warp owns up to four (token, query head) rows.  Keys are taken in tiles of 32 that are aligned to
 // absolute positions (0-31, 32-63, ...), lane j of a tile scores key j, and the online softmax
@@ -271,6 +271,12 @@ static int launch_simt(const void* q, int ld, const void* kpool, const void* vpo
     return rb_launch_status();
 }
 
+// attention_f32.cu: the 32-bit path's kernel where it takes the head size and the pools lie on 16-byte boundaries (257 tokens as above: 42 us).
+int rb_attention_f32_takes(int D, const void* kpool, const void* vpool);
+int rb_attention_f32(const float* q, int ld, const float* kpool, const float* vpool, const int* pos, const int* tok_seg, const int* block_table,
+                     int bt_stride, int page_size, float* out, int T, int Hq, int Hkv, int D, float scale, int window, int chunk, float softcap,
+                     const float* slopes, const float* sink, const float* bias, int bias_n, int keep, cudaStream_t st);
+
 RB_EXPORT int rb_attention_simt_mod(const void* q, int ld, const void* kpool, const void* vpool,
                                 const int* pos, const int* tok_seg, const int* block_table,
                                 int bt_stride, int page_size, void* out, int act_dtype, int T,
@@ -280,6 +286,9 @@ RB_EXPORT int rb_attention_simt_mod(const void* q, int ld, const void* kpool, co
     if (bias != nullptr && bias_n < 1) return (int)cudaErrorInvalidValue;
     if ((window > 0 && chunk > 0) || keep < 0 || (keep > 0 && window <= 0)) return (int)cudaErrorInvalidValue;
     if (D > SIMT_MAX_D || D <= 0 || Hkv <= 0 || Hq % Hkv) return (int)cudaErrorInvalidValue;
+    if (act_dtype == RB_F32 && rb_attention_f32_takes(D, kpool, vpool))
+        return rb_attention_f32((const float*)q, ld, (const float*)kpool, (const float*)vpool, pos, tok_seg, block_table, bt_stride, page_size,
+                                (float*)out, T, Hq, Hkv, D, scale, window, chunk, softcap, slopes, sink, bias, bias_n, keep, st);
     auto launch = act_dtype == RB_F32 ? (D <= 128 ? launch_simt<float, 1> : launch_simt<float, 2>)
                                       : (D <= 128 ? launch_simt<bf16, 1> : launch_simt<bf16, 2>);
     return launch(q, ld, kpool, vpool, pos, tok_seg, block_table, bt_stride, page_size, out, T, Hq, Hkv, D, scale, window, chunk,
