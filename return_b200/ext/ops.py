@@ -582,6 +582,8 @@ def gemm_tc5_bmn(x: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int = 
 # 1,038 -> 874 us; a captured one of 16 tokens 283 -> 267, of 64 387 -> 381; feed-forwards of 1,024 x 3,072 28.8 -> 19.0), above it loses
 # (600 rows of 2,048 x 6,144: 46.8 -> 53.1), and so with more weights to stream (64 tokens through layers of 4,096: 318 -> 333), but for few rows of
 # long sums: with K at least twice N the weight tiles are few, and K is cut over a cluster (64 x 4,096 x 12,288 21.7 -> 20.4).
+# And beyond a thousand rows the library's is as much faster however small the product (2,048 rows of a router, 32 x 2,048: 4.8 us and 6.7).
+ROWS_MAX = 1024
 ROWS_MAX_WORK = 3300 << 20
 ROWS_MAX_WEIGHTS = 1 << 24
 ROWS_LONG_SUMS = 128
@@ -591,7 +593,7 @@ def rows_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the kernel for the rows of an ordinary step takes this product and is the fastest way."""
     M, K = x.shape
     N = w.shape[0]
-    if x.dtype != torch.bfloat16 or M * N * K > ROWS_MAX_WORK and not (M <= ROWS_LONG_SUMS and K >= 2 * N):
+    if x.dtype != torch.bfloat16 or M > ROWS_MAX or M * N * K > ROWS_MAX_WORK and not (M <= ROWS_LONG_SUMS and K >= 2 * N):
         return False
     return ((N * K <= ROWS_MAX_WEIGHTS or M <= ROWS_LONG_SUMS and K >= 2 * N) and K % 8 == 0
             and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
