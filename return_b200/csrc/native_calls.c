@@ -6,6 +6,8 @@
 // independent of each other, a callee reads only the words it declares and the caller takes the words off the stack again, so one form
 // with more words than any entry has serves them all.  Anything else in an argument list (another type, another number of arguments) goes
 // to the ctypes function that the Call was made from.  An entry of 22 arguments: 0.3 us (through ctypes 2.8).
+//
+// `fill` writes lists of integers into an int32 array, which numpy does at 40 ns a number (a step's pages and tokens: 2,000 of them) and this at 2.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stddef.h>
@@ -92,7 +94,36 @@ static PyObject* make(PyObject* module, PyObject* args) {
     return (PyObject*)c;
 }
 
-static PyMethodDef methods[] = {{"make", make, METH_VARARGS, "make(address, kinds, general) -> Call, or None where the form is too small"}, {NULL}};
+// fill(array, places, lists, most): the first `most` numbers of lists[i] to array[places[i]], array[places[i] + 1], ...  False, with any part
+// of them written, if something is no list or no plain integer of 32 bits, or lies outside the array: then the caller's own way says what it is.
+static PyObject* fill(PyObject* module, PyObject* args) {
+    PyObject *array, *places, *lists;
+    Py_ssize_t most;
+    if (!PyArg_ParseTuple(args, "OO!O!n", &array, &PyList_Type, &places, &PyList_Type, &lists, &most)) return NULL;
+    Py_buffer to;
+    if (PyObject_GetBuffer(array, &to, PyBUF_CONTIG | PyBUF_FORMAT) < 0) return NULL;
+    const Py_ssize_t room = to.len / 4, n = PyList_GET_SIZE(lists);
+    int fine = to.itemsize == 4 && to.format != NULL && to.format[0] == 'i' && PyList_GET_SIZE(places) == n;
+    int* out = (int*)to.buf;
+    for (Py_ssize_t r = 0; fine && r < n; ++r) {
+        PyObject *list = PyList_GET_ITEM(lists, r), *place = PyList_GET_ITEM(places, r);
+        if (!PyList_CheckExact(list) || !PyLong_CheckExact(place)) { fine = 0; break; }
+        const Py_ssize_t at = PyLong_AsSsize_t(place), count = PyList_GET_SIZE(list) < most ? PyList_GET_SIZE(list) : most;
+        if (at < 0 || count > room || at > room - count) { PyErr_Clear(); fine = 0; break; }
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            PyObject* item = PyList_GET_ITEM(list, i);
+            int over = 0;
+            const long v = PyLong_CheckExact(item) ? PyLong_AsLongAndOverflow(item, &over) : 0;
+            if (!PyLong_CheckExact(item) || over || v < -2147483647L - 1 || v > 2147483647L) { fine = 0; break; }
+            out[at + i] = (int)v;
+        }
+    }
+    PyBuffer_Release(&to);
+    return PyBool_FromLong(fine);
+}
+
+static PyMethodDef methods[] = {{"fill", fill, METH_VARARGS, "fill(int32 array, places, lists, most) -> whether all of it was plain integers"},
+                                {"make", make, METH_VARARGS, "make(address, kinds, general) -> Call, or None where the form is too small"}, {NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "return_b200_native_calls", NULL, -1, methods};
 
 PyMODINIT_FUNC PyInit_return_b200_native_calls(void) {

@@ -220,9 +220,8 @@ class Entries:
         return getattr(self.__dict__["_lib"], name)
 
 
-def native_calls(lib: ctypes.CDLL):
-    """The entries of a library whose ``argtypes`` are set (and which return an int) taken past ctypes: ``csrc/native_calls.c``.
-    ``lib`` itself stays as it is.  Where that cannot be compiled it is handed back, and does the same."""
+def native_module():
+    """The module of ``csrc/native_calls.c``, or None where it cannot be had."""
     global _native_calls
     with _lock:
         if _native_calls is None:
@@ -236,13 +235,20 @@ def native_calls(lib: ctypes.CDLL):
                     _native_calls = module
                 except ImportError:
                     pass
-    if not _native_calls:
+    return _native_calls or None
+
+
+def native_calls(lib: ctypes.CDLL):
+    """The entries of a library whose ``argtypes`` are set (and which return an int) taken past ctypes: ``csrc/native_calls.c``.
+    ``lib`` itself stays as it is.  Where that cannot be compiled it is handed back, and does the same."""
+    module = native_module()
+    if module is None:
         return lib
     kinds = {ctypes.c_void_p: "p", ctypes.c_int: "i", ctypes.c_longlong: "i", ctypes.c_float: "f"}
     calls = {}
     for name, fn in list(vars(lib).items()):
         if isinstance(fn, ctypes._CFuncPtr) and fn.argtypes is not None and fn.restype is ctypes.c_int and all(t in kinds for t in fn.argtypes):
-            call = _native_calls.make(ctypes.cast(fn, ctypes.c_void_p).value, "".join(kinds[t] for t in fn.argtypes), fn)
+            call = module.make(ctypes.cast(fn, ctypes.c_void_p).value, "".join(kinds[t] for t in fn.argtypes), fn)
             if call is not None:
                 calls[name] = call
     return Entries(lib, calls)
