@@ -84,7 +84,7 @@ def prefill_throughput(runner, tokens: int, iters: int, warmup: int, seed: int =
 # kinds, the names of this engine's kernels (and of the library's matrix products).
 PROFILE_BUCKETS = [
     ("decode_attn", ["attn_decode", "attn_combine"]),
-    ("prefill_attn", ["attn_prefill", "attention_simt", "tc5_merge"]),
+    ("prefill_attn", ["attn_prefill", "attention_simt", "attention_f32", "tc5_merge"]),
     ("gemm/matmul", ["gemm", "nvjet", "cutlass", "cublas", "matmul"]),
     ("rmsnorm", ["rmsnorm", "norm_rows"]),
     ("rope", ["rope"]),

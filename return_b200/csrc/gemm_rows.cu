@@ -35,6 +35,14 @@ struct Args {
     int blocks;                            // blocks of k of a box: KPS, or 1 where K is no multiple of 64
     int out_f32, gated, act, vec;          // gated: 0, or 1 + the gate; act: -1, or the activation; vec: output rows of whole 16-byte pieces
     int* status;
+    // FUSED only
+    const float* ssq_in; int ssq_count;    // shares of sum(v^2) of every row of x, or null: the sums are multiplied by 1 / sqrt(sum / norm_dim + eps)
+    int norm_dim; float eps;
+    float* stream;                         // [M, N], or null: v = stream + sums goes back there; out gets v (offset + norm_w), ssq_out a
+    const void* norm_w; int norm_w_dtype;  // tile's share of sum(v^2) (out and norm_w null: neither)
+    float offset;
+    float* ssq_out;
+    int ld_sums;
 };
 
 __device__ __forceinline__ unsigned cluster_ctarank() {
@@ -56,8 +64,12 @@ __device__ __forceinline__ void load_box(unsigned smem_dst, const CUtensorMap* m
         ::"r"(smem_dst), "l"(map), "r"(x), "r"(row), "r"(block), "r"(bar) : "memory");
 }
 
-// LS: log2 of the CTAs that share a tile's K
-template <int LS>
+// LS: log2 of the CTAs that share a tile's K.
+// FUSED: the norm before the product and the residual add behind it are folded in, as gemm_skinny.cu does for few rows: a layer is two launches
+// shorter, which is what bounds such a step launch by launch: 512 tokens through six layers of 1,024 x 3,072 643 -> 563 us, 100 and 8 decoded
+// ones 729 -> 645; captured, 16 decoded tokens 264 -> 248, 64 371 -> 355, 128 509 -> 492.  The rows' factors are worked out by two warps while
+// the others wait for the operands, the first rows of the stream are asked for before that, and a half warp has a row's 128 columns.
+template <int LS, bool FUSED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args g) {
     constexpr int SPLIT = 1 << LS;
@@ -65,6 +77,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) unsigned long long full[MAX_STAGES], empty[MAX_STAGES], done;
     __shared__ unsigned tmem_slot;
+    __shared__ float rstd_s[FUSED ? MAX_BN : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = LS > 0 ? (int)cluster_ctarank() : 0;
     const int n0 = ((int)blockIdx.x >> LS) * BM, m0 = (int)blockIdx.y * g.tile_m;
@@ -88,6 +101,26 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const unsigned tmem = tmem_slot;
     bool ok = true;
     pdl_wait();
+    const int share = bn >> LS;                             // rows of the tile that a CTA finishes: m0 + (slot << LS | rank)
+    const int end = min(g.M, m0 + g.tile_m);
+    // FUSED: this thread's eight columns (the same in all of its rows), their norm weights and the first row's part of the stream
+    const int fused_col = n0 + 8 * (tid & 15);
+    float w8[8], next8[8];
+    auto ask = [&](int slot) {
+        const int row = m0 + (slot << LS | rank);
+        if (slot < share && row < end && fused_col < g.N) {
+            const float4* f = reinterpret_cast<const float4*>(g.stream + (size_t)row * g.N + fused_col);
+            const float4 lo = f[0], hi = f[1];
+            next8[0] = lo.x; next8[1] = lo.y; next8[2] = lo.z; next8[3] = lo.w; next8[4] = hi.x; next8[5] = hi.y; next8[6] = hi.z; next8[7] = hi.w;
+        }
+    };
+    if (FUSED && g.stream != nullptr) {
+        ask(tid >> 4);
+        if (g.norm_w != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w8[i] = fused_col < g.N ? g.offset + load_as_f32(g.norm_w, g.norm_w_dtype, fused_col + i) : 0.f;
+        }
+    }
 
     if (warp == 0) {
         if (lane == 0) {                                    // ---- operands
@@ -128,12 +161,21 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     } else if (warp >= 4) {
         ok = mbar_wait(smem_u32(&done), 0);
         fence_after_sync();
+    } else if (FUSED && g.ssq_in != nullptr) {              // ---- the rows' factors
+        for (int slot = tid - 64; slot < share; slot += 64) {
+            const int row = m0 + (slot << LS | rank);
+            float sum = 0.f;
+            if (row < end) {
+                const float* f = g.ssq_in + (size_t)row * g.ld_sums;
+                for (int i = 0; i < g.ssq_count; ++i) sum += f[i];
+            }
+            rstd_s[slot] = 1.0f / sqrtf(sum / (float)g.norm_dim + g.eps);
+        }
     }
     pdl_trigger_late();
     // ---- the sums to shared memory, over the stages: [share of K][row of this CTA's][weight row]
     __syncwarp();
     if (LS > 0) cluster_sync_all();                         // nobody's MMAs read them any more
-    const int share = bn >> LS;                             // rows of the tile that a CTA finishes
     if (warp >= 4) {
         const int q = warp & 3;
         unsigned to[SPLIT];
@@ -201,14 +243,48 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             }
         }
     };
-    const int end = min(g.M, m0 + g.tile_m);
-    if (g.gated) {
+    if (FUSED && g.stream != nullptr) {
+        for (int slot = tid >> 4; slot < share; slot += THREADS / 16) {          // a half warp has the whole of a row's columns
+            const int row = m0 + (slot << LS | rank);
+            const bool live = row < end && fused_col < g.N;
+            float v[8], had[8], ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) had[i] = next8[i];
+            ask(slot + THREADS / 16);
+            if (live) {
+                eight(slot, tid & 15, v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[i] = g.ssq_in ? had[i] + v[i] * rstd_s[slot] : had[i] + v[i];
+                    ss += v[i] * v[i];
+                }
+                float4* f = reinterpret_cast<float4*>(g.stream + (size_t)row * g.N + fused_col);
+                f[0] = make_float4(v[0], v[1], v[2], v[3]);
+                f[1] = make_float4(v[4], v[5], v[6], v[7]);
+                if (g.norm_w != nullptr) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] *= w8[i];
+                    store(row, fused_col, v);
+                }
+            }
+            if (g.ssq_out != nullptr) {
+                const unsigned half = 0xffffu << (lane & 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(half, ss, o);
+                if ((lane & 15) == 0 && row < end) g.ssq_out[(size_t)row * g.ld_sums + ((int)blockIdx.x >> LS)] = ss;
+            }
+        }
+    } else if (g.gated) {
         for (int e = tid; e < share * (BM / 16); e += THREADS) {
             const int slot = e / (BM / 16), c = e % (BM / 16), row = m0 + (slot << LS | rank), col = (n0 >> 1) + 8 * c;
             if (row >= end || col >= width) continue;
             float gate[8], up[8], v[8];
             eight(slot, 2 * c, gate);
             eight(slot, 2 * c + 1, up);
+            if (FUSED && g.ssq_in != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { gate[i] *= rstd_s[slot]; up[i] *= rstd_s[slot]; }
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = gate[i] / (1.0f + expf(-rb_gate_arg(g.gated - 1, gate[i]))) * up[i];
             store(row, col, v);
@@ -219,6 +295,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (row >= end || col >= width) continue;
             float v[8];
             eight(slot, c, v);
+            if (FUSED && g.ssq_in != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] *= rstd_s[slot];
+            }
             if (g.act >= 0) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = rb_activate(g.act, v[i], nullptr, 0, 0);
@@ -244,11 +324,11 @@ bool make_map(CUtensorMap* map, const void* p, int rows, int K, long long ld, in
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int LS>
+template <int LS, bool FUSED>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, unsigned smem, cudaStream_t st) {
     static PerDevice configured;
     const int rc = configured.once([&](int) {
-        return cudaFuncSetAttribute(gemm_rows_kernel<LS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(RING + 1024));
+        return cudaFuncSetAttribute(gemm_rows_kernel<LS, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(RING + 1024));
     });
     if (rc) return rc;
     cudaLaunchAttribute attr[2];
@@ -265,7 +345,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, unsigned
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = RB_PDL_MODE == 3 ? 1 : 2;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<LS>, mw, mx, g);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<LS, FUSED>, mw, mx, g);
 }
 
 // Rows of a tile and CTAs of a cluster: the choice whose busiest SM is done first.
@@ -286,6 +366,29 @@ void pick(int M, int N, int K, int sms, int* tiles_m, int* ls) {
     }
 }
 
+// What the two entries share: the shape's choice, the maps, the launch.
+template <bool FUSED>
+int run(Args& g, const void* x, const void* w, int ldx, int ldw, int tiles, int ls, cudaStream_t st) {
+    const int M = g.M, N = g.N, K = g.K;
+    if (K <= 0 || K % 8 || ldx % 8 || ldw % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return (int)cudaErrorInvalidValue;
+    if (tiles < 0) pick(M, N, K, rb_num_sms(), &tiles, &ls);
+    if (tiles < 1 || ls < 0 || ls > 2 || tiles > 65535 || (M + tiles - 1) / tiles > MAX_BN) return (int)cudaErrorInvalidValue;
+    g.tile_m = (M + tiles - 1) / tiles;
+    g.bn = (g.tile_m + 15) & ~15;
+    g.blocks = K % BK == 0 ? KPS : 1;
+    const int all = (K + BK * KPS - 1) / (BK * KPS), per = (all + (1 << ls) - 1) >> ls;
+    g.stages = (int)(RING / stage_bytes(g.bn));
+    g.stages = g.stages > MAX_STAGES ? MAX_STAGES : g.stages;
+    g.stages = g.stages > per ? per : g.stages;
+    g.vec = g.ldo % 8 == 0 && ((uintptr_t)g.out % 16) == 0;
+    unsigned smem = g.stages * stage_bytes(g.bn);
+    if (smem < (unsigned)g.bn * BM * 4) smem = (unsigned)g.bn * BM * 4;               // the sums lie over the stages
+    CUtensorMap mw, mx;
+    if (!make_map(&mw, w, N, K, ldw, BM) || !make_map(&mx, x, M, K, ldx, g.bn)) return (int)cudaErrorInvalidValue;
+    if (ls == 0) return launch<0, FUSED>(mw, mx, g, smem + 1024, st);
+    return ls == 1 ? launch<1, FUSED>(mw, mx, g, smem + 1024, st) : launch<2, FUSED>(mw, mx, g, smem + 1024, st);
+}
+
 }  // namespace
 
 // out: bfloat16, or float32 with out_f32.  gated: 1 + the number of a gate (W's rows woven in eights, out [M, N / 2]), or 0; act: an activation's
@@ -294,25 +397,28 @@ void pick(int M, int N, int K, int sms, int* tiles_m, int* ls) {
 RB_EXPORT int rb_gemm_rows(const void* x, const void* w, void* out, int out_f32, int gated, int act, int M, int N, int K, int ldx, int ldw, int ldo,
                            int tiles, int ls, int* status, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
-    if (K <= 0 || K % 8 || ldx % 8 || ldw % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return (int)cudaErrorInvalidValue;
     if (gated && (N % 16 || gated < 0 || gated - 1 > GATE_GELU_TANH || act >= 0)) return (int)cudaErrorInvalidValue;
     if (act > ACT_NEG_EXP_EXP) return (int)cudaErrorInvalidValue;
-    if (tiles < 0) pick(M, N, K, rb_num_sms(), &tiles, &ls);
-    if (tiles < 1 || ls < 0 || ls > 2 || tiles > 65535 || (M + tiles - 1) / tiles > MAX_BN) return (int)cudaErrorInvalidValue;
     Args g = {};
     g.out = out; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.out_f32 = out_f32; g.gated = gated; g.act = act; g.status = status;
-    g.tile_m = (M + tiles - 1) / tiles;
-    g.bn = (g.tile_m + 15) & ~15;
-    g.blocks = K % BK == 0 ? KPS : 1;
-    const int all = (K + BK * KPS - 1) / (BK * KPS), per = (all + (1 << ls) - 1) >> ls;
-    g.stages = (int)(RING / stage_bytes(g.bn));
-    g.stages = g.stages > MAX_STAGES ? MAX_STAGES : g.stages;
-    g.stages = g.stages > per ? per : g.stages;
-    g.vec = ldo % 8 == 0 && ((uintptr_t)out % 16) == 0;
-    unsigned smem = g.stages * stage_bytes(g.bn);
-    if (smem < (unsigned)g.bn * BM * 4) smem = (unsigned)g.bn * BM * 4;               // the sums lie over the stages
-    CUtensorMap mw, mx;
-    if (!make_map(&mw, w, N, K, ldw, BM) || !make_map(&mx, x, M, K, ldx, g.bn)) return (int)cudaErrorInvalidValue;
-    if (ls == 0) return launch<0>(mw, mx, g, smem + 1024, st);
-    return ls == 1 ? launch<1>(mw, mx, g, smem + 1024, st) : launch<2>(mw, mx, g, smem + 1024, st);
+    return run<false>(g, x, w, ldx, ldw, tiles, ls, st);
+}
+
+// The product with the norm before it and the residual add behind it folded in (as rb_gemm_skinny_fused, for more rows).
+// ssq_in [M, ld_sums]: ssq_count shares of sum(v^2) a row, or null.  stream [M, N] float32, or null: with it out is null (no next norm) or gets
+// v (offset + norm_w) for the next product, and ssq_out [M, ld_sums] (or null) one share a tile of 128 columns.
+RB_EXPORT int rb_gemm_rows_fused(const void* x, const void* w, void* out, int gated, int M, int N, int K, int ldx, int ldw, int ldo,
+                                 const float* ssq_in, int ssq_count, int norm_dim, float eps, float* stream, const void* norm_w,
+                                 int norm_w_dtype, float offset, float* ssq_out, int ld_sums, int tiles, int ls, int* status, cudaStream_t st) {
+    if (M <= 0 || N <= 0) return 0;
+    if (gated && (N % 16 || gated < 0 || gated - 1 > GATE_GELU_TANH || stream != nullptr)) return (int)cudaErrorInvalidValue;
+    if (ssq_in != nullptr && (ssq_count < 1 || ssq_count > ld_sums || norm_dim < 1)) return (int)cudaErrorInvalidValue;
+    if (stream == nullptr && (out == nullptr || norm_w != nullptr || ssq_out != nullptr)) return (int)cudaErrorInvalidValue;
+    if (stream != nullptr && (N % 8 || ((uintptr_t)stream % 16) || (out == nullptr) != (norm_w == nullptr))) return (int)cudaErrorInvalidValue;
+    if (ssq_out != nullptr && (N + BM - 1) / BM > ld_sums) return (int)cudaErrorInvalidValue;
+    Args g = {};
+    g.out = out; g.M = M; g.N = N; g.K = K; g.ldo = ldo; g.gated = gated; g.act = -1; g.status = status;
+    g.ssq_in = ssq_in; g.ssq_count = ssq_count; g.norm_dim = norm_dim; g.eps = eps;
+    g.stream = stream; g.norm_w = norm_w; g.norm_w_dtype = norm_w_dtype; g.offset = offset; g.ssq_out = ssq_out; g.ld_sums = ld_sums;
+    return run<true>(g, x, w, ldx, ldw, tiles, ls, st);
 }

@@ -361,6 +361,7 @@ class RowSums:
     WIDTH = 512
 
     def __init__(self, parts: torch.Tensor, dim: int, count: int = 0):
+        assert parts.dtype == torch.float32 and parts.is_contiguous()
         self.parts, self.dim, self.count = parts, dim, count
 
 
@@ -474,6 +475,8 @@ def tc5_lib() -> ctypes.CDLL:
         lib.rb_tc5_gemm_simple.argtypes = [P, P, P, I, I, I, I, I, I, I, I, P, P]
         lib.rb_tc5_gemm_bmn.argtypes = [P, P, P, I, I, I, I, I, I, I, P, P]
         lib.rb_gemm_rows.argtypes = [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P]
+        lib.rb_gemm_rows_fused.argtypes = [P, P, P, I, I, I, I, I, I, I, P, I, I, ctypes.c_float, P, P, I, ctypes.c_float, P, I, I, I, P, P]
+        lib.rb_gemm_rows_fused.restype = c_int
         lib.rb_gemm_rows.restype = c_int
         lib.rb_tc5_gemm.restype = lib.rb_tc5_gemm_simple.restype = lib.rb_tc5_gemm_bmn.restype = c_int
         _tc5 = build.native_calls(lib)
@@ -589,14 +592,19 @@ ROWS_MAX_WEIGHTS = 1 << 24
 ROWS_LONG_SUMS = 128
 
 
+def rows_limit(N: int, K: int) -> int:
+    """The largest number of rows that the kernel for the rows of an ordinary step takes against N x K weights and is the fastest way."""
+    limit = ROWS_LONG_SUMS if K >= 2 * N else 0
+    if N * K <= ROWS_MAX_WEIGHTS:
+        limit = max(limit, min(ROWS_MAX, ROWS_MAX_WORK // (N * K)))
+    return limit
+
+
 def rows_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the kernel for the rows of an ordinary step takes this product and is the fastest way."""
-    M, K = x.shape
-    N = w.shape[0]
-    if x.dtype != torch.bfloat16 or M > ROWS_MAX or M * N * K > ROWS_MAX_WORK and not (M <= ROWS_LONG_SUMS and K >= 2 * N):
-        return False
-    return ((N * K <= ROWS_MAX_WEIGHTS or M <= ROWS_LONG_SUMS and K >= 2 * N) and K % 8 == 0
-            and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    N, K = w.shape
+    return (x.dtype == torch.bfloat16 and x.shape[0] <= rows_limit(N, K) and K % 8 == 0 and x.stride(0) % 8 == 0
+            and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False, act: Optional[str] = None, tiles: int = -1,
@@ -615,6 +623,54 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool =
                                 tiles, log2_split, _ptr(tc5_status(x.device)), _stream())
     _tc5_launched.add(x.device)
     _check(rc, "gemm_rows")
+
+
+def gemm_rows_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], gated: bool = False, scale=None, residual=None,
+                    tiles: int = -1, log2_split: int = -1) -> None:
+    """``gemm_skinny_fused`` for the rows of an ordinary step: the same arguments, RowSums of [rows, tiles of 128 columns]."""
+    M, K = x.shape
+    N = w.shape[0]
+    assert x.dtype == w.dtype == torch.bfloat16 and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
+    ssq_in, ssq_in_count, norm_dim, eps, ld_sums = None, 0, 0, 0.0, 0
+    if scale is not None:
+        sums_in, eps = scale
+        ssq_in, ssq_in_count, norm_dim = sums_in.parts, sums_in.count, sums_in.dim
+        assert ssq_in_count > 0 and ssq_in.shape[0] >= M
+        ld_sums = ssq_in.shape[1]
+    stream = norm_w = ssq_out = None
+    norm_w_dtype, offset = F32, 0.0
+    if residual is not None:
+        stream, next_norm, sums_out = residual
+        assert not gated and stream.dtype == torch.float32 and stream.is_contiguous() and stream.shape == (M, N)
+        if next_norm is not None:
+            norm_w, offset = next_norm
+            assert out is not None and norm_w.numel() == N and norm_w.is_contiguous()
+            norm_w_dtype = dtype_code(norm_w.dtype)
+        if sums_out is not None:
+            sums_out.count = (N + 127) // 128
+            ssq_out = sums_out.parts
+            assert sums_out.dim == N and ssq_out.shape[0] >= M and ssq_out.shape[1] >= sums_out.count and (ssq_in is None or ssq_out.shape[1] == ld_sums)
+            ld_sums = ssq_out.shape[1]
+    if out is not None:
+        assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and out.shape == (M, N // 2 if gated else N)
+    rc = tc5_lib().rb_gemm_rows_fused(_ptr(x), _ptr(w), _ptr(out), 1 if gated else 0, M, N, K, x.stride(0), w.stride(0),
+                                      out.stride(0) if out is not None else 0, _ptr(ssq_in), ssq_in_count, norm_dim, eps, _ptr(stream),
+                                      _ptr(norm_w), norm_w_dtype, offset, _ptr(ssq_out), ld_sums, tiles, log2_split,
+                                      _ptr(tc5_status(x.device)), _stream())
+    _tc5_launched.add(x.device)
+    _check(rc, "gemm_rows_fused")
+
+
+def row_sums(buffer, name: str, rows: int, dim: int, device) -> "RowSums":
+    """Room for the shares of a norm over rows of ``dim`` values (``buffer``: the step's), for the kernel that takes so many rows."""
+    shape = (8, RowSums.WIDTH) if rows <= SKINNY_MAX_ROWS else (rows, (dim + 127) // 128)
+    return RowSums(buffer(name, shape, torch.float32, device), dim)
+
+
+def linear_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], gated: bool = False, scale=None, residual=None) -> None:
+    """A product with the norm before it and the residual add behind it folded in, by the kernel that takes so many rows: up to
+    SKINNY_MAX_ROWS, or up to ``rows_limit``."""
+    (gemm_skinny_fused if x.shape[0] <= SKINNY_MAX_ROWS else gemm_rows_fused)(x, w, out, gated, scale, residual)
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[str] = None,

@@ -70,12 +70,12 @@ class PreNormBlock(Block):
         return None
 
     def _fused_plan(self, stream):
-        """For a step of few rows in bfloat16 the two norms and the two residual adds of the block cost no kernel of
-        their own: the product before a norm (the mixer's last, the feed-forward's last) adds into the stream
+        """For a step of few rows, or an ordinary number of them, in bfloat16 the two norms and the two residual adds of the
+        block cost no kernel of their own: the product before a norm (the mixer's last, the feed-forward's last) adds into the stream
         and leaves v * w and sum(v^2); the product after it (the gated one, the next block's first) scales by
-        rstd (csrc/gemm_skinny.cu).  Six launches a layer instead of eight.  That needs a mixer and a feed-forward
-        that expose their products, RMSNorms, and sizes the kernel takes; anything else runs part by part."""
-        if self.env.act_dtype != torch.bfloat16 or stream.shape[0] > ops.SKINNY_MAX_ROWS or self._scaled:
+        rstd (csrc/gemm_skinny.cu, csrc/gemm_rows.cu).  Six launches a layer of a decode step instead of eight.  That
+        needs a mixer and a feed-forward that expose their products, RMSNorms, and sizes the kernel takes; anything else runs part by part."""
+        if self.env.act_dtype != torch.bfloat16 or self._scaled or stream.shape[0] > ops.ROWS_MAX:
             return None
         plan = getattr(self, "_fused_parts", None)
         if plan is None:
@@ -90,40 +90,50 @@ class PreNormBlock(Block):
                 if (interleave == 8 and gate_up.shape[0] % 16 == 0 and w_out.shape[0] == stream.shape[1] == down.shape[0]
                         and all(w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0
                                 and w.data_ptr() % 16 == 0 for w in weights)):
-                    plan = (w_in, in_name, w_out, gate_up, down)
+                    most = min(ops.rows_limit(*w.shape) for w in weights)           # rows that one kernel or the other takes in all four
+                    plan = (w_in, in_name, w_out, gate_up, down, max(most, ops.SKINNY_MAX_ROWS))
             self._fused_parts = plan
-        return plan or None
+        if not plan or stream.shape[0] > plan[5]:
+            return None
+        return plan
 
     def _forward_fused(self, plan, stream, delta, ctx):
-        w_in, in_name, w_out, gate_up, down = plan
+        w_in, in_name, w_out, gate_up, down, _ = plan
         T, H = stream.shape
         dev, dt = stream.device, self.env.act_dtype
         n1, n2 = self.mixer_norm, self.feed_forward_norm
         held = ctx.batch.scratch
+        key = ("block.fused", in_name, T, H, w_in.shape[0], gate_up.shape[0])
+        work = held.get(key)
+        if work is None:                                       # the same for every block of these sizes: looked up once a step
+            work = held[key] = (
+                ctx.buffer(in_name, (T, w_in.shape[0]), dt, dev),
+                ctx.buffer("block.rows_mid", (T, H), dt, dev), ops.row_sums(ctx.buffer, "block.sums_mid", T, H, dev),
+                ctx.buffer("block.gated_act", (T, gate_up.shape[0] // 2), dt, dev),
+                ctx.buffer("block.rows_out", (T, H), dt, dev), ops.row_sums(ctx.buffer, "block.sums_out", T, H, dev))
+        proj, rows2, sums2, act, rows3, sums3 = work
         # what the block before this one left for this block's first norm (made for this position of the schedule)
         pre = held.pop("block.prenormed", None)
-        proj = ctx.buffer(in_name, (T, w_in.shape[0]), dt, dev)
         if delta is None and pre is not None and pre["position"] == ctx.position:
-            ops.gemm_skinny_fused(pre["rows"], w_in, proj, scale=(pre["sums"], n1.spec.eps))
+            ops.linear_fused(pre["rows"], w_in, proj, scale=(pre["sums"], n1.spec.eps))
         else:
             a = ctx.buffer("block.normed", (T, H), dt, dev)
             n1.add_forward(stream, delta, a)                   # stream += delta; a = norm(stream)
-            ops.gemm_skinny(a, w_in, proj)
+            ops.linear(a, w_in, proj)
         mixed = self.mixer.core(proj, ctx)
-        rows2 = ctx.buffer("block.rows_mid", (T, H), dt, dev)
-        sums2 = ops.RowSums(ctx.buffer("block.sums_mid", (8, ops.RowSums.WIDTH), torch.float32, dev), H)
-        ops.gemm_skinny_fused(mixed, w_out, rows2, residual=(stream, (n2.p_weight, n2.spec.offset), sums2))
-        act = ctx.buffer("block.gated_act", (T, gate_up.shape[0] // 2), dt, dev)
-        ops.gemm_skinny_fused(rows2, gate_up, act, gated=True, scale=(sums2, n2.spec.eps))
+        ops.linear_fused(mixed, w_out, rows2, residual=(stream, (n2.p_weight, n2.spec.offset), sums2))
+        ops.linear_fused(rows2, gate_up, act, gated=True, scale=(sums2, n2.spec.eps))
         nxt = ctx.next_block.first_norm() if ctx.next_block is not None and hasattr(ctx.next_block, "first_norm") else None
         if nxt is not None and nxt[3] != H:
             nxt = None
+        if nxt is None and T > ops.SKINNY_MAX_ROWS:            # what follows adds it anyway
+            y = ctx.buffer("block.delta", (T, H), dt, dev)
+            ops.linear(act, down, y)
+            return y
         if nxt is None:
-            ops.gemm_skinny_fused(act, down, None, residual=(stream, None, None))
+            ops.linear_fused(act, down, None, residual=(stream, None, None))
         else:
-            rows3 = ctx.buffer("block.rows_out", (T, H), dt, dev)
-            sums3 = ops.RowSums(ctx.buffer("block.sums_out", (8, ops.RowSums.WIDTH), torch.float32, dev), H)
-            ops.gemm_skinny_fused(act, down, rows3, residual=(stream, (nxt[0], nxt[2]), sums3))
+            ops.linear_fused(act, down, rows3, residual=(stream, (nxt[0], nxt[2]), sums3))
             held["block.prenormed"] = {"rows": rows3, "sums": sums3, "position": ctx.position + 1}
         return None                                            # the stream already holds this block's output
 

@@ -78,3 +78,61 @@ def test_what_the_kernel_does_not_take_goes_to_the_library():
     out = torch.empty(40, 100, device=DEV, dtype=torch.bfloat16)
     ops.linear(x, w, out)
     _close(out, exact, size, 100)
+
+
+@pytest.mark.parametrize("M,H,Q,I,offset,wdt", [(9, 96, 64, 48, 0.0, torch.float32), (33, 136, 136, 128, 1.0, torch.bfloat16), (130, 1024, 512, 200, 0.0, torch.bfloat16),
+                                                (257, 264, 1024, 64, 0.5, torch.float32)])
+def test_norms_and_residual_adds_inside_the_products(M, H, Q, I, offset, wdt):
+    """Product + residual add, then the gated and a plain product on the rows it left, each step against 64 bits from what the step before it
+    really left."""
+    ops = _ops()
+    o, w_o, exact, size = _inputs(M, H, Q, M + H)
+    g = torch.Generator(device=DEV).manual_seed(M)
+    stream0 = torch.empty(M, H, device=DEV).normal_(std=2.0, generator=g)
+    norm = torch.empty(H, device=DEV).normal_(generator=g).to(wdt)
+    woven = torch.empty(2 * I, H, device=DEV).normal_(std=0.05, generator=g).bfloat16()
+    eps, tiles_n = 1e-5, (H + 127) // 128
+    least = (M + 255) // 256
+    for tiles, ls in [(-1, -1)] + [(t, l) for t in (least, least + 2) for l in (0, 1, 2)]:
+        shape = dict(tiles=tiles, log2_split=ls)
+        stream, rows = stream0.clone(), torch.full((M, H), float("nan"), device=DEV, dtype=torch.bfloat16)
+        sums = ops.RowSums(torch.full((M, tiles_n), float("nan"), device=DEV), H)
+        ops.gemm_rows_fused(o, w_o, rows, residual=(stream, (norm, offset), sums), **shape)
+        only = stream0.clone()
+        ops.gemm_rows_fused(o, w_o, None, residual=(only, None, None), **shape)
+        assert torch.equal(only, stream)
+        want = stream0.double() + exact
+        assert ((stream.double() - want).abs() <= want.abs() * 2.0 ** -23 + size * (Q / 16 + 4) * 2.0 ** -23).all()
+        left = stream.double() * (norm.double() + offset)
+        assert ((rows.double() - left).abs() <= left.abs() * (2.0 ** -8 + 2.0 ** -21) + 1e-37).all()
+        ssq = stream.double().square().sum(1)
+        assert sums.count == tiles_n
+        assert ((sums.parts[:, :tiles_n].double().sum(1) - ssq).abs() <= ssq * 16 * 2.0 ** -23).all()
+        # the rows it left, times the norm's factor: eight products' and three more roundings of the factor
+        rstd = (1.0 / (ssq / H + eps).sqrt())[:, None]
+        p, psize = rows.double() @ woven.double().T * rstd, rows.double().abs() @ woven.double().abs().T * rstd
+        plain = torch.full((M, 2 * I), float("nan"), device=DEV, dtype=torch.bfloat16)
+        ops.gemm_rows_fused(rows, woven, plain, scale=(sums, eps), **shape)
+        _close(plain, p, psize + p.abs(), H + 64)
+        gate, up = p.view(M, -1, 2, 8).unbind(2)
+        err = ((psize + p.abs()) * ((H + 64) / 16 + 4) * 2.0 ** -23).view(M, -1, 2, 8)
+        unit = gate * torch.sigmoid(gate)
+        act = torch.full((M, I), float("nan"), device=DEV, dtype=torch.bfloat16)
+        ops.gemm_rows_fused(rows, woven, act, gated=True, scale=(sums, eps), **shape)
+        tol = 1.1 * err[:, :, 0] * up.abs() + (unit.abs() + 1.1 * err[:, :, 0]) * err[:, :, 1] + (unit * up).abs() * (2.0 ** -8 + 2.0 ** -20) + 1e-37
+        assert ((act.double() - (unit * up).reshape(M, I)).abs() <= tol.reshape(M, I)).all()
+        # and a product that scales and adds at once
+        again = stream.clone()
+        ops.gemm_rows_fused(rows[:, :H], w_back := woven[:H] if 2 * I >= H else woven.repeat(H // (2 * I) + 1, 1)[:H].contiguous(), None,
+                            scale=(sums, eps), residual=(again, None, None), **shape)
+        q, qsize = rows.double() @ w_back.double().T * rstd, rows.double().abs() @ w_back.double().abs().T * rstd
+        want = stream.double() + q
+        assert ((again.double() - want).abs() <= want.abs() * 2.0 ** -23 + (qsize + q.abs()) * ((H + 64) / 16 + 4) * 2.0 ** -23).all()
+    ops.check_status(torch.device("cuda:0"))
+
+
+def test_fused_product_refuses_what_it_cannot_take():
+    ops = _ops()
+    x, w = torch.zeros(16, 64, device=DEV).bfloat16(), torch.zeros(130, 64, device=DEV).bfloat16()
+    with pytest.raises(Exception):                            # a row of the stream that is no whole 16-byte pieces
+        ops.gemm_rows_fused(x, w, None, residual=(torch.zeros(16, 130, device=DEV), None, None))
