@@ -16,7 +16,7 @@
 // All arithmetic keeps float32's precision.  The products run as bfloat16 matrix instructions on operands split into three
 // bfloat16 parts (x = h + m + l, 24 bits), six of the nine products (hh, hm, mh, hl, lh, mm; the rest is below 2^-24), the five small
 // ones in an accumulator of their own.  Per flop that is as fast as three TF32 products, which would keep 22 bits, and 1.3 times
-// the CUDA cores' peak, of which register blocks this small reach a third (gemm_f32.cu).
+// the CUDA cores' peak, of which register blocks this small reach a third.
 #include "tc5.cuh"
 
 #define CHUNK_DECAY 0            // the modes of recurrent.cu
@@ -521,12 +521,12 @@ chunk_prep_kernel(const ChunkArgs a) {
 // meet in shared memory.  U = T (v - ...) is made by the first four warps, the outputs by the last four (while the next chunk's U is
 // made), and every warp updates eight of the state's rows, which it keeps in float32 registers, and leaves their three parts for
 // the next chunk.  Chunks come by bulk copies, two ahead; every wait for one is bounded (status word).  Bound by the latency of
-// a chunk's steps one behind the other: 2.4 us a chunk of the delta rule with keys of 128 (64 chunks of 16 heads of 128 x 128: 152 us;
-// the matrix instructions alone would be 0.75 us a chunk), 1.6 us of the others (102 us).  With cp.async by all threads in the place of the
+// a chunk's steps one behind the other: 2.3 us a chunk of the delta rule with keys of 128 (64 chunks of 16 heads of 128 x 128: 149 us;
+// the matrix instructions alone would be 0.75 us a chunk), 1.6 us of the others (100 us).  With cp.async by all threads in the place of the
 // bulk copies and the outputs finished in their own chunk: 187 and 128 us; with eight warps instead of sixteen and the values'
-// conversion behind their load: 167 and 184.  The first kernel takes 60 and 42 us there; token by token it was 893 and 508.
-// Whether everything was an ordinary number is looked at once, behind the last chunk: 2 % of a layer (309.6 us a delta-rule layer of 2,048 tokens,
-// 303.7 without; at every chunk's barrier 314.4).
+// conversion behind their load: 167 and 184; with the outputs' sums and the checks of U and of the state on the chain: 157 and 107.
+// The first kernel takes 54 and 38 us there (62 and 45 with two CTAs an SM instead of three); token by token it was 893 and 508.
+// Whether everything was an ordinary number is asked of the outputs only and answered once, behind the last chunk.
 constexpr int STAGES = 3;
 
 __device__ __forceinline__ void bulk_copy(unsigned smem, const float* gmem, unsigned bytes, unsigned bar) {
