@@ -97,6 +97,20 @@ def test_swiglu(act, I):
         assert torch.equal(out2, out)
 
 
+@pytest.mark.parametrize("T,I", [(1, 4), (3, 1020), (2, 1024), (5, 1032)])
+def test_swiglu_of_float32_in_pieces_has_the_bits_of_the_general_kernel(T, I):
+    """Rows of one block of columns and of a bit more; a start that is no 16-byte boundary takes the general kernel."""
+    ops = _ops()
+    gu = 3 * torch.randn(T, 2 * I, device=DEV)
+    apart = torch.empty(T * 2 * I + 1, device=DEV)[1:].view(T, 2 * I)
+    apart.copy_(gu)
+    for interleave in (0, 8) if I % 8 == 0 else (0,):
+        out, general = torch.full((T, I), float("nan"), device=DEV), torch.empty(T, I, device=DEV)
+        ops.swiglu(gu, out, interleave=interleave)
+        ops.swiglu(apart, general, interleave=interleave)
+        assert torch.equal(out, general)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 7, 5), (3, 130, 257), (65, 64, 16), (100, 200, 96), (2, 384, 96)])
 def test_gemm_f32_is_exact_float32(M, N, K):
     ops = _ops()
