@@ -141,12 +141,12 @@ class Engine:
                 logits = self.runner.step(entries, tokens_dev if launched > committed else None)
                 params = [(r.temperature, r.top_k, r.top_p, uniform_draw(r.seed, len(r.output) + launched - committed))
                           for r in reqs]
-                tokens_dev = self.sampler.launch(logits, params, launched % Sampler.SLOTS)
+                tokens_dev = self.sampler.launch(logits, params, launched % Sampler.SLOTS, status=True)
                 launched += 1
                 continue
             if committed == launched:
                 break
-            toks, lps = self.sampler.fetch(committed % Sampler.SLOTS)
+            toks, lps = self.sampler.fetch(committed % Sampler.SLOTS)   # raises where a kernel's bounded wait gave up
             committed += 1
             for r, t, lp in zip(reqs, toks, lps):
                 if r.finish_reason is not None:

@@ -52,7 +52,7 @@ class ModelRunner:
         self.staging = BatchStaging(self.env.device)
         self.vocab_size = model.spec.vocab_size
         self.tilings = model.batch_tilings()   # the tables of row blocks that the model's parts read, by name
-        self._graphs = {}                   # (decode batch size, what the parts fixed) -> (graph, static batch, static logits)
+        self._graphs = {}                   # (decode batch size, what the parts fixed) -> (graph, static batch, static logits, its kernels' StatusWatch)
         self._graph_keys = {}               # (decode batch size, span of context lengths) -> key of _graphs
         self._graph_pool = None
         self.launches_per_replay = {}       # decode batch size -> kernels of this package in its graph
@@ -149,11 +149,12 @@ class ModelRunner:
         entry = self._graphs.get(key)
         if entry is None:
             entry = self._capture(key)
-        graph, static, logits = entry
+        graph, static, logits, watch = entry
         static.fill(host)
         if device_tokens is not None:
             static.tokens[:m].copy_(device_tokens[:m], non_blocking=True)     # after the upload, in stream order
         graph.replay()
+        watch.replayed()
         if host.num_want == m and (host.want_rows == range(m)).all():
             return logits[:m]
         return logits.index_select(0, torch.as_tensor(host.want_rows, dtype=torch.int64).to(logits.device))
@@ -189,12 +190,12 @@ class ModelRunner:
         torch.cuda.synchronize(self.env.device)
         graph = torch.cuda.CUDAGraph()
         before = ops.launch_count
-        with torch.cuda.graph(graph, pool=self._graph_pool):
+        with ops.StatusWatch(self.env.device) as watch, torch.cuda.graph(graph, pool=self._graph_pool):
             logits = self.model.forward(static, self.storage)
         self.launches_per_replay[n] = ops.launch_count - before
         if self._graph_pool is None:
             self._graph_pool = graph.pool()
-        self._graphs[key] = (graph, static, logits)
+        self._graphs[key] = (graph, static, logits, watch)
         return self._graphs[key]
 
     def capture_decode_graphs(self, batch_sizes=None) -> int:

@@ -315,8 +315,7 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int = -1
     assert w.shape[1] == K and out.shape == (M, N)
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     rc = core().rb_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                            kind, _ptr(tc5_status(x.device)), _stream())
-    _tc5_launched.add(x.device)
+                            kind, _status_word(x.device), _stream())
     _check(rc, "gemm_f32")
 
 
@@ -498,6 +497,52 @@ def tc5_status(device) -> torch.Tensor:
 _tc5_launched = set()          # devices on which a kernel with bounded waits ran since the status word was last read
 
 
+def _status_word(device):
+    """The pointer that a launch hands to a kernel with bounded waits; ``check_status`` then reads the word."""
+    _tc5_launched.add(device)
+    return _ptr(tc5_status(device))
+
+
+class StatusWatch:
+    """``with StatusWatch(device) as watch: <capture>`` finds out whether the captured launches include kernels with bounded waits.  A
+    replayed graph runs no Python, so whoever replays such a graph calls ``watch.replayed()`` beside it."""
+
+    def __init__(self, device):
+        self.device, self.waits = torch.device(device), False
+
+    def __enter__(self):
+        self._before = self.device in _tc5_launched
+        _tc5_launched.discard(self.device)
+        return self
+
+    def __exit__(self, *exc):
+        self.waits = self.device in _tc5_launched
+        if self._before:
+            _tc5_launched.add(self.device)
+
+    def replayed(self) -> None:
+        if self.waits:
+            _tc5_launched.add(self.device)
+
+
+def copy_status(device, to: torch.Tensor) -> bool:
+    """Copies the status word to ``to`` (pinned) in stream order, if a kernel with bounded waits ran on ``device`` since it was last
+    read: for a caller that does not want to wait for the device now, and hands what arrived to ``raise_status``."""
+    device = torch.device(device)
+    if device not in _tc5_launched:
+        return False
+    to.copy_(tc5_status(device), non_blocking=True)
+    return True
+
+
+def raise_status(device, code: int) -> None:
+    """Raises ``KernelError`` if ``code``, a status word as it was read, says that a bounded wait gave up."""
+    if code != 0:
+        tc5_status(torch.device(device)).zero_()
+        raise KernelError(f"a kernel on {device} gave up a bounded wait (an mbarrier, or the other CTAs of its grid) or "
+                          f"found its shared memory misaligned (status {code}); the step's output is not valid")
+
+
 def check_status(device) -> None:
     """Reads the status word of the tcgen05 kernels if one of them ran on ``device`` since the last check, and
     raises ``KernelError`` if a bounded wait gave up (the kernel's output is then not to be trusted).  It
@@ -506,14 +551,7 @@ def check_status(device) -> None:
     if device not in _tc5_launched:
         return
     _tc5_launched.discard(device)
-    t = _tc5_status.get(device)
-    if t is None:
-        return
-    code = int(t.item())
-    if code != 0:
-        t.zero_()
-        raise KernelError(f"a kernel on {device} gave up a bounded wait (an mbarrier, or the other CTAs of its grid) or "
-                          f"found its shared memory misaligned (status {code}); the step's output is not valid")
+    raise_status(device, int(tc5_status(device).item()))
 
 
 def gemm_tc5(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False, simple_bn: int = 0,
@@ -526,16 +564,15 @@ def gemm_tc5(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = 
     assert x.dtype == w.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32)
     assert w.shape[1] == K and out.shape == (M, N // 2 if gated else N)
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
-    status = tc5_status(x.device)
+    status = _status_word(x.device)
     f32 = 1 if out.dtype == torch.float32 else 0
     if simple_bn:
         rc = tc5_lib().rb_tc5_gemm_simple(_ptr(x), _ptr(w), _ptr(out), f32, simple_bn, M, N, K, x.stride(0),
-                                          w.stride(0), out.stride(0), _ptr(status), _stream())
+                                          w.stride(0), out.stride(0), status, _stream())
     else:
         fn = tc5_lib().rb_tc5_gemm_pair if pair else tc5_lib().rb_tc5_gemm
         rc = fn(_ptr(x), _ptr(w), _ptr(out), f32, _gated_code(gated, act), M, N, K, x.stride(0),
-                w.stride(0), out.stride(0), _ptr(status), _stream())
-    _tc5_launched.add(x.device)
+                w.stride(0), out.stride(0), status, _stream())
     _check(rc, "gemm_tc5")
 
 
@@ -559,7 +596,7 @@ def gemm_stream(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     _check(tc5_lib().rb_gemm_stream(_ptr(x), _ptr(w), _ptr(out), 1 if out.dtype == torch.float32 else 0,
                                     1 if gated else 0, M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                                    _ptr(tc5_status(x.device)), _stream()), "gemm_stream")
+                                    _status_word(x.device), _stream()), "gemm_stream")
 
 
 def gemm_stream_plan(M: int, N: int, K: int, gated: bool = False):
@@ -576,7 +613,7 @@ def gemm_tc5_bmn(x: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int = 
     N = b.shape[1]
     assert x.dtype == b.dtype == torch.bfloat16 and out.dtype == torch.float32 and b.shape[0] == K
     _check(tc5_lib().rb_tc5_gemm_bmn(_ptr(x), _ptr(b), _ptr(out), bn, M, N, K, x.stride(0), b.stride(0), out.stride(0),
-                                     _ptr(tc5_status(x.device)), _stream()), "gemm_tc5_bmn")
+                                     _status_word(x.device), _stream()), "gemm_tc5_bmn")
 
 
 # Where the kernel for the rows of an ordinary step is the fastest way.  As kernels alone the library's are 5-25 % faster from some 30 rows on
@@ -620,8 +657,7 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool =
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
     rc = tc5_lib().rb_gemm_rows(_ptr(x), _ptr(w), _ptr(out), 1 if out.dtype == torch.float32 else 0, _gated_code(gated, act or "silu"),
                                 ACTIVATIONS[act] if act is not None and not gated else -1, M, N, K, x.stride(0), w.stride(0), out.stride(0),
-                                tiles, log2_split, _ptr(tc5_status(x.device)), _stream())
-    _tc5_launched.add(x.device)
+                                tiles, log2_split, _status_word(x.device), _stream())
     _check(rc, "gemm_rows")
 
 
@@ -656,8 +692,7 @@ def gemm_rows_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
     rc = tc5_lib().rb_gemm_rows_fused(_ptr(x), _ptr(w), _ptr(out), 1 if gated else 0, M, N, K, x.stride(0), w.stride(0),
                                       out.stride(0) if out is not None else 0, _ptr(ssq_in), ssq_in_count, norm_dim, eps, _ptr(stream),
                                       _ptr(norm_w), norm_w_dtype, offset, _ptr(ssq_out), ld_sums, tiles, log2_split,
-                                      _ptr(tc5_status(x.device)), _stream())
-    _tc5_launched.add(x.device)
+                                      _status_word(x.device), _stream())
     _check(rc, "gemm_rows_fused")
 
 
@@ -853,7 +888,6 @@ def attention_prefill_tc5(qkv, k_pool, v_pool, tiles, cu_q, seg_pos0, block_tabl
     assert tiles.dtype == torch.int32 and tiles.is_contiguous()
     lib = attention_tc5_lib(head_dim)
     T = qkv.shape[0]
-    _tc5_launched.add(qkv.device)
     scratch = None
     if num_splits > 1:
         key = ("attention.prefill_split_scratch", num_splits, T, num_heads, head_dim)
@@ -865,7 +899,7 @@ def attention_prefill_tc5(qkv, k_pool, v_pool, tiles, cu_q, seg_pos0, block_tabl
     _check(lib.rb_attn_prefill_tc5_mod(_ptr(qkv), qkv.stride(0), _ptr(k_pool), _ptr(v_pool), _ptr(tiles),
                                        tiles.shape[0], _ptr(cu_q), _ptr(seg_pos0), _ptr(block_table),
                                        block_table.stride(0), page_size, _ptr(out), num_heads, num_kv_heads, scale,
-                                       int(window or 0), num_splits, _ptr(scratch), T, _ptr(tc5_status(qkv.device)),
+                                       int(window or 0), num_splits, _ptr(scratch), T, _status_word(qkv.device),
                                        _sink_ptr(sink, num_heads), int(chunk or 0), float(softcap or 0.0),
                                        _sink_ptr(slopes, num_heads), *_bias_args(bias, num_heads), int(keep or 0), int(share), _stream()),
            "attention_prefill_tc5", 2 if num_splits > 1 else 1)
@@ -1410,7 +1444,6 @@ def chunked_scan(mode: int, q, k, v, gate_a, gate_b, state, s_off: int, batch, c
         assert extra is not None and extra.dtype == torch.float32 and extra.is_contiguous()
         assert extra.numel() == (heads * dim if mode == SCAN_BONUS else heads)
     lib = recurrent_lib()
-    _tc5_launched.add(out.device)
     per = lib.rb_chunked_scan_floats(mode, heads, dim)
     window = max(1, min(chunks, CHUNK_SCRATCH_BYTES // (4 * per)))
     scratch = (buffer or (lambda name, shape, dtype, device: torch.empty(shape, dtype=dtype, device=device)))(
@@ -1420,7 +1453,7 @@ def chunked_scan(mode: int, q, k, v, gate_a, gate_b, state, s_off: int, batch, c
             mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), _is_f32(q), _is_f32(k), _is_f32(v),
             _ptr(gate_a), _ptr(gate_b), _ptr(extra), 1.0, _ptr(state), state.stride(0), s_off, _ptr(batch.cu_q), _ptr(batch.seg_slot),
             _ptr(scratch), _ptr(out), heads, kv_heads, dim, vdim, batch.num_segments, min_tokens, batch.num_segments if longs is None else longs, first, min(window, chunks - first),
-            _ptr(tc5_status(out.device)), _stream()), "chunked_scan", 2)
+            _status_word(out.device), _stream()), "chunked_scan", 2)
 
 
 def scan_pieces_combine(pieces, state, s_off: int, decay, cu_piece, seg_first, seg_slot, per_head: int, total: int,
@@ -1991,9 +2024,8 @@ def moe_tc5_gemm(x_sorted, w, offsets, out, act: Optional[str] = None) -> None:
     places = out.shape[0]
     assert x_sorted.dtype == w.dtype == out.dtype == torch.bfloat16 and x_sorted.stride(1) == 1 and w.is_contiguous()
     assert x_sorted.shape == (places, K) and out.shape[1] == N and out.stride(1) == 1
-    _tc5_launched.add(x_sorted.device)
     _check(moe_tc5_lib().rb_moe_tc5_gemm(_ptr(x_sorted), x_sorted.stride(0), _ptr(w), _ptr(offsets), E, _ptr(out), out.stride(0),
-                                         places, N, K, _act_code(act), _ptr(tc5_status(x_sorted.device)), _stream()), "moe_tc5_gemm")
+                                         places, N, K, _act_code(act), _status_word(x_sorted.device), _stream()), "moe_tc5_gemm")
 
 
 def moe_tc5_gated(x_sorted, w, offsets, out, limit: float, alpha: float, shift: float = 1.0, weight=None, pair_at=None) -> None:
@@ -2005,10 +2037,9 @@ def moe_tc5_gated(x_sorted, w, offsets, out, limit: float, alpha: float, shift: 
     assert x_sorted.shape == (places, K) and N == 2 * out.shape[1] and out.stride(1) == 1
     assert weight is None or (weight.dtype == torch.float32 and weight.numel() == places and weight.is_contiguous())
     assert pair_at is None or (pair_at.dtype == torch.int32 and pair_at.numel() == places)
-    _tc5_launched.add(x_sorted.device)
     _check(moe_tc5_lib().rb_moe_tc5_gated(_ptr(x_sorted), x_sorted.stride(0), _ptr(w), _ptr(offsets), E, _ptr(out), out.stride(0), places,
                                           N // 2, K, float(limit), float(alpha), float(shift), _ptr(weight), _ptr(pair_at),
-                                          _ptr(tc5_status(x_sorted.device)), _stream()), "moe_tc5_gated")
+                                          _status_word(x_sorted.device), _stream()), "moe_tc5_gated")
 
 
 # From this many (token, expert) pairs on, a step's experts run as tiles on the tensor cores over the pairs sorted by

@@ -51,11 +51,15 @@ class Sampler:
         self._out_host = [torch.empty(2 * n, dtype=torch.float32).pin_memory() for _ in range(self.SLOTS)]
         self._done = [torch.cuda.Event() for _ in range(self.SLOTS)]
         self._rows = [0] * self.SLOTS
+        self._status = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(self.SLOTS)]
+        self._has_status = [False] * self.SLOTS
 
-    def launch(self, logits: torch.Tensor, params: Sequence[Tuple[float, int, float, float]], slot: int = 0) -> torch.Tensor:
+    def launch(self, logits: torch.Tensor, params: Sequence[Tuple[float, int, float, float]], slot: int = 0,
+               status: bool = False) -> torch.Tensor:
         """Starts the sampling of one token per row; ``params``: per row (temperature, top_k, top_p,
         uniform draw).  Returns the tokens as an int32 device tensor (valid in stream order until the
-        next launch); ``fetch(slot)`` waits and brings them to the host."""
+        next launch); ``fetch(slot)`` waits and brings them to the host.  ``status``: the word in which kernels say that a
+        bounded wait gave up comes along, and ``fetch`` raises ``KernelError`` if one did."""
         n = logits.shape[0]
         assert n == len(params) and n > 0
         if n > self._cap:
@@ -73,6 +77,7 @@ class Sampler:
         lps = self._out_dev[n:2 * n]
         ops.sample(logits, d[0:n], d[n:2 * n].view(torch.int32), d[2 * n:3 * n], d[3 * n:4 * n], toks, lps)
         self._out_host[slot][:2 * n].copy_(self._out_dev[:2 * n], non_blocking=True)
+        self._has_status[slot] = status and ops.copy_status(self.device, self._status[slot])
         self._done[slot].record()
         self._rows[slot] = n
         return toks
@@ -81,6 +86,8 @@ class Sampler:
         """Tokens and log-probabilities of the launch in ``slot``, once they have arrived."""
         n = self._rows[slot]
         self._done[slot].synchronize()
+        if self._has_status[slot]:
+            ops.raise_status(self.device, int(self._status[slot][0]))
         out = self._out_host[slot].numpy()
         return out[:n].view(np.int32).tolist(), out[n:2 * n].tolist()
 
