@@ -114,6 +114,7 @@ attention_f32_kernel(const Args a) {
     const int by_head = blockIdx.x % (a.Hkv * splits), nth = blockIdx.x / (a.Hkv * splits), columns = (a.T + a.tb - 1) / a.tb;
     const int t0 = (nth % columns) * a.tb + nth / columns;
     if (t0 >= a.T) return;
+    pdl_wait();                                                        // the tables may be the work of the kernel before this one
     const int seg = a.tok_seg[t0], p0 = a.pos[t0];
     if (t0 > 0 && a.tok_seg[t0 - 1] == seg && a.pos[t0 - 1] == p0 - 1 && p0 % a.tb != 0) return;   // an earlier token's CTA takes this one along
     const int until = a.tb - p0 % a.tb;
@@ -131,7 +132,6 @@ attention_f32_kernel(const Args a) {
     float* inv_s = alpha_s + ROWS;
     __shared__ int page_of[2][KEYS], from_s[ROWS], to_s[ROWS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t2 = 2 * (lane & 3);
-    pdl_wait();
     const int* bt = a.block_table + (size_t)seg * a.bt_stride;
     const size_t head_stride = (size_t)a.page_size * D;
     auto q_row = [&](int row) { return a.q + (size_t)(t0 + row / nh) * a.ld + (size_t)(kvh * G + g0 + row % nh) * D; };

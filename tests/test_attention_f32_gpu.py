@@ -90,3 +90,27 @@ def test_rows_do_not_depend_on_their_block():
     for t in (0, 15, 16, 17, 64, 129, 130, 132, 133, 149, 150):
         assert torch.equal(run(rows[t:t + 1])[0], whole[t]), t
     assert torch.equal(run(rows.flip(0)), whole.flip(0))
+
+
+def test_tables_written_by_the_kernel_just_before():
+    """The launch overlaps the kernel before it, so the tables are read behind the wait for that kernel."""
+    from return_b200.ext import ops
+    pg = Paged([130, 70, 1], [130, 3, 1], 4, 2, 64, 16, torch.float32, seed=4)
+    order = torch.randperm(134, generator=torch.Generator().manual_seed(1)).to(DEV)
+    sets = [(pg.qkv, pg.pos, pg.tok_seg), tuple(t[order].contiguous() for t in (pg.qkv, pg.pos, pg.tok_seg))]
+    tables = types.SimpleNamespace(pos=torch.zeros_like(pg.pos), tok_seg=torch.zeros_like(pg.tok_seg))
+
+    def run(k, out):
+        qkv, pos, seg = sets[k]
+        torch.add(pos, 0, out=tables.pos)
+        torch.add(seg, 0, out=tables.tok_seg)
+        ops.paged_attention(qkv, pg.kpool, pg.vpool, tables, pg.bt, 16, out, 4, 2, 64, 0.125)
+
+    outs = [torch.full((134, 256), float("nan"), device=DEV) for _ in range(40)]
+    for i, out in enumerate(outs):
+        run(i & 1, out)
+        if i < 2:
+            torch.cuda.synchronize()
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[1], outs[0][order])
+    for i, out in enumerate(outs):
+        assert torch.equal(out, outs[i & 1]), i
