@@ -439,7 +439,7 @@ def gated_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, interleave
     if interleave == 8 and x.shape[0] >= PAIR_MIN_ROWS and pair_ok(x, w, out):
         gemm_tc5(x, w, out, gated=True, pair=True, act=act)
         return
-    if interleave == 8 and w.shape[0] % 16 == 0 and out.dtype == torch.bfloat16 and rows_ok(x, w):
+    if interleave == 8 and w.shape[0] % 16 == 0 and out.dtype == torch.bfloat16 and rows_ok(x, w, out, w.shape[0] // 2):
         gemm_rows(x, w, out, gated=True, act=act)
         return
     if ctx is not None:
@@ -637,11 +637,17 @@ def rows_limit(N: int, K: int) -> int:
     return limit
 
 
-def rows_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether the kernel for the rows of an ordinary step takes this product and is the fastest way."""
+def rows_ok(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, width: int = 0) -> bool:
+    """Whether the kernel for the rows of an ordinary step takes this product (into ``out``, of ``width`` columns), and is the fastest way.
+    What it does not take goes to the library, which copies or refuses: columns that do not lie side by side, rows that overlap (a stride
+    of zero among them), nothing to add up, several devices, an output of another shape."""
     N, K = w.shape
-    return (x.dtype == torch.bfloat16 and x.shape[0] <= rows_limit(N, K) and K % 8 == 0 and x.stride(0) % 8 == 0
-            and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+    return (0 < N * K and x.dtype == w.dtype == torch.bfloat16 and x.shape[0] <= rows_limit(N, K) and x.shape[1] == K and K % 8 == 0
+            and x.stride(1) == 1 and w.stride(1) == 1 and K <= x.stride(0) < 1 << 31 and K <= w.stride(0) < 1 << 31
+            and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+            and x.get_device() == w.get_device()
+            and (out is None or (out.shape == (x.shape[0], width) and out.dtype in (torch.bfloat16, torch.float32) and out.stride(1) == 1
+                                 and width <= out.stride(0) < 1 << 31 and out.get_device() == x.get_device())))
 
 
 def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False, act: Optional[str] = None, tiles: int = -1,
@@ -726,7 +732,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[st
     if skinny_ok(x, w):
         gemm_skinny(x, w, out, act=act, bias=bias)
         return
-    if act != "neg_exp_exp" and rows_ok(x, w):
+    if act != "neg_exp_exp" and rows_ok(x, w, out, w.shape[0]):
         gemm_rows(x, w, out, act=act)
         return
     if out.dtype == torch.float32:

@@ -136,3 +136,27 @@ def test_fused_product_refuses_what_it_cannot_take():
     x, w = torch.zeros(16, 64, device=DEV).bfloat16(), torch.zeros(130, 64, device=DEV).bfloat16()
     with pytest.raises(Exception):                            # a row of the stream that is no whole 16-byte pieces
         ops.gemm_rows_fused(x, w, None, residual=(torch.zeros(16, 130, device=DEV), None, None))
+
+
+def test_operands_that_only_the_library_takes():
+    """Strides and sizes that go past the kernel: as ``torch.mm`` takes them."""
+    ops = _ops()
+    M, N, K = 40, 64, 128
+    x, w, _, _ = _inputs(M, N, K, 6)
+    x = x.contiguous()
+    wide = torch.randn(M, 2 * K, device=DEV).bfloat16()
+    row_out = torch.empty(N, M, device=DEV, dtype=torch.bfloat16).t()
+    forms = [(x, w.t().contiguous().t(), None), (x.t().contiguous().t(), w, None), (wide[:, ::2], w, None), (x[:1].expand(M, K), w, None),
+             (wide.reshape(-1).as_strided((M, K), (8, 1)), w, None), (x, w[:1].expand(N, K), None), (x, w, row_out), (x[:, :0], w[:, :0], None), (x, w[:0], None)]
+    for i, (a, b, out) in enumerate(forms):
+        for dtype in (torch.bfloat16, torch.float32) if out is None else (torch.bfloat16,):
+            o = torch.full((M, b.shape[0]), 7.0, device=DEV, dtype=dtype) if out is None else out
+            ops.linear(a, b, o)
+            _close(o, a.double() @ b.double().T, a.double().abs() @ b.double().abs().T, K)
+    unit = torch.empty(M, N // 2, device=DEV, dtype=torch.bfloat16)
+    ops.gated_linear(x.t().contiguous().t(), w, unit, 8)
+    want = torch.empty_like(unit)
+    ops.gated_linear(x, w, want, 8)
+    assert (unit.float() - want.float()).norm() <= 2e-2 * want.float().norm()       # (the library's way rounds the two sums to bfloat16 first)
+    with pytest.raises(Exception):
+        ops.linear(x, w, torch.empty(1, N, device=DEV, dtype=torch.bfloat16).expand(M, N))
