@@ -126,6 +126,8 @@ class PreNormBlock(Block):
         nxt = ctx.next_block.first_norm() if ctx.next_block is not None and hasattr(ctx.next_block, "first_norm") else None
         if nxt is not None and nxt[3] != H:
             nxt = None
+        if T > ops.SKINNY_MAX_ROWS and not (isinstance(ctx.next_block, PreNormBlock) and ctx.next_block._fused_plan(stream)):
+            nxt = None                                         # the next block norms the stream itself: nobody would read what is left here
         if nxt is None and T > ops.SKINNY_MAX_ROWS:            # what follows adds it anyway
             y = ctx.buffer("block.delta", (T, H), dt, dev)
             ops.linear(act, down, y)
