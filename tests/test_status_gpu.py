@@ -38,7 +38,7 @@ def test_replayed_step(tmp_path, dtype, n):
     _raise_word()
     with pytest.raises(ops.KernelError, match="bounded wait"):
         eng.step()
-    eng.step()                                                # the word was read and put back
+    assert int(ops.tc5_status(DEV)) == 0                      # read and put back
 
 
 @pytest.mark.parametrize("dtype,n", [("bfloat16", 12), ("float32", 3)])
