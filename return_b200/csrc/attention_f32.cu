@@ -2,10 +2,11 @@
 // absolute positions, an online softmax a row, CTAs of up to 32 rows of neighbouring tokens that share a key/value head), its two
 // products on the matrix instructions in float32's precision.
 //
-// Operands are split into three bfloat16 parts (24 bits), six of nine products are made (the rest is below 2^-24 of a product), the
+// Operands are multiplied by 2^16 and split into three bfloat16 parts (which then hold every bit of every float32, small ones too: bfloat16 ends
+// at 2^-133), six of nine products are made (the rest is below 2^-24 of a product), the
 // largest in an accumulator of its own; a tile's 128 products of a score, or 32 of an output, are summed there, all else on the CUDA cores,
 // which round to nearest.  A row of the products is worked out by itself and in one order, so the result for a token does not
-// depend on how the prompt was cut into steps or on what else is in the batch: it is bit-identical.  An infinity or a NaN has no
+// depend on how the prompt was cut into steps or on what else is in the batch: it is bit-identical.  An infinity, a NaN or a number beyond 2^112 has no
 // parts: where a score or an output's sum over a tile is no finite number, it is made again from the operands, one FFMA behind the
 // other over what the row sees, so a value reaches only the rows that see it.
 //
@@ -24,6 +25,9 @@ namespace {
 constexpr int ROWS = 32, KEYS = 32, WARPS = 8, RW = 4;
 constexpr int SP = KEYS + 8;              // floats of a row of scores: eight-byte reads of four rows by four lanes hit all banks
 
+constexpr float UP = 65536.f, DOWN = 1.f / (UP * UP);                  // what operands are multiplied by, and sums
+constexpr unsigned long long UP2 = 0x4780000047800000ull;             // UP twice
+
 struct Parts { unsigned h, m, l; };       // of two neighbouring values, the first in the low half
 __device__ __forceinline__ unsigned pack2(float lo, float hi) {
     unsigned r;
@@ -40,6 +44,10 @@ __device__ __forceinline__ Parts split(float x, float y) {
     y -= __uint_as_float(p.m & 0xffff0000u);
     p.l = pack2(x, y);
     return p;
+}
+__device__ __forceinline__ Parts split_up(float x, float y) {         // of both times UP, one instruction
+    asm("{\n.reg .b64 v;\nmov.b64 v, {%0, %1};\nmul.rn.f32x2 v, v, %2;\nmov.b64 {%0, %1}, v;\n}" : "+f"(x), "+f"(y) : "l"(UP2));
+    return split(x, y);
 }
 __device__ __forceinline__ void mma(float (&c)[4], const uint4& a, unsigned b0, unsigned b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -60,7 +68,7 @@ struct Sums {                             // the product of the leading parts, t
         mma(mm, a.h, p.m, r.m);
         mma(hl, a.m, p.h, r.h);
     }
-    __device__ __forceinline__ float get(int i) const { return big[i] + ((mm[i] + hl[i]) + lh[i]); }
+    __device__ __forceinline__ float get(int i) const { return (big[i] + ((mm[i] + hl[i]) + lh[i])) * DOWN; }
 };
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= FLT_MAX; }
 
@@ -98,7 +106,7 @@ __device__ __noinline__ float chain(const float* a, const float* b, int n) {
 __device__ __noinline__ float chain_seen(const float* p, const float* v, int pitch, int from, int to, int kept, const int* page) {
     float x = 0.f;
     for (int j = 0; j < KEYS; ++j)
-        if (page[j] >= 0 && j <= to && (j >= from || j < kept)) x = fmaf(p[j], v[j * pitch], x);
+        if (page[j] >= 0 && j <= to && (j >= from || j < kept)) x = fmaf(p[j] * (1.f / UP), v[j * pitch], x);
     return x;
 }
 
@@ -176,7 +184,7 @@ attention_f32_kernel(const Args a) {
             const int row = ra + (i & 2 ? 8 : 0), at = d + (i & 1) + (i & 4 ? 8 : 0);
             x[i] = row < rows ? q_row(row)[at] : 0.f;
         }
-        const Parts p0_ = split(x[0], x[1]), p1 = split(x[2], x[3]), p2 = split(x[4], x[5]), p3 = split(x[6], x[7]);
+        const Parts p0_ = split_up(x[0], x[1]), p1 = split_up(x[2], x[3]), p2 = split_up(x[4], x[5]), p3 = split_up(x[6], x[7]);
         uint4* to = reinterpret_cast<uint4*>(qp + c * 384) + lane;
         to[0] = make_uint4(p0_.h, p1.h, p2.h, p3.h);
         to[32] = make_uint4(p0_.m, p1.m, p2.m, p3.m);
@@ -222,7 +230,7 @@ attention_f32_kernel(const Args a) {
             for (int k = 0; k < KT; ++k) {
                 const First x = {qa[k * 96], qa[k * 96 + 32], qa[k * 96 + 64]};
                 const float2 b0 = *reinterpret_cast<const float2*>(kr + 16 * k), b1 = *reinterpret_cast<const float2*>(kr + 16 * k + 8);
-                s.add(x, split(b0.x, b0.y), split(b1.x, b1.y));
+                s.add(x, split_up(b0.x, b0.y), split_up(b1.x, b1.y));
             }
 #pragma unroll
             for (int e = 0; e < 4; e += 2) {
@@ -275,7 +283,7 @@ attention_f32_kernel(const Args a) {
                 const float e = expf(sc[i] - mx[i]);
                 pj[i] = valid[i] ? e : 0.f;
                 sum[i] = pj[i];
-                Ps[(r0 + i) * SP + lane] = pj[i];
+                Ps[(r0 + i) * SP + lane] = pj[i] * UP;
             }
 #pragma unroll
             for (int w = 16; w > 0; w >>= 1)
@@ -314,8 +322,8 @@ attention_f32_kernel(const Args a) {
                 for (int j = 0; j < NT; ++j) {
                     const int col = 8 * (warp + WARPS * j) + g;
                     const float* vr = vs + (16 * k + t2) * VP + (col < D ? col : 0);
-                    v0[j] = split(vr[0], vr[VP]);
-                    v1[j] = split(vr[8 * VP], vr[9 * VP]);
+                    v0[j] = split_up(vr[0], vr[VP]);
+                    v1[j] = split_up(vr[8 * VP], vr[9 * VP]);
                 }
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {

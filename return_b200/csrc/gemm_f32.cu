@@ -1,6 +1,6 @@
 // Matrix product of the 32-bit path: C[M,N] = A[M,K] * W[N,K]^T in float32's precision, on the fifth-generation tensor cores.
 //
-// Every operand is split into three bfloat16 parts, x = h + m + l (24 bits: nothing of a float32 is lost), and six of the nine
+// Every operand is multiplied by 2^16 and split into three bfloat16 parts, 2^16 x = h + m + l, and six of the nine
 // products are made (hh, hm, mh, hl, mm, lh; the other three are below 2^-24 of a product), each exactly, the largest in an
 // accumulator of its own.  A tensor core's accumulator cuts off what it cannot hold instead of rounding, so it sums 128 values of k
 // at most; from there on sums are made on the CUDA cores, which round to nearest.  An element's sum has one order: K is
@@ -9,8 +9,10 @@
 // which of the shapes below computed it.  Error against 64 bits (2-norm over that of the result, normal operands): 1.3e-7 at K = 1,024,
 // 1.4e-7 at 3,072, where a chain of FFMAs over k has 5.7e-7 and 9.9e-7.
 //
-// An infinity or a NaN has no parts, and neither has a number beyond 3.38e38: where a result is no finite number, its
-// sum is made once more from the operands themselves, one FFMA behind the other over k.
+// The factor is there for small operands: bfloat16 ends at 2^-133, where the last bits of a number below 2^-109 would lie; times 2^16
+// the parts hold every bit of every float32.  (It takes the warps that split one more instruction a pair: 2,048 x 4,096 x 1,024 145 -> 153 us.)
+// An infinity or a NaN has no parts, and neither has a number beyond 2^112, and sums end at 2^96: where a result is no finite
+// number, it is made once more from the operands themselves, one FFMA behind the other over k.
 #include <float.h>
 
 #include "tc5.cuh"
@@ -38,6 +40,8 @@ constexpr int BM = 128;                    // weight rows of a CTA
 constexpr int RUN = 2;                     // blocks that one accumulator sums
 constexpr int GROUPS = 4;                  // groups of blocks of one sum
 constexpr int STAGES = 2;
+constexpr float UP = 65536.f, DOWN = 1.f / (UP * UP);                      // what operands are multiplied by, and sums
+constexpr unsigned long long UP2 = 0x4780000047800000ull;                 // UP twice
 constexpr int CONV = 256, DRAIN = 256, W_DRAIN = 8, W_MMA = 16, THREADS = 19 * 32;
 
 template <int BN> struct Shape {
@@ -82,8 +86,12 @@ __device__ __forceinline__ void tmem_ld8(unsigned taddr, unsigned (&r)[8]) {
 __device__ __forceinline__ void less(unsigned parts, float& x, float& y) {
     asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\nsub.rn.f32.bf16 %0, lo, %0;\nsub.rn.f32.bf16 %1, hi, %1;\n}" : "+f"(x), "+f"(y) : "r"(parts));
 }
+__device__ __forceinline__ void scaled_up(float& x, float& y) {          // times UP, both in one instruction
+    asm("{\n.reg .b64 v;\nmov.b64 v, {%0, %1};\nmul.rn.f32x2 v, v, %2;\nmov.b64 {%0, %1}, v;\n}" : "+f"(x), "+f"(y) : "l"(UP2));
+}
 __device__ __forceinline__ unsigned upper(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
 __device__ __forceinline__ void split(float x, float y, unsigned& h, unsigned& m, unsigned& l) {
+    scaled_up(x, y);
     h = __byte_perm(__float_as_uint(x) + 0x8000u, __float_as_uint(y) + 0x8000u, 0x7632);
     less(h, x, y);
     m = upper(x, y);
@@ -270,6 +278,7 @@ gemm_f32_kernel(const Args g) {
     auto leave = [&](int t, int r, float v) {               // tile row t, weight row r of the tile
         const int n = n0 + r;
         if (t < rows && n < g.N) {
+            v *= DOWN;
             if (!(fabsf(v) <= FLT_MAX)) v = chain(g.A + (size_t)(m0 + t) * g.lda, g.W + (size_t)n * g.ldw, g.K);
             g.C[(size_t)(m0 + t) * g.ldc + n] = v;
         }

@@ -114,3 +114,26 @@ def test_tables_written_by_the_kernel_just_before():
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[1], outs[0][order])
     for i, out in enumerate(outs):
         assert torch.equal(out, outs[i & 1]), i
+
+
+@pytest.mark.parametrize("q_up,k_up,v_up", [(100, -118, 0), (0, 0, -115), (-118, 105, 60)])
+def test_small_operands_keep_their_24_bits(q_up, k_up, v_up):
+    """Queries, keys and values times powers of two: the same scores and the same softmax, also where an operand's last bits lie below
+    bfloat16's smallest number."""
+    from return_b200.ext import ops
+    pg = Paged([100, 70], [100, 30], 4, 2, 64, 16, torch.float32, seed=12)
+    plain, _ = _both(pg, 4, 2, 64, 16)
+    q_cols = 4 * 64
+    pg.qkv[:, :q_cols] *= 2.0 ** q_up
+    pg.kpool *= 2.0 ** k_up
+    pg.vpool *= 2.0 ** v_up
+    batch = types.SimpleNamespace(pos=pg.pos, tok_seg=pg.tok_seg)
+    outs = []
+    for k, v in ((pg.kpool, pg.vpool), (_off(pg.kpool), _off(pg.vpool))):
+        out = torch.full((130, q_cols), float("nan"), device=DEV)
+        ops.paged_attention(pg.qkv, k, v, batch, pg.bt, 16, out, 4, 2, 64, 0.125 * 2.0 ** -(q_up + k_up))
+        outs.append(out.double() * 2.0 ** -v_up)
+    got, want = outs
+    assert torch.isfinite(got).all()
+    assert (got - want).abs().max() <= 2e-6 * max(1.0, float(want.abs().max()))
+    assert (got - plain.double()).abs().max() <= 2e-6 * max(1.0, float(want.abs().max()))

@@ -78,3 +78,28 @@ def test_numbers_without_parts(kind):
     assert torch.equal(got[want.isinf()], want[want.isinf()])
     fine = want.isfinite()
     assert ((got - want).abs()[fine] <= 1e-4 * want.abs()[fine] + 1e-3).all()
+
+
+@pytest.mark.parametrize("x_up,w_up", [(-120, 100), (-60, 60), (-140, 110), (-110, -25), (90, 3)])
+@pytest.mark.parametrize("kind", [-1, 0, 5, 11])
+def test_small_and_large_operands_keep_their_24_bits(x_up, w_up, kind):
+    """Powers of two times ordinary operands, down to numbers with fewer bits than 24 and products next to the smallest.  Where nothing leaves
+    the range the bits are those of the ordinary operands, and everywhere the error is theirs (and a rounding to float32's smallest
+    step for a result that small)."""
+    ops = _ops()
+    torch.manual_seed(9)
+    M, N, K = 37, 130, 260
+    x, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV).clamp(-3.9, 3.9)
+    plain, out = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_f32(x, w, plain, kind=kind)
+    xs, ws = (x.double() * 2.0 ** x_up).float(), (w.double() * 2.0 ** w_up).float()
+    ops.gemm_f32(xs, ws, out, kind=kind)
+    ops.check_status(x.device)
+    if x_up > -100 and x_up + w_up < 90:
+        assert torch.equal(out.double(), plain.double() * 2.0 ** (x_up + w_up))
+    exact, size = xs.double() @ ws.double().T, xs.double().abs() @ ws.double().abs().T
+    roundings = 3 * 2.0 ** -24 + 13 * 2.0 ** -23 + (K / 128 + 4) * 2.0 ** -24
+    if x_up == 90:                                            # sums beyond 2^96: a chain of K fused multiply-adds
+        roundings = K * 2.0 ** -24
+    assert ((out.double() - exact).abs() <= size * roundings + 2.0 ** -149).all()
+    assert exact.abs().max() > 0 and torch.isfinite(out).all()
