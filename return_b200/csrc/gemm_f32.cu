@@ -166,7 +166,7 @@ gemm_f32_kernel(const Args g) {
         const unsigned to0 = sw128_offset(r0, lane & 7);
         const float* w0 = g.W + (size_t)(n0 + r0) * g.ldw + k0;
         const float* a0 = g.A + (size_t)(m0 + r0) * g.lda + k0;
-        const int w_step = ROWS * g.ldw, a_step = ROWS * g.lda;
+        const size_t w_step = (size_t)ROWS * g.ldw, a_step = (size_t)ROWS * g.lda;
         unsigned live = 0;                                  // a bit a row: it exists
 #pragma unroll
         for (int u = 0; u < S::TASKS; ++u)
@@ -175,7 +175,7 @@ gemm_f32_kernel(const Args g) {
 #pragma unroll
         for (int u = 0; u < S::TASKS; ++u) x[u] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
         auto fetch = [&](int u, int b) {
-            const float* p = (u < W_TASKS ? w0 + (size_t)u * w_step : a0 + (size_t)(u - W_TASKS) * a_step) + b * BK;
+            const float* p = (u < W_TASKS ? w0 + u * w_step : a0 + (u - W_TASKS) * a_step) + b * BK;
             if (live >> u & 1) x[u] = WHOLE ? whole_piece(p) : part_of_piece(p, g.K - b * BK - k0);
         };
         if (b_begin < b_end) {
@@ -363,7 +363,6 @@ int pick(int M, int N, int K, int sms) {
     for (int kind = 0; kind < 12; ++kind) {
         const int bn = WIDTHS[kind / 3], split = SPLITS[kind % 3];
         const long long tiles_m = (M + bn - 1) / bn, ctas = tiles_m * ((N + BM - 1) / BM) * split, rounds = (ctas + sms - 1) / sms;
-        if (tiles_m > 65535) continue;                      // where the grid ends
         const long long blocks = GROUPS / split * per < nb ? GROUPS / split * per : nb;
         const long long cost = rounds * (blocks * BLOCK_COST[kind / 3] + FIXED_COST[kind / 3] + (split > 1 ? EXCHANGE_COST : 0));
         if (best_cost < 0 || cost < best_cost) { best = kind; best_cost = cost; }
@@ -381,10 +380,15 @@ RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N
     const int whole = K % BK == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
     const int sms = rb_num_sms();
     if (sms <= 0) return (int)cudaErrorInvalidDevice;
-    if (kind < 0) kind = pick(M, N, K, sms);
     if (kind >= 12) return (int)cudaErrorInvalidValue;
+    constexpr int MOST = 65535 * 16;                        // rows of a launch: its grid ends there with the narrowest tiles
+    for (long long m = MOST; m < M; m += MOST) {
+        const int rc = rb_gemm_f32(A + m * lda, W, C + m * ldc, (int)(M - m < MOST ? M - m : MOST), N, K, lda, ldw, ldc, kind, status, st);
+        if (rc) return rc;
+    }
+    if (M > MOST) M = MOST;
+    if (kind < 0) kind = pick(M, N, K, sms);
     const int bn = WIDTHS[kind / 3], tiles = (M + bn - 1) / bn;
-    if (tiles > 65535) return (int)cudaErrorInvalidValue;
     const Args g = {A, W, C, M, N, K, lda, ldw, ldc, whole, (M + tiles - 1) / tiles, status};
     switch (kind) {
         case 0: return launch<80, 1>(g, st);

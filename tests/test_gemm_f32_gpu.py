@@ -103,3 +103,36 @@ def test_small_and_large_operands_keep_their_24_bits(x_up, w_up, kind):
         roundings = K * 2.0 ** -24
     assert ((out.double() - exact).abs() <= size * roundings + 2.0 ** -149).all()
     assert exact.abs().max() > 0 and torch.isfinite(out).all()
+
+
+def test_rows_far_apart():
+    """32 rows times their stride pass 31 bits.  (The rows lie in 9 GB of which only they are touched.)"""
+    ops = _ops()
+    torch.manual_seed(1)
+    M, N, K, ld = 34, 130, 128, 1 << 26
+    far = torch.empty(ld * (M - 1) + K, device=DEV).as_strided((M, K), (ld, 1))
+    near, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    far.copy_(near)
+    out, want = torch.full((M, N), float("nan"), device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_f32(near, w, want)
+    ops.gemm_f32(far, w, out)
+    assert torch.equal(out, want)
+    out = torch.full((N, M), float("nan"), device=DEV)
+    ops.gemm_f32(w, far, out)                                 # as weight rows
+    assert (out - want.t()).abs().max() <= 1e-4
+    ops.check_status(far.device)
+
+
+def test_more_rows_than_a_launch_has_tiles():
+    ops = _ops()
+    torch.manual_seed(2)
+    M, K = 65535 * 16 + 19, 100
+    x, w = torch.randn(M, K, device=DEV), torch.randn(3, K, device=DEV)
+    for kind in (-1, 9):
+        out = torch.full((M, 3), float("nan"), device=DEV)
+        ops.gemm_f32(x, w, out, kind=kind)
+        ends = torch.cat((torch.arange(40), torch.arange(65535 * 16 - 40, M))).to(DEV)
+        want = torch.empty(len(ends), 3, device=DEV)
+        ops.gemm_f32(x[ends], w, want, kind=kind)
+        assert torch.equal(out[ends], want) and torch.isfinite(out).all()
+    ops.check_status(x.device)
