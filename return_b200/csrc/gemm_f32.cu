@@ -57,10 +57,13 @@ template <int BN> struct Shape {
     static_assert(BN % 16 == 0 && BUF <= 256 && GROUPS * (BN / 2) * BM * 4 <= STAGES * (int)STAGE_BYTES, "sizes of an MMA and of the exchange");
 };
 
+// What a row of both operands is: whole blocks of 64; whole pieces of four values, 16 bytes aligned like those; anything.
+constexpr int ROW_WHOLE = 0, ROW_QUADS = 1, ROW_ANY = 2;
+
 struct Args {
     const float* A; const float* W; float* C;
     int M, N, K, lda, ldw, ldc;
-    int whole;                             // rows of whole blocks of 64, 16 bytes aligned
+    int row;                               // ROW_WHOLE, ROW_QUADS or ROW_ANY
     int tile_m;                            // rows of C of a tile: at most BN
     int* status;
 };
@@ -110,14 +113,18 @@ struct Piece { float4 lo, hi; };           // eight values of k of a row
 __device__ __forceinline__ Piece whole_piece(const float* p) {
     return {*reinterpret_cast<const float4*>(p), *reinterpret_cast<const float4*>(p + 4)};
 }
-__device__ __forceinline__ Piece part_of_piece(const float* p, int left) {       // `left`: values that exist from p on
+__device__ __forceinline__ Piece quads_of_piece(const float* p, int left) {      // `left`: values that exist from p on, a multiple of four
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    return {left > 0 ? *reinterpret_cast<const float4*>(p) : none, left > 4 ? *reinterpret_cast<const float4*>(p + 4) : none};
+}
+__device__ __forceinline__ Piece part_of_piece(const float* p, int left) {
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = i < left ? p[i] : 0.f;
     return {make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7])};
 }
 
-template <int BN, int SPLIT, bool WHOLE>
+template <int BN, int SPLIT, int ROW>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_kernel(const Args g) {
     using S = Shape<BN>;
@@ -176,7 +183,8 @@ gemm_f32_kernel(const Args g) {
         for (int u = 0; u < S::TASKS; ++u) x[u] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
         auto fetch = [&](int u, int b) {
             const float* p = (u < W_TASKS ? w0 + u * w_step : a0 + (u - W_TASKS) * a_step) + b * BK;
-            if (live >> u & 1) x[u] = WHOLE ? whole_piece(p) : part_of_piece(p, g.K - b * BK - k0);
+            const int left = g.K - b * BK - k0;
+            if (live >> u & 1) x[u] = ROW == ROW_WHOLE ? whole_piece(p) : ROW == ROW_QUADS ? quads_of_piece(p, left) : part_of_piece(p, left);
         };
         if (b_begin < b_end) {
 #pragma unroll
@@ -323,12 +331,12 @@ gemm_f32_kernel(const Args g) {
     if (warp == W_MMA) tmem_dealloc(tmem, S::TMEM);
 }
 
-template <int BN, int SPLIT, bool WHOLE>
+template <int BN, int SPLIT, int ROW>
 int launch_as(const Args& g, cudaStream_t st) {
     constexpr unsigned smem = SPLIT > 1 ? Shape<BN>::CLUSTER_BYTES : Shape<BN>::NEED_BYTES;
     static PerDevice configured;
     const int rc = configured.once([&](int) {
-        return cudaFuncSetAttribute(gemm_f32_kernel<BN, SPLIT, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return cudaFuncSetAttribute(gemm_f32_kernel<BN, SPLIT, ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
     if (rc) return rc;
     cudaLaunchAttribute attr[2];
@@ -345,11 +353,14 @@ int launch_as(const Args& g, cudaStream_t st) {
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = RB_PDL_MODE == 3 ? 1 : 2;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BN, SPLIT, WHOLE>, g);
+    return (int)cudaLaunchKernelEx(&cfg, gemm_f32_kernel<BN, SPLIT, ROW>, g);
 }
 
 template <int BN, int SPLIT>
-int launch(const Args& g, cudaStream_t st) { return g.whole ? launch_as<BN, SPLIT, true>(g, st) : launch_as<BN, SPLIT, false>(g, st); }
+int launch(const Args& g, cudaStream_t st) {
+    if (g.row == ROW_WHOLE) return launch_as<BN, SPLIT, ROW_WHOLE>(g, st);
+    return g.row == ROW_QUADS ? launch_as<BN, SPLIT, ROW_QUADS>(g, st) : launch_as<BN, SPLIT, ROW_ANY>(g, st);
+}
 
 // Which shape: the one whose busiest SM is done first.  Measured, in units of 10 ns: what a CTA takes for a block of 64, for its set-up
 // and end, and for the exchange of a cluster's sums.  One round of CTAs after the other: 240 of them take twice what 148 do.
@@ -377,7 +388,8 @@ int pick(int M, int N, int K, int sms) {
 RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K,
                           int lda, int ldw, int ldc, int kind, int* status, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
-    const int whole = K % BK == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    const bool quads = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+    const int row = !quads ? ROW_ANY : K % BK == 0 ? ROW_WHOLE : ROW_QUADS;
     const int sms = rb_num_sms();
     if (sms <= 0) return (int)cudaErrorInvalidDevice;
     if (kind >= 12) return (int)cudaErrorInvalidValue;
@@ -389,7 +401,7 @@ RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N
     if (M > MOST) M = MOST;
     if (kind < 0) kind = pick(M, N, K, sms);
     const int bn = WIDTHS[kind / 3], tiles = (M + bn - 1) / bn;
-    const Args g = {A, W, C, M, N, K, lda, ldw, ldc, whole, (M + tiles - 1) / tiles, status};
+    const Args g = {A, W, C, M, N, K, lda, ldw, ldc, row, (M + tiles - 1) / tiles, status};
     switch (kind) {
         case 0: return launch<80, 1>(g, st);
         case 1: return launch<80, 2>(g, st);

@@ -136,3 +136,22 @@ def test_more_rows_than_a_launch_has_tiles():
         ops.gemm_f32(x[ends], w, want, kind=kind)
         assert torch.equal(out[ends], want) and torch.isfinite(out).all()
     ops.check_status(x.device)
+
+
+@pytest.mark.parametrize("K", [132, 188, 196, 252, 316, 1000])
+def test_rows_of_whole_pieces_of_four(K):
+    """They are fetched 16 bytes at a time and give the bits that they give one value at a time; what lies behind a row is not read."""
+    ops = _ops()
+    torch.manual_seed(K)
+    M, N = 85, 140
+    wide = torch.full((M + N, K + 4), float("nan"), device=DEV)
+    wide[:, :K] = torch.randn(M + N, K, device=DEV)
+    x, w = wide[:M, :K], wide[M:, :K]
+    off = torch.empty((M + N) * (K + 4) + 1, device=DEV)[1:].view(M + N, K + 4)
+    off.copy_(wide)
+    for kind in (-1, 0, 4, 11):
+        out, want = torch.full((M, N), float("nan"), device=DEV), torch.empty(M, N, device=DEV)
+        ops.gemm_f32(x, w, out, kind=kind)
+        ops.gemm_f32(off[:M, :K], off[M:, :K], want, kind=kind)
+        assert torch.equal(out, want) and torch.isfinite(out).all()
+    ops.check_status(x.device)
