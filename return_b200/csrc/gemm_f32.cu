@@ -383,6 +383,10 @@ int pick(int M, int N, int K, int sms) {
 
 }  // namespace
 
+// gemm_f32_short.cu: sums of few values
+int rb_gemm_f32_short_takes(int K);
+int rb_gemm_f32_short(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, int kind, int sms, cudaStream_t st);
+
 // kind: -1 the engine's choice; 0..11 a shape, 3 * (place in WIDTHS) + (place in SPLITS) (measurements and tests; any choice gives the same
 // bits).  status: one int in device memory, set to 1 if a wait inside the kernel gave up.
 RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K,
@@ -393,6 +397,7 @@ RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N
     const int sms = rb_num_sms();
     if (sms <= 0) return (int)cudaErrorInvalidDevice;
     if (kind >= 12) return (int)cudaErrorInvalidValue;
+    if (rb_gemm_f32_short_takes(K)) return rb_gemm_f32_short(A, W, C, M, N, K, lda, ldw, ldc, kind, sms, st);
     constexpr int MOST = 65535 * 16;                        // rows of a launch: its grid ends there with the narrowest tiles
     for (long long m = MOST; m < M; m += MOST) {
         const int rc = rb_gemm_f32(A + m * lda, W, C + m * ldc, (int)(M - m < MOST ? M - m : MOST), N, K, lda, ldw, ldc, kind, status, st);

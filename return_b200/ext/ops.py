@@ -69,7 +69,7 @@ PDL_MODE = 2
 
 _core = None
 
-_CORE_SOURCES = ["elementwise.cu", "gemm_f32.cu", "gemm_skinny.cu", "rope_cache.cu", "attention_simt.cu", "attention_f32.cu", "sampling.cu",
+_CORE_SOURCES = ["elementwise.cu", "gemm_f32.cu", "gemm_f32_short.cu", "gemm_skinny.cu", "rope_cache.cu", "attention_simt.cu", "attention_f32.cu", "sampling.cu",
                  "attention_prep.cu"]
 
 
