@@ -42,7 +42,7 @@ def _ptr(t: Optional[torch.Tensor]):
 try:                                                  # the raw handle, without building a Stream object
     _raw_stream, _device_index = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
 except AttributeError:                                # a torch without these: the public way, slower
-    _raw_stream = None
+    _raw_stream, _device_index = None, torch.cuda.current_device
 
 
 def _stream():
@@ -494,6 +494,12 @@ def tc5_status(device) -> torch.Tensor:
     return t
 
 
+def _with_index(device) -> torch.device:
+    """A device as tensors name it: "cuda" is the current one."""
+    device = torch.device(device)
+    return torch.device("cuda", _device_index()) if device.type == "cuda" and device.index is None else device
+
+
 _tc5_launched = set()          # devices on which a kernel with bounded waits ran since the status word was last read
 
 
@@ -508,7 +514,7 @@ class StatusWatch:
     replayed graph runs no Python, so whoever replays such a graph calls ``watch.replayed()`` beside it."""
 
     def __init__(self, device):
-        self.device, self.waits = torch.device(device), False
+        self.device, self.waits = _with_index(device), False
 
     def __enter__(self):
         self._before = self.device in _tc5_launched
@@ -528,7 +534,7 @@ class StatusWatch:
 def copy_status(device, to: torch.Tensor) -> bool:
     """Copies the status word to ``to`` (pinned) in stream order, if a kernel with bounded waits ran on ``device`` since it was last
     read: for a caller that does not want to wait for the device now, and hands what arrived to ``raise_status``."""
-    device = torch.device(device)
+    device = _with_index(device)
     if device not in _tc5_launched:
         return False
     to.copy_(tc5_status(device), non_blocking=True)
@@ -538,7 +544,7 @@ def copy_status(device, to: torch.Tensor) -> bool:
 def raise_status(device, code: int) -> None:
     """Raises ``KernelError`` if ``code``, a status word as it was read, says that a bounded wait gave up."""
     if code != 0:
-        tc5_status(torch.device(device)).zero_()
+        tc5_status(_with_index(device)).zero_()
         raise KernelError(f"a kernel on {device} gave up a bounded wait (an mbarrier, or the other CTAs of its grid) or "
                           f"found its shared memory misaligned (status {code}); the step's output is not valid")
 
@@ -547,7 +553,7 @@ def check_status(device) -> None:
     """Reads the status word of the tcgen05 kernels if one of them ran on ``device`` since the last check, and
     raises ``KernelError`` if a bounded wait gave up (the kernel's output is then not to be trusted).  It
     synchronises, so callers use it where they wait for the step anyway (after sampling, after a replayed step)."""
-    device = torch.device(device)
+    device = _with_index(device)
     if device not in _tc5_launched:
         return
     _tc5_launched.discard(device)

@@ -45,3 +45,19 @@ def test_the_word_that_comes_along(word):
         ops.raise_status(DEV, int(to))
     ops.raise_status(DEV, 0)
     assert int(word) == 0
+
+
+def test_a_device_without_an_index_is_the_current_one(word, monkeypatch):
+    monkeypatch.setattr(ops, "_device_index", lambda: 0)
+    for ask in (lambda: ops.check_status("cuda"), lambda: ops.check_status(torch.device("cuda")), lambda: ops.raise_status("cuda", int(word))):
+        ops._tc5_launched.add(DEV)
+        word.fill_(1)
+        with pytest.raises(ops.KernelError):
+            ask()
+        assert int(word) == 0
+    to = torch.zeros(1, dtype=torch.int32)
+    ops._tc5_launched.add(DEV)
+    assert ops.copy_status("cuda", to)
+    with ops.StatusWatch("cuda") as watch:
+        ops._tc5_launched.add(DEV)
+    assert watch.waits
