@@ -24,6 +24,7 @@ constexpr int BK = 64;                     // one 128-byte swizzle row
 constexpr int KPS = 2;                     // blocks of k of a stage
 constexpr int MAX_BN = 256, MAX_STAGES = 8;
 constexpr unsigned RING = 196 * 1024;      // bytes for stages
+constexpr unsigned TWO_AN_SM = 80 * 1024;  // of so many bytes no third CTA fits an SM
 constexpr int THREADS = 384;               // warp 0: TMA, 1: MMAs, 4 to 11: accumulators; all of them at the end
 
 __host__ __device__ constexpr unsigned stage_bytes(int bn) { return KPS * (unsigned)(BM + bn) * BK * 2; }
@@ -383,6 +384,9 @@ int run(Args& g, const void* x, const void* w, int ldx, int ldw, int tiles, int 
     g.vec = g.ldo % 8 == 0 && ((uintptr_t)g.out % 16) == 0;
     unsigned smem = g.stages * stage_bytes(g.bn);
     if (smem < (unsigned)g.bn * BM * 4) smem = (unsigned)g.bn * BM * 4;               // the sums lie over the stages
+    // CTAs of a cluster wait for each other while they hold tensor memory, so an SM takes no more of them than it has columns for: two of 256,
+    // four of 128 (52 KB each at least, so no fifth fits), and five, which is all that their threads leave room for, of fewer.
+    if (ls > 0 && g.bn > 128 && smem < TWO_AN_SM) smem = TWO_AN_SM;
     CUtensorMap mw, mx;
     if (!make_map(&mw, w, N, K, ldw, BM) || !make_map(&mx, x, M, K, ldx, g.bn)) return (int)cudaErrorInvalidValue;
     if (ls == 0) return launch<0, FUSED>(mw, mx, g, smem + 1024, st);

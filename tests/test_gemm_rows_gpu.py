@@ -160,3 +160,14 @@ def test_operands_that_only_the_library_takes():
     assert (unit.float() - want.float()).norm() <= 2e-2 * want.float().norm()       # (the library's way rounds the two sums to bfloat16 first)
     with pytest.raises(Exception):
         ops.linear(x, w, torch.empty(1, N, device=DEV, dtype=torch.bfloat16).expand(M, N))
+
+
+def test_clusters_share_an_sm_only_where_all_find_tensor_memory():
+    """Tiles of 144 rows hold 256 columns of tensor memory in few bytes of shared memory (one stage): more CTAs than SMs, in clusters."""
+    ops = _ops()
+    x, w, exact, size = _inputs(144, 128 * 400, 256, 3)
+    for ls in (1, 2):
+        out = torch.empty(144, 128 * 400, device=DEV)
+        ops.gemm_rows(x, w, out, tiles=1, log2_split=ls)
+        _close(out, exact, size, 256)
+    ops.check_status(x.device)
