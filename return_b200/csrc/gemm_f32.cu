@@ -363,17 +363,35 @@ int launch(const Args& g, cudaStream_t st) {
 }
 
 // Which shape: the one whose busiest SM is done first.  Measured, in units of 10 ns: what a CTA takes for a block of 64, for its set-up
-// and end, and for the exchange of a cluster's sums.  One round of CTAs after the other: 240 of them take twice what 148 do.
+// and end, and for the exchange of a cluster's sums.  One round of CTAs after the other: 240 of them take twice what 148 do
+// (fewer than 148 where they come in clusters).
 constexpr int WIDTHS[4] = {80, 64, 32, 16}, BLOCK_COST[4] = {108, 91, 74, 69}, FIXED_COST[4] = {670, 630, 450, 430}, SPLITS[3] = {1, 2, 4};
 constexpr int EXCHANGE_COST = 120;
 
-int pick(int M, int N, int K, int sms) {
+// CTAs that the device holds at once, by the place in SPLITS.
+bool resident(int (&ctas)[3]) {
+    static PerDevice asked;
+    static int of_device[PerDevice::MAX_DEVICES][3] = {};
+    const int rc = asked.once([&](int dev) {
+        of_device[dev][0] = rb_num_sms();
+        of_device[dev][1] = rb_cluster_ctas((const void*)gemm_f32_kernel<16, 2, ROW_WHOLE>, 2, THREADS, Shape<16>::CLUSTER_BYTES);
+        of_device[dev][2] = rb_cluster_ctas((const void*)gemm_f32_kernel<16, 4, ROW_WHOLE>, 4, THREADS, Shape<16>::CLUSTER_BYTES);
+        return of_device[dev][0] < 1 ? cudaErrorInvalidDevice : cudaSuccess;
+    });
+    int dev = 0;
+    if (rc || cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (int l = 0; l < 3; ++l) ctas[l] = of_device[dev][l];
+    return true;
+}
+
+int pick(int M, int N, int K, const int (&held)[3]) {
     int best = 0;
     long long best_cost = -1;
     const long long nb = (K + BK - 1) / BK, per = (nb + GROUPS - 1) / GROUPS;
     for (int kind = 0; kind < 12; ++kind) {
+        if (held[kind % 3] < 1) continue;
         const int bn = WIDTHS[kind / 3], split = SPLITS[kind % 3];
-        const long long tiles_m = (M + bn - 1) / bn, ctas = tiles_m * ((N + BM - 1) / BM) * split, rounds = (ctas + sms - 1) / sms;
+        const long long tiles_m = (M + bn - 1) / bn, ctas = tiles_m * ((N + BM - 1) / BM) * split, rounds = (ctas + held[kind % 3] - 1) / held[kind % 3];
         const long long blocks = GROUPS / split * per < nb ? GROUPS / split * per : nb;
         const long long cost = rounds * (blocks * BLOCK_COST[kind / 3] + FIXED_COST[kind / 3] + (split > 1 ? EXCHANGE_COST : 0));
         if (best_cost < 0 || cost < best_cost) { best = kind; best_cost = cost; }
@@ -404,7 +422,11 @@ RB_EXPORT int rb_gemm_f32(const float* A, const float* W, float* C, int M, int N
         if (rc) return rc;
     }
     if (M > MOST) M = MOST;
-    if (kind < 0) kind = pick(M, N, K, sms);
+    if (kind < 0) {
+        int held[3];
+        if (!resident(held)) return (int)cudaErrorInvalidConfiguration;
+        kind = pick(M, N, K, held);
+    }
     const int bn = WIDTHS[kind / 3], tiles = (M + bn - 1) / bn;
     const Args g = {A, W, C, M, N, K, lda, ldw, ldc, row, (M + tiles - 1) / tiles, status};
     switch (kind) {

@@ -349,8 +349,24 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& g, unsigned
     return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<LS, FUSED>, mw, mx, g);
 }
 
+// CTAs that the device holds at once, by log2 of their cluster's size: 148 SMs hold 148 in pairs and 132 in fours.
+bool resident(int (&ctas)[3]) {
+    static PerDevice asked;
+    static int of_device[PerDevice::MAX_DEVICES][3] = {};
+    const int rc = asked.once([&](int dev) {
+        of_device[dev][0] = rb_num_sms();
+        of_device[dev][1] = rb_cluster_ctas((const void*)gemm_rows_kernel<1, false>, 2, THREADS, RING + 1024);
+        of_device[dev][2] = rb_cluster_ctas((const void*)gemm_rows_kernel<2, false>, 4, THREADS, RING + 1024);
+        return of_device[dev][0] < 1 ? cudaErrorInvalidDevice : cudaSuccess;
+    });
+    int dev = 0;
+    if (rc || cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (int l = 0; l < 3; ++l) ctas[l] = of_device[dev][l];
+    return true;
+}
+
 // Rows of a tile and CTAs of a cluster: the choice whose busiest SM is done first.
-void pick(int M, int N, int K, int sms, int* tiles_m, int* ls) {
+void pick(int M, int N, int K, const int (&ctas)[3], int* tiles_m, int* ls) {
     long long best = -1;
     const long long all = (K + BK * KPS - 1) / (BK * KPS), tiles_n = (N + BM - 1) / BM;
     const int least = (M + MAX_BN - 1) / MAX_BN;
@@ -359,7 +375,8 @@ void pick(int M, int N, int K, int sms, int* tiles_m, int* ls) {
         if (t > least && (M + t - 2) / (t - 1) <= 32) break;      // narrower still gains nothing
         for (int l = 0; l < 3; ++l) {
             if (all >> l < 2 && l > 0) break;
-            const long long rounds = (tiles_n * t * (1 << l) + sms - 1) / sms;
+            if (ctas[l] < 1) continue;
+            const long long rounds = (tiles_n * t * (1 << l) + ctas[l] - 1) / ctas[l];
             const long long mma = 8 * (bn > 108 ? bn / 2 : 54) + 300, load = (BM + bn) * 6;
             const long long cost = rounds * (((all + (1 << l) - 1) >> l) * (mma > load ? mma : load) + 5000 + bn * 16 + (l > 0 ? 1500 : 0));
             if (best < 0 || cost < best) { best = cost; *tiles_m = t; *ls = l; }
@@ -372,7 +389,11 @@ template <bool FUSED>
 int run(Args& g, const void* x, const void* w, int ldx, int ldw, int tiles, int ls, cudaStream_t st) {
     const int M = g.M, N = g.N, K = g.K;
     if (K <= 0 || K % 8 || ldx % 8 || ldw % 8 || ((uintptr_t)x % 16) || ((uintptr_t)w % 16)) return (int)cudaErrorInvalidValue;
-    if (tiles < 0) pick(M, N, K, rb_num_sms(), &tiles, &ls);
+    if (tiles < 0) {
+        int ctas[3];
+        if (!resident(ctas)) return (int)cudaErrorInvalidConfiguration;
+        pick(M, N, K, ctas, &tiles, &ls);
+    }
     if (tiles < 1 || ls < 0 || ls > 2 || tiles > 65535 || (M + tiles - 1) / tiles > MAX_BN) return (int)cudaErrorInvalidValue;
     g.tile_m = (M + tiles - 1) / tiles;
     g.bn = (g.tile_m + 15) & ~15;
