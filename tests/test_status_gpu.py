@@ -9,6 +9,20 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
 
 
+@pytest.fixture
+def engine(tmp_path):
+    """An engine whose graphs go when the test ends: the errors that it expects keep frames alive, and a graph that is collected while another is
+    captured spoils that capture."""
+    made = []
+
+    def make(dtype, n):
+        made.append(_engine(tmp_path, dtype, n))
+        return made[0]
+
+    yield make
+    made[0].runner._graphs.clear()
+
+
 def _engine(tmp_path, dtype, n, max_new=12):
     from return_b200.engine.config import EngineConfig
     from return_b200.engine.engine import Engine
@@ -27,9 +41,9 @@ def _raise_word():
 
 # a step of 12 tokens in bfloat16 runs the rows' products, one of 3 in float32 the split ones
 @pytest.mark.parametrize("dtype,n", [("bfloat16", 12), ("float32", 3)])
-def test_replayed_step(tmp_path, dtype, n):
+def test_replayed_step(engine, dtype, n):
     from return_b200.ext import ops
-    eng = _engine(tmp_path, dtype, n)
+    eng = engine(dtype, n)
     while not eng._can_run_ahead():
         eng.step()
     eng.step()                                                # captures
@@ -42,9 +56,9 @@ def test_replayed_step(tmp_path, dtype, n):
 
 
 @pytest.mark.parametrize("dtype,n", [("bfloat16", 12), ("float32", 3)])
-def test_steps_that_run_ahead(tmp_path, monkeypatch, dtype, n):
+def test_steps_that_run_ahead(engine, monkeypatch, dtype, n):
     from return_b200.ext import ops
-    eng = _engine(tmp_path, dtype, n)
+    eng = engine(dtype, n)
     while not eng._can_run_ahead():
         eng.step()
     calls, step = [], eng.runner.step
@@ -63,9 +77,9 @@ def test_steps_that_run_ahead(tmp_path, monkeypatch, dtype, n):
     assert all(len(r.output) - before[r.id] <= 2 for r in eng.scheduler.running)       # nothing of the third step was given out
 
 
-def test_a_graph_without_such_kernels_asks_for_nothing(tmp_path):
+def test_a_graph_without_such_kernels_asks_for_nothing(engine):
     from return_b200.ext import ops
-    eng = _engine(tmp_path, "bfloat16", 3)                    # weight streaming and decode attention: no wait
+    eng = engine("bfloat16", 3)                    # weight streaming and decode attention: no wait
     while not eng._can_run_ahead():
         eng.step()
     eng.step()
