@@ -184,13 +184,13 @@ class ModelRunner:
                                    tilings=self.tilings)
         side = torch.cuda.Stream(device=self.env.device)
         side.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(side):                      # warm-up outside the capture
+        with ops.captured_step(), torch.cuda.stream(side):  # warm-up outside the capture, with its kernels
             self.model.forward(static, self.storage)
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize(self.env.device)
         graph = torch.cuda.CUDAGraph()
         before = ops.launch_count
-        with ops.StatusWatch(self.env.device) as watch, torch.cuda.graph(graph, pool=self._graph_pool):
+        with ops.captured_step(), ops.StatusWatch(self.env.device) as watch, torch.cuda.graph(graph, pool=self._graph_pool):
             logits = self.model.forward(static, self.storage)
         self.launches_per_replay[n] = ops.launch_count - before
         if self._graph_pool is None:

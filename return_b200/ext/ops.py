@@ -8,7 +8,10 @@ library (rollout/monkey_patch/qwen3.py:21-22,29-31,56).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import functools
+import threading
 from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
@@ -439,9 +442,11 @@ def gated_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, interleave
     if interleave == 8 and x.shape[0] >= PAIR_MIN_ROWS and pair_ok(x, w, out):
         gemm_tc5(x, w, out, gated=True, pair=True, act=act)
         return
-    if interleave == 8 and w.shape[0] % 16 == 0 and out.dtype == torch.bfloat16 and rows_ok(x, w, out, w.shape[0] // 2):
-        gemm_rows(x, w, out, gated=True, act=act)
-        return
+    if interleave == 8 and x.shape[0] > SKINNY_MAX_ROWS and w.shape[0] % 16 == 0 and out.dtype == torch.bfloat16 and x.is_cuda:
+        form = _rows_form(x, w, out, True)
+        if form is not None:
+            _launch_rows(form, x.device, _gated_code(True, act), -1)
+            return
     if ctx is not None:
         gu = ctx.buffer("gated_linear.gate_up", (x.shape[0], w.shape[0]), x.dtype, x.device)
     else:
@@ -506,7 +511,7 @@ _tc5_launched = set()          # devices on which a kernel with bounded waits ra
 def _status_word(device):
     """The pointer that a launch hands to a kernel with bounded waits; ``check_status`` then reads the word."""
     _tc5_launched.add(device)
-    return _ptr(tc5_status(device))
+    return tc5_status(device).data_ptr()
 
 
 class StatusWatch:
@@ -622,38 +627,107 @@ def gemm_tc5_bmn(x: torch.Tensor, b: torch.Tensor, out: torch.Tensor, bn: int = 
                                      _status_word(x.device), _stream()), "gemm_tc5_bmn")
 
 
-# Where the kernel for the rows of an ordinary step is the fastest way.  As kernels alone the library's are 5-25 % faster from some 30 rows on
-# (512 x 6,144 x 1,024 8.2 us against 9.9, 64 x 2,048 x 2,048 5.7 and 6.0), but a launch through torch takes the host 10 us against
-# 3 and does not overlap the kernel before it: up to this much work the step gains (a step of 512 tokens through six layers of 1,024
-# 1,038 -> 874 us; a captured one of 16 tokens 283 -> 267, of 64 387 -> 381; feed-forwards of 1,024 x 3,072 28.8 -> 19.0), above it loses
-# (600 rows of 2,048 x 6,144: 46.8 -> 53.1), and so with more weights to stream (64 tokens through layers of 4,096: 318 -> 333), but for few rows of
-# long sums: with K at least twice N the weight tiles are few, and K is cut over a cluster (64 x 4,096 x 12,288 21.7 -> 20.4).
-# And beyond a thousand rows the library's is as much faster however small the product (2,048 rows of a router, 32 x 2,048: 4.8 us and 6.7).
+# Where the kernel for the rows of an ordinary step is the fastest way.  As a kernel alone the library's is 5 to 40 % faster from some 30 rows on
+# (us, library / this: 64 x 4,096 x 1,024 5.0 / 5.9, 512 x 6,144 x 1,024 8.3 / 9.9, 384 x 2,048 x 2,048 6.8 / 9.5), but launched one by one a product
+# through torch takes the host 10 us against 6, the gated unit in the epilogue saves a launch more, and a layer whose four products take the
+# norms and adds in saves four more (csrc/gemm_rows.cu).  Steps of several launches wait for the host: up to this much work they gain (six layers of
+# 1,024 x 3,072, 512 tokens: 794 / 584, 768 tokens 738 / 666; three of 2,048 x 4,096, 200 tokens: 508 / 401; four mixers of 1,024 with states, 512
+# tokens: 1,070 / 905; with a limit of 1.25 G for a product outside such a layer 996).  Products one behind the other with nothing between them
+# would gain to 1.25 G only (256 x 2,048 x 2,048 9.8 / 8.2, 512 10.0 / 11.6, 256 x 4,096 x 2,048 10.1 / 12.1), gated ones to 2 to 4 G
+# (512 x 6,144 x 1,024 13.6 / 12.5, 640 14.5 / 13.9; 128 x 8,192 x 2,048 13.6 / 12.4, 200 14.3 / 15.9).  Above, a step loses
+# (560 tokens of 1,024 x 3,072, 3.4 G: 809 / 817; 600 rows of 2,048 x 6,144, 7 G: 46.8 / 53.1).
+# With more weights than ROWS_MAX_WEIGHTS to stream the library is faster, but for few rows of long sums: with K at least twice N the weight
+# tiles are few, and K is cut over a cluster (64 x 4,096 x 12,288 25.5 / 22.0).  Beyond a thousand rows it is, however small the product.
+# In a captured step a launch costs the host nothing, and only what the kernel saves on the device counts (us a product behind a norm, library / this):
+#   a layer     128 rows (us a layer less: 3.4 to 1.9 at 64 rows, 2.6 to 0.3 at 128; at 192 between 1.6 less and 2.2 more; 512 to 2,048 wide)
+#   gated       64 (48 x 6,144 x 1,024 9.5 / 9.2, 64 x 8,192 x 2,048 13.2 / 12.9; 128 x 8,192 x 1,024 10.7 / 11.6)
+#   a product   64 where the sums are long and the columns not too few (64 x 2,048 x 6,144 13.5 / 12.9, 16 x 1,024 x 3,072 10.4 / 8.2); the others
+#               lose from the first rows on (16 x 4,096 x 1,024 6.8 / 7.0, 64 7.0 / 7.8; 32 x 1,024 x 512 4.6 / 5.5)
 ROWS_MAX = 1024
 ROWS_MAX_WORK = 3300 << 20
 ROWS_MAX_WEIGHTS = 1 << 24
 ROWS_LONG_SUMS = 128
+ROWS_CAPTURED_LAYER = 128
+ROWS_CAPTURED = 64
+
+
+class _Step(threading.local):
+    captured = False
+
+
+_step = _Step()
+
+
+@contextlib.contextmanager
+def captured_step():
+    """What this thread launches inside belongs to a step that is captured in a graph (its warm-up among it, which then runs the kernels
+    that the graph will hold): products are chosen for that."""
+    before, _step.captured = _step.captured, True
+    try:
+        yield
+    finally:
+        _step.captured = before
 
 
 def rows_limit(N: int, K: int) -> int:
-    """The largest number of rows that the kernel for the rows of an ordinary step takes against N x K weights and is the fastest way."""
+    """The largest number of rows that the kernel for the rows of an ordinary step takes against N x K weights and is the fastest way, launched
+    one by one."""
     limit = ROWS_LONG_SUMS if K >= 2 * N else 0
     if N * K <= ROWS_MAX_WEIGHTS:
         limit = max(limit, min(ROWS_MAX, ROWS_MAX_WORK // (N * K)))
     return limit
 
 
-def rows_ok(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, width: int = 0) -> bool:
-    """Whether the kernel for the rows of an ordinary step takes this product (into ``out``, of ``width`` columns), and is the fastest way.
-    What it does not take goes to the library, which copies or refuses: columns that do not lie side by side, rows that overlap (a stride
-    of zero among them), nothing to add up, several devices, an output of another shape."""
-    N, K = w.shape
-    return (0 < N * K and x.dtype == w.dtype == torch.bfloat16 and x.shape[0] <= rows_limit(N, K) and x.shape[1] == K and K % 8 == 0
-            and x.stride(1) == 1 and w.stride(1) == 1 and K <= x.stride(0) < 1 << 31 and K <= w.stride(0) < 1 << 31
-            and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
-            and x.get_device() == w.get_device()
-            and (out is None or (out.shape == (x.shape[0], width) and out.dtype in (torch.bfloat16, torch.float32) and out.stride(1) == 1
-                                 and width <= out.stride(0) < 1 << 31 and out.get_device() == x.get_device())))
+def layer_rows_limit(limit: int) -> int:
+    """The most rows of a layer whose products take the norms and residual adds in, ``limit`` the least of their ``rows_limit``."""
+    return min(limit, ROWS_CAPTURED_LAYER) if _step.captured else limit
+
+
+@functools.lru_cache(maxsize=1024)
+def _rows_limit_alone(N: int, K: int, gated: bool, captured: bool) -> int:
+    if K <= 0 or N <= 0 or K % 8:
+        return -1
+    limit = rows_limit(N, K)
+    if captured:
+        return min(limit, ROWS_CAPTURED) if gated or (K >= 2 * N and N >= 1024) else -1
+    return limit
+
+
+def _rows_form(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], gated: bool):
+    """What the kernel for the rows of an ordinary step takes of this product (pointers, sizes, strides), if it takes it and is the fastest way;
+    else None.  What it does not take goes to the library, which copies or refuses: columns that do not lie side by side, rows that overlap
+    (a stride of zero among them), nothing to add up, several devices, an output of another shape.  (Every attribute is asked for once: a step
+    launched one by one waits for the host.)"""
+    (M, Kx), (N, K) = x.shape, w.shape
+    if M > _rows_limit_alone(N, K, gated, _step.captured):
+        return None
+    (sx, x1), (sw, w1) = x.stride(), w.stride()
+    px, pw = x.data_ptr(), w.data_ptr()
+    if not (Kx == K and x1 == w1 == 1 and K <= sx <= _INT_MAX and K <= sw <= _INT_MAX and (sx | sw) % 8 == 0 and (px | pw) % 16 == 0
+            and x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16):
+        return None
+    device = x.get_device()
+    if w.get_device() != device:
+        return None
+    if out is None:
+        return px, pw, None, 0, M, N, K, sx, sw, 0
+    width, f32, (so, o1) = N // 2 if gated else N, out.dtype is torch.float32, out.stride()
+    if o1 == 1 and width <= so <= _INT_MAX and out.shape == (M, width) and out.get_device() == device and (f32 or out.dtype is torch.bfloat16):
+        return px, pw, out.data_ptr(), 1 if f32 else 0, M, N, K, sx, sw, so
+    return None
+
+
+_INT_MAX = 2 ** 31 - 1
+
+
+def rows_ok(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, gated: bool = False) -> bool:
+    """Whether the kernel for the rows of an ordinary step takes this product (into ``out``), and is the fastest way."""
+    return _rows_form(x, w, out, gated) is not None
+
+
+def _launch_rows(form, device, gated: int, act: int) -> None:
+    px, pw, po, f32, M, N, K, sx, sw, so = form
+    _check(tc5_lib().rb_gemm_rows(px, pw, po, f32, gated, act, M, N, K, sx, sw, so, -1, -1, _status_word(device), _stream()), "gemm_rows")
 
 
 def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool = False, act: Optional[str] = None, tiles: int = -1,
@@ -735,12 +809,15 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act: Optional[st
     if not x.is_cuda:
         raise KernelError("the engine's kernels run on a CUDA device only; got a CPU tensor")
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-    if skinny_ok(x, w):
-        gemm_skinny(x, w, out, act=act, bias=bias)
-        return
-    if act != "neg_exp_exp" and rows_ok(x, w, out, w.shape[0]):
-        gemm_rows(x, w, out, act=act)
-        return
+    if x.shape[0] <= SKINNY_MAX_ROWS:
+        if skinny_ok(x, w):
+            gemm_skinny(x, w, out, act=act, bias=bias)
+            return
+    elif act != "neg_exp_exp":
+        form = _rows_form(x, w, out, False)
+        if form is not None:
+            _launch_rows(form, x.device, 0, ACTIVATIONS[act] if act is not None else -1)
+            return
     if out.dtype == torch.float32:
         torch.mm(x, w.t(), out_dtype=torch.float32, out=out)
     else:

@@ -91,9 +91,9 @@ class PreNormBlock(Block):
                         and all(w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and w.stride(1) == 1 and w.stride(0) % 8 == 0
                                 and w.data_ptr() % 16 == 0 for w in weights)):
                     most = min(ops.rows_limit(*w.shape) for w in weights)           # rows that one kernel or the other takes in all four
-                    plan = (w_in, in_name, w_out, gate_up, down, max(most, ops.SKINNY_MAX_ROWS))
+                    plan = (w_in, in_name, w_out, gate_up, down, most)
             self._fused_parts = plan
-        if not plan or stream.shape[0] > plan[5]:
+        if not plan or stream.shape[0] > max(ops.layer_rows_limit(plan[5]), ops.SKINNY_MAX_ROWS):
             return None
         return plan
 
