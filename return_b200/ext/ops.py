@@ -750,9 +750,8 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool =
 def gemm_rows_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], gated: bool = False, scale=None, residual=None,
                     tiles: int = -1, log2_split: int = -1) -> None:
     """``gemm_skinny_fused`` for the rows of an ordinary step: the same arguments, RowSums of [rows, tiles of 128 columns]."""
-    M, K = x.shape
-    N = w.shape[0]
-    assert x.dtype == w.dtype == torch.bfloat16 and w.shape[1] == K and x.stride(1) == 1 and w.stride(1) == 1
+    (M, K), (N, Kw), (sx, x1), (sw, w1) = x.shape, w.shape, x.stride(), w.stride()
+    assert x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and Kw == K and x1 == 1 and w1 == 1
     ssq_in, ssq_in_count, norm_dim, eps, ld_sums = None, 0, 0, 0.0, 0
     if scale is not None:
         sums_in, eps = scale
@@ -773,10 +772,12 @@ def gemm_rows_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor
             ssq_out = sums_out.parts
             assert sums_out.dim == N and ssq_out.shape[0] >= M and ssq_out.shape[1] >= sums_out.count and (ssq_in is None or ssq_out.shape[1] == ld_sums)
             ld_sums = ssq_out.shape[1]
+    so = 0
     if out is not None:
-        assert out.dtype == torch.bfloat16 and out.stride(1) == 1 and out.shape == (M, N // 2 if gated else N)
-    rc = tc5_lib().rb_gemm_rows_fused(_ptr(x), _ptr(w), _ptr(out), 1 if gated else 0, M, N, K, x.stride(0), w.stride(0),
-                                      out.stride(0) if out is not None else 0, _ptr(ssq_in), ssq_in_count, norm_dim, eps, _ptr(stream),
+        so, o1 = out.stride()
+        assert out.dtype is torch.bfloat16 and o1 == 1 and out.shape == (M, N // 2 if gated else N)
+    rc = tc5_lib().rb_gemm_rows_fused(_ptr(x), _ptr(w), _ptr(out), 1 if gated else 0, M, N, K, sx, sw, so,
+                                      _ptr(ssq_in), ssq_in_count, norm_dim, eps, _ptr(stream),
                                       _ptr(norm_w), norm_w_dtype, offset, _ptr(ssq_out), ld_sums, tiles, log2_split,
                                       _status_word(x.device), _stream())
     _check(rc, "gemm_rows_fused")

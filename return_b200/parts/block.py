@@ -25,6 +25,7 @@ class PreNormBlock(Block):
         self._children = {"mixer": self.mixer, "mixer_norm": self.mixer_norm}
         if self.feed_forward is not None:
             self._children.update({"feed_forward": self.feed_forward, "feed_forward_norm": self.feed_forward_norm})
+        self._fused_parts = None                               # what _fused_plan found, or False
         # a sublayer's output times a factor, or a layer without a feed-forward: the adds run in the kernel that takes
         # a factor per addend (csrc/recurrent.cu, add_dual_norm), which wants RMSNorms
         self._scaled = (self.residual_scale != 1.0 or self.feed_forward is None or bool(getattr(spec, "float_outputs", False)))
@@ -75,9 +76,10 @@ class PreNormBlock(Block):
         and leaves v * w and sum(v^2); the product after it (the gated one, the next block's first) scales by
         rstd (csrc/gemm_skinny.cu, csrc/gemm_rows.cu).  Six launches a layer of a decode step instead of eight.  That
         needs a mixer and a feed-forward that expose their products, RMSNorms, and sizes the kernel takes; anything else runs part by part."""
-        if self.env.act_dtype != torch.bfloat16 or self._scaled or stream.shape[0] > ops.ROWS_MAX:
+        T = stream.shape[0]
+        if T > ops.ROWS_MAX or self._scaled or self.env.act_dtype != torch.bfloat16:
             return None
-        plan = getattr(self, "_fused_parts", None)
+        plan = self._fused_parts
         if plan is None:
             plan = False
             mixer, ff = self.mixer, self.feed_forward
@@ -93,7 +95,7 @@ class PreNormBlock(Block):
                     most = min(ops.rows_limit(*w.shape) for w in weights)           # rows that one kernel or the other takes in all four
                     plan = (w_in, in_name, w_out, gate_up, down, most)
             self._fused_parts = plan
-        if not plan or stream.shape[0] > max(ops.layer_rows_limit(plan[5]), ops.SKINNY_MAX_ROWS):
+        if not plan or (T > ops.SKINNY_MAX_ROWS and T > ops.layer_rows_limit(plan[5])):
             return None
         return plan
 
@@ -123,11 +125,13 @@ class PreNormBlock(Block):
         mixed = self.mixer.core(proj, ctx)
         ops.linear_fused(mixed, w_out, rows2, residual=(stream, (n2.p_weight, n2.spec.offset), sums2))
         ops.linear_fused(rows2, gate_up, act, gated=True, scale=(sums2, n2.spec.eps))
-        nxt = ctx.next_block.first_norm() if ctx.next_block is not None and hasattr(ctx.next_block, "first_norm") else None
+        follower = ctx.next_block
+        if T > ops.SKINNY_MAX_ROWS and not (isinstance(follower, PreNormBlock) and follower._fused_plan(stream)):
+            nxt = None                                         # it norms the stream itself: nobody would read what is left here
+        else:
+            nxt = follower.first_norm() if follower is not None and hasattr(follower, "first_norm") else None
         if nxt is not None and nxt[3] != H:
             nxt = None
-        if T > ops.SKINNY_MAX_ROWS and not (isinstance(ctx.next_block, PreNormBlock) and ctx.next_block._fused_plan(stream)):
-            nxt = None                                         # the next block norms the stream itself: nobody would read what is left here
         if nxt is None and T > ops.SKINNY_MAX_ROWS:            # what follows adds it anyway
             y = ctx.buffer("block.delta", (T, H), dt, dev)
             ops.linear(act, down, y)
