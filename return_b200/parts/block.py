@@ -42,6 +42,7 @@ class PreNormBlock(Block):
                 for name, p in part.params().items()}
 
     def bind(self, tensors):
+        self._fused_parts = None                               # holds the weights
         for child, part in self._children.items():
             prefix = child + "."
             part.bind({k[len(prefix):]: v for k, v in tensors.items() if k.startswith(prefix)})

@@ -22,10 +22,14 @@ def _model(widths, seed=0):
     spec = qwen3.decoder_spec(cfg, 512)
     layers = tuple(dataclasses.replace(b, feed_forward=dataclasses.replace(b.feed_forward, intermediate_size=w)) for b, w in zip(spec.layers, widths))
     model = DecoderModel(dataclasses.replace(spec, layers=layers), BuildEnv(torch.bfloat16, DEV))
-    g = torch.Generator(device=DEV).manual_seed(seed)
-    model.bind({n: torch.empty(p.shape, device=DEV).normal_(1.0 if len(p.shape) == 1 else 0.0, 0.1 if len(p.shape) == 1 else 0.03, generator=g).bfloat16()
-                for n, p in model.params().items()})
+    model.bind(_weights(model, seed))
     return model
+
+
+def _weights(model, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return {n: torch.empty(p.shape, device=DEV).normal_(1.0 if len(p.shape) == 1 else 0.0, 0.1 if len(p.shape) == 1 else 0.03, generator=g).bfloat16()
+            for n, p in model.params().items()}
 
 
 def _step(model, T, monkeypatch=None):
@@ -67,3 +71,13 @@ def test_what_a_layer_leaves_is_read(monkeypatch, widths, left, T):
     monkeypatch.setattr(ops, "_rows_form", lambda *a: None)
     want, _, _ = _step(_model(widths), T)
     assert torch.isfinite(got).all() and (got - want).norm() <= 2e-2 * want.norm()
+
+
+@pytest.mark.parametrize("T", [3, 9, 100])
+def test_weights_bound_again_are_used(T):
+    model = _model((512, 512))
+    old, _, _ = _step(model, T)
+    model.bind(_weights(model, 7))
+    got, _, _ = _step(model, T)
+    want, _, _ = _step(_model((512, 512), 7), T)
+    assert torch.equal(got, want) and not torch.equal(got, old)
