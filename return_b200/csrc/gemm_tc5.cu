@@ -372,20 +372,6 @@ constexpr int PR_STAGES = 3;              // x 64 KB (measured at 2,048 x 24,576
 constexpr unsigned PR_A_BYTES = BM * BK * 2, PR_B_BYTES = PR_HALF * BK * 2, PR_BLOCK_BYTES = PR_A_BYTES + PR_B_BYTES;
 constexpr unsigned PR_STAGE_BYTES = PR_KPS * PR_BLOCK_BYTES;
 
-__device__ __forceinline__ unsigned cluster_ctarank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the address, in the cluster's shared window, of the same variable in CTA `rank`
-__device__ __forceinline__ unsigned map_to_cta(unsigned smem_addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void mbar_arrive_in_cluster(unsigned cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

@@ -42,6 +42,22 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
 // (tcgen05.mma operand reads, TMA) after this fence
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---------------------------------------------------------------------------------- clusters
+__device__ __forceinline__ unsigned cluster_ctarank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address, in the cluster's shared window, of the same variable in CTA `rank`
+__device__ __forceinline__ unsigned map_to_cta(unsigned smem_addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+
 // ---------------------------------------------------------------------------------- tensor memory
 // One warp allocates `cols` columns (a power of two, 32..512); the base address lands in *slot.
 __device__ __forceinline__ void tmem_alloc(unsigned slot_smem, unsigned cols) {
