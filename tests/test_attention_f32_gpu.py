@@ -42,14 +42,15 @@ def test_options_and_edges(Hq, Hkv, D, P, options):
     assert (got - want).abs().max() <= 2e-6 * max(1.0, float(want.abs().max()))
 
 
-def test_error_is_no_larger_than_the_chains():
-    pg = Paged([400, 300], [400, 60], 4, 2, 128, 16, torch.float32, seed=3)
-    got, chain = _both(pg, 4, 2, 128, 16)
+@pytest.mark.parametrize("D", [32, 64, 96, 128])
+def test_error_is_no_larger_than_the_chains(D):
+    pg = Paged([400, 300], [400, 60], 4, 2, D, 16, torch.float32, seed=3)
+    got, chain = _both(pg, 4, 2, D, 16)
     err = [0.0, 0.0]
     row = 0
     for i, (n, ql) in enumerate(zip(pg.kv_lens, pg.q_lens)):
         q, k, v = pg.q[i].double(), pg.k[i].double().repeat_interleave(2, 1), pg.v[i].double().repeat_interleave(2, 1)
-        s = torch.einsum("qhd,nhd->hqn", q, k) * 128 ** -0.5
+        s = torch.einsum("qhd,nhd->hqn", q, k) * D ** -0.5
         s = s.masked_fill(torch.arange(n)[None] > torch.arange(n - ql, n)[:, None], float("-inf"))
         want = torch.einsum("hqn,nhd->qhd", torch.softmax(s, -1), v).reshape(ql, -1).to(DEV)
         for j, o in enumerate((got, chain)):

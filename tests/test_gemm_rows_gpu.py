@@ -64,10 +64,12 @@ def test_activation_on_the_sums(act):
     x, w, exact, _ = _inputs(70, 136, 256, 4)
     f = {"relu2": lambda v: torch.relu(v) ** 2, "tanh": torch.tanh, "silu": lambda v: v * torch.sigmoid(v),
          "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[act]
-    out = torch.empty(70, 136, device=DEV, dtype=torch.bfloat16)
-    ops.linear(x, w, out, act=act)
     want = f(exact)
-    assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+    assert ops.rows_ok(x, w)
+    for product in (ops.gemm_rows, ops.linear):               # the kernel, and the way to it
+        out = torch.full((70, 136), float("nan"), device=DEV, dtype=torch.bfloat16)
+        product(x, w, out, act=act)
+        assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
     ops.check_status(x.device)
 
 
@@ -131,11 +133,41 @@ def test_norms_and_residual_adds_inside_the_products(M, H, Q, I, offset, wdt):
     ops.check_status(torch.device("cuda:0"))
 
 
-def test_fused_product_refuses_what_it_cannot_take():
+def test_products_refuse_what_they_cannot_take():
+    """Before anything is launched: each is an error of the entry itself."""
     ops = _ops()
-    x, w = torch.zeros(16, 64, device=DEV).bfloat16(), torch.zeros(130, 64, device=DEV).bfloat16()
-    with pytest.raises(Exception):                            # a row of the stream that is no whole 16-byte pieces
-        ops.gemm_rows_fused(x, w, None, residual=(torch.zeros(16, 130, device=DEV), None, None))
+    x, w = torch.zeros(16, 64, device=DEV).bfloat16(), torch.zeros(128, 64, device=DEV).bfloat16()
+    out, stream, norm = torch.zeros(16, 128, device=DEV).bfloat16(), torch.zeros(16, 128, device=DEV), torch.ones(128, device=DEV)
+    sums = ops.RowSums(torch.zeros(16, 1, device=DEV), 128)
+    ops.gemm_rows_fused(x, w, out, residual=(stream, (norm, 0.0), sums))
+    def zeros(*shape):
+        return torch.zeros(*shape, device=DEV).bfloat16()
+
+    refused = [
+        # a row of the stream is no whole 16-byte pieces; K is no multiple of 8; rows lie off 16-byte boundaries
+        lambda: ops.gemm_rows_fused(x, zeros(130, 64), None, residual=(torch.zeros(16, 130, device=DEV), None, None)),
+        lambda: ops.gemm_rows(x[:, :60], w[:, :60], out),
+        lambda: ops.gemm_rows(x[:, 1:57], w[:, :56], out),
+        # a tile of 300 rows; a cluster of eight CTAs; gate and up rows in no whole blocks
+        lambda: ops.gemm_rows(zeros(300, 64), w, zeros(300, 128), tiles=1, log2_split=0),
+        lambda: ops.gemm_rows(x, w, out, tiles=1, log2_split=3),
+        lambda: ops.gemm_rows_fused(x, zeros(136, 64), out[:, :68], gated=True, scale=(sums, 1e-6)),
+    ]
+    for call in refused:
+        with pytest.raises(ops.KernelError):
+            call()
+    narrow = ops.RowSums(torch.zeros(16, 1, device=DEV), 256)
+    gaps = torch.zeros(16, 129, device=DEV)[:, :128]
+    refused = [
+        # room for one share a row instead of two; a stream with gaps; a next norm and nowhere to put its rows
+        lambda: ops.gemm_rows_fused(x, zeros(256, 64), None, residual=(torch.zeros(16, 256, device=DEV), None, narrow)),
+        lambda: ops.gemm_rows_fused(x, w, None, residual=(gaps, None, None)),
+        lambda: ops.gemm_rows_fused(x, w, None, residual=(stream, (norm, 0.0), None)),
+    ]
+    for call in refused:
+        with pytest.raises(AssertionError):
+            call()
+    ops.check_status(x.device)
 
 
 def test_operands_that_only_the_library_takes():

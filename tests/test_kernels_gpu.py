@@ -135,8 +135,8 @@ def test_gemm_f32_is_exact_float32(M, N, K):
 @pytest.mark.parametrize("M,N,K", [(1, 33, 132), (2, 64, 4), (4, 100, 1030), (5, 65, 36), (33, 129, 100), (130, 257, 31), (257, 96, 256)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_gemm_f32_kernels_agree(M, N, K, offset):
-    """Every tile size and the kernel for few rows against each other (bit by bit) and against float64, at the edges of tiles and
-    stages; ``offset`` puts the operands off 16-byte boundaries.  A sum of K products in float32 is off by at most K / 2^24 times
+    """Every shape against each other (bit by bit) and against float64, for short sums and long ones and at the edges of tiles and
+    blocks; ``offset`` puts the operands off 16-byte boundaries.  A sum of K products in float32 is off by at most K / 2^24 times
     the sum of their sizes."""
     ops = _ops()
     wide = torch.randn(M + N, K + 3, device=DEV)
@@ -144,7 +144,7 @@ def test_gemm_f32_kernels_agree(M, N, K, offset):
     if offset == 0 and K % 4 == 0:
         x, w = x.contiguous(), w.contiguous()
     outs = []
-    for kind in (-1, 0, 1, 2, 3) + ((4,) if M <= 4 else ()):
+    for kind in range(-1, 12):
         outs.append(torch.full((M, N), float("nan"), device=DEV))
         ops.gemm_f32(x, w, outs[-1], kind=kind)
         assert torch.equal(outs[-1], outs[0])
