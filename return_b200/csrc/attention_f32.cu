@@ -2,9 +2,9 @@
 // absolute positions, an online softmax a row, CTAs of up to 32 rows of neighbouring tokens that share a key/value head), its two
 // products on the matrix instructions in float32's precision.
 //
-// Operands are multiplied by 2^16 and split into three bfloat16 parts (which then hold every bit of every float32, small ones too: bfloat16 ends
-// at 2^-133), six of nine products are made (the rest is below 2^-24 of a product), the
-// largest in an accumulator of its own; a tile's 128 products of a score, or 32 of an output, are summed there, all else on the CUDA cores,
+// Operands are multiplied by 2^16 and split into three bfloat16 parts (which then hold every bit of every float32, small ones too:
+// bfloat16 ends at 2^-133), six of nine products are made (the rest is below 2^-24 of a product), the largest in an accumulator of its own;
+// a tile's 128 products of a score, or 32 of an output, are summed there, all else on the CUDA cores,
 // which round to nearest.  A row of the products is worked out by itself and in one order, so the result for a token does not
 // depend on how the prompt was cut into steps or on what else is in the batch: it is bit-identical.  An infinity, a NaN or a number beyond 2^112 has no
 // parts: where a score or an output's sum over a tile is no finite number, it is made again from the operands, one FFMA behind the
@@ -12,9 +12,10 @@
 //
 // Eight warps.  Scores: a warp a 16 x 8 part of rows by keys, K's parts made as they are read.  Softmax: a warp four rows, a lane a key,
 // the rows' reductions in step.  Outputs: a warp up to two blocks of eight columns for all rows, V's parts made once, accumulators in registers.
-// Bound by what a tile of 32 keys waits for one behind the other (three barriers, 1,550 + 1,300 + 2,100 cycles of the three parts, of which
-// the matrix instructions are 1,600).  Measured (16 query and 8 key/value heads of 128), us, attention_simt.cu / this: 257 tokens of three
-// requests 67 / 42, 219 64 / 33, 1,000 420 / 216, one token behind 2,000 281 / 183.  P's parts made by the softmax's warps, and two sets of
+// Bound by what a tile of 32 keys waits for one behind the other: three parts and three barriers, 3 us a tile (one token behind 2,000 walks 63
+// tiles in 188 us), at half of the issue slots and 6.5 % of the tensor pipe (ncu).  Measured (16 query and 8 key/value heads of 128), us,
+// attention_simt.cu / this: 257 tokens of three requests 67 / 46, 219 64 / 35, 1,000 420 / 222, one token behind 2,000 281 / 188 (the factor's part
+// of it 2 to 9 %).  P's parts made by the softmax's warps, and two sets of
 // score accumulators: 2 to 10 % slower.
 #include <float.h>
 

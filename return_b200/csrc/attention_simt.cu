@@ -271,7 +271,7 @@ static int launch_simt(const void* q, int ld, const void* kpool, const void* vpo
     return rb_launch_status();
 }
 
-// attention_f32.cu: the 32-bit path's kernel where it takes the head size and the pools lie on 16-byte boundaries (257 tokens as above: 42 us).
+// attention_f32.cu: the 32-bit path's kernel where it takes the head size and the pools lie on 16-byte boundaries (257 tokens as above: 46 us).
 int rb_attention_f32_takes(int D, const void* kpool, const void* vpool);
 int rb_attention_f32(const float* q, int ld, const float* kpool, const float* vpool, const int* pos, const int* tok_seg, const int* block_table,
                      int bt_stride, int page_size, float* out, int T, int Hq, int Hkv, int D, float scale, int window, int chunk, float softcap,

@@ -28,13 +28,14 @@ using namespace tc5;
 //   one          thread issues the MMAs.
 // The tokens' parts lie below each other, so that one MMA multiplies the weights' leading parts with all three of them (N = 3 BN),
 // one the middle parts with two, one the last with one: three instructions for six products, which counts because an instruction
-// takes 54 cycles at least.  Two stages of parts, two sets of accumulators.  A tile takes 26 cycles a row of both operands and block
-// of 64 at BN = 80, four times what its MMAs take: bound by the warps that split, of which six more do not fit the registers.  The thread
-// that issues the MMAs halves what its scheduler has left (measured with the warps' clocks), so no warp that splits shares it: 257 x 4,096 x
+// takes 54 cycles at least.  Two stages of parts, two sets of accumulators.  A block of 64 takes a CTA 1.2 us at BN = 80 (2,048 x 4,096 x 1,024
+// is six tiles one behind the other on an SM, 25.6 us each, 6.7 of them set-up and end), of which the tensor pipe works less than half (24 % of
+// a launch of 257 x 4,096 x 1,024, ncu): bound by the warps that split, of which six more do not fit the registers.  The thread that issues the MMAs halves what its scheduler has left (measured with the warps' clocks), so no warp that splits shares it: 257 x 4,096 x
 // 1,024 took 29.8 us with two of them there, and 37.8 with the path for ragged rows in the same loop, whose code then did not stay in
 // the instruction cache.  Splitting by conversions, by integer rounding or by bfloat16-minus-float32 subtractions made no difference.
-// Now 27.4 us (tiles of FFMAs: 87); 257 x 6,144 x 1,024 42 (128), 257 x 1,024 x 3,072 22 (77), 2,048 x 4,096 x 1,024 148 (397),
-// 3 x 8,192 x 1,024 11 (18), 16 x 1,024 x 3,072 17 (75).
+// Now 26.8 us (tiles of FFMAs: 86); 257 x 6,144 x 1,024 43 (128), 257 x 1,024 x 3,072 22 (77), 2,048 x 4,096 x 1,024 153 (397), 2,048 x 4,096 x
+// 1,000, in pieces of four, 182 (409; one value at a time 311), x 3,001 673 (1,657),
+// 3 x 8,192 x 1,024 11 (18), 16 x 1,024 x 3,072 13 (75).
 constexpr int BK = 64;                     // values of k of a block: one 128-byte swizzle row of bfloat16
 constexpr int BM = 128;                    // weight rows of a CTA
 constexpr int RUN = 2;                     // blocks that one accumulator sums

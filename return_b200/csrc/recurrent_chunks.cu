@@ -14,7 +14,7 @@
 // still holds up those behind it.  The state stays in registers and S0 goes through matrix instructions.
 //
 // All arithmetic keeps float32's precision.  The products run as bfloat16 matrix instructions on operands split into three
-// bfloat16 parts (x = h + m + l, 24 bits), six of the nine products (hh, hm, mh, hl, lh, mm; the rest is below 2^-24), the five small
+// bfloat16 parts (x = h + m + l, 24 bits down to 2^-109, below which bfloat16 ends before they do), six of the nine products (hh, hm, mh, hl, lh, mm; the rest is below 2^-24), the five small
 // ones in an accumulator of their own.  Per flop that is as fast as three TF32 products, which would keep 22 bits, and 1.3 times
 // the CUDA cores' peak, of which register blocks this small reach a third.
 #include "tc5.cuh"

@@ -310,8 +310,9 @@ def softcap(x: torch.Tensor, cap: float) -> None:
 # ------------------------------------------------------------------------------- matrix products
 
 def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int = -1) -> None:
-    """out[M, N] = x[M, K] @ w[N, K]^T in float32's precision (operands split into three bfloat16 parts each, tensor cores; fixed
-    order over K).  ``kind``: 0-11 one shape of tile and split, -1 the one that suits the sizes; all give the same bits."""
+    """out[M, N] = x[M, K] @ w[N, K]^T in float32's precision (operands split into three bfloat16 parts each, tensor cores; up to 96
+    values of K multiply-adds; fixed order over K).  ``kind``: 0-11 one shape of tile and split, -1 the one that suits the sizes; all give the
+    same bits."""
     M, K = x.shape
     N = w.shape[0]
     assert x.dtype == w.dtype == out.dtype == torch.float32
@@ -323,8 +324,8 @@ def gemm_f32(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, kind: int = -1
 
 
 SKINNY_KERNEL_MAX_ROWS = 32     # what the kernel takes
-SKINNY_MAX_ROWS = 8             # what the engine gives it: beyond 8 rows the library is faster (38 us against 58 at
-                                # 16 rows and 106 at 32, for N = 24576, K = 4096)
+SKINNY_MAX_ROWS = 8             # what the engine gives it: beyond 8 rows the kernel for the rows of an ordinary step or the library is faster
+                                # (the library 38 us against 58 at 16 rows and 106 at 32, for N = 24576, K = 4096)
 
 
 def _gated_code(gated: bool, act: str = "silu") -> int:
@@ -434,7 +435,7 @@ def pair_ok(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
 def gated_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, interleave: int, ctx=None, act: str = "silu") -> None:
     """out[T, I] = act(x @ gate^T) * (x @ up^T), ``act`` one of ``GATES``, for the fused weight ``w`` [2I, K] of a gated
     feed-forward.  With the interleaved layout the product's epilogue does the gating where an own kernel
-    is the fastest: for few rows (weight streaming) and for many (tcgen05, pairs of CTAs); otherwise a product
+    is the fastest: for few rows (weight streaming), for those of an ordinary step (``gemm_rows``) and for many (tcgen05, pairs of CTAs); otherwise a product
     into a [T, 2I] buffer (from ``ctx``, a parts.base.LayerContext, if given) is followed by the SwiGLU kernel."""
     if interleave == 8 and skinny_ok(x, w):
         gemm_skinny(x, w, out, gated=True, act=act)
@@ -1235,8 +1236,8 @@ def paged_attention(qkv, k_pool, v_pool, batch, block_table, page_size, out, num
                     keep=0) -> None:
     """Attention of every token of the step over its request's cached keys (its own included).
 
-    float32: the CUDA-core kernel, whose result does not depend on how the work was cut.
-    bfloat16: the tensor-core kernels, one for prompt portions and one (split over the keys) for
+    float32: one kernel for all tokens (products of split operands for heads of 32, 64, 96 and 128, multiply-adds for others), whose result
+    does not depend on how the work was cut.  bfloat16: the tensor-core kernels, one for prompt portions and one (split over the keys) for
     single decoded tokens.
 
     Options of the score: ``window`` (the last n keys, and with ``keep`` also the sequence's first ``keep`` keys) or ``chunk`` (the keys of the query's own block of n positions,
