@@ -434,3 +434,14 @@ RB_EXPORT int rb_gemm_rows_fused(const void* x, const void* w, void* out, int ga
     g.stream = stream; g.norm_w = norm_w; g.norm_w_dtype = norm_w_dtype; g.offset = offset; g.ssq_out = ssq_out; g.ld_sums = ld_sums;
     return run<true>(g, x, w, ldx, ldw, tiles, ls, st);
 }
+
+// The engine's choice for a product, on the current device: tiles that M falls into, log2 of the CTAs that share K, CTAs of the grid, and how many of them
+// the device holds at once.
+RB_EXPORT int rb_gemm_rows_plan(int M, int N, int K, int* out) {
+    int ctas[3];
+    if (M <= 0 || N <= 0 || K <= 0 || !resident(ctas)) return (int)cudaErrorInvalidValue;
+    pick(M, N, K, ctas, &out[0], &out[1]);
+    out[2] = (out[0] * ((N + BM - 1) / BM)) << out[1];
+    out[3] = ctas[out[1]];
+    return 0;
+}

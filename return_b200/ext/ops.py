@@ -483,6 +483,8 @@ def tc5_lib() -> ctypes.CDLL:
         lib.rb_gemm_rows_fused.argtypes = [P, P, P, I, I, I, I, I, I, I, P, I, I, ctypes.c_float, P, P, I, ctypes.c_float, P, I, I, I, P, P]
         lib.rb_gemm_rows_fused.restype = c_int
         lib.rb_gemm_rows.restype = c_int
+        lib.rb_gemm_rows_plan.argtypes = [I, I, I, P]
+        lib.rb_gemm_rows_plan.restype = c_int
         lib.rb_tc5_gemm.restype = lib.rb_tc5_gemm_simple.restype = lib.rb_tc5_gemm_bmn.restype = c_int
         _tc5 = build.native_calls(lib)
     return _tc5
@@ -746,6 +748,14 @@ def gemm_rows(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool =
                                 ACTIVATIONS[act] if act is not None and not gated else -1, M, N, K, x.stride(0), w.stride(0), out.stride(0),
                                 tiles, log2_split, _status_word(x.device), _stream())
     _check(rc, "gemm_rows")
+
+
+def gemm_rows_plan(M: int, N: int, K: int):
+    """(tiles that M falls into, log2 of the CTAs that share K, CTAs, how many of them the device holds at once) of ``gemm_rows``."""
+    buf = (c_int * 4)()
+    if tc5_lib().rb_gemm_rows_plan(M, N, K, ctypes.addressof(buf)):
+        raise KernelError("gemm_rows_plan: no such product")
+    return tuple(buf)
 
 
 def gemm_rows_fused(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], gated: bool = False, scale=None, residual=None,

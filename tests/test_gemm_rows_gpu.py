@@ -203,3 +203,15 @@ def test_clusters_share_an_sm_only_where_all_find_tensor_memory():
         ops.gemm_rows(x, w, out, tiles=1, log2_split=ls)
         _close(out, exact, size, 256)
     ops.check_status(x.device)
+
+
+def test_shapes_fill_the_device_once():
+    """A device holds fewer CTAs in fours than it has SMs.  A product that fits it in one round of another shape does not take two of these."""
+    ops = _ops()
+    for N in (768, 1024, 1152, 1536, 2048, 3072, 4608):
+        for K in (1024, 2048, 4096):
+            for M in range(16, 257, 16):
+                tiles, ls, ctas, held = ops.gemm_rows_plan(M, N, K)
+                assert ctas == tiles * ((N + 127) // 128) << ls and ctas <= held, (M, N, K, tiles, ls, ctas, held)
+    with pytest.raises(ops.KernelError):
+        ops.gemm_rows_plan(16, 128, 0)
