@@ -359,8 +359,8 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gated: bool
 class RowSums:
     """Where a product in its residual form leaves each CTA's share of sum(v^2) per token, for the norm that follows:
     the product that takes the normed rows multiplies its result by rstd = 1 / sqrt(sum / dim + eps) instead of
-    anyone norming them.  ``parts``: float32 [8, width]; ``count``: the shares that were written; ``dim``: the length
-    of the normed row."""
+    anyone norming them.  ``parts``: float32, a row a token ([8, width], or [rows, tiles of 128 columns] for more than 8 rows); ``count``: the
+    shares that were written; ``dim``: the length of the normed row."""
     WIDTH = 512
 
     def __init__(self, parts: torch.Tensor, dim: int, count: int = 0):
